@@ -319,6 +319,21 @@ def test_sgemm_true_fp32(M, N, K):
     assert torch.equal(out2.cpu(), ops.linear(wide[:, 4: 4 + K].contiguous(), w.to(DEV)).cpu())
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 17, 32, 33, 64, 65, 129, 513])
+@pytest.mark.parametrize("N,K", [(16, 16), (17, 132), (130, 2052), (2048, 260), (300, 77), (9000, 36)])
+def test_sgemm_every_kernel_gives_the_same_bits(M, N, K):
+    """Few rows, many rows, every tile, K with and without whole quads: one chain of multiply-adds per output, so a row has
+    the bits it has alone; K roundings of at most 2^-24 of the running sum bound its error."""
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(10)
+    a, w = torch.randn(M, K), torch.randn(N, K)
+    out = ops.linear(a.to(DEV), w.to(DEV)).cpu()
+    bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
+    assert bool(((out.double() - a.double() @ w.double().t()).abs() <= bound).all())
+    for m in {0, M // 2, M - 1}:
+        assert torch.equal(ops.linear(a[m:m + 1].to(DEV), w.to(DEV)).cpu()[0], out[m])
+
+
 def test_sgemm_keeps_what_tf32_would_lose():
     """Inputs with 20 significant bits: a reduced-precision matrix mode would round them to 10."""
     from photon_infer_b200.kernels import ops
