@@ -857,6 +857,16 @@ def test_attention_tcgen05_far_key_and_page_edges():
         assert not torch.isnan(out.float()).any()
 
 
+@pytest.mark.parametrize("n_q,n_kv,d", [(32, 8, 64), (6, 2, 128), (5, 5, 64)])
+@pytest.mark.parametrize("longs", [(0,), (31,), (32,), (69,), (0, 31, 32, 63, 64, 69), tuple(range(70))])
+def test_attention_tcgen05_finds_the_portions_among_many_requests(n_q, n_kv, d, longs):
+    """A block finds its request 32 at a time: portions at the edges of those groups, first, last, alone and everywhere,
+    with one tile, whole tiles and a partly filled last one, beside requests of few rows (at 5/5 heads up to 16 tokens)."""
+    few = 16 * n_kv // n_q
+    steps = [(i % 7, (20, 128, 150, 33)[i % 4]) if i in longs else (i % 5, 1 + i % few) for i in range(70)]
+    _tc_attention_case(n_q, n_kv, d, 16, None, [a + b for a, b in steps], steps)
+
+
 def test_attention_tcgen05_refuses_other_sizes():
     from photon_infer_b200.errors import PhotonError
     from photon_infer_b200.kernels import ops
