@@ -330,6 +330,60 @@ delta_out_kernel(const float* __restrict__ o, const TZ* z, long z_stride, const 
   }
 }
 
+// The same with four numbers at a time and the head in registers, QUADS groups of four a lane: for heads of up to 512 numbers on
+// 16-byte (float) and 8-byte (bfloat16) boundaries.  2,048 rows of 16 heads of 128 (42 MB): 20 us with 4-byte accesses.
+__device__ __forceinline__ void delta_load4(const float* p, float* f) {
+  const float4 r = *reinterpret_cast<const float4*>(p);
+  f[0] = r.x; f[1] = r.y; f[2] = r.z; f[3] = r.w;
+}
+__device__ __forceinline__ void delta_load4(const bf16* p, float* f) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+__device__ __forceinline__ void delta_store4(float* p, const float* f) { *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]); }
+__device__ __forceinline__ void delta_store4(bf16* p, const float* f) {
+  __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+
+template <typename TZ, typename TO, int QUADS>
+__global__ void __launch_bounds__(256)
+delta_out_vec_kernel(const float* __restrict__ o, const TZ* z, long z_stride, const float* __restrict__ norm_w, float eps,
+                     TO* __restrict__ out, long out_stride, int T, int H, int vdim) {
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long item = (long)blockIdx.x * 8 + warp;
+  if (item >= (long)T * H) return;
+  const int t = (int)(item / H), h = (int)(item - (long)t * H);
+  const float* row = o + ((size_t)t * H + h) * vdim;
+  const TZ* zr = z + (size_t)t * z_stride + (size_t)h * vdim;
+  float x[QUADS][4], g[QUADS][4];
+#pragma unroll
+  for (int u = 0; u < QUADS; ++u) {
+    const int i = (u * 32 + lane) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { x[u][e] = 0.f; g[u][e] = 0.f; }
+    if (i < vdim) { delta_load4(row + i, x[u]); delta_load4(zr + i, g[u]); }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int u = 0; u < QUADS; ++u)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss += x[u][e] * x[u][e];
+  ss = warp_sum(ss);
+  const float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
+#pragma unroll
+  for (int u = 0; u < QUADS; ++u) {
+    const int i = (u * 32 + lane) * 4;
+    if (i >= vdim) continue;
+    float y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = x[u][e] * inv * norm_w[i + e] * (g[u][e] / (1.0f + expf(-g[u][e])));
+    delta_store4(out + (size_t)t * out_stride + (size_t)h * vdim + i, y);
+  }
+}
+
 // x [T][>= C] of x_dtype (row stride x_stride): the projected q, k, v side by side; taps_w float [C][taps];
 // state float [num_slots][state_stride], a request's convolution rows at conv_offset; y float [T][C]: q, k (unit
 // vectors, q scaled) and v after the convolution.  Then the state's rows are brought up to date.
@@ -420,6 +474,18 @@ PHOTON_API int photon_delta_out(const float* o, const void* z, long z_stride, in
   if (T <= 0) return 0;
   const long items = (long)T * H;
   dim3 grid((unsigned)((items + 3) / 4));
+  // four numbers at a time where everything lies on their boundaries
+  const uintptr_t za = z_dtype == PHOTON_F32 ? 15 : 7, oa = out_dtype == PHOTON_F32 ? 15 : 7;
+  if (vdim % 4 == 0 && vdim <= 512 && z_stride % 4 == 0 && out_stride % 4 == 0 && ((uintptr_t)o & 15) == 0 && ((uintptr_t)z & za) == 0 &&
+      ((uintptr_t)out & oa) == 0) {
+    const dim3 vgrid((unsigned)((items + 7) / 8));
+#define DOUT_VEC(TZ, TO, Q) return launch_pdl(delta_out_vec_kernel<TZ, TO, Q>, vgrid, dim3(256), 0, stream, o, (const TZ*)z, z_stride, norm_w, \
+                                              eps, (TO*)out, out_stride, T, H, vdim)
+#define DOUT_VECS(TZ, TO) do { if (vdim <= 128) DOUT_VEC(TZ, TO, 1); if (vdim <= 256) DOUT_VEC(TZ, TO, 2); DOUT_VEC(TZ, TO, 4); } while (0)
+    if (z_dtype == PHOTON_F32 && out_dtype == PHOTON_F32) DOUT_VECS(float, float);
+    if (z_dtype == PHOTON_F32 && out_dtype == PHOTON_BF16) DOUT_VECS(float, bf16);
+    if (z_dtype == PHOTON_BF16 && out_dtype == PHOTON_BF16) DOUT_VECS(bf16, bf16);
+  }
 #define DOUT_GO(TZ, TO) return launch_pdl(delta_out_kernel<TZ, TO>, grid, dim3(128), 0, stream, o, (const TZ*)z, z_stride, norm_w, eps, \
                                           (TO*)out, out_stride, T, H, vdim)
   if (z_dtype == PHOTON_F32 && out_dtype == PHOTON_F32) DOUT_GO(float, float);

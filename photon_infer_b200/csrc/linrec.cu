@@ -28,8 +28,7 @@
 // Every token's arithmetic is the same chain whatever the step brought before it, and the cut of a head's columns
 // into blocks changes no column's arithmetic, so a request's numbers depend neither on how it was cut into steps nor
 // on the batch.
-#include "common.cuh"
-#include <math.h>
+#include "linrec.cuh"
 
 // ---------------------------------------------------------------- short causal convolution
 template <typename TI>
@@ -132,17 +131,6 @@ PHOTON_API int photon_conv_state(const void* x, long x_stride, int x_dtype, int 
 #define LR_CHUNK 16
 #define LR_COLS 16
 #define LR_THREADS 128
-
-__device__ __forceinline__ float lr_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float lr_logsigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ void lr_cp4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-__device__ __forceinline__ void lr_cp16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-__device__ __forceinline__ void lr_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int K> __device__ __forceinline__ void lr_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(K) : "memory"); }
 
 // Mode 2's inputs.
 __device__ __forceinline__ float lr_silu(float x) { return x / (1.0f + expf(-x)); }
@@ -415,45 +403,7 @@ static int linrec_launch(int rpl, dim3 grid, cudaStream_t stream, const float* q
 // d = v - S, S += k d, o += q S; the lanes' shares of the read-outs meet by shuffles in one tree over the lanes, so every
 // token's arithmetic is the same chain wherever its step starts.  (Two columns a lane and eight warps take the same time for
 // one request of 2,048 tokens and 16 heads of 128 x 128, and a tenth more for 32 heads.)
-#define LRR_C 4                 // columns of a lane: 2 or 4
 #define LRR_THREADS (512 / LRR_C)
-typedef unsigned long long lr_pair;
-struct alignas(LRR_C * 4) LrCols { float x[LRR_C]; };   // the lane's columns of one row
-__device__ __forceinline__ lr_pair lr_dup(float x) { lr_pair d; asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(x)); return d; }
-__device__ __forceinline__ lr_pair lr_mul2(lr_pair a, lr_pair b) { lr_pair d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ lr_pair lr_fma2(lr_pair a, lr_pair b, lr_pair c) {
-  lr_pair d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ float lr_sum2(lr_pair a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
-  return x + y;
-}
-__device__ __forceinline__ lr_pair lr_make(float x, float y) { lr_pair d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y)); return d; }
-__device__ __forceinline__ void lr_split(lr_pair a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
-
-// The lanes' shares of NV sums meet over the distances D, D / 2 .. 1: while a lane holds several sums it keeps half of them (the
-// upper half where the distance's bit of its number is set) and hands over the others.
-template <int D, int NV, int M>
-__device__ __forceinline__ void lr_meet(float (&val)[M], int sub) {
-  if constexpr (D > 0) {
-    if constexpr (NV > 1) {
-      const bool up = sub & D;
-#pragma unroll
-      for (int i = 0; i < NV / 2; ++i) {
-        const float own = up ? val[i + NV / 2] : val[i], other = up ? val[i] : val[i + NV / 2];
-        val[i] = own + __shfl_xor_sync(0xffffffffu, other, D);
-      }
-      lr_meet<D / 2, NV / 2>(val, sub);
-    } else {
-      val[0] += __shfl_xor_sync(0xffffffffu, val[0], D);
-      lr_meet<D / 2, 1>(val, sub);
-    }
-  }
-}
-
 template <int L, int R>
 __global__ void __launch_bounds__(LRR_THREADS)
 linrec_rows_kernel(const float* __restrict__ q, long q_stride, const float* __restrict__ k, long k_stride,

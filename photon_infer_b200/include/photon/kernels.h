@@ -238,6 +238,11 @@ PHOTON_EXPORT int photon_delta_out(const float* o, const void* z, long z_stride,
 PHOTON_EXPORT int photon_group_rmsnorm(const void* x, long x_stride, int x_dtype, const float* gate, long gate_stride, int gate_mode,
                      float* residual, const void* w, int w_dtype, void* out, long out_stride, int out_dtype, int T, int H,
                      int groups, float eps, const void* x_bias, int xb_dtype, cudaStream_t stream);
+/* The norm alone, a warp per part, without a stream: x / den (float [T][groups], may be null), the gate before or behind.  Parts of up
+ * to 1,024 numbers, a multiple of 4, on 16-byte (float) or 8-byte (bfloat16) boundaries. */
+PHOTON_EXPORT int photon_part_rmsnorm(const void* x, long x_stride, int x_dtype, const float* den, const float* gate, long gate_stride,
+                     int gate_mode, const void* w, int w_dtype, void* out, long out_stride, int out_dtype, int T, int H,
+                     int groups, float eps, cudaStream_t stream);
 /* out = a N(z) + b N(z^2) + c N(z^3) + e with N(u) = u / sqrt(mean(u^2) + eps) over the row; coef [4] = (a, b, c, e). */
 PHOTON_EXPORT int photon_polynorm(const void* z, long z_stride, int z_dtype, const void* coef, int coef_dtype, void* out,
                      long out_stride, int out_dtype, int T, int F, float eps, cudaStream_t stream);
@@ -299,6 +304,20 @@ PHOTON_EXPORT int photon_linrec(int mode, const float* q, long q_stride, const f
 PHOTON_EXPORT int photon_linrec_gates(const float* q, long q_stride, const float* z, long z_stride, const float* bias,
                            const float* lower, float* q_out, float* k_out, long out_stride, int T, int C, cudaStream_t stream);
 
+/* ------------------------------------------------------------------ linrec_segments.cu: long portions in segments side by side */
+/* Blocks of one (segment, head); floats of scratch. */
+PHOTON_EXPORT int photon_linrec_segment_blocks(int N, int dv);
+PHOTON_EXPORT long photon_linrec_segments_scratch(int mode, int T, int S, int segs, int H, int N, int dv);
+/* As photon_linrec (mode 2: q and k from photon_linrec_gates), requests cut into up to `segs` segments of `seg` tokens (a
+ * multiple of 16).  mode 3: S_t = diag(a_t) S_(t-1) + k v^T with a [T][qk_heads * N]; ga .. p2 unused.  mode 1: den [T][H] gets
+ * what the outputs are to be divided by.  scratch: 16-byte aligned. */
+PHOTON_EXPORT int photon_linrec_segments(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
+                              long v_stride, const float* a, long a_stride, const float* ga, const float* gb, long g_stride,
+                              const float* p0, const float* p1, const float* p2, float cap, float q_scale,
+                              const int* cu_tokens, const int* state_slots, float* state, long state_stride, int num_slots,
+                              float* out, long out_stride, float* den, float* scratch, int T, int S, int H, int qk_heads,
+                              int N, int dv, int seg, int segs, int* err, cudaStream_t stream);
+
 /* ------------------------------------------------------------------ attention_talk.cu: attention whose heads' scores are mixed */
 /* Bias (float, may be null) on q [T][H * d] and k [T][G * d] of in_dtype, rotation of the first rot_dims numbers of a head
  * (number j with j + rot_dims / 2, angle positions[t] * inv_freq[j]); q_out of out_dtype; the rotated key goes to k_cache, the
@@ -343,15 +362,11 @@ PHOTON_EXPORT int photon_gla_recurrent(const void* q, const void* k, const void*
                          int norm_w_dtype, float eps, float tau, float qscale, const int* cu_tokens, const int* state_slots,
                          float* state, int num_slots, void* out, long out_stride, int S, int heads, int dim, int vdim,
                          int skip_from, int* err, cudaStream_t stream);
-/* One long prompt portion (tokens first .. first + count - 1 of the step, state slot `slot`, negative: from zero, nothing
- * stored) in chunks of `chunk` tokens that run side by side.  scratch: float [count * heads * (vdim + dim) + 4 +
- * ceil(count / chunk) * heads * dim * vdim], 16-byte aligned.  photon_gla_recurrent leaves requests of skip_from tokens or more
- * (skip_from > 0) to this path. */
-PHOTON_EXPORT int photon_gla_chunked(const void* q, const void* k, const void* v, const void* g, const void* low, long in_stride,
-                       int dtype, int rank, const void* w_a2, const void* b_a2, int b_a2_dtype, const void* norm_w,
-                       int norm_w_dtype, float eps, float tau, float qscale, int first, int count, int chunk, int slot,
-                       float* state, int num_slots, float* scratch, void* out, long out_stride, int heads, int dim, int vdim,
-                       int* err, cudaStream_t stream);
+/* The inputs of a long portion in 32-bit (photon_linrec_segments walks them): q, k [T][nd] and v [T][nv] as float and the
+ * decays exp(log_sigmoid(w_a2 low + b_a2) / tau) [T][nd], all with row stride out_stride. */
+PHOTON_EXPORT int photon_gla_prep(const void* q, const void* k, const void* v, const void* low, long in_stride, int dtype, int rank,
+                       const void* w_a2, const void* b_a2, int b_a2_dtype, float tau, float* q_out, float* k_out, float* v_out,
+                       float* a_out, long out_stride, int T, int nd, int nv, cudaStream_t stream);
 
 /* ------------------------------------------------------------------ moe.cu: routed experts */
 /* Router: logits = Wr h + bias in 32-bit; ids/weights [T][top]: the top experts and the softmax over their logits;

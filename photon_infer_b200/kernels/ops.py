@@ -1443,6 +1443,35 @@ def group_rmsnorm(x: Optional[torch.Tensor], weight: Optional[torch.Tensor], eps
              _dtype_code(x_bias) if x_bias is not None else F32, _stream()), "group_rmsnorm")
 
 
+def part_rmsnorm_supported(x: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor, groups: int) -> bool:
+    """The sizes of ``part_rmsnorm``: parts of up to 1,024 numbers, quads of numbers on their natural boundaries."""
+    gs = x.shape[1] // groups
+    quads = lambda t: t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0
+    return gs % 4 == 0 and gs <= 1024 and quads(x) and quads(out) and (gate is None or quads(gate))
+
+
+def part_rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, groups: int, out: torch.Tensor, gate: Optional[torch.Tensor] = None,
+                 gate_mode: Optional[str] = None, den: Optional[torch.Tensor] = None) -> None:
+    """``group_rmsnorm`` without a stream, with a warp per part of ``x [T, H]``: for many rows.  ``den`` (float32 ``[T, groups]``):
+    every part is divided by its number first."""
+    _cuda(x, weight, out, gate, den)
+    T, H = x.shape
+    if groups <= 0 or H % groups or x.stride(1) != 1 or out.shape != (T, H) or out.stride(1) != 1 or weight.numel() != H \
+            or not weight.is_contiguous():
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "part_rmsnorm: x and out [T, H] in equal parts, weight [H]")
+    if gate_mode not in GATE_MODES or (gate is None) != (gate_mode is None) or \
+            (gate is not None and (gate.dtype != torch.float32 or gate.shape != (T, H) or gate.stride(1) != 1)):
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "part_rmsnorm: a float32 [T, H] gate goes with a gate mode")
+    if den is not None and (den.dtype != torch.float32 or den.shape != (T, groups) or not den.is_contiguous()):
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "part_rmsnorm: den must be contiguous float32 [T, groups]")
+    f = _fn("row_norms", "photon_part_rmsnorm",
+            [c_void_p, c_long, c_int, c_void_p, c_void_p, c_long, c_int, c_void_p, c_int, c_void_p, c_long, c_int, c_int, c_int, c_int,
+             c_float, c_void_p])
+    _check(f(_ptr(x), x.stride(0), _dtype_code(x), _ptr(den), _ptr(gate), gate.stride(0) if gate is not None else 0, GATE_MODES[gate_mode],
+             _ptr(weight), _dtype_code(weight), _ptr(out), out.stride(0), _dtype_code(out), T, H, int(groups), float(eps), _stream()),
+           "part_rmsnorm")
+
+
 def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor) -> None:
     """``out = a N(z) + b N(z^2) + c N(z^3) + e`` per row, powers element by element, ``N(u) = u / sqrt(mean(u^2) + eps)``;
     ``coef [4] = (a, b, c, e)``."""
@@ -1689,6 +1718,87 @@ def linrec(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate_a:
              _ptr(err), _stream()), "linrec")
 
 
+#: A bfloat16 step in which some request brings at least this many tokens cuts its recurrences into segments: two of 64 tokens are the
+#: fewest that gain (one request of 300 tokens, gated linear attention, 16 heads of 128 x 128: 50 us in segments).
+LINREC_SEGMENTS_MIN_TOKENS = 128
+LINREC_SEGMENT_MODES = {"state_space": 0, "matrix_memory": 1, "forget_write": 2, "decay_rows": 3}
+
+
+def linrec_segments_supported(dim: int, longest: int) -> bool:
+    """Whether the recurrences of a bfloat16 step run in segments: states of up to 512 rows, a request with enough tokens."""
+    return dim <= 512 and longest >= LINREC_SEGMENTS_MIN_TOKENS
+
+
+def linrec_segment_tokens(query_lens, heads: int, dim: int, vdim: int, sms: int) -> int:
+    """Tokens of a segment, a multiple of 16: the fewest with which the requests' segments fit the GPU at once at two blocks a
+    streaming multiprocessor (one block more would wait for a whole segment), but no fewer than 64 (every segment but the first costs a
+    pass over its tokens without queries and a fold of its end state)."""
+    blocks = heads * int(load_module("linrec_segments").photon_linrec_segment_blocks(dim, vdim))
+    places = max(1, 2 * sms // blocks)
+    seg = max(64, -(-sum(query_lens) // (16 * places)) * 16)
+    longest = max(query_lens)
+    while seg < longest and sum(-(-n // seg) for n in query_lens) > places:
+        seg += 16
+    return seg
+
+
+def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: Optional[torch.Tensor], gate_a: Optional[torch.Tensor],
+                    gate_b: Optional[torch.Tensor], p0: Optional[torch.Tensor], p1: Optional[torch.Tensor], p2: Optional[torch.Tensor],
+                    cap: float, q_scale: float, cu_tokens: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor, out: torch.Tensor,
+                    query_lens, heads: int, qk_heads: int, dim: int, vdim: int, err: Optional[torch.Tensor],
+                    segment: Optional[int] = None) -> Optional[torch.Tensor]:
+    """``linrec`` for a step with long portions: every request is cut into segments that run side by side, a first pass from
+    zero states and a second one from the states that the first pass's ends add up to.  The arithmetic of a token is that of ``linrec``;
+    a segment's start is one multiply-add per segment before it away from the state that ``linrec`` would have reached.  ``forget_write``:
+    ``q`` and ``k`` as ``linrec_gates`` leaves them.  ``decay_rows``: ``S <- diag(a) S + k v^T``, ``a [T, qk_heads * dim]``.
+    ``matrix_memory``: ``out`` is not divided; returns ``[T, heads]``, what it is to be divided by.  ``query_lens``: the requests'
+    tokens in the step (host)."""
+    _cuda(q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, err)
+    if mode not in LINREC_SEGMENT_MODES:
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, f"linrec_segments: unknown mode {mode!r}")
+    T, S = q.shape[0], len(query_lens)
+    for t, w, what in ((q, qk_heads * dim, "q"), (k, qk_heads * dim, "k"), (v, heads * vdim, "v"), (a, qk_heads * dim, "a"),
+                       (gate_a, heads, "gate_a"), (gate_b, heads, "gate_b"), (out, heads * vdim, "out")):
+        if t is not None and (t.dtype != torch.float32 or t.shape != (T, w) or t.stride(1) != 1):
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"linrec_segments: {what} must be a float32 [T, {w}] view")
+    if gate_b is not None and (gate_a is None or gate_b.stride(0) != gate_a.stride(0)):
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: both gates must have one row stride")
+    if (mode == "matrix_memory") != (gate_b is not None) or (mode in ("state_space", "matrix_memory")) != (gate_a is not None) \
+            or (mode == "decay_rows") != (a is not None):
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, "linrec_segments: the matrix memory has two gates per head, the state-space layer one, "
+                          "the others none beside their rows' gates or decays")
+    for t, what in ((p0, "p0"), (p1, "p1"), (p2, "p2")):
+        if t is not None and (t.dtype != torch.float32 or t.numel() != heads or not t.is_contiguous()):
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"linrec_segments: {what} must be float32 [{heads}]")
+    if mode in ("state_space", "matrix_memory") and (p0 is None or p1 is None or (p2 is None and mode == "state_space")):
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, "linrec_segments: the gates' parameters are missing")
+    need = heads * dim * vdim + (heads * dim + heads if mode == "matrix_memory" else 0)
+    if state.dtype != torch.float32 or state.dim() != 2 or not state.is_contiguous() or state.shape[1] < need:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: state must be contiguous float32 [slots, row]")
+    _int32(cu_tokens, "cu_tokens")
+    _int32(state_slots, "state_slots")
+    if cu_tokens.numel() < S + 1 or state_slots.numel() < S or sum(query_lens) > T:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: cu_tokens and state_slots must cover every request")
+    seg = int(segment) if segment else linrec_segment_tokens(query_lens, heads, dim, vdim, sm_count(q.device))
+    segs = max(1, -(-max(query_lens, default=1) // seg))
+    code = LINREC_SEGMENT_MODES[mode]
+    size = load_module("linrec_segments").photon_linrec_segments_scratch
+    size.restype, size.argtypes = c_long, [c_int] * 7
+    scratch = torch.empty(size(code, T, S, segs, heads, dim, vdim), dtype=torch.float32, device=q.device)
+    den = torch.empty((T, heads), dtype=torch.float32, device=q.device) if mode == "matrix_memory" else None
+    f = _fn("linrec_segments", "photon_linrec_segments",
+            [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_long, c_void_p, c_void_p,
+             c_void_p, c_float, c_float, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(code, _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(a), a.stride(0) if a is not None else 0,
+             _ptr(gate_a), _ptr(gate_b), gate_a.stride(0) if gate_a is not None else 0, _ptr(p0), _ptr(p1), _ptr(p2), float(cap),
+             float(q_scale), _ptr(cu_tokens), _ptr(state_slots), _ptr(state), state.stride(0), state.shape[0], _ptr(out), out.stride(0),
+             _ptr(den), _ptr(scratch), T, S, heads, qk_heads, dim, vdim, seg, segs, _ptr(err), _stream()), "linrec_segments")
+    global _launch_count
+    _launch_count += (mode in ("state_space", "matrix_memory")) + (segs > 1)
+    return den
+
+
 # ----------------------------------------------------------------------------- attention whose heads' scores are mixed
 
 def talk_prep(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Tensor], q_bias: Optional[torch.Tensor], k_bias: Optional[torch.Tensor],
@@ -1842,7 +1952,7 @@ def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Te
     logits ``w_a2 low + b_a2``, the per-head norm and the output gate.  ``q, k [T, heads * dim]``,
     ``v, g [T, heads * vdim]`` and ``low [T, rank]`` are sections of one fused row (same row stride),
     ``w_a2 [heads * dim, rank]``, ``state [slots, heads, dim, vdim]`` float32, ``out [T, heads * vdim]``.
-    ``skip_from`` > 0: requests that bring that many tokens or more are left alone (``gla_chunked`` runs them)."""
+    ``skip_from`` > 0: requests that bring that many tokens or more are left alone (the caller runs them)."""
     _cuda(q, k, v, g, low, w_a2, b_a2, norm_w, cu_tokens, state_slots, state, out, err)
     T = q.shape[0]
     rank = low.shape[1]
@@ -1868,46 +1978,24 @@ def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Te
              int(skip_from), _ptr(err), _stream()), "gla_recurrent")
 
 
-GLA_CHUNK = 32              # tokens of a chunk of the chunk-parallel recurrence (measured: 64 -> 521 us, 32 -> 420 us, 16 -> 515 us at 2,048 tokens, 16 heads of 128 x 128)
-
-
-def gla_chunked_supported(dim: int, vdim: int, rank: int = 64) -> bool:
-    """A block shape of the chunk kernel exists (columns x row groups within 512 threads, the groups a power of two),
-    and the shared memory of the two chunk kernels fits."""
-    for rpt in (8, 16, 32, 64):
-        groups = -(-dim // rpt)
-        p = 1
-        while p < groups:
-            p *= 2
-        if p <= 32 and vdim * p <= 512 and dim <= 512:
-            local = (3 * GLA_CHUNK * groups * (rpt + 4) + GLA_CHUNK * vdim + dim * (rank + 2)) * 4
-            out = (dim * vdim + 4 + (GLA_CHUNK + 4) * dim + GLA_CHUNK * vdim) * 4
-            return local <= 220 * 1024 and out <= 200 * 1024
-    return False
-
-
-def gla_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, low: torch.Tensor, w_a2: torch.Tensor,
-                b_a2: torch.Tensor, norm_w: torch.Tensor, eps: float, tau: float, qscale: float, first: int, count: int,
-                slot: int, state: torch.Tensor, out: torch.Tensor, heads: int, dim: int, vdim: int,
-                err: Optional[torch.Tensor]) -> None:
-    """One long prompt portion (tokens ``first .. first + count - 1`` of the step's rows, state slot ``slot``) with its
-    chunks of ``GLA_CHUNK`` tokens side by side: each chunk's own recurrence from zero, a scan over the chunks' end
-    states, and the start states' share of the outputs with the norm and the gate.  Same tensors as
-    ``gla_recurrent``; the sums differ from its sums in their order only."""
-    _cuda(q, k, v, g, low, w_a2, b_a2, norm_w, state, out, err)
-    rank = low.shape[1]
-    chunks = -(-count // GLA_CHUNK)
-    scratch = torch.empty(count * heads * (vdim + dim) + 4 + chunks * heads * dim * vdim, dtype=torch.float32, device=q.device)
-    f = _fn("gla", "photon_gla_chunked",
-            [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
-             c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_long,
-             c_int, c_int, c_int, c_void_p, c_void_p])
-    _check(f(_ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(low), q.stride(0), _dtype_code(q), rank, _ptr(w_a2), _ptr(b_a2),
-             _dtype_code(b_a2), _ptr(norm_w), _dtype_code(norm_w), float(eps), float(tau), float(qscale), int(first),
-             int(count), GLA_CHUNK, int(slot), _ptr(state), state.shape[0], _ptr(scratch), _ptr(out), out.stride(0), heads,
-             dim, vdim, _ptr(err), _stream()), "gla_chunked")
-    global _launch_count
-    _launch_count += 2
+def gla_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, low: torch.Tensor, w_a2: torch.Tensor, b_a2: torch.Tensor, tau: float):
+    """The inputs of a long portion in 32-bit, as ``linrec_segments`` walks them: ``q``, ``k [T, heads * dim]`` and ``v [T, heads *
+    vdim]`` (views of one fused row) as float32 and the decays ``exp(log_sigmoid(w_a2 low + b_a2) / tau)``; returns ``(q, k, v, a)``."""
+    _cuda(q, k, v, low, w_a2, b_a2)
+    T, nd, nv, rank = q.shape[0], q.shape[1], v.shape[1], low.shape[1]
+    for t, w, what in ((q, nd, "q"), (k, nd, "k"), (v, nv, "v"), (low, rank, "low")):
+        if t.shape != (T, w) or t.stride(1) != 1 or t.stride(0) != q.stride(0) or t.dtype != q.dtype:
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"gla_prep: {what} must be [T, {w}] with the row stride of q")
+    if w_a2.shape != (nd, rank) or w_a2.dtype != q.dtype or not w_a2.is_contiguous() or b_a2.numel() != nd or not b_a2.is_contiguous():
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "gla_prep: w_a2 [heads * dim, rank] of q's dtype, b_a2 [heads * dim]")
+    rows = torch.empty((T, 3 * nd + nv), dtype=torch.float32, device=q.device)
+    qo, ko, ao, vo = rows[:, :nd], rows[:, nd:2 * nd], rows[:, 2 * nd:3 * nd], rows[:, 3 * nd:]
+    f = _fn("gla", "photon_gla_prep",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p,
+             c_void_p, c_long, c_int, c_int, c_int, c_void_p])
+    _check(f(_ptr(q), _ptr(k), _ptr(v), _ptr(low), q.stride(0), _dtype_code(q), rank, _ptr(w_a2), _ptr(b_a2), _dtype_code(b_a2), float(tau),
+             _ptr(qo), _ptr(ko), _ptr(vo), _ptr(ao), rows.stride(0), T, nd, nv, _stream()), "gla_prep")
+    return qo, ko, vo, ao
 
 
 # ----------------------------------------------------------------------------- routed experts

@@ -9,8 +9,9 @@
 ``silu(W_g h)`` and projected by ``W_o``.  The state starts at zero, is 32-bit, and lives in the request's state
 slot between steps; decays, their logarithms and the recurrence itself are 32-bit.
 
-One fused product gives ``[q | k | v | g | W_a1 h]``; one kernel forms the decay logits from the low-rank part,
-runs the recurrence over the tokens of a step and applies the norm and the gate in its epilogue.
+One fused product gives ``[q | k | v | g | W_a1 h]``.  For few tokens one kernel forms the decay logits from the low-rank part,
+runs the recurrence over the tokens of a step and applies the norm and the gate in its epilogue; a step with a long portion
+forms the decays of all tokens first, runs the recurrence in segments side by side (``linrec_segments.cu``), and then norm and gate.
 """
 from __future__ import annotations
 
@@ -25,7 +26,7 @@ from .registry import register_mixer
 
 
 class GatedLinearAttention(Mixer):
-    kernel_modules = ("gla",)
+    kernel_modules = ("gla", "linrec_segments", "delta")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, tau: float, eps: float,
@@ -33,7 +34,7 @@ class GatedLinearAttention(Mixer):
         self.hidden_size, self.heads, self.dim, self.vdim = hidden_size, heads, dim, vdim
         self.tau, self.eps = float(tau), float(eps)
         self.decay_rank = decay_rank            # None: the weight file decides
-        self.w_in = self.w_a2 = self.b_a2 = self.norm = self.w_o = None
+        self.w_in = self.w_a2 = self.b_a2 = self.norm = self.norm32 = self.w_o = None
 
     def required_kernels(self, dtype):
         mods = list(self.kernel_modules)
@@ -58,6 +59,7 @@ class GatedLinearAttention(Mixer):
         self.w_a2 = tensors["a2"].contiguous()
         self.b_a2 = tensors["a2.b"].contiguous()
         self.norm = tensors["norm"].contiguous()
+        self.norm32 = self.norm.to(torch.float32)
         self.w_o = tensors["o"].contiguous()
 
     def weight_bytes(self) -> int:
@@ -74,36 +76,22 @@ class GatedLinearAttention(Mixer):
         v, g = fused[:, 2 * nd:2 * nd + nv], fused[:, 2 * nd + nv:2 * nd + 2 * nv]
         low = fused[:, 2 * nd + 2 * nv:]
         out = torch.empty((T, nv), dtype=h.dtype, device=h.device)
-        # long bfloat16 prompt portions run their chunks side by side; everything else (and the float32 run, whose sums
-        # depend on nothing but the token's place in its request) goes token by token
-        skip = 0
+        # a step with a long bfloat16 portion runs in segments of tokens side by side; everything else (and the float32 run, whose
+        # sums depend on nothing but the token's place in its request) goes token by token
         lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and max(lens) >= CHUNKED_MIN_TOKENS and ops.gla_chunked_supported(self.dim, self.vdim, self.decay_rank or 64):
-            skip = CHUNKED_MIN_TOKENS
-            slots = self._host_slots(ctx)
-            t = 0
-            for s, m in enumerate(lens):
-                if m >= skip:
-                    ops.gla_chunked(q, k, v, g, low, self.w_a2, self.b_a2, self.norm, self.eps, self.tau, self.dim ** -0.5,
-                                    t, m, slots[s], cache.state, out, self.heads, self.dim, self.vdim, ctx.error_flag)
-                t += m
-        if skip == 0 or min(lens) < skip:
+        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported(self.dim, max(lens)):
+            q, k, v, a = ops.gla_prep(q, k, v, low, self.w_a2, self.b_a2, self.tau)
+            o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
+            state = cache.state.view(cache.state.shape[0], -1)
+            ops.linrec_segments("decay_rows", q, k, v, a, None, None, None, None, None, 0.0, self.dim ** -0.5, ctx.cu_tokens, ctx.state_slots,
+                                state, o, lens, self.heads, self.heads, self.dim, self.vdim, ctx.error_flag)
+            ops.delta_out(o, g, self.norm32, self.eps, out, self.heads, self.vdim)
+        else:
             ops.gla_recurrent(q, k, v, g, low, self.w_a2, self.b_a2, self.norm, self.eps, self.tau, self.dim ** -0.5,
                               ctx.cu_tokens, ctx.state_slots, cache.state, out, ctx.num_seqs, self.heads, self.dim, self.vdim,
-                              ctx.error_flag, skip_from=skip)
+                              ctx.error_flag)
         return project(out, self.w_o)
 
-
-    @staticmethod
-    def _host_slots(ctx: StepContext):
-        """The requests' state slots on the host (the chunked path takes a request's slot as a launch argument)."""
-        if ctx.host_state_slots:
-            return list(ctx.host_state_slots)
-        return ctx.state_slots.cpu().tolist()
-
-
-#: A request that brings at least this many tokens to a bfloat16 step runs chunk-parallel.
-CHUNKED_MIN_TOKENS = 128
 
 register_mixer("gla", GatedLinearAttention)
 register_mixer("gla_2", GatedLinearAttention)

@@ -29,7 +29,7 @@ DEFAULT_NAMES = {"q": "q", "f": "f", "f_bias": "f.b", "lower": "lower", "v": "v"
 
 
 class Hgrn2Mixer(Mixer):
-    kernel_modules = ("linrec", "row_norms")
+    kernel_modules = ("linrec", "linrec_segments", "row_norms")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, eps: float, names: Optional[Dict[str, str]] = None):
@@ -73,8 +73,14 @@ class Hgrn2Mixer(Mixer):
             ops.linrec_gates(q, k, bias, lower, y[:, :nd], y[:, nd:])
             q, k, bias, lower = y[:, :nd], y[:, nd:], None, None
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
-        ops.linrec("forget_write", q, k, v, None, None, bias, lower, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o,
-                   ctx.num_seqs, H, H, self.dim, self.vdim, ctx.error_flag)
+        lens = list(ctx.host_query_lens)
+        if h.dtype == torch.bfloat16 and lens and bias is None and ops.linrec_segments_supported(self.dim, max(lens)):
+            # long portions: segments of tokens side by side
+            ops.linrec_segments("forget_write", q, k, v, None, None, None, None, None, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots,
+                                cache.state, o, lens, H, H, self.dim, self.vdim, ctx.error_flag)
+        else:
+            ops.linrec("forget_write", q, k, v, None, None, bias, lower, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o,
+                       ctx.num_seqs, H, H, self.dim, self.vdim, ctx.error_flag)
         out = torch.empty((T, nv), dtype=h.dtype, device=h.device)
         ops.group_rmsnorm(o, self.norm, self.eps, H, out=out)
         return project(out, self.w_o)

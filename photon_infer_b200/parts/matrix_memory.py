@@ -32,7 +32,7 @@ DEFAULT_NAMES = {"q": "q", "k": "k", "v": "v", "g": "g", "o": "o", "norm": "norm
 
 
 class MatrixMemoryMixer(Mixer):
-    kernel_modules = ("linrec", "row_norms")
+    kernel_modules = ("linrec", "linrec_segments", "row_norms")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, gate_cap: float, eps: float,
@@ -74,6 +74,19 @@ class MatrixMemoryMixer(Mixer):
         rows = project(h, self.w_in, out_dtype=torch.float32)       # [q | k | v | g | i | f]
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
         g0 = 2 * nd + nv
+        lens = list(ctx.host_query_lens)
+        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported(self.dim, max(lens)):
+            # long portions: segments of tokens side by side; the division rides in the norm
+            den = ops.linrec_segments("matrix_memory", rows[:, :nd], rows[:, nd:2 * nd], rows[:, 2 * nd:g0], None, rows[:, g0 + nv:g0 + nv + H],
+                                      rows[:, g0 + nv + H:], self.i_bias, self.f_bias, None, self.gate_cap, self.dim ** -0.5, ctx.cu_tokens,
+                                      ctx.state_slots, cache.state, o, lens, H, H, self.dim, self.vdim, ctx.error_flag)
+            out, gate = torch.empty((T, nv), dtype=h.dtype, device=h.device), rows[:, g0:g0 + nv]
+            if ops.part_rmsnorm_supported(o, gate, out, H):
+                ops.part_rmsnorm(o, self.norm, self.eps, H, out, gate=gate, gate_mode="sigmoid_after", den=den)
+            else:
+                o.view(T, H, self.vdim).div_(den.unsqueeze(-1))
+                ops.group_rmsnorm(o, self.norm, self.eps, H, out=out, gate=gate, gate_mode="sigmoid_after")
+            return project(out, self.w_o, out_dtype=torch.float32)
         ops.linrec("matrix_memory", rows[:, :nd], rows[:, nd:2 * nd], rows[:, 2 * nd:g0], rows[:, g0 + nv:g0 + nv + H],
                    rows[:, g0 + nv + H:], self.i_bias, self.f_bias, None, self.gate_cap, self.dim ** -0.5, ctx.cu_tokens,
                    ctx.state_slots, cache.state, o, ctx.num_seqs, H, H, self.dim, self.vdim, ctx.error_flag)

@@ -32,7 +32,7 @@ DEFAULT_NAMES = {"in": "in", "conv": "conv", "conv_bias": "conv.b", "dt_bias": "
 
 
 class StateSpaceMixer(Mixer):
-    kernel_modules = ("linrec", "row_norms")
+    kernel_modules = ("linrec", "linrec_segments", "row_norms")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, vdim: int, state: int, taps: int, eps: float, groups: int = 1,
@@ -88,11 +88,22 @@ class StateSpaceMixer(Mixer):
         ops.conv_silu(rows[:, inner:inner + C], self.taps_w, self.conv_bias, ctx.token_seq, ctx.cu_tokens, ctx.state_slots,
                       cache.state, self.heads * self.state * self.vdim, y, ctx.num_seqs, ctx.error_flag)
         o = torch.empty((T, inner), dtype=torch.float32, device=h.device)
-        ops.linrec("state_space", y[:, inner + GN:], y[:, inner:inner + GN], y[:, :inner], rows[:, inner + C:], None,
-                   self.a_log, self.dt_bias, self.d_skip, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o,
-                   ctx.num_seqs, self.heads, self.groups, self.state, self.vdim, ctx.error_flag)
-        out = torch.empty((T, inner), dtype=h.dtype, device=h.device)
-        ops.group_rmsnorm(o, self.norm, self.eps, self.norm_groups, out=out, gate=rows[:, :inner], gate_mode="silu_before")
+        lens = list(ctx.host_query_lens)
+        long = h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported(self.state, max(lens))
+        if long:
+            # long portions: segments of tokens side by side
+            ops.linrec_segments("state_space", y[:, inner + GN:], y[:, inner:inner + GN], y[:, :inner], None, rows[:, inner + C:], None,
+                                self.a_log, self.dt_bias, self.d_skip, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o, lens,
+                                self.heads, self.groups, self.state, self.vdim, ctx.error_flag)
+        else:
+            ops.linrec("state_space", y[:, inner + GN:], y[:, inner:inner + GN], y[:, :inner], rows[:, inner + C:], None,
+                       self.a_log, self.dt_bias, self.d_skip, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o,
+                       ctx.num_seqs, self.heads, self.groups, self.state, self.vdim, ctx.error_flag)
+        out, gate = torch.empty((T, inner), dtype=h.dtype, device=h.device), rows[:, :inner]
+        if long and ops.part_rmsnorm_supported(o, gate, out, self.norm_groups):
+            ops.part_rmsnorm(o, self.norm, self.eps, self.norm_groups, out, gate=gate, gate_mode="silu_before")
+        else:
+            ops.group_rmsnorm(o, self.norm, self.eps, self.norm_groups, out=out, gate=gate, gate_mode="silu_before")
         return project(out, self.w_o, out_dtype=torch.float32)
 
 
