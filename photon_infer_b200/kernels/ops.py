@@ -1385,6 +1385,48 @@ def delta_recurrent(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_b
              _stream()), "delta_recurrent")
 
 
+#: A bfloat16 step in which some request brings at least this many tokens runs the delta rule 32 tokens at a time.
+DELTA_CHUNKED_MIN_TOKENS = 64
+
+
+def delta_chunked_supported(dim: int, vdim: int, longest: int) -> bool:
+    """Whether the delta rule of a bfloat16 step runs in chunks: heads of up to 128 and 256 numbers, a request with enough tokens."""
+    return dim <= 128 and vdim <= 256 and longest >= DELTA_CHUNKED_MIN_TOKENS
+
+
+def delta_chunked(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, cu_tokens: torch.Tensor,
+                  state_slots: torch.Tensor, state: torch.Tensor, o: torch.Tensor, query_lens, qk_heads: int, heads: int, dim: int, vdim: int,
+                  err: Optional[torch.Tensor]) -> None:
+    """``delta_recurrent`` for steps with long portions: what the tokens of a chunk of 32 do to each other is formed for all chunks
+    side by side, and the state walks from chunk to chunk in matrix products.  ``query_lens``: the requests' tokens in the step (host)."""
+    _cuda(y, ab, a_log, dt_bias, cu_tokens, state_slots, state, o, err)
+    T, S = y.shape[0], len(query_lens)
+    C = 2 * qk_heads * dim + heads * vdim
+    if y.dtype != torch.float32 or y.shape != (T, C) or not y.is_contiguous() or ab.shape != (T, 2 * heads) or ab.stride(1) != 1 \
+            or o.dtype != torch.float32 or o.shape != (T, heads * vdim) or not o.is_contiguous():
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "delta_chunked: y float32 [T, channels], ab [T, 2 heads], o float32 [T, heads * vdim]")
+    for t in (a_log, dt_bias):
+        if t.dtype != torch.float32 or t.numel() != heads or not t.is_contiguous():
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, "delta_chunked: A_log and dt_bias must be float32 [heads]")
+    if state.dtype != torch.float32 or state.dim() != 2 or not state.is_contiguous() or state.shape[1] < heads * dim * vdim:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "delta_chunked: state must be contiguous float32 [slots, row]")
+    _int32(cu_tokens, "cu_tokens")
+    _int32(state_slots, "state_slots")
+    if cu_tokens.numel() < S + 1 or state_slots.numel() < S or sum(query_lens) > T:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "delta_chunked: cu_tokens and state_slots must cover every request")
+    size = load_module("delta_chunked").photon_delta_chunked_scratch
+    size.restype, size.argtypes = c_long, [c_int] * 4
+    scratch = torch.empty(size(T, S, heads, vdim), dtype=torch.float32, device=y.device)
+    f = _fn("delta_chunked", "photon_delta_chunked",
+            [c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_int,
+             c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(_ptr(y), _ptr(ab), ab.stride(0), _dtype_code(ab), _ptr(a_log), _ptr(dt_bias), _ptr(cu_tokens), _ptr(state_slots), _ptr(state),
+             state.stride(0), state.shape[0], _ptr(o), _ptr(scratch), T, S, max(query_lens, default=0), qk_heads, heads, dim, vdim, _ptr(err),
+             _stream()), "delta_chunked")
+    global _launch_count
+    _launch_count += 1
+
+
 def delta_out(o: torch.Tensor, z: torch.Tensor, norm_w: torch.Tensor, eps: float, out: torch.Tensor, heads: int, vdim: int) -> None:
     """``out = o / sqrt(mean(o^2) + eps) * norm_w * silu(z)`` per head over ``vdim``; ``o`` float32, ``z`` a view."""
     _cuda(o, z, norm_w, out)

@@ -14,7 +14,7 @@ rows) starts at zero, is 32-bit, and lives in the request's state slot between s
 projections is 32-bit.
 
 One fused product gives ``[q | k | v | W_g h | W_a h | W_b h]`` as 32-bit rows; then the convolution kernel, the
-recurrence over the tokens of the step (one block per request and head), and norm and gate.
+recurrence over the tokens of the step (token by token, or 32 tokens at a time for long bfloat16 portions), and norm and gate.
 """
 from __future__ import annotations
 
@@ -32,7 +32,7 @@ DEFAULT_NAMES = {"q": "q", "k": "k", "v": "v", "g": "g", "o": "o", "a": "a", "b"
 
 
 class GatedDeltaRule(Mixer):
-    kernel_modules = ("delta",)
+    kernel_modules = ("delta", "delta_chunked")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, taps: int, eps: float,
@@ -94,8 +94,15 @@ class GatedDeltaRule(Mixer):
         ops.delta_conv(rows[:, :C], self.taps_w, ctx.token_seq, ctx.cu_tokens, ctx.state_slots, state,
                        self.heads * self.dim * self.vdim, y, ctx.num_seqs, self.qk_heads, H, self.dim, self.vdim, ctx.error_flag)
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
-        ops.delta_recurrent(y, rows[:, C + nv:C + nv + 2 * H], self.a_log, self.dt_bias, ctx.cu_tokens, ctx.state_slots, state,
-                            o, ctx.num_seqs, self.qk_heads, H, self.dim, self.vdim, ctx.error_flag)
+        ab = rows[:, C + nv:C + nv + 2 * H]
+        lens = list(ctx.host_query_lens)
+        if h.dtype == torch.bfloat16 and lens and ops.delta_chunked_supported(self.dim, self.vdim, max(lens)):
+            # long portions: 32 tokens at a time in matrix products
+            ops.delta_chunked(y, ab, self.a_log, self.dt_bias, ctx.cu_tokens, ctx.state_slots, state, o, lens, self.qk_heads, H, self.dim,
+                              self.vdim, ctx.error_flag)
+        else:
+            ops.delta_recurrent(y, ab, self.a_log, self.dt_bias, ctx.cu_tokens, ctx.state_slots, state,
+                                o, ctx.num_seqs, self.qk_heads, H, self.dim, self.vdim, ctx.error_flag)
         out = torch.empty((T, nv), dtype=h.dtype, device=h.device)
         ops.delta_out(o, rows[:, C:C + nv], self.norm, self.eps, out, H, self.vdim)
         return project(out, self.w_o)
