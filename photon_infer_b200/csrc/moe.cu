@@ -23,77 +23,12 @@
 #define MOE_BM 32          // rows of a tile of the grouped products
 
 // ---------------------------------------------------------------- router
-// A block owns `tok` consecutive tokens (at most its number of warps, at most 8): a warp takes every nwarp-th row of
-// the router and forms that row's logit for all of the block's tokens at once, so the row is read once per block.
-// Then warp i chooses for token i.  A logit's sum has the same order whatever `tok` and the number of warps are.  Measured on B200 with 2,048
-// tokens, 16 experts, rows of 2,048 (the call with its memset): one token per block 57 us, two 47, four 41, eight 59
-// (256 blocks, each walking its rows in sequence, are too few); 8 tokens: one per block 22 us, eight in one block 61.
-// Few tokens (TOK 1): one per block, a warp per row (up to 32), four loads of the row in flight.
-#define MOE_ROUTE_TOK 8
-template <typename T, int TOK>
-__global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) moe_route_kernel(const T* __restrict__ h, long h_stride, const T* __restrict__ Wr,
-                                 const void* __restrict__ bias, int bias_bf16, int H, int E, int top,
-                                 int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int T_,
-                                 int mode, int n_groups, int keep_groups, float route_scale,
-                                 const T* __restrict__ Wsg, float* __restrict__ shared_gate, int tok,
-                                 const float* __restrict__ correction, int real, const float* __restrict__ given) {
-  extern __shared__ float logits[];                     // per token: E (+ 1: the shared expert's gate) + n_groups flags (mode 3: + E)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-  const int t0 = blockIdx.x * tok;
-  const int ntok = min(tok, T_ - t0);
-  const int LS = E + 1 + n_groups + (mode == 3 ? E : 0);
-  constexpr int V = 16 / sizeof(T);                      // elements of a 16-byte load
-  const bool vec = (H % V == 0) && ((uintptr_t)h % 16 == 0) && (h_stride % V == 0) && ((uintptr_t)Wr % 16 == 0) &&
-                   ((uintptr_t)Wsg % 16 == 0);
-  if (given) {                                           // the logits come from a product of their own
-    for (int i = threadIdx.x; i < ntok * E; i += blockDim.x) {
-      const int u = i / E, e = i - u * E;
-      logits[u * LS + e] = given[(size_t)(t0 + u) * E + e] + (bias ? load_w(bias, bias_bf16, e) : 0.f);
-    }
-  }
-  for (int e = given ? E + warp : warp; e < E + (Wsg ? 1 : 0); e += nwarp) {
-    const T* w = e < E ? Wr + (size_t)e * H : Wsg;
-    float acc[TOK];
-#pragma unroll
-    for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
-    if (vec) {
-#pragma unroll (TOK == 1 ? 4 : 1)
-      for (int k = lane * V; k < H; k += 32 * V) {
-        const uint4 wv = *reinterpret_cast<const uint4*>(w + k);
-        const T* wp = reinterpret_cast<const T*>(&wv);
-#pragma unroll
-        for (int i = 0; i < TOK; ++i) {
-          if (i < ntok) {
-            const uint4 xv = *reinterpret_cast<const uint4*>(h + (size_t)(t0 + i) * h_stride + k);
-            const T* xp = reinterpret_cast<const T*>(&xv);
-#pragma unroll
-            for (int u = 0; u < V; ++u) acc[i] = fmaf(to_f32(xp[u]), to_f32(wp[u]), acc[i]);
-          }
-        }
-      }
-    } else {
-      for (int k = lane; k < H; k += 32) {
-        const float wk = to_f32(w[k]);
-#pragma unroll
-        for (int i = 0; i < TOK; ++i)
-          if (i < ntok) acc[i] = fmaf(to_f32(h[(size_t)(t0 + i) * h_stride + k]), wk, acc[i]);
-      }
-    }
-    const float add = (bias && e < E) ? load_w(bias, bias_bf16, e) : 0.f;
-#pragma unroll
-    for (int i = 0; i < TOK; ++i) {
-      if (i < ntok) {
-        const float v = warp_sum(acc[i]);
-        if (lane == 0) logits[i * LS + e] = v + add;
-      }
-    }
-  }
-  __syncthreads();
-  if (warp >= ntok) return;
-  const int t = t0 + warp;                               // this warp's token
-  float* lg = logits + warp * LS;
+// What a warp does once its token's logits stand in lg [E (+ 1: the shared expert's gate) + n_groups flags (mode 3: + E)].
+__device__ __forceinline__ void moe_choose(float* lg, int t, int lane, int E, int top, int* __restrict__ ids, float* __restrict__ weights,
+                                           int* __restrict__ counts, int mode, int n_groups, int keep_groups, float route_scale,
+                                           bool has_gate, float* __restrict__ shared_gate, const float* __restrict__ correction, int real) {
   const bool first = lane == 0;
-  if (first && Wsg) shared_gate[t] = 1.0f / (1.0f + expf(-lg[E]));
+  if (first && has_gate) shared_gate[t] = 1.0f / (1.0f + expf(-lg[E]));
   if (mode == 3) {
     // Scores are the softmax over all experts; the choice goes by score + correction, the weights are the chosen scores as
     // they are, times route_scale.  Lane i keeps the experts i, i + 32, ..; equal choice scores: the lower index.
@@ -252,6 +187,140 @@ __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) moe_route_kernel(const 
   }
 }
 
+// A block owns `tok` consecutive tokens (at most its number of warps, at most 8): a warp takes every nwarp-th row of
+// the router and forms that row's logit for all of the block's tokens at once, so the row is read once per block.
+// Then warp i chooses for token i.  A logit's sum has the same order whatever `tok` and the number of warps are.  Measured on B200 with 2,048
+// tokens, 16 experts, rows of 2,048 (the call with its memset): one token per block 57 us, two 47, four 41, eight 59
+// (256 blocks, each walking its rows in sequence, are too few); 8 tokens: one per block 22 us, eight in one block 61.
+// Few tokens (TOK 1): one per block, a warp per row (up to 32), four loads of the row in flight.
+#define MOE_ROUTE_TOK 8
+template <typename T, int TOK>
+__global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) moe_route_kernel(const T* __restrict__ h, long h_stride, const T* __restrict__ Wr,
+                                 const void* __restrict__ bias, int bias_bf16, int H, int E, int top,
+                                 int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int T_,
+                                 int mode, int n_groups, int keep_groups, float route_scale,
+                                 const T* __restrict__ Wsg, float* __restrict__ shared_gate, int tok,
+                                 const float* __restrict__ correction, int real, const float* __restrict__ given) {
+  extern __shared__ float logits[];                     // per token: E (+ 1: the shared expert's gate) + n_groups flags (mode 3: + E)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  const int t0 = blockIdx.x * tok;
+  const int ntok = min(tok, T_ - t0);
+  const int LS = E + 1 + n_groups + (mode == 3 ? E : 0);
+  constexpr int V = 16 / sizeof(T);                      // elements of a 16-byte load
+  const bool vec = (H % V == 0) && ((uintptr_t)h % 16 == 0) && (h_stride % V == 0) && ((uintptr_t)Wr % 16 == 0) &&
+                   ((uintptr_t)Wsg % 16 == 0);
+  if (given) {                                           // the logits come from a product of their own
+    for (int i = threadIdx.x; i < ntok * E; i += blockDim.x) {
+      const int u = i / E, e = i - u * E;
+      logits[u * LS + e] = given[(size_t)(t0 + u) * E + e] + (bias ? load_w(bias, bias_bf16, e) : 0.f);
+    }
+  }
+  for (int e = given ? E + warp : warp; e < E + (Wsg ? 1 : 0); e += nwarp) {
+    const T* w = e < E ? Wr + (size_t)e * H : Wsg;
+    float acc[TOK];
+#pragma unroll
+    for (int i = 0; i < TOK; ++i) acc[i] = 0.f;
+    if (vec) {
+#pragma unroll (TOK == 1 ? 4 : 1)
+      for (int k = lane * V; k < H; k += 32 * V) {
+        const uint4 wv = *reinterpret_cast<const uint4*>(w + k);
+        const T* wp = reinterpret_cast<const T*>(&wv);
+#pragma unroll
+        for (int i = 0; i < TOK; ++i) {
+          if (i < ntok) {
+            const uint4 xv = *reinterpret_cast<const uint4*>(h + (size_t)(t0 + i) * h_stride + k);
+            const T* xp = reinterpret_cast<const T*>(&xv);
+#pragma unroll
+            for (int u = 0; u < V; ++u) acc[i] = fmaf(to_f32(xp[u]), to_f32(wp[u]), acc[i]);
+          }
+        }
+      }
+    } else {
+      for (int k = lane; k < H; k += 32) {
+        const float wk = to_f32(w[k]);
+#pragma unroll
+        for (int i = 0; i < TOK; ++i)
+          if (i < ntok) acc[i] = fmaf(to_f32(h[(size_t)(t0 + i) * h_stride + k]), wk, acc[i]);
+      }
+    }
+    const float add = (bias && e < E) ? load_w(bias, bias_bf16, e) : 0.f;
+#pragma unroll
+    for (int i = 0; i < TOK; ++i) {
+      if (i < ntok) {
+        const float v = warp_sum(acc[i]);
+        if (lane == 0) logits[i * LS + e] = v + add;
+      }
+    }
+  }
+  __syncthreads();
+  if (warp >= ntok) return;
+  moe_choose(logits + warp * LS, t0 + warp, lane, E, top, ids, weights, counts, mode, n_groups, keep_groups, route_scale, Wsg != nullptr,
+             shared_gate, correction, real);
+}
+
+// Many bfloat16 tokens: a block forms the logits of 16 of them on the tensor cores (mma.m16n8k16: products of bfloat16 numbers
+// are exact, 16 of them are added up inside and everything beyond by 32-bit additions here), its eight warps taking every eighth
+// 32-wide piece of the rows with 16-byte loads (a lane's eight numbers are the k positions 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of two
+// products, for tokens and router rows alike), then a warp chooses for two tokens.  Bound by the latency of the rows' loads.
+// 2,048 tokens, 16 experts, rows of 2,048 (8.4 MB), beside the shared expert's products on another stream: 26 us; the kernel
+// above, which reads every router row from L2 once per four tokens, 36 us.
+#define MOE_ROUTE_MANY 16
+template <int NT>
+__global__ void __launch_bounds__(256)
+moe_route_many_kernel(const bf16* __restrict__ h, long h_stride, const bf16* __restrict__ Wr, const void* __restrict__ bias, int bias_bf16,
+                      int H, int E, int top, int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int T_, int mode,
+                      int n_groups, int keep_groups, float route_scale, const bf16* __restrict__ Wsg, float* __restrict__ shared_gate,
+                      const float* __restrict__ correction, int real) {
+  extern __shared__ float logits[];                     // [16][LS], then [8 warps][16][NT * 8] partial sums
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int t0 = blockIdx.x * MOE_ROUTE_MANY, ntok = min(MOE_ROUTE_MANY, T_ - t0);
+  const int LS = E + 1 + n_groups + (mode == 3 ? E : 0), outs = E + (Wsg ? 1 : 0);
+  float* part = logits + MOE_ROUTE_MANY * LS;
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  const bf16* r0 = g < ntok ? h + (size_t)(t0 + g) * h_stride + 8 * t : nullptr;
+  const bf16* r1 = g + 8 < ntok ? h + (size_t)(t0 + g + 8) * h_stride + 8 * t : nullptr;
+  const bf16* rw[NT];
+  float acc[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    const int e = n * 8 + g;
+    rw[n] = e < E ? Wr + (size_t)e * H + 8 * t : e < outs ? Wsg + 8 * t : nullptr;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+  }
+#pragma unroll 2
+  for (int k = warp * 32; k < H; k += 256) {
+    const uint4 x0 = r0 ? *reinterpret_cast<const uint4*>(r0 + k) : none, x1 = r1 ? *reinterpret_cast<const uint4*>(r1 + k) : none;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      const uint4 w = rw[n] ? *reinterpret_cast<const uint4*>(rw[n] + k) : none;
+      float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+          : "+f"(d[0][0]), "+f"(d[0][1]), "+f"(d[0][2]), "+f"(d[0][3]) : "r"(x0.x), "r"(x1.x), "r"(x0.y), "r"(x1.y), "r"(w.x), "r"(w.y));
+      asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+          : "+f"(d[1][0]), "+f"(d[1][1]), "+f"(d[1][2]), "+f"(d[1][3]) : "r"(x0.z), "r"(x1.z), "r"(x0.w), "r"(x1.w), "r"(w.z), "r"(w.w));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[n][i] += d[0][i] + d[1][i];
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[(warp * 16 + g + (i >> 1) * 8) * (NT * 8) + n * 8 + 2 * t + (i & 1)] = acc[n][i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < ntok * outs; i += 256) {
+    const int u = i / outs, e = i - u * outs;
+    double v = bias && e < E ? (double)load_w(bias, bias_bf16, e) : 0.0;   // one rounding for the sum over the warps
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += (double)part[(w * 16 + u) * (NT * 8) + e];
+    logits[u * LS + e] = (float)v;
+  }
+  __syncthreads();
+  for (int u = warp; u < ntok; u += 8)
+    moe_choose(logits + u * LS, t0 + u, lane, E, top, ids, weights, counts, mode, n_groups, keep_groups, route_scale, Wsg != nullptr,
+               shared_gate, correction, real);
+}
+
 // h [T][H] (row stride in elements), Wr [E][H] of the same type, bias [E] (may be null).  ids, weights [T][top];
 // counts [E] is cleared first and then holds the number of (token, choice) pairs of every expert.
 PHOTON_API int photon_moe_route(const void* h, long h_stride, int dtype, const void* Wr, const void* bias, int bias_dtype,
@@ -292,6 +361,21 @@ PHOTON_API int photon_moe_route_ex(const void* h, long h_stride, int dtype, cons
   cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)buckets * sizeof(int), stream);
   if (e != cudaSuccess) return (int)e;
   const int blocks = (T_ + tok - 1) / tok;
+  // 64 outputs are what a warp's registers hold; rows that its 16-byte loads cannot read, other types and logits that were formed
+  // before go to the kernel above
+  const int tiles = (E + (Wsg ? 1 : 0) + 7) / 8;
+  if (!few && dtype == PHOTON_BF16 && logits == nullptr && tiles <= 8 && H % 32 == 0 && h_stride % 8 == 0 && ((uintptr_t)h & 15) == 0 &&
+      ((uintptr_t)Wr & 15) == 0 && ((uintptr_t)Wsg & 15) == 0) {
+    const int nt = tiles <= 2 ? 2 : tiles <= 3 ? 3 : tiles <= 4 ? 4 : 8;
+    const size_t room = ((size_t)MOE_ROUTE_MANY * (E + 1 + n_groups + (mode == 3 ? E : 0)) + (size_t)8 * 16 * nt * 8) * sizeof(float);
+#define MOE_MANY(NT) do { \
+      if (room > 48 * 1024 && (e = cudaFuncSetAttribute(moe_route_many_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room)) != cudaSuccess) return (int)e; \
+      moe_route_many_kernel<NT><<<(T_ + MOE_ROUTE_MANY - 1) / MOE_ROUTE_MANY, 256, room, stream>>>((const bf16*)h, h_stride, (const bf16*)Wr, bias, \
+          bias_dtype == PHOTON_BF16, H, E, top, ids, weights, counts, T_, mode, n_groups, keep_groups, route_scale, (const bf16*)Wsg, shared_gate, \
+          correction, real); } while (0)
+    if (nt == 2) MOE_MANY(2); else if (nt == 3) MOE_MANY(3); else if (nt == 4) MOE_MANY(4); else MOE_MANY(8);
+    return launch_status();
+  }
 #define MOE_ROUTE(T, TOK) moe_route_kernel<T, TOK><<<blocks, warps * 32, smem, stream>>>((const T*)h, h_stride, (const T*)Wr, bias, \
       bias_dtype == PHOTON_BF16, H, E, top, ids, weights, counts, T_, mode, n_groups, keep_groups, route_scale, (const T*)Wsg, shared_gate, \
       tok, correction, real, logits)
@@ -349,7 +433,8 @@ PHOTON_API int photon_moe_align(const int* ids, const int* counts, int n, int E,
                                 int* tiles, int* num_tiles, cudaStream_t stream) {
   if (n <= 0 || E <= 0) return 0;
   if (real != E && real != E - 1) return PHOTON_ERR_ARGUMENT;
-  moe_align_kernel<<<E, 256, 0, stream>>>(ids, counts, n, E, real, offsets, sorted, place, tiles, num_tiles);
+  // a block walks all pairs: 4,096 of them take 8 us with 1,024 threads, 10 with 256
+  moe_align_kernel<<<E, n >= 1024 ? 1024 : 256, 0, stream>>>(ids, counts, n, E, real, offsets, sorted, place, tiles, num_tiles);
   return launch_status();
 }
 

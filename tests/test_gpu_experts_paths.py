@@ -1,0 +1,32 @@
+"""Routed experts: the router's logits of many tokens on the tensor cores."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("T,H,E,gate", [(64, 32, 2, False), (65, 64, 8, True), (79, 288, 16, False), (2049, 2048, 16, True), (130, 96, 33, True),
+                                        (100, 160, 63, True), (100, 160, 64, True)])
+@pytest.mark.parametrize("scoring", ["softmax_chosen", "softmax_all", "sigmoid", "softmax_raw"])
+def test_router_of_many_tokens(T, H, E, gate, scoring):
+    """The choice and the weights against 64 bits; a choice may differ only where two scores are closer than the logits' rounding
+    (products of bfloat16 numbers are exact: H additions of at most 2^-23 of the sum of magnitudes)."""
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(T + E)
+    h, wr, b = torch.randn(T, H, device=DEV).bfloat16(), (torch.randn(E, H, device=DEV) * H ** -0.5).bfloat16(), torch.randn(E, device=DEV) * 0.1
+    wsg = (torch.randn(1, H, device=DEV) * H ** -0.5).bfloat16() if gate else None
+    got = ops.moe_route(h, wr, b, 2, scoring, w_shared_gate=wsg)
+    ids, weights, counts = got[:3]
+    z = h.double() @ wr.double().t() + b.double()
+    err = H * 2.0 ** -23 * (h.double().abs() @ wr.double().abs().t()).max()
+    score = {"softmax_chosen": z, "softmax_all": torch.softmax(z, -1), "sigmoid": torch.sigmoid(z), "softmax_raw": torch.softmax(z, -1)}[scoring]
+    top, want = torch.topk(z, 2, dim=-1)
+    chosen = z.gather(1, ids.long())
+    assert float((chosen - top).abs().max()) <= 2 * float(err)
+    s = score.gather(1, ids.long())
+    w = {"softmax_chosen": torch.softmax(s, -1), "softmax_all": s / s.sum(-1, keepdim=True), "sigmoid": s, "softmax_raw": s}[scoring]
+    assert float((weights.double() - w).abs().max()) < 2e-5
+    assert torch.equal(counts.cpu().long(), torch.bincount(ids.flatten().long().cpu(), minlength=E))
+    if gate:
+        assert float((got[3].double().flatten() - torch.sigmoid(h.double() @ wsg[0].double())).abs().max()) < 2e-5
