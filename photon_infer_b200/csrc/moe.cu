@@ -721,58 +721,106 @@ PHOTON_API int photon_moe_glu(const void* gate_up, void* out, int dtype, int n, 
 }
 
 // ---------------------------------------------------------------- few rows: one matrix-vector product per pair
-// A decode step brings a handful of (token, choice) pairs, each to another expert as a rule: nothing is sorted,
-// block (c, p) streams the rows c * 32 .. of pair p's expert matrix once, 16 bytes per lane and load, against the
-// pair's input row in shared memory; a warp owns four output features at a time and adds its lanes' sums up.
-#define GEMV_COLS 32
+// A decode step brings a handful of (token, choice) pairs: nothing is sorted, a warp streams GEMV_ROWS rows of an expert's matrix
+// side by side (gate and up of half as many columns), 16 bytes per lane and load, against the pair's input row in shared memory,
+// and adds its lanes' sums up.  Pairs that chose the same expert can share a block: the first of every SHARE of them (in the
+// order of the pairs, at most 64) multiplies the rows with the inputs of all of them, the others' blocks return.  A pair's sums
+// are formed in the same order either way.  Bound by the bytes of the experts that were chosen, as long as those pairs that are
+// not shared don't read them from L2 over and over.  Gate and up, then down, of 16 experts, random choices, us (in brackets one
+// row, or gate and up of one column, at a time and nothing shared): width and expert size 2,048: 2 pairs 9 + 8 (13 + 8), 8 pairs
+// 25 + 15 (29 + 19), 16 pairs 41 + 23 (50 + 23), 32 pairs 55 + 31 (71 + 40), 64 pairs 93 + 49 (129 + 66); 4,096: 8 pairs 80 + 43
+// (100 + 41), 16 pairs 115 + 64 (155 + 70), 64 pairs 357 + 182 (583 + 291; the gate and up matrices at 6.5 TB/s: 164).  Two rows
+// side by side: 55 + 33 at 32 pairs, 96 + 52 at 64.  Four pieces of a row ahead instead of two: 68 + 37, 119 + 60 when shared.
+#define GEMV_ROWS 4
+#define GEMV_SHARE 4
+// From this many pairs on some are likely to share: 2,048 wide, 8 pairs 31 + 17 us shared and 25 + 15 alone, 16 pairs 41 + 23 both,
+// 32 pairs 55 + 31 and 67 + 34; 4,096 wide, 8 pairs 82 + 43 and 80 + 43, 16 pairs 115 + 64 and 155 + 77.
+#define GEMV_SHARE_FROM 16
 
-template <typename TO, bool GLU>
+template <typename TO, bool GLU, int SHARE>
 __global__ void __launch_bounds__(256)
 moe_gemv_kernel(const bf16* __restrict__ x, long ldx, int x_div, const int* __restrict__ ids, const bf16* __restrict__ W,
                 TO* __restrict__ out, long ldo, int N, int K, int act, const float* __restrict__ weights, float limit,
-                float slope, int experts) {
-  extern __shared__ __align__(16) bf16 xs[];
+                float slope, int experts, int n) {
+  extern __shared__ __align__(16) bf16 xs[];             // [SHARE][K]
+  constexpr int R = GEMV_ROWS, C = GLU ? R / 2 : R;
   const int p = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int e = ids[p];
   if (e >= experts) return;                              // an identity expert: nothing to multiply
+  int pair[SHARE], count = 1;
+  pair[0] = p;
+  if (SHARE > 1) {                                       // n <= 64
+    const unsigned lo = __ballot_sync(0xffffffffu, lane < n && ids[lane < n ? lane : 0] == e);
+    const unsigned hi = __ballot_sync(0xffffffffu, lane + 32 < n && ids[lane + 32 < n ? lane + 32 : 0] == e);
+    unsigned long long same = (unsigned long long)hi << 32 | lo;
+    if (__popcll(same & ((1ull << p) - 1)) % SHARE != 0) return;
+    same &= ~((2ull << p) - 1);                          // the pairs behind this one
+#pragma unroll
+    for (int j = 1; j < SHARE; ++j) {
+      pair[j] = p;
+      if (same) { pair[j] = __ffsll(same) - 1; same &= same - 1; count = j + 1; }
+    }
+  }
   const int cols = GLU ? N / 2 : N;
-  const bf16* xr = x + (size_t)(p / x_div) * ldx;
-  for (int i = threadIdx.x * 8; i < K; i += blockDim.x * 8)
-    *reinterpret_cast<uint4*>(xs + i) = *reinterpret_cast<const uint4*>(xr + i);
+#pragma unroll
+  for (int j = 0; j < SHARE; ++j) {
+    if (j < count) {
+      const bf16* xr = x + (size_t)(pair[j] / x_div) * ldx;
+      for (int i = threadIdx.x * 8; i < K; i += blockDim.x * 8)
+        *reinterpret_cast<uint4*>(xs + (size_t)j * K + i) = *reinterpret_cast<const uint4*>(xr + i);
+    }
+  }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bf16* We = W + (size_t)e * N * K;
+  const int col = (blockIdx.x * 8 + warp) * C;
+  if (col >= cols) return;                               // the whole warp
+  const bf16* w[R];                                      // rows behind the last column repeat it
 #pragma unroll
-  for (int c = 0; c < GEMV_COLS / 8; ++c) {
-    const int col = blockIdx.x * GEMV_COLS + c * 8 + warp;
-    if (col >= cols) continue;                           // the whole warp
-    float a0 = 0.f, a1 = 0.f;
-    const bf16* w0 = We + (size_t)col * K;
-    const bf16* w1 = We + (size_t)(col + cols) * K;
-    for (int k = lane * 8; k < K; k += 256) {
-      const uint4 xv = *reinterpret_cast<const uint4*>(xs + k);
-      const uint4 wv = *reinterpret_cast<const uint4*>(w0 + k);
-      const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
-      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv);
+  for (int r = 0; r < R; ++r)
+    w[r] = W + ((size_t)e * N + min(col + r % C, cols - 1) + (r / C) * cols) * K;
+  float a[SHARE][R];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 xf = __bfloat1622float2(xp[i]), wf = __bfloat1622float2(wp[i]);
-        a0 = fmaf(xf.x, wf.x, a0); a0 = fmaf(xf.y, wf.y, a0);
-      }
-      if (GLU) {
-        const uint4 uv = *reinterpret_cast<const uint4*>(w1 + k);
-        const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&uv);
+  for (int j = 0; j < SHARE; ++j)
+#pragma unroll
+    for (int r = 0; r < R; ++r) a[j][r] = 0.f;
+#pragma unroll 2
+  for (int k = lane * 8; k < K; k += 256) {
+    uint4 wv[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) wv[r] = *reinterpret_cast<const uint4*>(w[r] + k);
+#pragma unroll
+    for (int j = 0; j < SHARE; ++j) {
+      if (j < count) {
+        const uint4 xv = *reinterpret_cast<const uint4*>(xs + (size_t)j * K + k);
+        const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float2 xf = __bfloat1622float2(xp[i]), uf = __bfloat1622float2(up[i]);
-          a1 = fmaf(xf.x, uf.x, a1); a1 = fmaf(xf.y, uf.y, a1);
+          const float2 xf = __bfloat1622float2(xp[i]);
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const float2 wf = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wv[r])[i]);
+            a[j][r] = fmaf(xf.x, wf.x, a[j][r]); a[j][r] = fmaf(xf.y, wf.y, a[j][r]);
+          }
         }
       }
     }
-    a0 = warp_sum(a0);
-    if (GLU) a1 = warp_sum(a1);
-    if (weights) { const float f = weights[p]; a0 *= f; a1 *= f; }   // the pair's input factor
-    if (lane == 0) out[(size_t)p * ldo + col] = from_f32<TO>(GLU ? moe_glu_pair(a0, a1, act, limit, slope) : moe_act(a0, act));
+  }
+#pragma unroll
+  for (int j = 0; j < SHARE; ++j) {
+    if (j < count) {
+      const float f = weights ? weights[pair[j]] : 1.f;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        a[j][r] = warp_sum(a[j][r]);
+        if (weights) a[j][r] *= f;                       // the pair's input factor
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          if (col + c < cols)
+            out[(size_t)pair[j] * ldo + col + c] = from_f32<TO>(GLU ? moe_glu_pair(a[j][c], a[j][(GLU ? C : 0) + c], act, limit, slope) : moe_act(a[j][c], act));
+      }
+    }
   }
 }
 
@@ -787,12 +835,17 @@ PHOTON_API int photon_moe_gemv(const void* x, long ldx, int x_div, const int* id
   if (K <= 0 || x_div <= 0 || (glu && (N & 1)) || (act == PHOTON_ACT_CLAMPED_SWISH && !glu)) return PHOTON_ERR_ARGUMENT;
   if (K % 8 || ldx % 8 || (uintptr_t)x % 16 || (uintptr_t)W % 16 || n > 65535 || (size_t)K * 2 > 96 * 1024) return PHOTON_ERR_UNSUPPORTED;
   const int cols = glu ? N / 2 : N;
-  dim3 grid((cols + GEMV_COLS - 1) / GEMV_COLS, n);
-  const size_t smem = (size_t)K * sizeof(bf16);
-#define MOE_GEMV(TO, GLU) do { \
-    if (smem > 48 * 1024) { cudaError_t e_ = cudaFuncSetAttribute(moe_gemv_kernel<TO, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+  const int block_cols = 8 * (glu ? GEMV_ROWS / 2 : GEMV_ROWS);
+  dim3 grid((cols + block_cols - 1) / block_cols, n);
+  // sharing needs the ids of all pairs in one look and the rows of all its pairs in shared memory
+  const bool share = n >= GEMV_SHARE_FROM && n <= 64 && (size_t)GEMV_SHARE * K * sizeof(bf16) <= 96 * 1024;
+  const size_t smem = (size_t)(share ? GEMV_SHARE : 1) * K * sizeof(bf16);
+#define MOE_GEMV_GO(TO, GLU, SHARE) do { \
+    if (smem > 48 * 1024) { cudaError_t e_ = cudaFuncSetAttribute(moe_gemv_kernel<TO, GLU, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
                             if (e_ != cudaSuccess) return (int)e_; } \
-    moe_gemv_kernel<TO, GLU><<<grid, 256, smem, stream>>>((const bf16*)x, ldx, x_div, ids, (const bf16*)W, (TO*)out, ldo, N, K, act, weights, limit, slope, experts); } while (0)
+    moe_gemv_kernel<TO, GLU, SHARE><<<grid, 256, smem, stream>>>((const bf16*)x, ldx, x_div, ids, (const bf16*)W, (TO*)out, ldo, N, K, act, weights, \
+                                                                 limit, slope, experts, n); } while (0)
+#define MOE_GEMV(TO, GLU) do { if (share) MOE_GEMV_GO(TO, GLU, GEMV_SHARE); else MOE_GEMV_GO(TO, GLU, 1); } while (0)
   if (out_dtype == PHOTON_BF16) { if (glu) MOE_GEMV(bf16, true); else MOE_GEMV(bf16, false); }
   else if (out_dtype == PHOTON_F32) { if (glu) MOE_GEMV(float, true); else MOE_GEMV(float, false); }
   else return PHOTON_ERR_ARGUMENT;

@@ -1,9 +1,39 @@
-"""Routed experts: the router's logits of many tokens on the tensor cores."""
+"""Routed experts: pairs that share an expert's rows in the matrix-vector products of a decode step, and the router's logits of
+many tokens on the tensor cores."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("pairs", [[0], [3, 3], [2, 2, 2, 2, 2] * 3, [0, 5, 0, 1, 5, 0, 0, 0, 5, 3, 3, 0, 5, 5, 5, 5], [4] * 64,
+                                   [i * 7 % 6 for i in range(64)], [i % 2 * 5 for i in range(33)], [1] * 31 + [2] + [1] * 9,
+                                   [7, 0, 7, 0], [7, 0] * 12, [i % 5 for i in range(70)]])
+@pytest.mark.parametrize("glu", [False, True])
+def test_pairs_of_one_expert_get_the_bits_that_they_get_alone(pairs, glu):
+    """Groups of one, of exactly four, of more, at the ends of the 64 pairs that are seen at once, beyond them, and ids behind the
+    last expert (identity experts), whose rows stay as they are."""
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(len(pairs))
+    E, N, K = 6, 74, 264
+    w = torch.randn(E, N, K, device=DEV).bfloat16()
+    x = torch.randn((len(pairs) + 1) // 2, K, device=DEV).bfloat16()
+    f = torch.rand(len(pairs), device=DEV)
+    ids = torch.tensor(pairs, dtype=torch.int32, device=DEV)
+    cols = N // 2 if glu else N
+    act = dict(glu=True, activation="silu") if glu else {}
+    out = torch.full((len(pairs), cols), 9.0, device=DEV)
+    ops.moe_gemv(x, 2, ids, w, out, weights=f, **act)
+    for p, e in enumerate(pairs):
+        one = torch.full((1, cols), 9.0, device=DEV)
+        ops.moe_gemv(x[p // 2:p // 2 + 1], 1, ids[p:p + 1], w, one, weights=f[p:p + 1], **act)
+        assert torch.equal(one[0], out[p]), p
+        if e >= E:
+            assert bool((out[p] == 9.0).all())
+        elif not glu:
+            want = (w[e].double() @ x[p // 2].double()) * f[p].double()
+            assert float((out[p].double() - want).abs().max()) < K * 2.0 ** -24 * float((w[e].double().abs() @ x[p // 2].double().abs()).max())
 
 
 @pytest.mark.parametrize("T,H,E,gate", [(64, 32, 2, False), (65, 64, 8, True), (79, 288, 16, False), (2049, 2048, 16, True), (130, 96, 33, True),
