@@ -21,6 +21,10 @@
 // own row (attention over a cached latent: the latent is key and value at once, the rest of the row is a
 // rotated key part).  And the query heads that share a key/value head are cut into chunks of `hb` heads per
 // block, so that any number of query heads may share one key/value head.
+//
+// Bound by latency: a block's tiles follow one another, and few blocks are there when tokens are decoded.  Keys and values come
+// in 16-byte loads and a product's operands 16 numbers ahead: two decoded 32-bit tokens behind 500 keys (16 tiles, 4 heads of 64 a
+// block) in a layer's step 103 us; with 4-byte loads of the values, a division for the offset of each, and the product not unrolled 231.
 #include "common.cuh"
 #include <math.h>
 
@@ -51,7 +55,7 @@ paged_attention_kernel(const T* __restrict__ q, long q_stride, T* __restrict__ o
   float* mrun = sc + hb * ATT_TILE;          // hb
   float* lsum = mrun + hb;                   // hb
   float* corr = lsum + hb;                   // hb
-  long long* kbase = (long long*)(corr + hb + ((hb & 1) & ((d + 1) & 1)));   // TILE; 8-byte aligned: an odd number of floats
+  long long* krow = (long long*)(corr + hb + ((hb & 1) & ((d + 1) & 1)));   // TILE; 8-byte aligned: an odd number of floats
                                                                             // (hb * (d + 3) of them, mod 2) gets one more
   if (shared_kv) vs = ks;
 
@@ -93,21 +97,22 @@ paged_attention_kernel(const T* __restrict__ q, long q_stride, T* __restrict__ o
   }
   constexpr int VEC = 16 / sizeof(T);
   const bool vec = (d % VEC == 0) && ((uintptr_t)k_cache % 16 == 0);
+  const bool vec_v = (dv % VEC == 0) && ((uintptr_t)v_cache % 16 == 0);
   for (int vt = vt_lo; vt < vt_hi; ++vt) {
     const int tile0 = (vt < kept_tiles ? vt : tile_lo + vt - kept_tiles) * ATT_TILE;
     __syncthreads();                          // previous tile fully consumed; qs ready on the first pass
     if (tid < ATT_TILE) {
       const int kk = tile0 + tid;
-      long long base = -1;
+      long long row = -1;
       if (kk <= p && (kk >= kstart || kk < keep_first)) {
         const int page = table[kk / page_size];
         if (page < 0 || page >= num_pages) {
           report_error(err, PHOTON_DEV_BAD_PAGE, t, kk, page);
         } else {
-          base = (((long long)page * n_kv + g) * page_size + (kk % page_size)) * d;
+          row = ((long long)page * n_kv + g) * page_size + (kk % page_size);
         }
       }
-      kbase[tid] = base;
+      krow[tid] = row;
     }
     __syncthreads();
     if (vec) {
@@ -115,9 +120,9 @@ paged_attention_kernel(const T* __restrict__ q, long q_stride, T* __restrict__ o
 #pragma unroll 4
       for (int i = tid; i < ATT_TILE * per_key; i += ATT_THREADS) {
         const int key = i / per_key, j = (i - key * per_key) * VEC;
-        const long long base = kbase[key];
+        const long long row = krow[key];
         uint4 raw = make_uint4(0, 0, 0, 0);
-        if (base >= 0) raw = *reinterpret_cast<const uint4*>(k_cache + base + j);
+        if (row >= 0) raw = *reinterpret_cast<const uint4*>(k_cache + row * d + j);
         const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
         for (int u = 0; u < VEC; ++u) ks[key * (d + 1) + j + u] = to_f32(e[u]);
@@ -125,15 +130,27 @@ paged_attention_kernel(const T* __restrict__ q, long q_stride, T* __restrict__ o
     } else {
       for (int i = tid; i < ATT_TILE * d; i += ATT_THREADS) {
         const int key = i / d, j = i - key * d;
-        const long long base = kbase[key];
-        ks[key * (d + 1) + j] = base >= 0 ? to_f32(k_cache[base + j]) : 0.f;
+        const long long row = krow[key];
+        ks[key * (d + 1) + j] = row >= 0 ? to_f32(k_cache[row * d + j]) : 0.f;
       }
     }
-    if (!shared_kv) {
+    if (!shared_kv && vec_v) {
+      const int per_key = dv / VEC;
+#pragma unroll 4
+      for (int i = tid; i < ATT_TILE * per_key; i += ATT_THREADS) {
+        const int key = i / per_key, j = (i - key * per_key) * VEC;
+        const long long row = krow[key];
+        uint4 raw = make_uint4(0, 0, 0, 0);
+        if (row >= 0) raw = *reinterpret_cast<const uint4*>(v_cache + row * dv + j);
+        const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+        for (int u = 0; u < VEC; ++u) vs[key * dv + j + u] = to_f32(e[u]);
+      }
+    } else if (!shared_kv) {
       for (int i = tid; i < ATT_TILE * dv; i += ATT_THREADS) {
         const int key = i / dv, j = i - key * dv;
-        const long long base = kbase[key];
-        vs[key * dv + j] = base >= 0 ? to_f32(v_cache[base / d * dv + j]) : 0.f;
+        const long long row = krow[key];
+        vs[key * dv + j] = row >= 0 ? to_f32(v_cache[row * dv + j]) : 0.f;
       }
     }
     __syncthreads();
@@ -141,10 +158,11 @@ paged_attention_kernel(const T* __restrict__ q, long q_stride, T* __restrict__ o
     for (int i = tid; i < G * ATT_TILE; i += ATT_THREADS) {
       const int h = i / ATT_TILE, key = i - h * ATT_TILE;
       float s = -INFINITY;
-      if (kbase[key] >= 0) {
+      if (krow[key] >= 0) {
         const float* qh = qs + h * d;
         const float* kr = ks + key * (d + 1);
         float dot = 0.f;
+#pragma unroll 16
         for (int j = 0; j < d; ++j) dot += qh[j] * kr[j];
         s = dot * scale;
         if (softcap > 0.f) s = softcap * tanhf(s / softcap);
