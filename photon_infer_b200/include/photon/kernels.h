@@ -140,6 +140,14 @@ PHOTON_EXPORT int photon_paged_attention_ex(const void* q, long q_stride, void* 
                               int window, float scale, int splits, float* part, int* err, int keep_first, const float* sinks,
                               float softcap, const void* gate, long gate_stride, cudaStream_t stream);
 
+/* ------------------------------------------------------------------ attention_rows.cu: prompt portions in true 32-bit */
+/* photon_paged_attention's results, bit for bit, for float q, out [T][n_q * d] and caches [num_pages][n_kv][page_size][d]: a block walks
+ * the keys for several tokens of one request.  cu_tokens [num_seqs + 1]: where every request's tokens begin, T at the end.  d 64 or
+ * 128, up to 32 query heads per key/value head, 16-byte aligned rows; others: PHOTON_ERR_UNSUPPORTED. */
+PHOTON_EXPORT int photon_attention_rows(const float* q, long q_stride, float* out, long out_stride, const float* k_cache, const float* v_cache,
+                              const int* block_table, int max_pages, const int* cu_tokens, const int* positions, int T_, int num_seqs,
+                              int n_q, int n_kv, int d, int page_size, int num_pages, float scale, int* err, cudaStream_t stream);
+
 /* ------------------------------------------------------------------ latent.cu: attention over a cached latent */
 /* One pass over a token's fused down-projection row down[t] = [query latent (q_rank) | key/value latent (kv_rank) |
  * shared key part (rot)]: cq[t] = rmsnorm(query latent) * q_norm_w; the cache row at slot_mapping[t] becomes

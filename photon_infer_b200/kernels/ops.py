@@ -486,6 +486,38 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v
         _launch_count += 1
 
 
+def attention_rows_supported(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, n_q: int, n_kv: int,
+                             head_dim: int) -> bool:
+    """Whether ``attention_rows`` takes the call: float32, heads of 64 or 128, up to 32 query heads per key/value head, caches and
+    rows in 16-byte pieces."""
+    return (q.dtype == torch.float32 and head_dim in (64, 128) and n_kv > 0 and n_q % n_kv == 0 and n_q // n_kv <= 32
+            and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0 and v_cache.shape == k_cache.shape
+            and all(t.dtype == torch.float32 and t.data_ptr() % 16 == 0 for t in (q, out, k_cache, v_cache)))
+
+
+def attention_rows(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
+                   cu_tokens: torch.Tensor, positions: torch.Tensor, num_seqs: int, n_q: int, n_kv: int, head_dim: int, scale: float,
+                   err: Optional[torch.Tensor]) -> None:
+    """``paged_attention``'s results, bit for bit, with a block for several tokens of a request (float32, no window): request ``s`` has
+    the tokens ``cu_tokens[s] .. cu_tokens[s + 1]`` of the step."""
+    _cuda(q, out, k_cache, v_cache, block_table, cu_tokens, positions, err)
+    T = q.shape[0]
+    if q.shape[1] != n_q * head_dim or q.stride(1) != 1 or out.shape != (T, n_q * head_dim) or out.stride(1) != 1:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "attention_rows: q and out must be [T, n_q * head_dim]")
+    if k_cache.shape[3] != head_dim or k_cache.shape[1] != n_kv or cu_tokens.numel() < num_seqs + 1:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "attention_rows: the caches are [pages, n_kv, page_size, head_dim], cu_tokens [requests + 1]")
+    if not attention_rows_supported(q, out, k_cache, v_cache, n_q, n_kv, head_dim):
+        raise PhotonError(ErrorCode.UNSUPPORTED_SIZE, "attention_rows: float32, heads of 64 or 128, at most 32 per key/value head, aligned rows")
+    for name, t in (("block_table", block_table), ("cu_tokens", cu_tokens), ("positions", positions)):
+        _int32(t, name)
+    f = _fn("attention_rows", "photon_attention_rows",
+            [c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+             c_int, c_int, c_float, c_void_p, c_void_p])
+    _check(f(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1],
+             _ptr(cu_tokens), _ptr(positions), T, num_seqs, n_q, n_kv, head_dim, k_cache.shape[2], k_cache.shape[0], float(scale), _ptr(err),
+             _stream()), "attention_rows")
+
+
 _ticket_buffers = {}
 
 

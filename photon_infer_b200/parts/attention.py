@@ -152,8 +152,23 @@ class PagedAttention(Mixer):
             attend_tensor_cores(self, q, out, ctx, cache)
             return
         group = ctx.groups[cache.group]
+        if self.window is None and rows_together(ctx, q, out, cache, self.n_q, self.n_kv, self.head_dim):
+            ops.attention_rows(q, out, cache.k, cache.v, group.block_table, ctx.cu_tokens, ctx.positions, ctx.num_seqs,
+                               self.n_q, self.n_kv, self.head_dim, self.scale, ctx.error_flag)
+            return
         ops.paged_attention(q, out, cache.k, cache.v, group.block_table, ctx.token_seq, ctx.positions,
                             self.n_q, self.n_kv, self.head_dim, self.window, self.scale, ctx.error_flag)
+
+
+def rows_together(ctx: StepContext, q: torch.Tensor, out: torch.Tensor, cache: LayerCache, n_q: int, n_kv: int, head_dim: int) -> bool:
+    """Whether prompt portions in 32-bit take the kernel whose blocks walk the keys for several tokens (``ops.attention_rows``: the
+    general kernel's bits).  A block of it needs as long for a tile of keys however few of its rows there are, so it wants as many
+    (token, head) rows as would fill the chip with the general kernel's blocks, or many heads per key/value head.  Both on a B200, us,
+    general kernel first, 32/8 heads of 64: 512 tokens 264 and 88; 64 tokens behind 500: 91 and 79; 16 requests of 3 behind 500: 77 and 67;
+    4 tokens behind 500: 66 and 66; 16 tokens 6 and 11; 8/8 heads: 64 tokens behind 500: 72 and 79; 32/1 heads: 4 tokens behind 500: 234
+    and 71."""
+    return (ctx.max_query_len > 1 and (q.shape[0] * n_q >= 1024 or n_q >= 16 * n_kv)
+            and ops.attention_rows_supported(q, out, cache.k, cache.v, n_q, n_kv, head_dim))
 
 
 def attend_tensor_cores(mixer, q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: LayerCache,

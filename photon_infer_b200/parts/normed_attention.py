@@ -22,7 +22,7 @@ from typing import Dict, List, Optional
 import torch
 
 from ..kernels import ops
-from .attention import attend_tensor_cores
+from .attention import attend_tensor_cores, rows_together
 from .base import LayerCache, Mixer, PagedCacheSpec, StepContext, TensorSpec
 from .linear import project
 from .registry import register_mixer
@@ -158,6 +158,11 @@ class NormedAttention(Mixer):
                                 gate=gate)
             return
         group = ctx.groups[cache.group]
+        plain = self.window is None and not self.keep_first and self.sinks is None and not self.softcap and gate is None
+        if plain and rows_together(ctx, q, out, cache, self.n_q, self.n_kv, self.head_dim):
+            ops.attention_rows(q, out, cache.k, cache.v, group.block_table, ctx.cu_tokens, ctx.positions, ctx.num_seqs,
+                               self.n_q, self.n_kv, self.head_dim, self.scale, ctx.error_flag)
+            return
         splits = 1
         if q.dtype == torch.bfloat16 and ctx.max_query_len == 1:
             keys = ctx.max_context_len if self.window is None else min(self.window + self.keep_first + 1, ctx.max_context_len)
