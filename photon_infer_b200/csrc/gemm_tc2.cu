@@ -378,7 +378,7 @@ static int t2_launch(const void* x, long ldx, const void* W, long ldw, void* out
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = photon_pdl_enabled(stream) ? 2 : 1;
+  cfg.numAttrs = photon_pdl_enabled() ? 2 : 1;
   cudaError_t e;
 #define T2_GO(EPI_) cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<EPI_>, map_a, map_w, out, ldo, M, N, K, I, tiles_n, num_tiles, err, Q)
   switch (epilogue) {
