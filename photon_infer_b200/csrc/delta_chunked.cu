@@ -26,9 +26,13 @@
 // stages that each thread fills for itself; the four warps' partial sums of W S0 and Q S0 meet in shared memory, one
 // barrier a chunk.
 //
-// Measured, 2,048 tokens, 16 heads of 128 x 128: prep 103 us, walk 176 us, against 616 us for the token-by-token kernel, whose chain
-// from one token to the next is 300 ns; 64 tokens 18 + 9 us against 22 us and more for its walk.  The error against 64 bits is
+// Measured, 2,048 tokens, 16 heads of 128 x 128: prep 52 us, walk 176 us, against 616 us for the token-by-token kernel, whose chain
+// from one token to the next is 300 ns; 64 tokens 10 + 8 us against 22 us and more for its walk.  The error against 64 bits is
 // 2.4e-7 (outputs) and 1.8e-7 (state) where the token-by-token kernel has 2.6e-7 and 2.1e-7.
+// What bounds the prep: its blocks' loads and stores (100 MB, 15 us of them) and the gaps between a block's steps; with the keys and queries
+// read 4 bytes at a time in turn, and the values only when the substitution asks for them, it took 103 us.  Three or four blocks an SM
+// instead of two take the same time.  What bounds the walk: 156 products of 16 x 8 x 8 a chunk and scheduler at 33 cycles each; eight
+// warps of 16 rows instead of four of 32 take 181 us.
 #include "common.cuh"
 #include <math.h>
 
@@ -67,6 +71,26 @@ dc_prep_kernel(const float* __restrict__ y, const void* ab, long ab_stride, int 
   if (n <= 0) return;
   const int C = 2 * Gq * dim + H * dv, hq = h / (H / Gq);
   float* dst = scratch + ((size_t)dc_place(cu_tokens, s, c) * H + h) * dc_floats(dvp);
+  // Keys, queries and values (at first U0's place holds them) all at once, zeros behind the heads' sizes and the chunk's end.
+  const bool pieces = dim % 4 == 0 && dv % 4 == 0 && C % 4 == 0 && (uintptr_t)y % 16 == 0;
+  auto bring = [&](float* to, int ld, int width, int from, int held) {
+    if (pieces) {
+      for (int i = tid; i < DC * (width / 4); i += 256) {
+        const int t = i / (width / 4), d = i % (width / 4) * 4;
+        const bool there = t < n && d < held;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to + t * ld + d)),
+                     "l"(there ? y + (size_t)(t0 + t) * C + from + d : y), "r"(there ? 16 : 0) : "memory");
+      }
+    } else {
+      for (int i = tid; i < DC * width; i += 256) {
+        const int t = i / width, d = i % width;
+        to[t * ld + d] = t < n && d < held ? y[(size_t)(t0 + t) * C + from + d] : 0.f;
+      }
+    }
+  };
+  bring(ks, DP_LD, DC_D, (Gq + hq) * dim, dim);
+  bring(qs, DP_LD, DC_D, hq * dim, dim);
+  bring(us, dvp + 4, dvp, 2 * Gq * dim + h * dv, dv);
   if (tid < 32) {
     // the chunk's gates: tokens behind its end decay nothing and write nothing
     float lgate = 0.f, beta = 0.f;
@@ -91,17 +115,7 @@ dc_prep_kernel(const float* __restrict__ y, const void* ab, long ab_stride, int 
     tail_s[tid] = expf((float)(end - d));
     if (tid == 31) dst[3 * DC_MAT + DC * DC + (size_t)DC * dvp] = b_s[31];
   }
-  for (int i = tid; i < DC * DC_D; i += 256) {
-    const int t = i / DC_D, d = i % DC_D;
-    float kk = 0.f, qq = 0.f;
-    if (t < n && d < dim) {
-      const float* row = y + (size_t)(t0 + t) * C;
-      qq = row[hq * dim + d];
-      kk = row[(Gq + hq) * dim + d];
-    }
-    ks[t * DP_LD + d] = kk;
-    qs[t * DP_LD + d] = qq;
-  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   {
     // L and A: thread (t, j) has the pairs (t, j), (t, j + 8) ..
@@ -153,7 +167,7 @@ dc_prep_kernel(const float* __restrict__ y, const void* ab, long ab_stride, int 
     for (int t = 0; t < DC; ++t) {
       float r;
       if (isw) r = b_s[t] * ks[t * DP_LD + col];
-      else r = t < n && vc < dv ? y[(size_t)(t0 + t) * C + 2 * Gq * dim + (size_t)h * dv + vc] : 0.f;
+      else r = us[t * (dvp + 4) + vc];
       x[t] = beta_s[t] * r;
     }
 #pragma unroll
