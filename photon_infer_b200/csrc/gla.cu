@@ -158,6 +158,253 @@ __global__ void __launch_bounds__(MAXT) gla_recurrent_kernel(const T* __restrict
   }
 }
 
+// ---------------------------------------------------------------- one chunk of a long portion, from a zero state
+// Everything the chunk needs is brought into shared memory at once (decayed inputs of all its tokens, formed side
+// by side), the walk over its tokens then touches no global memory but its results and meets no barrier: thread
+// j * RP + r keeps rows r * RPT .. of column j, and the RP partial sums of a column lie in neighbouring lanes and
+// meet by shuffles.  Leaves the chunk's own outputs o_loc [T][heads][vdim] (no norm yet), the decay from the chunk's
+// start through every token b [T][heads][dim], and the chunk's end state s_loc [chunks][heads][dim][vdim].
+template <typename T, int RPT>
+__global__ void __launch_bounds__(512)
+gla_chunk_local_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+                       const T* __restrict__ low, long in_stride, int rank, const T* __restrict__ w_a2,
+                       const void* __restrict__ b_a2, int b_bf16, float inv_tau, float qscale, int first, int count,
+                       int chunk, float* __restrict__ o_loc, float* __restrict__ b_out, float* __restrict__ s_loc,
+                       int heads, int dim, int vdim, int RP) {
+  extern __shared__ __align__(16) float sm[];
+  const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, nthreads = blockDim.x;
+  const int R = (dim + RPT - 1) / RPT;
+  const int gs = RPT + 4;                  // a row group's stride: groups start in different banks
+  const int dimp = R * gs;
+  const int t0 = first + c * chunk, n = min(first + count, t0 + chunk) - t0;
+  float* qf = sm;                          // chunk x dimp
+  float* kf = qf + chunk * dimp;
+  float* af = kf + chunk * dimp;
+  float* vf = af + chunk * dimp;           // chunk x vdim
+  float* wa = vf + chunk * vdim;           // dim x (rank + 1)
+  float* ba = wa + dim * (rank + 1);       // dim
+  for (int i = tid; i < dim * rank; i += nthreads) wa[(i / rank) * (rank + 1) + i % rank] = to_f32(w_a2[(size_t)h * dim * rank + i]);
+  for (int i = tid; i < dim; i += nthreads) ba[i] = load_w(b_a2, b_bf16, (size_t)h * dim + i);
+  for (int i = tid; i < 3 * chunk * dimp; i += nthreads) sm[i] = 0.f;
+  __syncthreads();
+  for (int e = tid; e < n * dim; e += nthreads) {
+    const int t = e / dim, i = e - t * dim;
+    const size_t off = (size_t)(t0 + t) * in_stride + (size_t)h * dim + i;
+    const T* lw = low + (size_t)(t0 + t) * in_stride;
+    float zz = 0.f;
+    for (int r = 0; r < rank; ++r) zz = fmaf(to_f32(lw[r]), wa[i * (rank + 1) + r], zz);
+    zz += ba[i];
+    const float ls = fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)));            // log(sigmoid(z))
+    const int at = t * dimp + (i / RPT) * gs + i % RPT;
+    qf[at] = to_f32(q[off]) * qscale;
+    kf[at] = to_f32(k[off]);
+    af[at] = expf(ls * inv_tau);
+  }
+  for (int e = tid; e < n * vdim; e += nthreads) {
+    const int t = e / vdim, j = e - t * vdim;
+    vf[e] = to_f32(v[(size_t)(t0 + t) * in_stride + (size_t)h * vdim + j]);
+  }
+  __syncthreads();
+  if (tid < dim) {                          // the decay since the chunk's start, channel by channel
+    float cum = 1.f;
+    const int at = (tid / RPT) * gs + tid % RPT;
+    for (int t = 0; t < n; ++t) {
+      cum *= af[t * dimp + at];
+      b_out[((size_t)(t0 + t) * heads + h) * dim + tid] = cum;
+    }
+  }
+  const int j = tid / RP, r = tid % RP;
+  const bool active = j < vdim && r < R;
+  float st[RPT];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) st[i] = 0.f;
+  const int g0 = (r < R ? r : 0) * gs;
+  for (int t = 0; t < n; ++t) {
+    float o = 0.f, o2 = 0.f;
+    if (active) {
+      const float vcur = vf[t * vdim + j];
+      const float4* qb = reinterpret_cast<const float4*>(qf + t * dimp + g0);
+      const float4* kb = reinterpret_cast<const float4*>(kf + t * dimp + g0);
+      const float4* ab = reinterpret_cast<const float4*>(af + t * dimp + g0);
+#pragma unroll
+      for (int i = 0; i < RPT / 4; ++i) {
+        const float4 a4 = ab[i], k4 = kb[i], q4 = qb[i];
+        st[4 * i] = fmaf(a4.x, st[4 * i], k4.x * vcur);
+        st[4 * i + 1] = fmaf(a4.y, st[4 * i + 1], k4.y * vcur);
+        st[4 * i + 2] = fmaf(a4.z, st[4 * i + 2], k4.z * vcur);
+        st[4 * i + 3] = fmaf(a4.w, st[4 * i + 3], k4.w * vcur);
+        o = fmaf(st[4 * i], q4.x, o);
+        o2 = fmaf(st[4 * i + 1], q4.y, o2);
+        o = fmaf(st[4 * i + 2], q4.z, o);
+        o2 = fmaf(st[4 * i + 3], q4.w, o2);
+      }
+      o += o2;
+    }
+    for (int d = 1; d < RP; d <<= 1) o += __shfl_xor_sync(0xffffffffu, o, d);   // RP lanes of a column, fixed order
+    if (active && r == 0) o_loc[((size_t)(t0 + t) * heads + h) * vdim + j] = o;
+  }
+  if (active) {
+    float* S = s_loc + ((size_t)c * heads + h) * dim * vdim;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+      if (r * RPT + i < dim) S[(size_t)(r * RPT + i) * vdim + j] = st[i];
+  }
+}
+
+template <typename T, int RPT>
+static int gla_chunk_local_launch(const void* q, const void* k, const void* v, const void* low, long in_stride, int rank,
+                                  const void* w_a2, const void* b_a2, int bb, float it, float qscale, int first, int count,
+                                  int chunk, float* o_loc, float* b, float* s_loc, int heads, int dim, int vdim, int rp,
+                                  int chunks, cudaStream_t stream) {
+  const int R = (dim + RPT - 1) / RPT;
+  const size_t smem = ((size_t)3 * chunk * R * (RPT + 4) + (size_t)chunk * vdim + (size_t)dim * (rank + 2)) * sizeof(float);
+  int threads = (vdim * rp + 31) / 32 * 32;
+  if (threads < dim) threads = (dim + 31) / 32 * 32;
+  if (threads > 512 || smem > 220 * 1024) return PHOTON_ERR_UNSUPPORTED;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(gla_chunk_local_kernel<T, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  gla_chunk_local_kernel<T, RPT><<<dim3(chunks, heads), threads, smem, stream>>>(
+      (const T*)q, (const T*)k, (const T*)v, (const T*)low, in_stride, rank, (const T*)w_a2, b_a2, bb, it, qscale, first,
+      count, chunk, o_loc, b, s_loc, heads, dim, vdim, rp);
+  return launch_status();
+}
+
+// Rows per thread of the chunk kernel: the fewest with which the block (columns x row groups, the groups rounded up to a
+// power of two so that they meet by shuffles) stays within 512 threads.  0: no shape fits.
+static inline int gla_chunk_rows(int dim, int vdim, int* rp) {
+  for (int r = 8; r <= 64; r *= 2) {
+    const int R = (dim + r - 1) / r;
+    int p = 1;
+    while (p < R) p <<= 1;
+    if (p <= 32 && (long)vdim * p <= 512 && dim <= 512) { *rp = p; return r; }
+  }
+  return 0;
+}
+
+// The states at the chunks' starts, one (i, j) element per thread, chunk after chunk: start[0] is the state in the
+// request's slot (zero for a negative slot), start[c + 1] = b_end[c] * start[c] + s_loc[c]; s_loc[c] is overwritten
+// with start[c], and the state after the last chunk goes back into the slot.
+__global__ void gla_chunk_scan_kernel(float* s_loc, const float* __restrict__ b, int first, int count,
+                                      int chunk, int chunks, float* __restrict__ state, int slot, int heads, int dim,
+                                      int vdim) {
+  const int h = blockIdx.y;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= dim * vdim) return;
+  const int i = e / vdim;
+  float* S = slot >= 0 ? state + ((size_t)slot * heads + h) * dim * vdim : nullptr;
+  float cur = S ? S[e] : 0.f;
+  auto decay_of = [&](int c) { return b[((size_t)(min(first + count, first + (c + 1) * chunk) - 1) * heads + h) * dim + i]; };
+  auto end_of = [&](int c) { return s_loc[((size_t)c * heads + h) * dim * vdim + e]; };
+  // four chunks' values are on their way before the first of them is used
+  constexpr int AHEAD = 4;
+  float bd[AHEAD], le[AHEAD];
+#pragma unroll
+  for (int u = 0; u < AHEAD; ++u) { bd[u] = u < chunks ? decay_of(u) : 0.f; le[u] = u < chunks ? end_of(u) : 0.f; }
+  for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+    float nb[AHEAD], nl[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int c = c0 + AHEAD + u;
+      nb[u] = c < chunks ? decay_of(c) : 0.f;
+      nl[u] = c < chunks ? end_of(c) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int c = c0 + u;
+      if (c < chunks) {
+        s_loc[((size_t)c * heads + h) * dim * vdim + e] = cur;
+        cur = fmaf(bd[u], cur, le[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) { bd[u] = nb[u]; le[u] = nl[u]; }
+  }
+  if (S) S[e] = cur;
+}
+
+// What the state at the chunk's start adds to every token of the chunk, o_t += sum_i (q_t[i] b_t[i]) start[i][:],
+// then the head's norm and the gate.  One block per (chunk, head); the start state and the decayed queries in shared
+// memory.
+template <typename T>
+__global__ void __launch_bounds__(256)
+gla_chunk_out_kernel(const T* __restrict__ q, const T* __restrict__ g, long in_stride, const float* __restrict__ b,
+                     const float* __restrict__ o_loc, const float* __restrict__ s_start, const void* __restrict__ norm_w,
+                     int norm_w_bf16, float eps, float qscale, int first, int count, int chunk, T* __restrict__ out,
+                     long out_stride, int heads, int dim, int vdim) {
+  extern __shared__ float sm[];
+  const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const int t0 = first + c * chunk, n = min(first + count, t0 + chunk) - t0;
+  float* Ss = sm;                         // dim x vdim
+  const int qld = chunk + 4;                  // a channel's stride in qb: neighbouring channels start four banks apart
+  float* qb = Ss + ((dim * vdim + 3) & ~3);   // dim x qld, 16-byte aligned
+  float* os = qb + qld * dim;             // chunk x vdim
+  const float* src = s_start + ((size_t)c * heads + h) * dim * vdim;
+  if ((dim * vdim) % 4 == 0) {
+    for (int e = tid; e < dim * vdim / 4; e += 256) reinterpret_cast<float4*>(Ss)[e] = reinterpret_cast<const float4*>(src)[e];
+  } else {
+    for (int e = tid; e < dim * vdim; e += 256) Ss[e] = src[e];
+  }
+  // the decayed queries, transposed: qb[i][t], so that eight tokens of one channel are two 16-byte reads
+  for (int e = tid; e < chunk * dim; e += 256) {
+    const int t = e / dim, i = e - t * dim;
+    qb[i * qld + t] = t < n ? to_f32(q[(size_t)(t0 + t) * in_stride + (size_t)h * dim + i]) * qscale *
+                                    b[((size_t)(t0 + t) * heads + h) * dim + i] : 0.f;
+  }
+  __syncthreads();
+  // a thread owns four value columns and eight tokens: three 16-byte reads of shared memory serve 32 multiply-adds
+  const int groups = chunk / 8, quads = (vdim + 3) / 4;
+  const bool vec4 = (vdim & 3) == 0;
+  for (int e = tid; e < groups * quads; e += 256) {
+    const int tg = e / quads, j = (e - tg * quads) * 4;
+    float a[8][4];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int w = 0; w < 4; ++w) a[u][w] = 0.f;
+    for (int i = 0; i < dim; ++i) {
+      float sv[4];
+      if (vec4) {
+        const float4 s4 = *reinterpret_cast<const float4*>(Ss + i * vdim + j);
+        sv[0] = s4.x; sv[1] = s4.y; sv[2] = s4.z; sv[3] = s4.w;
+      } else {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) sv[w] = j + w < vdim ? Ss[i * vdim + j + w] : 0.f;
+      }
+      const float4 q0 = *reinterpret_cast<const float4*>(qb + i * qld + tg * 8);
+      const float4 q1 = *reinterpret_cast<const float4*>(qb + i * qld + tg * 8 + 4);
+      const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int w = 0; w < 4; ++w) a[u][w] = fmaf(qv[u], sv[w], a[u][w]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int t = tg * 8 + u;
+      if (t < n) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+          if (j + w < vdim) os[t * vdim + j + w] = a[u][w] + o_loc[((size_t)(t0 + t) * heads + h) * vdim + j + w];
+      }
+    }
+  }
+  __syncthreads();
+  const int warp = tid >> 5, lane = tid & 31;
+  for (int t = warp; t < n; t += 8) {
+    float ss = 0.f;
+    for (int j = lane; j < vdim; j += 32) ss += os[t * vdim + j] * os[t * vdim + j];
+    ss = warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)vdim + eps);
+    for (int j = lane; j < vdim; j += 32) {
+      const float gg = to_f32(g[(size_t)(t0 + t) * in_stride + (size_t)h * vdim + j]);
+      out[(size_t)(t0 + t) * out_stride + (size_t)h * vdim + j] =
+          from_f32<T>(os[t * vdim + j] * inv * load_w(norm_w, norm_w_bf16, j) * (gg / (1.0f + expf(-gg))));
+    }
+  }
+}
+
 // ---------------------------------------------------------------- the inputs of a long portion
 // Long portions run in segments (linrec_segments.cu, which walks 32-bit rows): q, k, v and the decays of all tokens as float,
 // two channels a thread, GP_TOK tokens a block, whose low-rank rows wait in shared memory.  Bound by memory: it reads 2 bytes and
@@ -333,4 +580,50 @@ PHOTON_API int photon_gla_recurrent(const void* q, const void* k, const void* v,
   if (maxt == 1024) { GLA_DISPATCH_T(1024) }
   if (maxt == 512) { GLA_DISPATCH_T(512) }
   GLA_DISPATCH_T(256)
+}
+
+// One long prompt portion (tokens first .. first + count - 1 of the step, state slot `slot`) in chunks that run side by
+// side: every chunk's own recurrence from zero, a scan over the chunks' end states, and the start states' share of the
+// outputs with the norm and the gate.  scratch: float [count * heads * (vdim + dim) + 4 + chunks * heads * dim * vdim]
+// with chunks = ceil(count / chunk), 16-byte aligned.  The sums differ from the token-by-token kernel's in their order only.
+PHOTON_API int photon_gla_chunked(const void* q, const void* k, const void* v, const void* g, const void* low,
+                                  long in_stride, int dtype, int rank, const void* w_a2, const void* b_a2, int b_a2_dtype,
+                                  const void* norm_w, int norm_w_dtype, float eps, float tau, float qscale, int first,
+                                  int count, int chunk, int slot, float* state, int num_slots, float* scratch, void* out,
+                                  long out_stride, int heads, int dim, int vdim, int* err, cudaStream_t stream) {
+  if (count <= 0) return 0;
+  if (heads <= 0 || dim <= 0 || vdim <= 0 || rank <= 0 || chunk <= 0 || chunk % 8 || !(tau > 0.f) || slot >= num_slots)
+    return PHOTON_ERR_ARGUMENT;
+  if (heads > 65535) return PHOTON_ERR_UNSUPPORTED;
+  const int chunks = (count + chunk - 1) / chunk;
+  const size_t smem_out = ((size_t)dim * vdim + 4 + (size_t)(chunk + 4) * dim + (size_t)chunk * vdim) * sizeof(float);
+  if (smem_out > 200 * 1024) return PHOTON_ERR_UNSUPPORTED;
+  // the scratch is indexed by the token's place in the step: its three parts are laid out for tokens first ..
+  float* o_loc = scratch - (size_t)first * heads * vdim;
+  float* b = scratch + (size_t)count * heads * vdim - (size_t)first * heads * dim;
+  float* s_loc = scratch + (((size_t)count * heads * (vdim + dim) + 3) & ~(size_t)3);   // 16-byte aligned: read four at a time
+  const int wb = norm_w_dtype == PHOTON_BF16, bb = b_a2_dtype == PHOTON_BF16;
+  const float it = 1.0f / tau;
+  int rp = 1;
+  const int rows = gla_chunk_rows(dim, vdim, &rp);
+  if (rows == 0) return PHOTON_ERR_UNSUPPORTED;
+  int st;
+#define GLA_LOCAL(T, RPT) gla_chunk_local_launch<T, RPT>(q, k, v, low, in_stride, rank, w_a2, b_a2, bb, it, qscale, first, \
+                                                         count, chunk, o_loc, b, s_loc, heads, dim, vdim, rp, chunks, stream)
+  if (dtype == PHOTON_BF16) st = rows == 8 ? GLA_LOCAL(bf16, 8) : rows == 16 ? GLA_LOCAL(bf16, 16) : rows == 32 ? GLA_LOCAL(bf16, 32) : GLA_LOCAL(bf16, 64);
+  else st = rows == 8 ? GLA_LOCAL(float, 8) : rows == 16 ? GLA_LOCAL(float, 16) : rows == 32 ? GLA_LOCAL(float, 32) : GLA_LOCAL(float, 64);
+  if (st != 0) return st;
+  gla_chunk_scan_kernel<<<dim3((dim * vdim + 255) / 256, heads), 256, 0, stream>>>(s_loc, b, first, count, chunk, chunks,
+                                                                                state, slot, heads, dim, vdim);
+  if ((st = launch_status()) != 0) return st;
+  if (dtype == PHOTON_BF16) {
+    if (smem_out > 48 * 1024) cudaFuncSetAttribute(gla_chunk_out_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_out);
+    gla_chunk_out_kernel<bf16><<<dim3(chunks, heads), 256, smem_out, stream>>>((const bf16*)q, (const bf16*)g, in_stride, b, o_loc,
+        s_loc, norm_w, wb, eps, qscale, first, count, chunk, (bf16*)out, out_stride, heads, dim, vdim);
+  } else {
+    if (smem_out > 48 * 1024) cudaFuncSetAttribute(gla_chunk_out_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_out);
+    gla_chunk_out_kernel<float><<<dim3(chunks, heads), 256, smem_out, stream>>>((const float*)q, (const float*)g, in_stride, b, o_loc,
+        s_loc, norm_w, wb, eps, qscale, first, count, chunk, (float*)out, out_stride, heads, dim, vdim);
+  }
+  return launch_status();
 }

@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) moe_route_kernel(const 
 // 2,048 tokens, 16 experts, rows of 2,048 (8.4 MB), beside the shared expert's products on another stream: 26 us; the kernel
 // above, which reads every router row from L2 once per four tokens, 36 us.
 #define MOE_ROUTE_MANY 16
+#define MOE_MANY_FROM 4000000L
 template <int NT>
 __global__ void __launch_bounds__(256)
 moe_route_many_kernel(const bf16* __restrict__ h, long h_stride, const bf16* __restrict__ Wr, const void* __restrict__ bias, int bias_bf16,
@@ -364,7 +365,9 @@ PHOTON_API int photon_moe_route_ex(const void* h, long h_stride, int dtype, cons
   // 64 outputs are what a warp's registers hold; rows that its 16-byte loads cannot read, other types and logits that were formed
   // before go to the kernel above
   const int tiles = (E + (Wsg ? 1 : 0) + 7) / 8;
-  if (!few && dtype == PHOTON_BF16 && logits == nullptr && tiles <= 8 && H % 32 == 0 && h_stride % 8 == 0 && ((uintptr_t)h & 15) == 0 &&
+  // .. and so do fewer numbers than MOE_MANY_FROM, whose few blocks of 16 tokens take as long as many (a routed feed-forward of 16 experts,
+  // us, that kernel first: 1,200 tokens x 2,048 217 and 226, 2,048 x 2,048 294 and 286, 1,200 x 4,096 600 and 588)
+  if (!few && (long)T_ * H >= MOE_MANY_FROM && dtype == PHOTON_BF16 && logits == nullptr && tiles <= 8 && H % 32 == 0 && h_stride % 8 == 0 && ((uintptr_t)h & 15) == 0 &&
       ((uintptr_t)Wr & 15) == 0 && ((uintptr_t)Wsg & 15) == 0) {
     const int nt = tiles <= 2 ? 2 : tiles <= 3 ? 3 : tiles <= 4 ? 4 : 8;
     const size_t room = ((size_t)MOE_ROUTE_MANY * (E + 1 + n_groups + (mode == 3 ? E : 0)) + (size_t)8 * 16 * nt * 8) * sizeof(float);

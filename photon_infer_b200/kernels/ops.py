@@ -1421,9 +1421,16 @@ def delta_recurrent(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_b
 DELTA_CHUNKED_MIN_TOKENS = 64
 
 
-def delta_chunked_supported(dim: int, vdim: int, longest: int) -> bool:
-    """Whether the delta rule of a bfloat16 step runs in chunks: heads of up to 128 and 256 numbers, a request with enough tokens."""
-    return dim <= 128 and vdim <= 256 and longest >= DELTA_CHUNKED_MIN_TOKENS
+#: .. and a step tokens x heads: below, a step waits for the host or for the token-by-token kernel's one launch (B200, a mixer's
+#: step, us, token by token first: 130 tokens x 16 heads 101 and 116, 2 x 130 x 16 98 and 117, 300 x 16 138 and 116).
+DELTA_CHUNKED_FROM = 4700
+
+
+def delta_chunked_supported(dim: int, vdim: int, query_lens, heads: int) -> bool:
+    """Whether the delta rule of a bfloat16 step runs in chunks: heads of up to 128 and 256 numbers, a request with enough tokens,
+    and a step with enough work."""
+    return (dim <= 128 and vdim <= 256 and max(query_lens) >= DELTA_CHUNKED_MIN_TOKENS
+            and sum(query_lens) * heads >= DELTA_CHUNKED_FROM)
 
 
 def delta_chunked(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, cu_tokens: torch.Tensor,
@@ -1798,9 +1805,22 @@ LINREC_SEGMENTS_MIN_TOKENS = 128
 LINREC_SEGMENT_MODES = {"state_space": 0, "matrix_memory": 1, "forget_write": 2, "decay_rows": 3}
 
 
-def linrec_segments_supported(dim: int, longest: int) -> bool:
-    """Whether the recurrences of a bfloat16 step run in segments: states of up to 512 rows, a request with enough tokens."""
-    return dim <= 512 and longest >= LINREC_SEGMENTS_MIN_TOKENS
+#: Tokens x heads of a step from which the segments are the faster way.  Below, a step waits for the host or for one pass over the
+#: tokens, and the segments' additional launches and second pass cost more than they save.  B200, heads of 128 x 128, a mixer's
+#: step, us, without segments first: gated linear attention 300 tokens x 16 heads 139 and 148, 3 x 130 x 16 250 and 148; matrix
+#: memory 3 x 130 x 16 105 and 132, 500 x 16 161 and 131; state space 500 x 16 151 and 154, 300 x 32 168 and 157.
+#: Forget and write: 600 x 16 146 and 149, 850 x 16 165 and 145, 2,000 x 16 332 and 245; its one-pass kernel fills the GPU from 32 (request,
+#: head) pairs on: 2 x 700 x 16 187 and 197, 2,000 x 32 574 and 557, 2 x 1,400 x 32 722 and 755.
+LINREC_SEGMENTS_FROM = {"decay_rows": 6000, "matrix_memory": 7000, "state_space": 9000, "forget_write": 12000}
+
+
+def linrec_segments_supported(mode: str, dim: int, query_lens, heads: int) -> bool:
+    """Whether the recurrences of a bfloat16 step run in segments: states of up to 512 rows, a request with enough tokens, and a
+    step with enough work."""
+    if mode == "forget_write" and len(query_lens) * heads >= 32:
+        return False
+    return (dim <= 512 and max(query_lens) >= LINREC_SEGMENTS_MIN_TOKENS
+            and sum(query_lens) * heads >= LINREC_SEGMENTS_FROM[mode])
 
 
 def linrec_segment_tokens(query_lens, heads: int, dim: int, vdim: int, sms: int) -> int:
@@ -2070,6 +2090,48 @@ def gla_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, low: torch.Tenso
     _check(f(_ptr(q), _ptr(k), _ptr(v), _ptr(low), q.stride(0), _dtype_code(q), rank, _ptr(w_a2), _ptr(b_a2), _dtype_code(b_a2), float(tau),
              _ptr(qo), _ptr(ko), _ptr(vo), _ptr(ao), rows.stride(0), T, nd, nv, _stream()), "gla_prep")
     return qo, ko, vo, ao
+
+
+GLA_CHUNK = 32              # tokens of a chunk of the chunk-parallel recurrence (measured: 64 -> 521 us, 32 -> 420 us, 16 -> 515 us at 2,048 tokens, 16 heads of 128 x 128)
+
+
+def gla_chunked_supported(dim: int, vdim: int, rank: int = 64) -> bool:
+    """A block shape of the chunk kernel exists (columns x row groups within 512 threads, the groups a power of two),
+    and the shared memory of the two chunk kernels fits."""
+    for rpt in (8, 16, 32, 64):
+        groups = -(-dim // rpt)
+        p = 1
+        while p < groups:
+            p *= 2
+        if p <= 32 and vdim * p <= 512 and dim <= 512:
+            local = (3 * GLA_CHUNK * groups * (rpt + 4) + GLA_CHUNK * vdim + dim * (rank + 2)) * 4
+            out = (dim * vdim + 4 + (GLA_CHUNK + 4) * dim + GLA_CHUNK * vdim) * 4
+            return local <= 220 * 1024 and out <= 200 * 1024
+    return False
+
+
+def gla_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, low: torch.Tensor, w_a2: torch.Tensor,
+                b_a2: torch.Tensor, norm_w: torch.Tensor, eps: float, tau: float, qscale: float, first: int, count: int,
+                slot: int, state: torch.Tensor, out: torch.Tensor, heads: int, dim: int, vdim: int,
+                err: Optional[torch.Tensor]) -> None:
+    """One long prompt portion (tokens ``first .. first + count - 1`` of the step's rows, state slot ``slot``) with its
+    chunks of ``GLA_CHUNK`` tokens side by side: each chunk's own recurrence from zero, a scan over the chunks' end
+    states, and the start states' share of the outputs with the norm and the gate.  Same tensors as
+    ``gla_recurrent``; the sums differ from its sums in their order only."""
+    _cuda(q, k, v, g, low, w_a2, b_a2, norm_w, state, out, err)
+    rank = low.shape[1]
+    chunks = -(-count // GLA_CHUNK)
+    scratch = torch.empty(count * heads * (vdim + dim) + 4 + chunks * heads * dim * vdim, dtype=torch.float32, device=q.device)
+    f = _fn("gla", "photon_gla_chunked",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
+             c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_long,
+             c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(_ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(low), q.stride(0), _dtype_code(q), rank, _ptr(w_a2), _ptr(b_a2),
+             _dtype_code(b_a2), _ptr(norm_w), _dtype_code(norm_w), float(eps), float(tau), float(qscale), int(first),
+             int(count), GLA_CHUNK, int(slot), _ptr(state), state.shape[0], _ptr(scratch), _ptr(out), out.stride(0), heads,
+             dim, vdim, _ptr(err), _stream()), "gla_chunked")
+    global _launch_count
+    _launch_count += 2
 
 
 # ----------------------------------------------------------------------------- routed experts

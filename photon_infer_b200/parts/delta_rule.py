@@ -96,7 +96,7 @@ class GatedDeltaRule(Mixer):
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
         ab = rows[:, C + nv:C + nv + 2 * H]
         lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and ops.delta_chunked_supported(self.dim, self.vdim, max(lens)):
+        if h.dtype == torch.bfloat16 and lens and ops.delta_chunked_supported(self.dim, self.vdim, lens, H):
             # long portions: 32 tokens at a time in matrix products
             ops.delta_chunked(y, ab, self.a_log, self.dt_bias, ctx.cu_tokens, ctx.state_slots, state, o, lens, self.qk_heads, H, self.dim,
                               self.vdim, ctx.error_flag)

@@ -79,18 +79,41 @@ class GatedLinearAttention(Mixer):
         # a step with a long bfloat16 portion runs in segments of tokens side by side; everything else (and the float32 run, whose
         # sums depend on nothing but the token's place in its request) goes token by token
         lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported(self.dim, max(lens)):
+        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("decay_rows", self.dim, lens, self.heads):
             q, k, v, a = ops.gla_prep(q, k, v, low, self.w_a2, self.b_a2, self.tau)
             o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
             state = cache.state.view(cache.state.shape[0], -1)
             ops.linrec_segments("decay_rows", q, k, v, a, None, None, None, None, None, 0.0, self.dim ** -0.5, ctx.cu_tokens, ctx.state_slots,
                                 state, o, lens, self.heads, self.heads, self.dim, self.vdim, ctx.error_flag)
             ops.delta_out(o, g, self.norm32, self.eps, out, self.heads, self.vdim)
-        else:
+            return project(out, self.w_o)
+        # smaller steps: portions of CHUNKED_MIN_TOKENS with their chunks side by side, the rest token by token
+        skip = 0
+        if h.dtype == torch.bfloat16 and lens and max(lens) >= CHUNKED_MIN_TOKENS and ops.gla_chunked_supported(self.dim, self.vdim, self.decay_rank or 64):
+            skip = CHUNKED_MIN_TOKENS
+            slots = self._host_slots(ctx)
+            t = 0
+            for s, m in enumerate(lens):
+                if m >= skip:
+                    ops.gla_chunked(q, k, v, g, low, self.w_a2, self.b_a2, self.norm, self.eps, self.tau, self.dim ** -0.5,
+                                    t, m, slots[s], cache.state, out, self.heads, self.dim, self.vdim, ctx.error_flag)
+                t += m
+        if skip == 0 or min(lens) < skip:
             ops.gla_recurrent(q, k, v, g, low, self.w_a2, self.b_a2, self.norm, self.eps, self.tau, self.dim ** -0.5,
                               ctx.cu_tokens, ctx.state_slots, cache.state, out, ctx.num_seqs, self.heads, self.dim, self.vdim,
-                              ctx.error_flag)
+                              ctx.error_flag, skip_from=skip)
         return project(out, self.w_o)
+
+    @staticmethod
+    def _host_slots(ctx: StepContext):
+        """The requests' state slots on the host (the chunked path takes a request's slot as a launch argument)."""
+        if ctx.host_state_slots:
+            return list(ctx.host_state_slots)
+        return ctx.state_slots.cpu().tolist()
+
+
+#: A request that brings at least this many tokens to a bfloat16 step runs chunk-parallel.
+CHUNKED_MIN_TOKENS = 128
 
 
 register_mixer("gla", GatedLinearAttention)

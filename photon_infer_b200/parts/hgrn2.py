@@ -74,7 +74,7 @@ class Hgrn2Mixer(Mixer):
             q, k, bias, lower = y[:, :nd], y[:, nd:], None, None
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
         lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and bias is None and ops.linrec_segments_supported(self.dim, max(lens)):
+        if h.dtype == torch.bfloat16 and lens and bias is None and ops.linrec_segments_supported("forget_write", self.dim, lens, H):
             # long portions: segments of tokens side by side
             ops.linrec_segments("forget_write", q, k, v, None, None, None, None, None, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots,
                                 cache.state, o, lens, H, H, self.dim, self.vdim, ctx.error_flag)

@@ -75,7 +75,7 @@ class MatrixMemoryMixer(Mixer):
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
         g0 = 2 * nd + nv
         lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported(self.dim, max(lens)):
+        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("matrix_memory", self.dim, lens, H):
             # long portions: segments of tokens side by side; the division rides in the norm
             den = ops.linrec_segments("matrix_memory", rows[:, :nd], rows[:, nd:2 * nd], rows[:, 2 * nd:g0], None, rows[:, g0 + nv:g0 + nv + H],
                                       rows[:, g0 + nv + H:], self.i_bias, self.f_bias, None, self.gate_cap, self.dim ** -0.5, ctx.cu_tokens,

@@ -89,7 +89,7 @@ class StateSpaceMixer(Mixer):
                       cache.state, self.heads * self.state * self.vdim, y, ctx.num_seqs, ctx.error_flag)
         o = torch.empty((T, inner), dtype=torch.float32, device=h.device)
         lens = list(ctx.host_query_lens)
-        long = h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported(self.state, max(lens))
+        long = h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("state_space", self.state, lens, self.heads)
         if long:
             # long portions: segments of tokens side by side
             ops.linrec_segments("state_space", y[:, inner + GN:], y[:, inner:inner + GN], y[:, :inner], None, rows[:, inner + C:], None,

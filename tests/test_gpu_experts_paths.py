@@ -37,7 +37,9 @@ def test_pairs_of_one_expert_get_the_bits_that_they_get_alone(pairs, glu):
 
 
 @pytest.mark.parametrize("T,H,E,gate", [(64, 32, 2, False), (65, 64, 8, True), (79, 288, 16, False), (2049, 2048, 16, True), (130, 96, 33, True),
-                                        (100, 160, 63, True), (100, 160, 64, True)])
+                                        (100, 160, 63, True), (100, 160, 64, True),
+                                        (125001, 32, 2, False), (62507, 64, 8, True), (13889, 288, 16, False), (41669, 96, 33, True),
+                                        (25011, 160, 63, True), (25003, 160, 64, True)])
 @pytest.mark.parametrize("scoring", ["softmax_chosen", "softmax_all", "sigmoid", "softmax_raw"])
 def test_router_of_many_tokens(T, H, E, gate, scoring):
     """The choice and the weights against 64 bits; a choice may differ only where two scores are closer than the logits' rounding
