@@ -31,8 +31,9 @@
 // 2.4e-7 (outputs) and 1.8e-7 (state) where the token-by-token kernel has 2.6e-7 and 2.1e-7.
 // What bounds the prep: its blocks' loads and stores (100 MB, 15 us of them) and the gaps between a block's steps; with the keys and queries
 // read 4 bytes at a time in turn, and the values only when the substitution asks for them, it took 103 us.  Three or four blocks an SM
-// instead of two take the same time.  What bounds the walk: 156 products of 16 x 8 x 8 a chunk and scheduler at 33 cycles each; eight
-// warps of 16 rows instead of four of 32 take 181 us.
+// instead of two take the same time.  The walk takes 2.75 us a chunk, 156 products of 16 x 8 x 8 and
+// their operands' splits for each scheduler; eight warps of 16 rows instead of four of 32 take 181 us, the same walk in plain 32-bit
+// multiply-adds (tiles of 4 x 4 from shared memory) 218 us.
 #include "common.cuh"
 #include <math.h>
 
