@@ -11,7 +11,8 @@ slot between steps; decays, their logarithms and the recurrence itself are 32-bi
 
 One fused product gives ``[q | k | v | g | W_a1 h]``.  For few tokens one kernel forms the decay logits from the low-rank part,
 runs the recurrence over the tokens of a step and applies the norm and the gate in its epilogue; a step with a long portion
-forms the decays of all tokens first, runs the recurrence in segments side by side (``linrec_segments.cu``), and then norm and gate.
+forms the decays of all tokens first, runs the recurrence in segments side by side (``linrec_segments.cu``), and then norm and gate.  Portions in
+between run chunks of 32 tokens from zero states side by side, joined by a scan.
 """
 from __future__ import annotations
 
