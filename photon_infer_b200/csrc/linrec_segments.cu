@@ -15,8 +15,11 @@
 // segment's start and L the running maximum from nothing, m_t = max(F_t + m_start, L_t), so both come from one scan per
 // segment, and keep_t = exp(f_t + (m_(t-1) - m_t)) holds whatever the last bits of m are.
 //
-// Everything is 32-bit as in the token-by-token kernels; a segment's walk is the same chain of operations, and what
-// differs is the fold (one multiply-add per segment and state element).
+// Everything is 32-bit as in the token-by-token kernels; what differs is the scale in which a chunk's state is held (below) and
+// the fold (one multiply-add per segment and state element, two where the decay is one number per row).  Decays near 1 are
+// carried by what they lack to 1 (ls_decay).  Error of the state against 64 bits, 2,048 tokens, token by token in brackets:
+// write gates of 1e-5 to 1e-2 that hardly change 2.3e-7 (3.3e-7), of 0.01 to 0.5 6.2e-8 (5.2e-8); row decays of 0.999 to
+// 0.9999 2.9e-7 (1.0e-6), of 0.96 1.2e-7 (1.4e-7).  With products of rounded decays the first was 5.8e-6, the third 2.7e-6.
 //
 // What bounds it: the FP32 pipe.  A packed multiply-add with three operands takes three cycles and a packed product two, so
 // the decay is taken out of the walk: over a chunk of 16 tokens the state is held relative to the product b_t of the decays
@@ -41,6 +44,20 @@
 
 struct alignas(16) LsCols { float x[LS_C]; };        // the lane's columns of one row
 
+// The product b of decays and what it lacks to 1, B = 1 - b, brought forward by a decay that lacks `gone` to 1 (`scaled` is that
+// decay times b).  Near 1 a product rounds to 2^-25 of itself at every token, always alike where the decays hardly change, which over
+// hundreds of tokens is far more than the state's own roundings; B keeps all its bits there.  Below 1/2 the product is the exact one.
+__device__ __forceinline__ void ls_decay(float scaled, float gone, float& b, float& B) {
+  B = fmaf(gone, b, B);
+  b = B < 0.5f ? 1.0f - B : scaled;
+}
+// A decay as one number: -B (minus zero for a decay of 1) where B lies between 0 and 1/2, else b (also behind a decay that the
+// rounding of a running maximum has put above 1).  x decays to fma(code, x, x or 0): the sign says which.
+__device__ __forceinline__ float ls_code(float b, float B) { return B >= 0.f && B < 0.5f ? -fabsf(B) : b; }
+__device__ __forceinline__ uint32_t ls_mask(float code) { return (uint32_t)(__float_as_int(code) >> 31); }
+__device__ __forceinline__ float ls_apply(float code, float x) { return fmaf(code, x, __uint_as_float(__float_as_uint(x) & ls_mask(code))); }
+__device__ __forceinline__ lr_pair ls_mask2(float c0, float c1) { return (lr_pair)ls_mask(c1) << 32 | ls_mask(c0); }
+
 struct LsArgs {
   const float* q; long q_stride;                     // [T][qk_heads * N]
   const float* k; long k_stride;                     // [T][qk_heads * N]: keys; mode 2: write gates
@@ -55,7 +72,7 @@ struct LsArgs {
   float* out; long out_stride;                       // [T][H * dv]; mode 1: before the division
   float* den;                                        // mode 1: [T][H], what the outputs are to be divided by
   float* ends;                                       // [S * segs][H][N * dv]
-  float* vecs;                                       // [S * segs][H][N]: mode 1 n at the end; modes 2, 3 the rows' decay
+  float* vecs;                                       // [S * segs][H][N]: mode 1 n at the end; modes 2, 3 the rows' decay (ls_code)
   float* scale;                                      // [S * segs][H][2]: mode 0 the decay; mode 1 F and L at the end
   float* first;                                      // [S][H][N * dv], then [S][H][N], then [S][H]: the state before the step
   int T, S, H, qk_heads, N, dv, seg, segs, vec;
@@ -151,7 +168,7 @@ ls_walk_kernel(const LsArgs A) {
   float* vs = as + (HAS_A ? 2 * LS_CHUNK * NP : 0);    // [2][CHUNK][BC]
   float* os = vs + 2 * LS_CHUNK * BC;                  // [CHUNK][BC], second pass
   __shared__ float keep_s[LS_CHUNK], take_s[LS_CHUNK], floor_s[LS_CHUNK], by_s[LS_CHUNK];
-  __shared__ __align__(16) float end_s[MODE < 2 ? 4 : NP];    // modes 2, 3: the rows' decay through the chunk
+  __shared__ __align__(16) float end_s[MODE < 2 ? 4 : NP];    // the decay through the chunk (ls_code), modes 2 and 3 per row
   __shared__ int plain_s;
   __shared__ float den_s[4][LS_CHUNK];
   const int N = A.N, dv = A.dv, H = A.H;
@@ -215,7 +232,7 @@ ls_walk_kernel(const LsArgs A) {
 
   lr_pair S[R / 2][LS_C];
   float m0 = 0.f;                                      // mode 1: the running maximum before the segment
-  float follow[RT];                                    // the thread's rows of n, or of the decay since the segment's start
+  float follow[RT], lacks[RT];                         // the thread's rows of n, or of the decay since the segment's start and 1 minus it
   {
     const bool zero = PASS == 1 && sg > 0;
     const bool kept = PASS == 2 && nseg > 1;           // the first pass put the state before the step aside: the last segment
@@ -239,7 +256,7 @@ ls_walk_kernel(const LsArgs A) {
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       const int r = tid + i * LS_THREADS;
-      follow[i] = 1.f;
+      follow[i] = 1.f; lacks[i] = 0.f;
       if (MODE == 1 && leads) {
         follow[i] = vec != nullptr && r < N ? vec[r] : 0.f;
         if (PASS == 1 && sg == 0 && r < N) first_n[r] = follow[i];
@@ -275,10 +292,12 @@ ls_walk_kernel(const LsArgs A) {
             load(em, j, e, x[e]);
             d[e] = SCALAR ? c1 : (row_of(j, e) < N ? ev[row_of(j, e)] : 0.f);
           }
-          const lr_pair dd = lr_make(d[0], d[1]);
+          const lr_pair dd = lr_make(d[0], d[1]), kept = ls_mask2(d[0], d[1]), one = lr_dup(1.0f);
 #pragma unroll
-          for (int c = 0; c < LS_C; ++c)
-            S[j][c] = lr_fma2(dd, S[j][c], lr_make(MODE == 1 ? c2 * x[0][c] : x[0][c], MODE == 1 ? c2 * x[1][c] : x[1][c]));
+          for (int c = 0; c < LS_C; ++c) {
+            const lr_pair end = lr_make(MODE == 1 ? c2 * x[0][c] : x[0][c], MODE == 1 ? c2 * x[1][c] : x[1][c]);
+            S[j][c] = lr_fma2(dd, S[j][c], SCALAR ? end : lr_fma2(one, S[j][c] & kept, end));
+          }
         }
       }
     }
@@ -356,7 +375,7 @@ ls_walk_kernel(const LsArgs A) {
     const int cnt = min(LS_CHUNK, b1 - base);
     // the chunk's gates (their raw numbers came in under the chunk before).  Tokens behind the chunk keep everything and take
     // nothing.
-    float gk = 1.f, gt = 0.f, gfl = 0.f, gb = 1.f;
+    float gk = 1.f, gt = 0.f, gfl = 0.f, gb = 1.f, gB = 0.f;
     int gplain = 0;
     if (SCALAR && warp == 0) {
       if (lane < cnt) {
@@ -369,11 +388,11 @@ ls_walk_kernel(const LsArgs A) {
         }
       }
       fetch_gates(base + LS_CHUNK);
-      gb = gk;                                         // the decay since the chunk's start
+      gb = gk; gB = 1.0f - gk;                         // the decay since the chunk's start
 #pragma unroll
       for (int o = 1; o < LS_CHUNK; o <<= 1) {
-        const float up = __shfl_up_sync(0xffffffffu, gb, o);
-        if (lane >= o) gb *= up;
+        float up = __shfl_up_sync(0xffffffffu, gb, o), upB = __shfl_up_sync(0xffffffffu, gB, o);
+        if (lane >= o) { ls_decay(gb * up, gB, up, upB); gb = up; gB = upB; }
       }
       gplain = !(__shfl_sync(0xffffffffu, gb, LS_CHUNK - 1) >= LS_SMALL);
       if (!gplain) gt = gt / gb;
@@ -383,6 +402,7 @@ ls_walk_kernel(const LsArgs A) {
     if (SCALAR && tid < LS_CHUNK) {
       keep_s[tid] = gk; take_s[tid] = gt; floor_s[tid] = gfl; by_s[tid] = gplain ? 1.f : gb;
       if (tid == 0) plain_s = gplain;
+      if (tid == LS_CHUNK - 1) end_s[0] = ls_code(gb, gB);
     }
     __syncthreads();                                   // this chunk has landed for every thread
     float* kd = ks + (size_t)stage * LS_CHUNK * NP;
@@ -394,15 +414,20 @@ ls_walk_kernel(const LsArgs A) {
       plain = plain_s != 0;
     } else {
       // a thread per row: the row's decays multiplied up, then its keys and queries brought into the chunk's scale
+      auto row_decay = [&](int at, float& b, float& B) {
+        const float x = HAS_A ? ad[at] : kd[at];           // the decay, or what it lacks to 1
+        ls_decay(HAS_A ? x * b : fmaf(-x, b, b), HAS_A ? 1.0f - x : x, b, B);
+      };
       float b_end[RT];
       bool small = false;
 #pragma unroll
       for (int i = 0; i < RT; ++i) {
         const int r = tid + i * LS_THREADS;
-        float bt = 1.f;
-        if (r < N) for (int tt = 0; tt < cnt; ++tt) bt *= HAS_A ? ad[tt * NP + r] : 1.0f - kd[tt * NP + r];
-        b_end[i] = bt;
-        follow[i] *= bt;
+        float bt = 1.f, Bt = 0.f;
+        if (r < N) for (int tt = 0; tt < cnt; ++tt) row_decay(tt * NP + r, bt, Bt);
+        b_end[i] = ls_code(bt, Bt);
+        const float f = follow[i];
+        ls_decay(ls_apply(b_end[i], f), Bt, follow[i], lacks[i]);
         small |= !(bt >= LS_SMALL);
       }
       plain = __syncthreads_or(small) != 0;
@@ -411,12 +436,12 @@ ls_walk_kernel(const LsArgs A) {
         for (int i = 0; i < RT; ++i) {
           const int r = tid + i * LS_THREADS;
           if (r < N) {
-            float bt = 1.f;
+            float bt = 1.f, Bt = 0.f;
 #pragma unroll 4
             for (int tt = 0; tt < cnt; ++tt) {
               const int at = tt * NP + r;
               const float kk = kd[at];
-              bt *= HAS_A ? ad[at] : 1.0f - kk;
+              row_decay(at, bt, Bt);
               kd[at] = kk / bt;
               if (HAS_Q) qd[at] *= bt;
             }
@@ -451,7 +476,7 @@ ls_walk_kernel(const LsArgs A) {
               if (HAS_Q) nq[tt] = fmaf(follow[i], qd[tt * NP + r], nq[tt]);
             }
           }
-          if (!plain) follow[i] *= by_s[LS_CHUNK - 1];
+          if (!plain) follow[i] = ls_apply(end_s[0], follow[i]);
         }
       }
       if (HAS_Q) {
@@ -543,16 +568,19 @@ ls_walk_kernel(const LsArgs A) {
             meet(t, val);
           }
         }
-        lr_pair e2[2];
-        if (SCALAR) e2[0] = e2[1] = lr_dup(by_s[LS_CHUNK - 1]);
+        lr_pair e2[2], kept[2];
+        if (SCALAR) { e2[0] = e2[1] = lr_dup(end_s[0]); kept[0] = kept[1] = ls_mask2(end_s[0], end_s[0]); }
 #pragma unroll
         for (int j = 0; j < R / 4; ++j) {
           if (!SCALAR) {
-            const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(end_s + (j * L + sub) * 4);
-            e2[0] = e.x; e2[1] = e.y;
+            const float4 e = *reinterpret_cast<const float4*>(end_s + (j * L + sub) * 4);
+            e2[0] = lr_make(e.x, e.y); e2[1] = lr_make(e.z, e.w);
+            kept[0] = ls_mask2(e.x, e.y); kept[1] = ls_mask2(e.z, e.w);
           }
 #pragma unroll
-          for (int c = 0; c < LS_C; ++c) { S[2 * j][c] = lr_mul2(e2[0], S[2 * j][c]); S[2 * j + 1][c] = lr_mul2(e2[1], S[2 * j + 1][c]); }
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int c = 0; c < LS_C; ++c) S[2 * j + i][c] = lr_fma2(e2[i], S[2 * j + i][c], S[2 * j + i][c] & kept[i]);
         }
       }
     }
@@ -605,7 +633,7 @@ ls_walk_kernel(const LsArgs A) {
   }
   if (leads && vec != nullptr && (MODE == 1 || (PASS == 1 && !SCALAR))) {
 #pragma unroll
-    for (int i = 0; i < RT; ++i) if (tid + i * LS_THREADS < N) vec[tid + i * LS_THREADS] = follow[i];
+    for (int i = 0; i < RT; ++i) if (tid + i * LS_THREADS < N) vec[tid + i * LS_THREADS] = MODE == 1 ? follow[i] : ls_code(follow[i], lacks[i]);
   }
 }
 

@@ -135,6 +135,60 @@ def test_running_maxima_far_from_zero():
         assert _rel(x, o.double()) < 5e-5
 
 
+@pytest.mark.parametrize("mode", ["state_space", "matrix_memory", "forget_write", "decay_rows"])
+@pytest.mark.parametrize("gates", ["constant", "nearly constant", "ordinary"])
+def test_slow_decays_keep_their_bits(mode, gates):
+    """2,048 tokens whose decays are nearly 1 (and ordinary ones), in segments of the length that a step gets: the error against 64 bits
+    is no larger than that of the walk token by token, or within two roundings of the state."""
+    from photon_infer_b200.kernels import ops
+    gen = torch.Generator().manual_seed(len(mode) + len(gates))
+    H, N, dv, T = 2, 64, 32, 2048
+    vary = {"constant": 0.0, "nearly constant": 0.01, "ordinary": 1.0}[gates]
+    slow = gates != "ordinary"
+    rand = lambda *shape: torch.randn(*shape, generator=gen)
+    q, k, v = rand(T, H * N), rand(T, H * N), rand(T, H * dv)
+    per_row = torch.rand(H * N, generator=gen)
+    a = ga = gb = p0 = p1 = p2 = None
+    if mode == "forget_write":                                   # write gates of 1e-5 to 1e-2, or of 0.01 to 0.5
+        k = (10.0 ** (-5 + 3 * per_row) if slow else 0.01 + 0.49 * per_row) * (1 + 0.5 * vary * torch.tanh(rand(T, H * N)))
+    elif mode == "decay_rows":
+        a = torch.exp(torch.nn.functional.logsigmoid((4 + 3 * per_row if slow else per_row) + vary * rand(T, H * N)) / 16)
+    elif mode == "state_space":
+        ga, p0, p1, p2 = -4 + vary * rand(T, H), torch.full((H,), -3.0 if slow else 0.0), torch.full((H,), 0.1), torch.ones(H)
+    else:
+        ga, gb, p0, p1 = 0.3 * rand(T, H), (6.0 if slow else 2.0) + vary * rand(T, H), torch.zeros(H), torch.tensor([0.0, 0.7])
+    memory, cap, scale = mode == "matrix_memory", 15.0, N ** -0.5
+    size = H * N * dv + (H * N + H if memory else 0)
+    dev = lambda x: None if x is None else x.to(DEV)
+    q, k, v, a, ga, gb, p0, p1, p2 = map(dev, (q, k, v, a, ga, gb, p0, p1, p2))
+    if memory:
+        gates_ab = torch.cat([ga, gb], dim=1)
+        ga, gb = gates_ab[:, :H], gates_ab[:, H:]
+    s1, o1 = torch.zeros(1, size, device=DEV), torch.empty(T, H * dv, device=DEV)
+    den = ops.linrec_segments(mode, q, k, v, a, ga, gb, p0, p1, p2, cap if memory else 0.0, scale, i32([0, T]), i32([0]), s1, o1, [T], H, H, N, dv,
+                              None)
+    if memory:
+        o1 = (o1.view(T, H, dv) / den.unsqueeze(-1)).view(T, H * dv)
+    s2, o2 = torch.zeros(1, size, device=DEV), torch.empty(T, H * dv, device=DEV)
+    if mode == "decay_rows":
+        S, rows = torch.zeros(H, N, dv, device=DEV), []
+        for t in range(T):
+            S = torch.addcmul(a[t].view(H, N, 1) * S, k[t].view(H, N, 1), v[t].view(H, 1, dv))
+            rows.append(torch.einsum("hnv,hn->hv", S, q[t].view(H, N)) * scale)
+        s2[0], o2 = S.flatten(), torch.stack(rows).flatten(1)
+    else:
+        ops.linrec(mode, q, k, v, ga, gb, p0, p1, p2, cap if memory else 0.0, scale, i32([0, T]), i32([0]), s2, o2, 1, H, H, N, dv, None)
+    d = lambda x: None if x is None else x.double()
+    heads = lambda x: None if x is None else x.double().view(T, H, -1)
+    zero = lambda *shape: torch.zeros(*shape, dtype=torch.float64, device=DEV)
+    want, S, n, m = _walk(mode, heads(q), heads(k), heads(v), heads(a), d(ga), d(gb), d(p0), d(p1), d(p2), cap, scale, zero(H, N, dv), zero(H, N),
+                          zero(H))
+    errors = [(_rel(o, want), _rel(s[0, :H * N * dv], S.flatten())) for o, s in ((o1, s1), (o2, s2))]
+    print("segments and walk (outputs, state):", errors)
+    assert errors[0][1] <= max(1.1 * errors[1][1], 2.0 ** -23), errors
+    assert errors[0][0] <= max(1.1 * errors[1][0], 2.0 ** -22), errors       # a sum of 64 such products behind it
+
+
 @pytest.mark.parametrize("mode", [None, "silu_before", "sigmoid_after"])
 @pytest.mark.parametrize("groups,gs", [(16, 128), (2, 1024), (3, 4), (1, 260), (9, 512)])
 def test_norm_of_parts(mode, groups, gs):
