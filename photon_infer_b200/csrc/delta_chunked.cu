@@ -20,6 +20,9 @@
 // Cores while surpassing the FP32 theoretical peak performance", 2022: it is the accumulation inside the tensor cores that
 // rounds coarsely).
 //
+// A token whose inputs are not finite reaches its own and later outputs only, as token by token; there it is NaN where the plain
+// rule may leave an infinity (the second part of an infinity's split is NaN).
+//
 // The walk keeps S^T [16 columns][128 rows] in accumulator registers, a warp 32 of the rows: an accumulator fragment with
 // the rows 2 t, 2 t + 1 of a lane is at once the A fragment of the next product, if the other operand's k index is read
 // in the same order.  Its operands lie in memory in that order, 16 bytes a lane, and travel by cp.async into a ring of three
@@ -35,6 +38,7 @@
 // their operands' splits for each scheduler; eight warps of 16 rows instead of four of 32 take 181 us, the same walk in plain 32-bit
 // multiply-adds (tiles of 4 x 4 from shared memory) 218 us.
 #include "common.cuh"
+#include <float.h>
 #include <math.h>
 
 #define DC 32                                          // tokens of a chunk
@@ -139,7 +143,7 @@ dc_prep_kernel(const float* __restrict__ y, const void* ab, long ab_stride, int 
       const float ratio = sx <= t ? expf((float)(lg[t] - lg[sx])) : 0.f;
       Ls[t * (DC + 4) + sx] = sx < t ? beta_s[t] * ratio * kk[u] : 0.f;
       // A [warp t / 8][sx / 16][lane (t % 8) * 4 + (sx % 8) / 2][(sx % 16) / 8 * 2 + sx % 2]
-      A[((t >> 3) * 2 + (sx >> 4)) * 128 + ((t & 7) * 4 + ((sx & 7) >> 1)) * 4 + ((sx >> 3) & 1) * 2 + (sx & 1)] = ratio * qk[u];
+      A[((t >> 3) * 2 + (sx >> 4)) * 128 + ((t & 7) * 4 + ((sx & 7) >> 1)) * 4 + ((sx >> 3) & 1) * 2 + (sx & 1)] = sx <= t ? ratio * qk[u] : 0.f;
     }
   }
   // Q and K of the walk, in its order of lanes (qs and ks are read by rows)
@@ -321,6 +325,8 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
     __syncthreads();                                   // the partial sums and U0 are there for every warp; the sums of the chunk before
     fetch(c + DC_STAGES - 1);                          // last are read no more, and neither is the stage that is filled now
     uint32_t uh[4][4], ul[4][4];
+    float uw[4] = {0.f, 0.f, 0.f, 0.f};                // U of the tokens whose outputs this warp forms
+    bool wild = false;                                 // infinities and NaN among them
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float4 u0 = d4[(3 * DC_MAT + DC * DC) / 4 + i * 32];
@@ -328,7 +334,12 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
       const float u[4] = {u0.x - ((p0.x + p1.x) + (p2.x + p3.x)), u0.y - ((p0.y + p1.y) + (p2.y + p3.y)),
                           u0.z - ((p0.z + p1.z) + (p2.z + p3.z)), u0.w - ((p0.w + p1.w) + (p2.w + p3.w))};
       dc_operand(u, uh[i], ul[i]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (i == w) { uw[e] = u[e]; wild |= !(fabsf(u[e]) <= FLT_MAX); }
+      }
     }
+    wild = __any_sync(0xffffffffu, wild);
     // the outputs of tokens 8 w .. 8 w + 7 and this warp's rows of the state, side by side
     DcAcc out, nw[4];
     {
@@ -354,13 +365,29 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
         dc_mma3(nw[1], uh[i], ul[i], k0.z, k0.w);
         dc_mma3(nw[2], uh[i], ul[i], k1.x, k1.y);
         dc_mma3(nw[3], uh[i], ul[i], k1.z, k1.w);
-        dc_mma3(out, uh[i], ul[i], u ? a.z : a.x, u ? a.w : a.y);
+        // A is zero for later tokens, but zero times their infinities would not be: tiles behind the warp's are left out, and its
+        // own one is a plain sum over the tokens that count where its U is not finite
+        if (i < w || (i == w && !wild)) dc_mma3(out, uh[i], ul[i], u ? a.z : a.x, u ? a.w : a.y);
       }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) st[j][e] = dc_sum(nw[j], e);
+    if (wild) {
+      // A [warp][s / 16][lane (t % 8) * 4 + (s % 8) / 2][(s % 16) / 8 * 2 + s % 2], s = 8 w + i
+      const float* a = reinterpret_cast<const float*>(d4 - lane) + 3 * DC_MAT + (w * 2 + (w >> 1)) * 128 + (w & 1) * 2;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int from = (lane & ~3) | (i >> 1);
+        const float u0 = __shfl_sync(0xffffffffu, uw[i & 1], from), u1 = __shfl_sync(0xffffffffu, uw[2 + (i & 1)], from);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int tt = 2 * t + (e & 1);
+          if (i <= tt) out.x[e] = fmaf(a[(tt * 4 + (i >> 1)) * 4 + (i & 1)], e < 2 ? u0 : u1, out.x[e]);
+        }
+      }
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int tok = c * DC + 8 * w + 2 * t + (e & 1), col = cb * DC_CB + g + (e >> 1) * 8;

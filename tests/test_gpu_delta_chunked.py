@@ -127,3 +127,36 @@ def test_convolution_of_many_tokens_gives_the_bits_of_few(H, G, dim, dv):
     whole = run([[(r, 0, n) for r, n in enumerate(lens)]])
     cut = run([[(0, 0, 33), (1, 0, 1)], [(0, 33, 37), (2, 0, 2)], [(4, 0, 60)], [(5, 0, 17)]])
     assert torch.equal(whole[0], cut[0]) and torch.equal(whole[1], cut[1])
+
+
+@pytest.mark.parametrize("what", ["key", "query", "value", "decay", "step size"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [0, 13, 31, 40, 95])
+def test_what_is_not_finite_reaches_no_earlier_token(what, bad, at):
+    """One number of a token is not finite: the outputs before it are those that they are without it (up to the rounding of the eight
+    tokens whose sums are then plain ones), and those that are not finite are the token-by-token kernel's."""
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(at)
+    T, H, G, dim, dv = 100, 4, 2, 128, 48
+    y = torch.randn(T, 2 * G * dim + H * dv, device=DEV)
+    y[:, :2 * G * dim] *= dim ** -0.5
+    ab = torch.randn(T, 2 * H, device=DEV)
+    a_log, dt_bias = torch.zeros(H, device=DEV), torch.full((H,), -3.0, device=DEV)
+    start = torch.randn(1, H * dim * dv, device=DEV)
+
+    def run(chunks, y, ab):
+        s, o = start.clone(), torch.empty(T, H * dv, device=DEV)
+        args = (y, ab, a_log, dt_bias, i32([0, T]), i32([0]), s, o)
+        ops.delta_chunked(*args, [T], G, H, dim, dv, None) if chunks else ops.delta_recurrent(*args, 1, G, H, dim, dv, None)
+        return o, s
+    clean = run(True, y, ab)[0]
+    if what in ("decay", "step size"):
+        ab[at, 1 if what == "decay" else H + 1] = bad
+    else:
+        y[at, {"key": G * dim + 5, "query": 5, "value": 2 * G * dim + dv + 7}[what]] = bad
+    (o, s), (want, after) = run(True, y, ab), run(False, y, ab)
+    assert torch.equal(o[:at // 8 * 8], clean[:at // 8 * 8])
+    assert at == 0 or _rel(o[:at], clean[:at].double()) < 1e-6
+    assert torch.equal(torch.isfinite(o), torch.isfinite(want)) and torch.equal(torch.isfinite(s), torch.isfinite(after))
+    fine = torch.isfinite(want)
+    assert _rel(o[fine], want[fine].double()) < 2e-5
