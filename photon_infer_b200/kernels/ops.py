@@ -2072,6 +2072,11 @@ def gla_recurrent(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Te
              int(skip_from), _ptr(err), _stream()), "gla_recurrent")
 
 
+def gla_prep_supported(tokens: int, rank: int) -> bool:
+    """The sizes of ``gla_prep``: the low-rank rows of its 16 tokens in 48 KB of shared memory, and its grid."""
+    return rank <= 768 and tokens <= 16 * 65535
+
+
 def gla_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, low: torch.Tensor, w_a2: torch.Tensor, b_a2: torch.Tensor, tau: float):
     """The inputs of a long portion in 32-bit, as ``linrec_segments`` walks them: ``q``, ``k [T, heads * dim]`` and ``v [T, heads *
     vdim]`` (views of one fused row) as float32 and the decays ``exp(log_sigmoid(w_a2 low + b_a2) / tau)``; returns ``(q, k, v, a)``."""

@@ -80,7 +80,8 @@ class GatedLinearAttention(Mixer):
         # a step with a long bfloat16 portion runs in segments of tokens side by side; everything else (and the float32 run, whose
         # sums depend on nothing but the token's place in its request) goes token by token
         lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("decay_rows", self.dim, lens, self.heads):
+        if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("decay_rows", self.dim, lens, self.heads) \
+                and ops.gla_prep_supported(T, low.shape[1]):
             q, k, v, a = ops.gla_prep(q, k, v, low, self.w_a2, self.b_a2, self.tau)
             o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
             state = cache.state.view(cache.state.shape[0], -1)
