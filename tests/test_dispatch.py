@@ -61,3 +61,18 @@ def test_weight_streaming_product_sizes():
     assert not ops.skinny_gemm_supported(torch.zeros(65, 2048, dtype=torch.bfloat16), w)
     assert not ops.skinny_gemm_supported(torch.zeros(33, 2048, dtype=torch.bfloat16), w, swiglu=True)
     assert not ops.skinny_gemm_supported(torch.zeros(8, 2044, dtype=torch.bfloat16), torch.zeros(16, 2044, dtype=torch.bfloat16))
+
+
+def test_the_switch_of_dependent_launches_takes_every_word_for_off(tmp_path):
+    """``PHOTON_PDL``: unset, empty and 1 leave the launches on, everything else turns them off."""
+    import os
+    import subprocess
+
+    from photon_infer_b200.csrc.build import CSRC_DIR, INCLUDE_DIR, find_nvcc
+    src, exe = tmp_path / "pdl.cu", tmp_path / "pdl"
+    src.write_text('#include "common.cuh"\n#include <cstdio>\nint main() { printf("%d", (int)photon_pdl_enabled()); return 0; }\n')
+    subprocess.run([find_nvcc(), "-std=c++17", "-I", CSRC_DIR, "-I", INCLUDE_DIR, "-o", str(exe), str(src)], check=True, capture_output=True)
+    env = {k: v for k, v in os.environ.items() if k != "PHOTON_PDL"}
+    said = lambda value: subprocess.run([str(exe)], env=dict(env, PHOTON_PDL=value), capture_output=True, text=True).stdout
+    assert subprocess.run([str(exe)], env=env, capture_output=True, text=True).stdout == "1"
+    assert [said(v) for v in ("", "1", "0", "off", "no", "false")] == ["1", "1", "0", "0", "0", "0"]
