@@ -486,11 +486,16 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v
         _launch_count += 1
 
 
+def attention_rows_heads(n_q: int, n_kv: int, head_dim: int) -> bool:
+    """The heads that ``attention_rows`` is written for."""
+    return head_dim in (64, 128) and n_kv > 0 and n_q % n_kv == 0 and n_q // n_kv <= 32
+
+
 def attention_rows_supported(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, n_q: int, n_kv: int,
                              head_dim: int) -> bool:
     """Whether ``attention_rows`` takes the call: float32, heads of 64 or 128, up to 32 query heads per key/value head, caches and
     rows in 16-byte pieces."""
-    return (q.dtype == torch.float32 and head_dim in (64, 128) and n_kv > 0 and n_q % n_kv == 0 and n_q // n_kv <= 32
+    return (q.dtype == torch.float32 and attention_rows_heads(n_q, n_kv, head_dim)
             and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0 and v_cache.shape == k_cache.shape
             and all(t.dtype == torch.float32 and t.data_ptr() % 16 == 0 for t in (q, out, k_cache, v_cache)))
 

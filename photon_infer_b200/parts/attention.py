@@ -52,6 +52,8 @@ class PagedAttention(Mixer):
             mods.append(("attention_tc", {"HEAD_DIM": self.head_dim}))
         if dtype == torch.bfloat16 and self.head_dim in (64, 128) and self.n_q // self.n_kv <= 16:
             mods.append(("attention_decode", {"HEAD_DIM": self.head_dim}))
+        if dtype == torch.float32 and self.window is None and ops.attention_rows_heads(self.n_q, self.n_kv, self.head_dim):
+            mods.append("attention_rows")
         return mods
 
     # -- weights: separate q/k/v in the file, one fused matrix on the device

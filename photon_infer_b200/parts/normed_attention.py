@@ -74,6 +74,9 @@ class NormedAttention(Mixer):
 
     def required_kernels(self, dtype):
         mods = list(self.kernel_modules)
+        if dtype == torch.float32 and self._plain and not self.output_gate and self.value_dim == self.head_dim \
+                and ops.attention_rows_heads(self.n_q, self.n_kv, self.head_dim):
+            mods.append("attention_rows")
         if dtype == torch.bfloat16:
             mods.extend(["gemm_skinny", "gemm_tc", "gemm_tc2"])
             if self._flash_ok(dtype):
@@ -84,6 +87,11 @@ class NormedAttention(Mixer):
                     and self.value_dim == self.head_dim and self.n_q // self.n_kv <= 16:
                 mods.append(("attention_decode", {"HEAD_DIM": self.head_dim}))     # long contexts without any of the rules
         return mods
+
+    @property
+    def _plain(self) -> bool:
+        """Attention without any of the rules."""
+        return self.window is None and not self.keep_first and not self.sink and not self.softcap
 
     def _flash_ok(self, dtype) -> bool:
         return ops.flash_attention_supported(dtype, self.head_dim, self.value_dim)
@@ -158,8 +166,7 @@ class NormedAttention(Mixer):
                                 gate=gate)
             return
         group = ctx.groups[cache.group]
-        plain = self.window is None and not self.keep_first and self.sinks is None and not self.softcap and gate is None
-        if plain and rows_together(ctx, q, out, cache, self.n_q, self.n_kv, self.head_dim):
+        if self._plain and gate is None and rows_together(ctx, q, out, cache, self.n_q, self.n_kv, self.head_dim):
             ops.attention_rows(q, out, cache.k, cache.v, group.block_table, ctx.cu_tokens, ctx.positions, ctx.num_seqs,
                                self.n_q, self.n_kv, self.head_dim, self.scale, ctx.error_flag)
             return

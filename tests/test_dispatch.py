@@ -76,3 +76,42 @@ def test_the_switch_of_dependent_launches_takes_every_word_for_off(tmp_path):
     said = lambda value: subprocess.run([str(exe)], env=dict(env, PHOTON_PDL=value), capture_output=True, text=True).stdout
     assert subprocess.run([str(exe)], env=env, capture_output=True, text=True).stdout == "1"
     assert [said(v) for v in ("", "1", "0", "off", "no", "false")] == ["1", "1", "0", "0", "0", "0"]
+
+
+def test_what_a_step_can_launch_is_built_at_load(monkeypatch):
+    """The kernels that attention's 32-bit portions go to are among the modules that a model compiles before its first step, and are
+    not where no step can go to them."""
+    from photon_infer_b200.parts.attention import PagedAttention
+    from photon_infer_b200.parts.normed_attention import NormedAttention
+
+    class Taken(Exception):
+        pass
+
+    def taken(*args, **kwargs):
+        raise Taken
+
+    monkeypatch.setattr(ops, "attention_rows", taken)
+    monkeypatch.setattr(ops, "paged_attention", lambda *args, **kwargs: None)
+    part = lambda cls, *heads, **k: cls(256, *heads, **(dict(k, eps=1e-5) if cls is NormedAttention else k))
+    for cls, extras in ((PagedAttention, ({}, {"window": 16})),
+                        (NormedAttention, ({}, {"window": 16}, {"window": 16, "keep_first": 2}, {"sink": True}, {"softcap": 30.0}, {"output_gate": True},
+                                           {"value_dim": 32}))):
+        for heads in ((4, 2, 64), (32, 1, 128), (33, 1, 64), (4, 2, 96)):
+            for extra in extras:
+                mixer = part(cls, *heads, **extra)
+                n_q, n_kv, d = heads
+                v = getattr(mixer, "value_dim", d)
+                q, out = torch.zeros(256, n_q * d), torch.zeros(256, n_q * v)
+                if getattr(mixer, "sink", False):
+                    mixer.sinks = torch.zeros(n_q)
+                gate = torch.zeros(256, n_q * v) if extra.get("output_gate") else None
+                ctx = type("Ctx", (), dict(max_query_len=256, num_seqs=1, num_tokens=256, cu_tokens=None, positions=None, token_seq=None,
+                                           error_flag=None, max_context_len=256, groups=[type("G", (), dict(block_table=None))]))
+                cache = type("C", (), dict(group=0, k=torch.zeros(4, n_kv, 16, d), v=torch.zeros(4, n_kv, 16, v)))
+                try:
+                    mixer.attend(q, out, ctx, cache, *([gate] if gate is not None else []))
+                    goes = False
+                except Taken:
+                    goes = True
+                assert goes == ("attention_rows" in mixer.required_kernels(torch.float32)), (cls, heads, extra)
+                assert "attention_rows" not in mixer.required_kernels(torch.bfloat16)
