@@ -215,13 +215,13 @@ delta_recurrent_kernel(const float* __restrict__ y, const float* x_ab, long ab_s
                        const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                        const int* __restrict__ cu_tokens, const int* __restrict__ state_slots, float* __restrict__ state,
                        long state_stride, int num_slots, float* __restrict__ o_out, int Gq, int H, int dim, int vdim, int vcols,
-                       int* err) {
+                       int skip_from, int* err) {
   extern __shared__ __align__(16) float sm[];
   pdl_wait();
   const int s = blockIdx.x, h = blockIdx.y, cg = blockIdx.z;
   const int tid = threadIdx.x, nthreads = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int t0 = cu_tokens[s], t1 = cu_tokens[s + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || (skip_from > 0 && t1 - t0 >= skip_from)) return;     // long portions may be left to delta_chunked.cu
   const int slot = state_slots[s];
   if (slot >= num_slots) {
     if (tid == 0 && cg == 0) report_error(err, PHOTON_DEV_BAD_SLOT, t0, slot, num_slots);
@@ -495,8 +495,8 @@ PHOTON_API int photon_delta_conv(const void* x, long x_stride, int x_dtype, cons
 template <int RPT, int RP>
 static int delta_recurrent_launch(const float* y, const void* ab, long ab_stride, int ab_bf16, const float* a_log,
                                   const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
-                                  long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim, int* err,
-                                  cudaStream_t stream) {
+                                  long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim,
+                                  int skip_from, int* err, cudaStream_t stream) {
   // Columns a block owns: at most 256 / RP, and few enough that the step has about one block an SM: the warps of a
   // block go to different schedulers of the SM, while the first warps of two blocks on one SM would share one, and a
   // warp that walks tokens wants a scheduler to itself.  A multiple of 8 where the head has that many.  The cut
@@ -522,16 +522,18 @@ static int delta_recurrent_launch(const float* y, const void* ab, long ab_stride
     if (e != cudaSuccess) return (int)e;
   }
   return launch_pdl(delta_recurrent_kernel<RPT, RP>, dim3(S, H, groups), dim3(threads), smem, stream, y, (const float*)ab, ab_stride,
-                    ab_bf16, a_log, dt_bias, cu_tokens, state_slots, state, state_stride, num_slots, o, Gq, H, dim, vdim, vcols, err);
+                    ab_bf16, a_log, dt_bias, cu_tokens, state_slots, state, state_stride, num_slots, o, Gq, H, dim, vdim, vcols, skip_from,
+                    err);
 }
 
 // y float [T][C] from photon_delta_conv; ab [T][>= 2 H] of ab_dtype (row stride ab_stride): the raw decay inputs of the
 // H heads, then the raw beta inputs; a_log, dt_bias float [H]; state as above with S [H][dim][vdim] at its start;
-// o float [T][H * vdim]: the read-outs before the norm.  dim up to 256.
-PHOTON_API int photon_delta_recurrent(const float* y, const void* ab, long ab_stride, int ab_dtype, const float* a_log,
-                                      const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
-                                      long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim,
-                                      int* err, cudaStream_t stream) {
+// o float [T][H * vdim]: the read-outs before the norm.  dim up to 256.  skip_from > 0: requests that bring that many tokens or
+// more are left alone.
+PHOTON_API int photon_delta_recurrent_ex(const float* y, const void* ab, long ab_stride, int ab_dtype, const float* a_log,
+                                         const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
+                                         long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim,
+                                         int skip_from, int* err, cudaStream_t stream) {
   if (S <= 0) return 0;
   if (Gq <= 0 || H <= 0 || H % Gq || dim <= 0 || vdim <= 0) return PHOTON_ERR_ARGUMENT;
   if (ab_dtype != PHOTON_F32 && ab_dtype != PHOTON_BF16) return PHOTON_ERR_ARGUMENT;
@@ -541,9 +543,17 @@ PHOTON_API int photon_delta_recurrent(const float* y, const void* ab, long ab_st
   // every level of shuffles lengthens the chain from one token to the next
 #define DELTA_TRY(RPT, RP) if (dim <= RPT * RP) \
     return delta_recurrent_launch<RPT, RP>(y, ab, ab_stride, bf, a_log, dt_bias, cu_tokens, state_slots, state, state_stride, num_slots, \
-                                           o, S, Gq, H, dim, vdim, err, stream)
+                                           o, S, Gq, H, dim, vdim, skip_from, err, stream)
   DELTA_TRY(4, 2); DELTA_TRY(4, 4); DELTA_TRY(8, 4); DELTA_TRY(16, 4); DELTA_TRY(32, 4); DELTA_TRY(64, 4);
   return PHOTON_ERR_UNSUPPORTED;
+}
+
+PHOTON_API int photon_delta_recurrent(const float* y, const void* ab, long ab_stride, int ab_dtype, const float* a_log,
+                                      const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
+                                      long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim,
+                                      int* err, cudaStream_t stream) {
+  return photon_delta_recurrent_ex(y, ab, ab_stride, ab_dtype, a_log, dt_bias, cu_tokens, state_slots, state, state_stride, num_slots, o, S, Gq, H,
+                                   dim, vdim, 0, err, stream);
 }
 
 // o float [T][H * vdim]; z [T][H * vdim] of z_dtype (row stride z_stride); norm_w float [vdim]; out [T][H * vdim] of out_dtype.

@@ -37,7 +37,7 @@
 // instead of two take the same time.  The walk takes 2.75 us a chunk, 156 products of 16 x 8 x 8 and
 // their operands' splits for each scheduler; eight warps of 16 rows instead of four of 32 take 181 us, the same walk in plain 32-bit
 // multiply-adds (tiles of 4 x 4 from shared memory) 218 us.
-#include "common.cuh"
+#include "portions.cuh"
 #include <float.h>
 #include <math.h>
 
@@ -51,9 +51,6 @@
 
 __device__ __forceinline__ float dc_softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
-// The chunk c of request s lies at this index: the requests' chunks follow each other, at most one place left free each.
-__device__ __forceinline__ long dc_place(const int* cu_tokens, int s, int c) { return cu_tokens[s] / DC + s + c; }
-
 // Scratch of a (chunk, head): W, Q, K [4 warps][4 token tiles][2][32 lanes][4]; A [4][2][32][4]; U0 [dvp / 16][4][32][4]; b_C.
 __host__ __device__ __forceinline__ long dc_floats(int dvp) { return 3L * DC_MAT + DC * DC + (long)DC * dvp + 4; }
 
@@ -62,8 +59,8 @@ __host__ __device__ __forceinline__ long dc_floats(int dvp) { return 3L * DC_MAT
 
 __global__ void __launch_bounds__(256, 2)
 dc_prep_kernel(const float* __restrict__ y, const void* ab, long ab_stride, int ab_bf16, const float* __restrict__ a_log,
-               const float* __restrict__ dt_bias, const int* __restrict__ cu_tokens, float* __restrict__ scratch, int Gq, int H, int dim,
-               int dv, int dvp) {
+               const float* __restrict__ dt_bias, const int* __restrict__ cu_tokens, int S, int from, float* __restrict__ scratch, int Gq,
+               int H, int dim, int dv, int dvp) {
   extern __shared__ __align__(16) float dp[];
   float* ks = dp;                                      // [DC][DP_LD]
   float* qs = ks + DC * DP_LD;                         // [DC][DP_LD]
@@ -71,11 +68,12 @@ dc_prep_kernel(const float* __restrict__ y, const void* ab, long ab_stride, int 
   float* us = Ls + DC * (DC + 4);                      // [DC][dvp + 4]
   __shared__ double lg[DC];
   __shared__ float beta_s[DC], b_s[DC], tail_s[DC];
-  const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z, tid = threadIdx.x;
-  const int t0 = cu_tokens[s] + c * DC, n = min(DC, cu_tokens[s + 1] - t0);
-  if (n <= 0) return;
+  const int h = blockIdx.y, tid = threadIdx.x;
+  const Portion at = find_portion<false>(cu_tokens, S, from, DC, blockIdx.x);
+  if (at.seq < 0) return;
+  const int t0 = cu_tokens[at.seq] + ((int)blockIdx.x - at.before) * DC, n = min(DC, cu_tokens[at.seq + 1] - t0);
   const int C = 2 * Gq * dim + H * dv, hq = h / (H / Gq);
-  float* dst = scratch + ((size_t)dc_place(cu_tokens, s, c) * H + h) * dc_floats(dvp);
+  float* dst = scratch + ((size_t)blockIdx.x * H + h) * dc_floats(dvp);
   // Keys, queries and values (at first U0's place holds them) all at once, zeros behind the heads' sizes and the chunk's end.
   const bool pieces = dim % 4 == 0 && dv % 4 == 0 && C % 4 == 0 && (uintptr_t)y % 16 == 0;
   auto bring = [&](float* to, int ld, int width, int from, int held) {
@@ -246,23 +244,25 @@ __device__ __forceinline__ void dc_operand(const float (&c)[4], uint32_t (&hi)[4
 }
 
 __global__ void __launch_bounds__(128)
-dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tokens, const int* __restrict__ state_slots,
-               float* __restrict__ state, long state_stride, int num_slots, float* __restrict__ o_out, int H, int dim, int dv, int dvp, int* err) {
+dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tokens, int num_seqs, int from, int places,
+               const int* __restrict__ state_slots, float* __restrict__ state, long state_stride, int num_slots, float* __restrict__ o_out, int H, int dim, int dv, int dvp, int* err) {
   extern __shared__ __align__(16) float dw[];
   float* red = dw + DC_STAGES * DC_STAGE;              // [2][4 warps][8 tiles][32 lanes][4]
-  const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
+  const int cb = blockIdx.x, h = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int t0 = cu_tokens[s], ntok = cu_tokens[s + 1] - t0;
-  if (ntok <= 0) return;
+  const Portion at = find_portion<true>(cu_tokens, num_seqs, from, DC, blockIdx.z);
+  const int s = at.seq;
+  if (s < 0) return;
+  const int t0 = cu_tokens[s], ntok = cu_tokens[s + 1] - t0, chunks = (ntok + DC - 1) / DC;
+  if (at.before + chunks > places) return;             // the caller counted other requests: nothing was formed for this one
   int slot = state_slots[s];
   if (slot >= num_slots) {
     if (tid == 0 && cb == 0) report_error(err, PHOTON_DEV_BAD_SLOT, t0, slot, num_slots);
     return;
   }
   float* S = slot >= 0 ? state + (size_t)slot * state_stride + (size_t)h * dim * dv : nullptr;
-  const int chunks = (ntok + DC - 1) / DC;
   const long per = dc_floats(dvp), step = per * H;
-  const float* src0 = scratch + ((size_t)dc_place(cu_tokens, s, 0) * H + h) * per;
+  const float* src0 = scratch + ((size_t)at.before * H + h) * per;
 
   // a thread's share of a chunk: 8 quads of W, of Q, of K, 2 of A, one of U0 (token tile w of the block's columns)
   auto fetch = [&](int c) {
@@ -406,33 +406,32 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
   }
 }
 
-// Scratch floats of photon_delta_chunked for T tokens of S requests.
-PHOTON_API long photon_delta_chunked_scratch(int T, int S, int H, int dv) {
-  return ((long)T / DC + S + 1) * H * dc_floats((dv + 15) / 16 * 16);
-}
+// Tokens of a chunk, and scratch floats of photon_delta_chunked for `chunks` of them.
+PHOTON_API int photon_delta_chunk(void) { return DC; }
+PHOTON_API long photon_delta_chunked_scratch(long chunks, int H, int dv) { return chunks * H * dc_floats((dv + 15) / 16 * 16); }
 
-// As photon_delta_recurrent, for steps with long portions: the same arguments, T tokens in all, `longest` tokens of a request at
-// most; scratch: photon_delta_chunked_scratch floats, 16-byte aligned.  dim up to 128, vdim up to 256.
+// As photon_delta_recurrent, for the requests that bring at least `from` tokens: `longs` of them, with `chunks` chunks of
+// photon_delta_chunk tokens (the last one of a request may be short); the others are left alone.  scratch:
+// photon_delta_chunked_scratch floats, 16-byte aligned.  dim up to 128, vdim up to 256.
 PHOTON_API int photon_delta_chunked(const float* y, const void* ab, long ab_stride, int ab_dtype, const float* a_log, const float* dt_bias,
                                     const int* cu_tokens, const int* state_slots, float* state, long state_stride, int num_slots, float* o,
-                                    float* scratch, int T, int S, int longest, int Gq, int H, int dim, int vdim, int* err,
+                                    float* scratch, int S, int from, int longs, int chunks, int Gq, int H, int dim, int vdim, int* err,
                                     cudaStream_t stream) {
-  if (S <= 0 || T <= 0) return 0;
-  if (Gq <= 0 || H <= 0 || H % Gq || dim <= 0 || vdim <= 0 || longest <= 0 || scratch == nullptr || ((uintptr_t)scratch & 15)) return PHOTON_ERR_ARGUMENT;
+  if (S <= 0 || longs <= 0 || chunks <= 0) return 0;
+  if (Gq <= 0 || H <= 0 || H % Gq || dim <= 0 || vdim <= 0 || scratch == nullptr || ((uintptr_t)scratch & 15)) return PHOTON_ERR_ARGUMENT;
   if (ab_dtype != PHOTON_F32 && ab_dtype != PHOTON_BF16) return PHOTON_ERR_ARGUMENT;
   const int dvp = (vdim + 15) / 16 * 16;
-  const long chunks = ((long)longest + DC - 1) / DC;
-  if (dim > DC_D || vdim > 256 || S > 65535 || H > 65535 || chunks > 0x7fffffffL) return PHOTON_ERR_UNSUPPORTED;
+  if (dim > DC_D || vdim > 256 || longs > 65535 || H > 65535) return PHOTON_ERR_UNSUPPORTED;
   const size_t smem1 = ((size_t)2 * DC * DP_LD + DC * (DC + 4) + DC * (dvp + 4)) * sizeof(float);
   const size_t smem2 = ((size_t)DC_STAGES * DC_STAGE + 2 * DC_RED) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(dc_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dc_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
   if (e != cudaSuccess) return (int)e;
-  dc_prep_kernel<<<dim3((unsigned)chunks, H, S), 256, smem1, stream>>>(y, ab, ab_stride, ab_dtype == PHOTON_BF16, a_log, dt_bias, cu_tokens, scratch,
-                                                                      Gq, H, dim, vdim, dvp);
+  dc_prep_kernel<<<dim3(chunks, H), 256, smem1, stream>>>(y, ab, ab_stride, ab_dtype == PHOTON_BF16, a_log, dt_bias, cu_tokens, S, from, scratch, Gq,
+                                                          H, dim, vdim, dvp);
   const int st = launch_status();
   if (st != 0) return st;
-  dc_walk_kernel<<<dim3(dvp / DC_CB, H, S), 128, smem2, stream>>>(scratch, cu_tokens, state_slots, state, state_stride, num_slots, o, H, dim, vdim,
-                                                                  dvp, err);
+  dc_walk_kernel<<<dim3(dvp / DC_CB, H, longs), 128, smem2, stream>>>(scratch, cu_tokens, S, from, chunks, state_slots, state, state_stride, num_slots, o, H,
+                                                                      dim, vdim, dvp, err);
   return launch_status();
 }

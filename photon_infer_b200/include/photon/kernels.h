@@ -233,13 +233,19 @@ PHOTON_EXPORT int photon_delta_recurrent(const float* y, const void* ab, long ab
                            const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
                            long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim, int* err,
                            cudaStream_t stream);
-/* delta_chunked.cu: the same for steps with long portions, 32 tokens at a time; T tokens in all, `longest` of one request at most;
- * scratch 16-byte aligned.  dim up to 128, vdim up to 256. */
-PHOTON_EXPORT long photon_delta_chunked_scratch(int T, int S, int H, int dv);
+/* The same; skip_from > 0: requests that bring that many tokens or more are left alone. */
+PHOTON_EXPORT int photon_delta_recurrent_ex(const float* y, const void* ab, long ab_stride, int ab_dtype, const float* a_log,
+                           const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
+                           long state_stride, int num_slots, float* o, int S, int Gq, int H, int dim, int vdim, int skip_from,
+                           int* err, cudaStream_t stream);
+/* delta_chunked.cu: the same for the requests that bring at least `from` tokens, photon_delta_chunk() of them at a time: `longs`
+ * requests with `chunks` chunks in all.  scratch 16-byte aligned.  dim up to 128, vdim up to 256. */
+PHOTON_EXPORT int photon_delta_chunk(void);
+PHOTON_EXPORT long photon_delta_chunked_scratch(long chunks, int H, int dv);
 PHOTON_EXPORT int photon_delta_chunked(const float* y, const void* ab, long ab_stride, int ab_dtype, const float* a_log,
                            const float* dt_bias, const int* cu_tokens, const int* state_slots, float* state,
-                           long state_stride, int num_slots, float* o, float* scratch, int T, int S, int longest, int Gq, int H,
-                           int dim, int vdim, int* err, cudaStream_t stream);
+                           long state_stride, int num_slots, float* o, float* scratch, int S, int from, int longs, int chunks,
+                           int Gq, int H, int dim, int vdim, int* err, cudaStream_t stream);
 /* out = o / sqrt(mean(o^2) + eps) * norm_w * silu(z) per head over vdim; z [T][H * vdim] of z_dtype, norm_w float [vdim]. */
 PHOTON_EXPORT int photon_delta_out(const float* o, const void* z, long z_stride, int z_dtype, const float* norm_w, float eps,
                      void* out, long out_stride, int out_dtype, int T, int H, int vdim, cudaStream_t stream);

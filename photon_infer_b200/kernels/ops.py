@@ -1396,11 +1396,12 @@ def delta_conv(x: torch.Tensor, taps_w: torch.Tensor, token_seq: torch.Tensor, c
 
 def delta_recurrent(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, cu_tokens: torch.Tensor,
                     state_slots: torch.Tensor, state: torch.Tensor, o: torch.Tensor, num_seqs: int, qk_heads: int, heads: int,
-                    dim: int, vdim: int, err: Optional[torch.Tensor]) -> None:
+                    dim: int, vdim: int, err: Optional[torch.Tensor], skip_from: int = 0) -> None:
     """The gated delta rule over the tokens of a step, request by request: ``y [T, C]`` from ``delta_conv``,
     ``ab [T, 2 heads]`` (a view with a row stride: the raw decay inputs, then the raw beta inputs), ``a_log``,
     ``dt_bias`` float32 ``[heads]``; ``o [T, heads * vdim]`` float32 receives the read-outs.  The state matrices are
-    the first ``heads * dim * vdim`` numbers of a request's state row."""
+    the first ``heads * dim * vdim`` numbers of a request's state row.  ``skip_from`` > 0: requests that bring that many tokens
+    or more are left alone (the caller runs them)."""
     _cuda(y, ab, a_log, dt_bias, cu_tokens, state_slots, state, o, err)
     T = y.shape[0]
     if ab.shape != (T, 2 * heads) or ab.stride(1) != 1:
@@ -1414,35 +1415,40 @@ def delta_recurrent(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_b
         raise PhotonError(ErrorCode.SHAPE_MISMATCH, "delta_recurrent: state must be contiguous float32 [slots, row]")
     _int32(cu_tokens, "cu_tokens")
     _int32(state_slots, "state_slots")
-    f = _fn("delta", "photon_delta_recurrent",
+    f = _fn("delta", "photon_delta_recurrent_ex",
             [c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_int,
-             c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+             c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(_ptr(y), _ptr(ab), ab.stride(0), _dtype_code(ab), _ptr(a_log), _ptr(dt_bias), _ptr(cu_tokens), _ptr(state_slots),
-             _ptr(state), state.stride(0), state.shape[0], _ptr(o), int(num_seqs), qk_heads, heads, dim, vdim, _ptr(err),
+             _ptr(state), state.stride(0), state.shape[0], _ptr(o), int(num_seqs), qk_heads, heads, dim, vdim, int(skip_from), _ptr(err),
              _stream()), "delta_recurrent")
 
 
-#: A bfloat16 step in which some request brings at least this many tokens runs the delta rule 32 tokens at a time.
+#: The requests of a bfloat16 step that bring at least this many tokens may run the delta rule 32 tokens at a time.
 DELTA_CHUNKED_MIN_TOKENS = 64
 
 
-#: .. and a step tokens x heads: below, a step waits for the host or for the token-by-token kernel's one launch (B200, a mixer's
-#: step, us, token by token first: 130 tokens x 16 heads 101 and 116, 2 x 130 x 16 98 and 117, 300 x 16 138 and 116).
+#: .. and such requests of a step together tokens x heads: below, a step waits for the host or for the token-by-token kernel's one
+#: launch (B200, a mixer's step, us, token by token first: 130 tokens x 16 heads 101 and 116, 2 x 130 x 16 98 and 117, 300 x 16 138
+#: and 116).
 DELTA_CHUNKED_FROM = 4700
 
 
-def delta_chunked_supported(dim: int, vdim: int, query_lens, heads: int) -> bool:
-    """Whether the delta rule of a bfloat16 step runs in chunks: heads of up to 128 and 256 numbers, a request with enough tokens,
-    and a step with enough work."""
-    return (dim <= 128 and vdim <= 256 and max(query_lens) >= DELTA_CHUNKED_MIN_TOKENS
-            and sum(query_lens) * heads >= DELTA_CHUNKED_FROM)
+def delta_chunked_from(dim: int, vdim: int, query_lens, heads: int) -> int:
+    """The tokens from which a request of a bfloat16 step runs the delta rule in chunks; 0: none does.  Heads of up to 128 and 256
+    numbers, and long requests with enough work; a request of fewer tokens stays in the token-by-token kernel, since it would cost a whole
+    chunk."""
+    if dim > 128 or vdim > 256 or max(query_lens) < DELTA_CHUNKED_MIN_TOKENS:
+        return 0
+    work = sum(n for n in query_lens if n >= DELTA_CHUNKED_MIN_TOKENS) * heads
+    return DELTA_CHUNKED_MIN_TOKENS if work >= DELTA_CHUNKED_FROM else 0
 
 
 def delta_chunked(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, cu_tokens: torch.Tensor,
                   state_slots: torch.Tensor, state: torch.Tensor, o: torch.Tensor, query_lens, qk_heads: int, heads: int, dim: int, vdim: int,
-                  err: Optional[torch.Tensor]) -> None:
-    """``delta_recurrent`` for steps with long portions: what the tokens of a chunk of 32 do to each other is formed for all chunks
-    side by side, and the state walks from chunk to chunk in matrix products.  ``query_lens``: the requests' tokens in the step (host)."""
+                  err: Optional[torch.Tensor], long_from: int = 1) -> None:
+    """``delta_recurrent`` for the requests that bring at least ``long_from`` tokens: what the tokens of a chunk of 32 do to each
+    other is formed for all chunks side by side, and the state walks from chunk to chunk in matrix products.  ``query_lens``: the
+    requests' tokens in the step (host)."""
     _cuda(y, ab, a_log, dt_bias, cu_tokens, state_slots, state, o, err)
     T, S = y.shape[0], len(query_lens)
     C = 2 * qk_heads * dim + heads * vdim
@@ -1458,15 +1464,17 @@ def delta_chunked(y: torch.Tensor, ab: torch.Tensor, a_log: torch.Tensor, dt_bia
     _int32(state_slots, "state_slots")
     if cu_tokens.numel() < S + 1 or state_slots.numel() < S or sum(query_lens) > T:
         raise PhotonError(ErrorCode.SHAPE_MISMATCH, "delta_chunked: cu_tokens and state_slots must cover every request")
-    size = load_module("delta_chunked").photon_delta_chunked_scratch
-    size.restype, size.argtypes = c_long, [c_int] * 4
-    scratch = torch.empty(size(T, S, heads, vdim), dtype=torch.float32, device=y.device)
+    lib = load_module("delta_chunked")
+    chunk, size = int(lib.photon_delta_chunk()), lib.photon_delta_chunked_scratch
+    size.restype, size.argtypes = c_long, [c_long, c_int, c_int]
+    pieces = [-(-n // chunk) for n in query_lens if n >= max(1, long_from)]
+    scratch = torch.empty(size(sum(pieces), heads, vdim), dtype=torch.float32, device=y.device)
     f = _fn("delta_chunked", "photon_delta_chunked",
             [c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_int,
-             c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(_ptr(y), _ptr(ab), ab.stride(0), _dtype_code(ab), _ptr(a_log), _ptr(dt_bias), _ptr(cu_tokens), _ptr(state_slots), _ptr(state),
-             state.stride(0), state.shape[0], _ptr(o), _ptr(scratch), T, S, max(query_lens, default=0), qk_heads, heads, dim, vdim, _ptr(err),
-             _stream()), "delta_chunked")
+             state.stride(0), state.shape[0], _ptr(o), _ptr(scratch), S, int(long_from), len(pieces), sum(pieces), qk_heads, heads, dim, vdim,
+             _ptr(err), _stream()), "delta_chunked")
     global _launch_count
     _launch_count += 1
 

@@ -95,14 +95,15 @@ class GatedDeltaRule(Mixer):
                        self.heads * self.dim * self.vdim, y, ctx.num_seqs, self.qk_heads, H, self.dim, self.vdim, ctx.error_flag)
         o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
         ab = rows[:, C + nv:C + nv + 2 * H]
-        lens = list(ctx.host_query_lens)
-        if h.dtype == torch.bfloat16 and lens and ops.delta_chunked_supported(self.dim, self.vdim, lens, H):
+        lens = ctx.host_query_lens
+        long = ops.delta_chunked_from(self.dim, self.vdim, lens, H) if h.dtype == torch.bfloat16 and lens else 0
+        if long:
             # long portions: 32 tokens at a time in matrix products
             ops.delta_chunked(y, ab, self.a_log, self.dt_bias, ctx.cu_tokens, ctx.state_slots, state, o, lens, self.qk_heads, H, self.dim,
-                              self.vdim, ctx.error_flag)
-        else:
+                              self.vdim, ctx.error_flag, long_from=long)
+        if not long or min(lens) < long:
             ops.delta_recurrent(y, ab, self.a_log, self.dt_bias, ctx.cu_tokens, ctx.state_slots, state,
-                                o, ctx.num_seqs, self.qk_heads, H, self.dim, self.vdim, ctx.error_flag)
+                                o, ctx.num_seqs, self.qk_heads, H, self.dim, self.vdim, ctx.error_flag, skip_from=long)
         out = torch.empty((T, nv), dtype=h.dtype, device=h.device)
         ops.delta_out(o, rows[:, C:C + nv], self.norm, self.eps, out, H, self.vdim)
         return project(out, self.w_o)
