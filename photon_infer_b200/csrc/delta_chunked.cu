@@ -325,8 +325,6 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
     __syncthreads();                                   // the partial sums and U0 are there for every warp; the sums of the chunk before
     fetch(c + DC_STAGES - 1);                          // last are read no more, and neither is the stage that is filled now
     uint32_t uh[4][4], ul[4][4];
-    float uw[4] = {0.f, 0.f, 0.f, 0.f};                // U of the tokens whose outputs this warp forms
-    bool wild = false;                                 // infinities and NaN among them
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float4 u0 = d4[(3 * DC_MAT + DC * DC) / 4 + i * 32];
@@ -334,12 +332,7 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
       const float u[4] = {u0.x - ((p0.x + p1.x) + (p2.x + p3.x)), u0.y - ((p0.y + p1.y) + (p2.y + p3.y)),
                           u0.z - ((p0.z + p1.z) + (p2.z + p3.z)), u0.w - ((p0.w + p1.w) + (p2.w + p3.w))};
       dc_operand(u, uh[i], ul[i]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (i == w) { uw[e] = u[e]; wild |= !(fabsf(u[e]) <= FLT_MAX); }
-      }
     }
-    wild = __any_sync(0xffffffffu, wild);
     // the outputs of tokens 8 w .. 8 w + 7 and this warp's rows of the state, side by side
     DcAcc out, nw[4];
     {
@@ -365,20 +358,43 @@ dc_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ cu_tok
         dc_mma3(nw[1], uh[i], ul[i], k0.z, k0.w);
         dc_mma3(nw[2], uh[i], ul[i], k1.x, k1.y);
         dc_mma3(nw[3], uh[i], ul[i], k1.z, k1.w);
-        // A is zero for later tokens, but zero times their infinities would not be: tiles behind the warp's are left out, and its
-        // own one is a plain sum over the tokens that count where its U is not finite
-        if (i < w || (i == w && !wild)) dc_mma3(out, uh[i], ul[i], u ? a.z : a.x, u ? a.w : a.y);
+        dc_mma3(out, uh[i], ul[i], u ? a.z : a.x, u ? a.w : a.y);
       }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) st[j][e] = dc_sum(nw[j], e);
-    if (wild) {
+    bool finite = true;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) finite &= fabsf(dc_sum(out, e)) <= FLT_MAX;
+    if (!__all_sync(0xffffffffu, finite)) {
+      // A is zero for later tokens, but zero times their infinities is not.  The warp's outputs again: the tiles of earlier tokens,
+      // then its own one, as a plain sum over the tokens that count if U is not finite there.
+      {
+        const float4 p0 = r4[(4 + w) * 32], p1 = r4[(12 + w) * 32], p2 = r4[(20 + w) * 32], p3 = r4[(28 + w) * 32];
+        dc_clear(out);
+        out.x[0] = (p0.x + p1.x) + (p2.x + p3.x); out.x[1] = (p0.y + p1.y) + (p2.y + p3.y);
+        out.x[2] = (p0.z + p1.z) + (p2.z + p3.z); out.x[3] = (p0.w + p1.w) + (p2.w + p3.w);
+      }
+      const float4 u0 = d4[(3 * DC_MAT + DC * DC) / 4 + w * 32];
+      const float4 p0 = r4[w * 32], p1 = r4[(8 + w) * 32], p2 = r4[(16 + w) * 32], p3 = r4[(24 + w) * 32];
+      const float uw[4] = {u0.x - ((p0.x + p1.x) + (p2.x + p3.x)), u0.y - ((p0.y + p1.y) + (p2.y + p3.y)),
+                           u0.z - ((p0.z + p1.z) + (p2.z + p3.z)), u0.w - ((p0.w + p1.w) + (p2.w + p3.w))};
+      bool wild = false;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) wild |= !(fabsf(uw[e]) <= FLT_MAX);
+      wild = __any_sync(0xffffffffu, wild);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 q = d4[3 * DC_MAT / 4 + (w * 2 + (i >> 1)) * 32];
+        if (i < w || (i == w && !wild)) dc_mma3(out, uh[i], ul[i], i & 1 ? q.z : q.x, i & 1 ? q.w : q.y);
+      }
       // A [warp][s / 16][lane (t % 8) * 4 + (s % 8) / 2][(s % 16) / 8 * 2 + s % 2], s = 8 w + i
       const float* a = reinterpret_cast<const float*>(d4 - lane) + 3 * DC_MAT + (w * 2 + (w >> 1)) * 128 + (w & 1) * 2;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
+        if (!wild) break;
         const int from = (lane & ~3) | (i >> 1);
         const float u0 = __shfl_sync(0xffffffffu, uw[i & 1], from), u1 = __shfl_sync(0xffffffffu, uw[2 + (i & 1)], from);
 #pragma unroll
