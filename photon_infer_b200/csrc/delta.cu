@@ -471,8 +471,10 @@ PHOTON_API int photon_delta_conv(const void* x, long x_stride, int x_dtype, cons
   const int C = 2 * Gq * dim + H * vdim;
   dim3 grid((2 * Gq + H + 3) / 4, T);
   int st;
-  // many tokens; a decode step's few keep a warp each, which is the shorter way for one token
-  if (x_dtype == PHOTON_F32 && taps == 4 && dim <= 128 && vdim <= 128 && T >= 64 && ((uintptr_t)taps_w & 15) == 0)
+  // many tokens of few requests; a decode step's few keep a warp each, which is the shorter way for one token, and so do steps with
+  // many requests: a request's first three tokens look up its slot and read its state's rows, which a warp does for one token after the
+  // other (a mixer's step, us, a warp per token first, 64 + 63 tokens of 64 requests x 16 heads 139 and 154, 128 + 63 182 and 195)
+  if (x_dtype == PHOTON_F32 && taps == 4 && dim <= 128 && vdim <= 128 && T >= 64 && T >= 16L * S && ((uintptr_t)taps_w & 15) == 0)
     st = launch_pdl(delta_conv_many_kernel, dim3(grid.x, (T + DCV_TOK - 1) / DCV_TOK), dim3(128), 0, stream, (const float*)x, x_stride, taps_w,
                     token_seq, cu_tokens, state_slots, (const float*)state, state_stride, conv_offset, num_slots, y, T, Gq, H, dim, vdim, err);
   else if (x_dtype == PHOTON_F32)
