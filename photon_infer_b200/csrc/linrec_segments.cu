@@ -6,6 +6,8 @@
 //   S_t = diag(a_t) S_(t-1) + k_t v_t^T             mode 3 (gated linear attention): a number per row
 //
 // The update is linear in the state, so a segment's end is (its decay) x (its start) + (its end from a zero start).
+// The requests' segments stand one behind the other in the grid, a request of few tokens is one segment; only requests of several
+// have room in scratch.
 //   1. ls_gates_kernel (modes 0, 1): the gates of all tokens, and what a segment does to the scale of the state.
 //   2. the walk, first pass: every segment but the last, from zero (the first from the request's state), keeps its
 //      end state and its decay in scratch.  No queries.
@@ -35,6 +37,7 @@
 // 32 tokens joined by a scan) -> 156 us and 37 us for its inputs.  Half of the time is the FP32 pipe; the rest is the barriers of a
 // chunk, the folds and the blocks' start, which two or three blocks an SM hide equally (100 us either way for the second pass).
 #include "linrec.cuh"
+#include "portions.cuh"
 
 #define LS_CHUNK 16
 #define LS_THREADS 128
@@ -71,11 +74,12 @@ struct LsArgs {
   float* state; long state_stride; int num_slots;
   float* out; long out_stride;                       // [T][H * dv]; mode 1: before the division
   float* den;                                        // mode 1: [T][H], what the outputs are to be divided by
-  float* ends;                                       // [S * segs][H][N * dv]
-  float* vecs;                                       // [S * segs][H][N]: mode 1 n at the end; modes 2, 3 the rows' decay (ls_code)
-  float* scale;                                      // [S * segs][H][2]: mode 0 the decay; mode 1 F and L at the end
-  float* first;                                      // [S][H][N * dv], then [S][H][N], then [S][H]: the state before the step
-  int T, S, H, qk_heads, N, dv, seg, segs, vec;
+  float* ends;                                       // [cut_segs][H][N * dv]: the requests of several segments
+  float* vecs;                                       // [cut_segs][H][N]: mode 1 n at the end; modes 2, 3 the rows' decay (ls_code)
+  float* scale;                                      // [segs][H][2]: mode 0 the decay; mode 1 F and L at the end
+  float* first;                                      // [cuts][H][N * dv], then [cuts][H][N]: the state of those requests before the step
+  float* first_m;                                    // [S][H]: mode 1, the running maximum before the step
+  int T, S, H, qk_heads, N, dv, seg, segs, cuts, cut_segs, vec;
   int* err;
 };
 
@@ -87,18 +91,17 @@ ls_gates_kernel(const float* __restrict__ ga, const float* __restrict__ gb, long
                 const float* __restrict__ p1, float cap, float* __restrict__ gates, LsArgs A) {
   const int lane = threadIdx.x & 31;
   const int h = blockIdx.y * 4 + (threadIdx.x >> 5);
-  const int s = blockIdx.x / A.segs, sg = blockIdx.x - s * A.segs;
-  if (h >= A.H) return;
+  const Portion place = find_portion<false>(A.cu_tokens, A.S, 1, A.seg, blockIdx.x);
+  const int s = place.seq, sg = (int)blockIdx.x - place.before;
+  if (h >= A.H || s < 0) return;
   const int t0 = A.cu_tokens[s], t1 = A.cu_tokens[s + 1];
   const int b0 = t0 + sg * A.seg, b1 = min(t1, b0 + A.seg);
   const size_t TH = (size_t)A.T * A.H;
   if (MODE == 1 && sg == 0 && lane == 0) {
     const int slot = A.state_slots[s];
-    const size_t SH = (size_t)A.S * A.H;
-    A.first[SH * A.N * A.dv + SH * A.N + (size_t)s * A.H + h] =
+    A.first_m[(size_t)s * A.H + h] =
         slot >= 0 && slot < A.num_slots ? A.state[(size_t)slot * A.state_stride + (size_t)A.H * A.N * (A.dv + 1) + h] : 0.f;
   }
-  if (b0 >= b1) return;
   const float a_h = MODE == 0 ? expf(p0[h]) : 0.f;
   double sum = 0.0;                                  // of dt or f over the segment's tokens before these 32
   float last = -INFINITY;                            // mode 1: L at the token before these 32
@@ -172,10 +175,14 @@ ls_walk_kernel(const LsArgs A) {
   __shared__ int plain_s;
   __shared__ float den_s[4][LS_CHUNK];
   const int N = A.N, dv = A.dv, H = A.H;
-  const int s = blockIdx.z / A.segs, sg = blockIdx.z - s * A.segs;
+  const Portion place = find_portion<false>(A.cu_tokens, A.S, 1, A.seg, blockIdx.z);
+  const int s = place.seq, sg = (int)blockIdx.z - place.before;
+  if (s < 0) return;
   const int t0 = A.cu_tokens[s], t1 = A.cu_tokens[s + 1];
   const int nseg = (t1 - t0 + A.seg - 1) / A.seg;
-  if (sg >= nseg || (PASS == 1 && sg == nseg - 1)) return;
+  if (PASS == 1 && sg == nseg - 1) return;
+  // a caller that counted other requests than cu_tokens holds has made no room for them
+  if (nseg > 1 && (place.cut_rank >= A.cuts || place.cut_before + nseg > A.cut_segs)) return;
   const int b0 = t0 + sg * A.seg, b1 = min(t1, b0 + A.seg);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane & (L - 1);
@@ -193,7 +200,9 @@ ls_walk_kernel(const LsArgs A) {
   float* row0 = slot >= 0 ? A.state + (size_t)slot * A.state_stride : nullptr;
   float* S_h = row0 ? row0 + (size_t)h * N * dv : nullptr;
   float* n_h = row0 ? row0 + (size_t)H * N * dv + (size_t)h * N : nullptr;           // mode 1
-  const size_t SH = (size_t)A.S * H, sh = (size_t)s * H + h;
+  const size_t SH = (size_t)A.cuts * H, sh = (size_t)place.cut_rank * H + h;
+  auto seg_at = [&](int i) { return (size_t)(place.cut_before + i) * H + h; };                         // the request's segment i in scratch
+  auto scale_at = [&](int i) { return A.scale + ((size_t)(place.before + i) * H + h) * 2; };
   float* first_S = A.first + sh * N * dv;
   float* first_n = A.first + SH * N * dv + sh * N;
   const bool wide = A.vec && c0 + col + LS_C <= dv;   // all of the lane's columns at a time
@@ -239,8 +248,8 @@ ls_walk_kernel(const LsArgs A) {
     const float* m = zero ? nullptr : kept ? first_S : S_h;                          // overwrites the slot
     const float* vec = zero ? nullptr : kept ? first_n : n_h;
     if (PASS == 2 && sg > 0) {
-      m = A.ends + (((size_t)s * A.segs) * H + h) * N * dv;
-      vec = A.vecs + (((size_t)s * A.segs) * H + h) * N;
+      m = A.ends + seg_at(0) * N * dv;
+      vec = A.vecs + seg_at(0) * N;
     }
 #pragma unroll
     for (int j = 0; j < R / 2; ++j) {
@@ -262,21 +271,19 @@ ls_walk_kernel(const LsArgs A) {
         if (PASS == 1 && sg == 0 && r < N) first_n[r] = follow[i];
       }
     }
-    if (MODE == 1) m0 = zero ? -INFINITY : A.first[SH * N * dv + SH * N + sh];
+    if (MODE == 1) m0 = zero ? -INFINITY : A.first_m[(size_t)s * H + h];
     if (PASS == 2 && sg > 0) {
       // S is the state at the end of segment 0; the segments after it, one behind the other
-      if (MODE == 1) {
-        const float* sc = A.scale + (((size_t)s * A.segs) * H + h) * 2;
-        m0 = fmaxf(sc[0] + m0, sc[1]);
-      }
+      if (MODE == 1) m0 = fmaxf(scale_at(0)[0] + m0, scale_at(0)[1]);
       for (int i = 1; i < sg; ++i) {
-        const size_t at = ((size_t)s * A.segs + i) * H + h;
+        const size_t at = seg_at(i);
+        const float* sc = scale_at(i);
         const float* em = A.ends + at * N * dv;
         const float* ev = A.vecs + at * N;
         float c1 = 1.f, c2 = 1.f;
-        if (MODE == 0) c1 = A.scale[at * 2];
+        if (MODE == 0) c1 = sc[0];
         if (MODE == 1) {
-          const float fm = A.scale[at * 2] + m0, lm = A.scale[at * 2 + 1];
+          const float fm = sc[0] + m0, lm = sc[1];
           const float mn = fmaxf(fm, lm);
           c1 = expf(fm - mn); c2 = expf(lm - mn); m0 = mn;
           if (leads) {
@@ -614,12 +621,12 @@ ls_walk_kernel(const LsArgs A) {
   float* m = nullptr;
   float* vec = nullptr;
   if (PASS == 1) {
-    m = A.ends + (((size_t)s * A.segs + sg) * H + h) * N * dv;
-    vec = A.vecs + (((size_t)s * A.segs + sg) * H + h) * N;
+    m = A.ends + seg_at(sg) * N * dv;
+    vec = A.vecs + seg_at(sg) * N;
   } else if (sg == nseg - 1) {
     m = S_h; vec = n_h;
     if (MODE == 1 && leads && tid == 0 && row0) {
-      const float* sc = A.scale + (((size_t)s * A.segs + sg) * H + h) * 2;
+      const float* sc = scale_at(sg);
       row0[(size_t)H * N * (dv + 1) + h] = fmaxf(sc[0] + m0, sc[1]);
     }
   }
@@ -643,13 +650,13 @@ static int ls_walk(LsArgs A, cudaStream_t stream) {
   const size_t smem = ((size_t)2 * LS_CHUNK * NP * (1 + (PASS == 2) + (MODE == 3)) + (2 + (PASS == 2)) * LS_CHUNK * BC) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(ls_walk_kernel<MODE, L, R, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  ls_walk_kernel<MODE, L, R, PASS><<<dim3((A.dv + BC - 1) / BC, A.H, A.S * A.segs), LS_THREADS, smem, stream>>>(A);
+  ls_walk_kernel<MODE, L, R, PASS><<<dim3((A.dv + BC - 1) / BC, A.H, A.segs), LS_THREADS, smem, stream>>>(A);
   return launch_status();
 }
 
 template <int MODE, int L, int R>
 static int ls_go(const LsArgs& A, cudaStream_t stream) {
-  if (A.segs > 1) {
+  if (A.cuts > 0) {
     const int st = ls_walk<MODE, L, R, 1>(A, stream);
     if (st != 0) return st;
   }
@@ -671,16 +678,27 @@ PHOTON_API int photon_linrec_segment_blocks(int N, int dv) {
   return (dv + bc - 1) / bc;
 }
 
-// Scratch floats of photon_linrec_segments: gates, ends, vectors, scales, the states before the step.
-PHOTON_API long photon_linrec_segments_scratch(int mode, int T, int S, int segs, int H, int N, int dv) {
-  const long pieces = (long)S * segs * H;
+// The parts of photon_linrec_segments' scratch in floats: gates, ends, vectors, scales, the states and the running maxima before
+// the step.
+static void ls_parts(int mode, int T, int S, int segs, int cuts, int cut_segs, int H, int N, int dv, long (&part)[6]) {
   auto four = [](long n) { return (n + 3) & ~3L; };
-  return four(mode == 0 ? 2L * T * H : mode == 1 ? 4L * T * H : 0) + four(pieces * N * dv) + four(pieces * N) + four(pieces * 2) +
-         four((long)S * H * ((long)N * dv + N + 1));
+  part[0] = four(mode == 0 ? 2L * T * H : mode == 1 ? 4L * T * H : 0);
+  part[1] = four((long)cut_segs * H * N * dv);
+  part[2] = four((long)cut_segs * H * N);
+  part[3] = four((long)segs * H * 2);
+  part[4] = four((long)cuts * H * ((long)N * dv + N));
+  part[5] = four((long)S * H);
 }
 
-// As photon_linrec, for requests cut into up to `segs` segments of `seg` tokens (a multiple of 16) each; mode 3: a float
-// [T][qk_heads * N] the rows' decays, ga .. p2 unused.  Mode 2: q and k as photon_linrec_gates leaves them.  Mode 1: den
+PHOTON_API long photon_linrec_segments_scratch(int mode, int T, int S, int segs, int cuts, int cut_segs, int H, int N, int dv) {
+  long part[6], sum = 0;
+  ls_parts(mode, T, S, segs, cuts, cut_segs, H, N, dv, part);
+  for (long p : part) sum += p;
+  return sum;
+}
+
+// As photon_linrec, for requests cut into segments of `seg` tokens (a multiple of 16): `segs` of them in all, `cut_segs` of which
+// belong to the `cuts` requests that have more than one; mode 3: a float [T][qk_heads * N] the rows' decays, ga .. p2 unused.  Mode 2: q and k as photon_linrec_gates leaves them.  Mode 1: den
 // float [T][H] gets what the outputs are to be divided by, and out is not divided.  scratch: photon_linrec_segments_scratch
 // floats, 16-byte aligned.  N up to 512.
 PHOTON_API int photon_linrec_segments(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
@@ -688,31 +706,34 @@ PHOTON_API int photon_linrec_segments(int mode, const float* q, long q_stride, c
                                       const float* p0, const float* p1, const float* p2, float cap, float q_scale,
                                       const int* cu_tokens, const int* state_slots, float* state, long state_stride, int num_slots,
                                       float* out, long out_stride, float* den, float* scratch, int T, int S, int H, int qk_heads,
-                                      int N, int dv, int seg, int segs, int* err, cudaStream_t stream) {
+                                      int N, int dv, int seg, int segs, int cuts, int cut_segs, int* err, cudaStream_t stream) {
   if (S <= 0 || T <= 0) return 0;
-  if (mode < 0 || mode > 3 || H <= 0 || qk_heads <= 0 || H % qk_heads || N <= 0 || dv <= 0 || seg <= 0 || seg % LS_CHUNK || segs <= 0)
+  if (mode < 0 || mode > 3 || H <= 0 || qk_heads <= 0 || H % qk_heads || N <= 0 || dv <= 0 || seg <= 0 || seg % LS_CHUNK || segs <= 0 ||
+      cuts < 0 || cut_segs < 0)
     return PHOTON_ERR_ARGUMENT;
   if (scratch == nullptr || ((uintptr_t)scratch & 15) || (mode == 1 && (!(cap > 0.f) || den == nullptr)) || (mode == 3) != (a != nullptr))
     return PHOTON_ERR_ARGUMENT;
-  if (N > 512 || H > 65535 || (long)S * segs > 65535) return PHOTON_ERR_UNSUPPORTED;
+  if (N > 512 || H > 65535 || segs > 65535) return PHOTON_ERR_UNSUPPORTED;
   LsArgs A;
   A.q = q; A.q_stride = q_stride; A.k = k; A.k_stride = k_stride; A.v = v; A.v_stride = v_stride; A.a = a; A.a_stride = a_stride;
   A.d_skip = p2; A.q_scale = q_scale; A.cu_tokens = cu_tokens; A.state_slots = state_slots; A.state = state; A.state_stride = state_stride;
   A.num_slots = num_slots; A.out = out; A.out_stride = out_stride; A.den = den;
-  A.T = T; A.S = S; A.H = H; A.qk_heads = qk_heads; A.N = N; A.dv = dv; A.seg = seg; A.segs = segs; A.err = err;
-  auto four = [](long n) { return (n + 3) & ~3L; };
-  const long pieces = (long)S * segs * H;
+  A.T = T; A.S = S; A.H = H; A.qk_heads = qk_heads; A.N = N; A.dv = dv; A.seg = seg; A.segs = segs; A.cuts = cuts;
+  A.cut_segs = cut_segs; A.err = err;
+  long part[6];
+  ls_parts(mode, T, S, segs, cuts, cut_segs, H, N, dv, part);
   float* gates = scratch;
   A.gates = gates;
-  A.ends = gates + four(mode == 0 ? 2L * T * H : mode == 1 ? 4L * T * H : 0);
-  A.vecs = A.ends + four(pieces * N * dv);
-  A.scale = A.vecs + four(pieces * N);
-  A.first = A.scale + four(pieces * 2);
+  A.ends = gates + part[0];
+  A.vecs = A.ends + part[1];
+  A.scale = A.vecs + part[2];
+  A.first = A.scale + part[3];
+  A.first_m = A.first + part[4];
   A.vec = N % 4 == 0 && dv % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && state_stride % 4 == 0 && out_stride % 4 == 0 &&
           ((uintptr_t)out & 15) == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)k & 15) == 0 && ((uintptr_t)v & 15) == 0 && ((uintptr_t)state & 15) == 0 &&
           (a == nullptr || (a_stride % 4 == 0 && ((uintptr_t)a & 15) == 0));
   if (mode < 2) {
-    const dim3 grid(S * segs, (H + 3) / 4);
+    const dim3 grid(segs, (H + 3) / 4);
     if (mode == 0) ls_gates_kernel<0><<<grid, 128, 0, stream>>>(ga, gb, g_stride, p0, p1, cap, gates, A);
     else ls_gates_kernel<1><<<grid, 128, 0, stream>>>(ga, gb, g_stride, p0, p1, cap, gates, A);
     const int st = launch_status();

@@ -6,6 +6,7 @@ struct Portion {
   int seq;      // the request; -1: no request holds the place
   int before;   // places of the long requests in front of it
   int rank;     // long requests in front of it
+  int cut_before, cut_rank;     // the same two, counting only requests with more than one place
 };
 
 // The requests that bring at least `from` tokens stand one behind the other, with a place for every `size` tokens begun; the others
@@ -14,7 +15,7 @@ struct Portion {
 template <bool BY_RANK>
 __device__ __forceinline__ Portion find_portion(const int* __restrict__ cu_tokens, int num_seqs, int from, int size, int at) {
   const int lane = threadIdx.x & 31;
-  Portion p = {-1, 0, 0};
+  Portion p = {-1, 0, 0, 0, 0};
   for (int s0 = 0; s0 < num_seqs; s0 += 32) {
     const int s = s0 + lane;
     int n = s < num_seqs ? cu_tokens[s + 1] - cu_tokens[s] : 0;
@@ -25,7 +26,7 @@ __device__ __forceinline__ Portion find_portion(const int* __restrict__ cu_token
       const int v = __shfl_up_sync(0xffffffffu, upto, o);
       if (lane >= o) upto += v;
     }
-    const unsigned longs = __ballot_sync(0xffffffffu, n > 0);
+    const unsigned longs = __ballot_sync(0xffffffffu, n > 0), cuts = __ballot_sync(0xffffffffu, n > 1);
     const int rank = p.rank + __popc(longs & ((1u << lane) - 1));
     const unsigned hit = __ballot_sync(0xffffffffu, n > 0 && (BY_RANK ? rank == at : p.before + upto > at));
     if (hit != 0) {
@@ -33,10 +34,14 @@ __device__ __forceinline__ Portion find_portion(const int* __restrict__ cu_token
       p.seq = s0 + l;
       p.before += __shfl_sync(0xffffffffu, upto - n, l);
       p.rank = __shfl_sync(0xffffffffu, rank, l);
+      p.cut_before += __reduce_add_sync(0xffffffffu, lane < l && n > 1 ? n : 0);
+      p.cut_rank += __popc(cuts & ((1u << l) - 1));
       return p;
     }
     p.before += __shfl_sync(0xffffffffu, upto, 31);
     p.rank += __popc(longs);
+    p.cut_before += __reduce_add_sync(0xffffffffu, n > 1 ? n : 0);
+    p.cut_rank += __popc(cuts);
   }
   return p;
 }

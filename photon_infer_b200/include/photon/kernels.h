@@ -328,16 +328,16 @@ PHOTON_EXPORT int photon_linrec_gates(const float* q, long q_stride, const float
 /* ------------------------------------------------------------------ linrec_segments.cu: long portions in segments side by side */
 /* Blocks of one (segment, head); floats of scratch. */
 PHOTON_EXPORT int photon_linrec_segment_blocks(int N, int dv);
-PHOTON_EXPORT long photon_linrec_segments_scratch(int mode, int T, int S, int segs, int H, int N, int dv);
-/* As photon_linrec (mode 2: q and k from photon_linrec_gates), requests cut into up to `segs` segments of `seg` tokens (a
- * multiple of 16).  mode 3: S_t = diag(a_t) S_(t-1) + k v^T with a [T][qk_heads * N]; ga .. p2 unused.  mode 1: den [T][H] gets
+PHOTON_EXPORT long photon_linrec_segments_scratch(int mode, int T, int S, int segs, int cuts, int cut_segs, int H, int N, int dv);
+/* As photon_linrec (mode 2: q and k from photon_linrec_gates), requests cut into segments of `seg` tokens (a multiple of 16): `segs`
+ * in all, `cut_segs` of which belong to the `cuts` requests that have more than one.  mode 3: S_t = diag(a_t) S_(t-1) + k v^T with a [T][qk_heads * N]; ga .. p2 unused.  mode 1: den [T][H] gets
  * what the outputs are to be divided by.  scratch: 16-byte aligned. */
 PHOTON_EXPORT int photon_linrec_segments(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
                               long v_stride, const float* a, long a_stride, const float* ga, const float* gb, long g_stride,
                               const float* p0, const float* p1, const float* p2, float cap, float q_scale,
                               const int* cu_tokens, const int* state_slots, float* state, long state_stride, int num_slots,
                               float* out, long out_stride, float* den, float* scratch, int T, int S, int H, int qk_heads,
-                              int N, int dv, int seg, int segs, int* err, cudaStream_t stream);
+                              int N, int dv, int seg, int segs, int cuts, int cut_segs, int* err, cudaStream_t stream);
 
 /* ------------------------------------------------------------------ attention_talk.cu: attention whose heads' scores are mixed */
 /* Bias (float, may be null) on q [T][H * d] and k [T][G * d] of in_dtype, rotation of the first rot_dims numbers of a head

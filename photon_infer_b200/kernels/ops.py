@@ -1818,7 +1818,7 @@ LINREC_SEGMENTS_MIN_TOKENS = 128
 LINREC_SEGMENT_MODES = {"state_space": 0, "matrix_memory": 1, "forget_write": 2, "decay_rows": 3}
 
 
-#: Tokens x heads of a step from which the segments are the faster way.  Below, a step waits for the host or for one pass over the
+#: Tokens x heads of a step with such a request from which the segments are the faster way.  Below, a step waits for the host or for one pass over the
 #: tokens, and the segments' additional launches and second pass cost more than they save.  B200, heads of 128 x 128, a mixer's
 #: step, us, without segments first: gated linear attention 300 tokens x 16 heads 139 and 148, 3 x 130 x 16 250 and 148; matrix
 #: memory 3 x 130 x 16 105 and 132, 500 x 16 161 and 131; state space 500 x 16 151 and 154, 300 x 32 168 and 157.
@@ -1830,23 +1830,36 @@ LINREC_SEGMENTS_FROM = {"decay_rows": 6000, "matrix_memory": 7000, "state_space"
 def linrec_segments_supported(mode: str, dim: int, query_lens, heads: int) -> bool:
     """Whether the recurrences of a bfloat16 step run in segments: states of up to 512 rows, a request with enough tokens, and a
     step with enough work."""
-    if mode == "forget_write" and len(query_lens) * heads >= 32:
+    if dim > 512 or max(query_lens) < LINREC_SEGMENTS_MIN_TOKENS or (mode == "forget_write" and len(query_lens) * heads >= 32):
         return False
-    return (dim <= 512 and max(query_lens) >= LINREC_SEGMENTS_MIN_TOKENS
-            and sum(query_lens) * heads >= LINREC_SEGMENTS_FROM[mode])
+    return sum(query_lens) * heads >= LINREC_SEGMENTS_FROM[mode]
 
 
-def linrec_segment_tokens(query_lens, heads: int, dim: int, vdim: int, sms: int) -> int:
-    """Tokens of a segment, a multiple of 16: the fewest with which the requests' segments fit the GPU at once at two blocks a
-    streaming multiprocessor (one block more would wait for a whole segment), but no fewer than 64 (every segment but the first costs a
-    pass over its tokens without queries and a fold of its end state)."""
-    blocks = heads * int(load_module("linrec_segments").photon_linrec_segment_blocks(dim, vdim))
-    places = max(1, 2 * sms // blocks)
-    seg = max(64, -(-sum(query_lens) // (16 * places)) * 16)
+def linrec_segment_blocks(dim: int, vdim: int) -> int:
+    """Blocks of one (segment, head)."""
+    return int(load_module("linrec_segments").photon_linrec_segment_blocks(dim, vdim))
+
+
+def linrec_segment_tokens(query_lens, heads: int, blocks: int, sms: int) -> int:
+    """Tokens of a segment, a multiple of 16: the fewest with which the segments of the step's long requests (at least 128 tokens, or
+    the longest) fit the GPU at once at two blocks a streaming multiprocessor (one block more would wait for a whole segment), but no fewer
+    than 64 (every segment but the first costs a pass over its tokens without queries and a fold of its end state).  The others are
+    done within a segment's time and take no place.  The longest request's tokens where there are no more places than long requests."""
     longest = max(query_lens)
-    while seg < longest and sum(-(-n // seg) for n in query_lens) > places:
-        seg += 16
-    return seg
+    longs = [n for n in query_lens if n >= LINREC_SEGMENTS_MIN_TOKENS] or [longest]
+    places, total = max(1, 2 * sms // (heads * blocks)), sum(longs)
+    whole = max(4, -(-longest // 16))
+    if places <= len(longs):
+        return whole * 16
+    # fewer sixteens than `low` cannot fit; `high` fits, since a request's last segment is less than one above its share
+    low, high = max(4, -(-total // (16 * places))), max(4, min(whole, -(-total // (16 * (places - len(longs))))))
+    while low < high:
+        mid = (low + high) // 2
+        if sum(-(-n // (16 * mid)) for n in longs) <= places:
+            high = mid
+        else:
+            low = mid + 1
+    return low * 16
 
 
 def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: Optional[torch.Tensor], gate_a: Optional[torch.Tensor],
@@ -1855,8 +1868,9 @@ def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
                     query_lens, heads: int, qk_heads: int, dim: int, vdim: int, err: Optional[torch.Tensor],
                     segment: Optional[int] = None) -> Optional[torch.Tensor]:
     """``linrec`` for a step with long portions: every request is cut into segments that run side by side, a first pass from
-    zero states and a second one from the states that the first pass's ends add up to.  The arithmetic of a token is that of ``linrec``;
-    a segment's start is one multiply-add per segment before it away from the state that ``linrec`` would have reached.  ``forget_write``:
+    zero states and a second one from the states that the first pass's ends add up to.  Everything is 32-bit; a chunk of 16 tokens holds its
+    state relative to its decays, and a segment's start is a multiply-add per segment before it away from the state that ``linrec`` would have
+    reached.  ``forget_write``:
     ``q`` and ``k`` as ``linrec_gates`` leaves them.  ``decay_rows``: ``S <- diag(a) S + k v^T``, ``a [T, qk_heads * dim]``.
     ``matrix_memory``: ``out`` is not divided; returns ``[T, heads]``, what it is to be divided by.  ``query_lens``: the requests'
     tokens in the step (host)."""
@@ -1886,23 +1900,26 @@ def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     _int32(state_slots, "state_slots")
     if cu_tokens.numel() < S + 1 or state_slots.numel() < S or sum(query_lens) > T:
         raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: cu_tokens and state_slots must cover every request")
-    seg = int(segment) if segment else linrec_segment_tokens(query_lens, heads, dim, vdim, sm_count(q.device))
-    segs = max(1, -(-max(query_lens, default=1) // seg))
+    seg = int(segment) if segment else linrec_segment_tokens(query_lens, heads, linrec_segment_blocks(dim, vdim), sm_count(q.device))
+    pieces = [-(-n // seg) for n in query_lens]
+    cut = [n for n in pieces if n > 1]
+    segs = max(1, sum(pieces))
     code = LINREC_SEGMENT_MODES[mode]
     size = load_module("linrec_segments").photon_linrec_segments_scratch
-    size.restype, size.argtypes = c_long, [c_int] * 7
-    scratch = torch.empty(size(code, T, S, segs, heads, dim, vdim), dtype=torch.float32, device=q.device)
+    size.restype, size.argtypes = c_long, [c_int] * 9
+    scratch = torch.empty(size(code, T, S, segs, len(cut), sum(cut), heads, dim, vdim), dtype=torch.float32, device=q.device)
     den = torch.empty((T, heads), dtype=torch.float32, device=q.device) if mode == "matrix_memory" else None
     f = _fn("linrec_segments", "photon_linrec_segments",
             [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_long, c_void_p, c_void_p,
              c_void_p, c_float, c_float, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int,
-             c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(code, _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(a), a.stride(0) if a is not None else 0,
              _ptr(gate_a), _ptr(gate_b), gate_a.stride(0) if gate_a is not None else 0, _ptr(p0), _ptr(p1), _ptr(p2), float(cap),
              float(q_scale), _ptr(cu_tokens), _ptr(state_slots), _ptr(state), state.stride(0), state.shape[0], _ptr(out), out.stride(0),
-             _ptr(den), _ptr(scratch), T, S, heads, qk_heads, dim, vdim, seg, segs, _ptr(err), _stream()), "linrec_segments")
+             _ptr(den), _ptr(scratch), T, S, heads, qk_heads, dim, vdim, seg, segs, len(cut), sum(cut), _ptr(err), _stream()),
+           "linrec_segments")
     global _launch_count
-    _launch_count += (mode in ("state_space", "matrix_memory")) + (segs > 1)
+    _launch_count += (mode in ("state_space", "matrix_memory")) + (len(cut) > 0)
     return den
 
 

@@ -63,6 +63,36 @@ def test_weight_streaming_product_sizes():
     assert not ops.skinny_gemm_supported(torch.zeros(8, 2044, dtype=torch.bfloat16), torch.zeros(16, 2044, dtype=torch.bfloat16))
 
 
+def test_the_delta_rule_chooses_per_request():
+    """What a request is run by depends on its own tokens; the long requests of a step together say whether there is enough work."""
+    assert ops.delta_chunked_from(128, 128, [256] + [1] * 31, 32) == ops.DELTA_CHUNKED_MIN_TOKENS
+    assert ops.delta_chunked_from(128, 128, [64] + [1] * 200, 32) == 0           # the decoded tokens are no work for the chunks
+    assert ops.delta_chunked_from(128, 128, [63] * 100, 32) == 0
+    assert ops.delta_chunked_from(129, 128, [4096], 32) == 0 and ops.delta_chunked_from(128, 257, [4096], 32) == 0
+
+
+def test_segments_are_the_shortest_whose_long_requests_fit_at_once():
+    """.. whatever stands beside the long requests."""
+    import random
+    rng = random.Random(1)
+    for _ in range(2000):
+        longs = [rng.randint(128, 4096) for _ in range(rng.choice((1, 1, 2, 3, 5, 9)))]
+        heads, blocks = rng.choice((1, 2, 4, 8, 16, 32)), rng.choice((1, 2, 4))
+        places, seg = max(1, 296 // (heads * blocks)), ops.linrec_segment_tokens(longs, heads, blocks, 148)
+        cut = lambda n: sum(-(-x // n) for x in longs)
+        assert seg % 16 == 0 and seg >= 64
+        if places <= len(longs):
+            assert cut(seg) == len(longs)                # as many segments as requests: nothing is cut
+        else:
+            assert cut(seg) <= places and (seg == 64 or cut(seg - 16) > places)
+        others = [rng.randint(0, 127) for _ in range(rng.randint(0, 70))]
+        mixed = longs + others
+        rng.shuffle(mixed)
+        assert ops.linrec_segment_tokens(mixed, heads, blocks, 148) == seg
+    assert ops.linrec_segment_tokens([2048] + [1] * 63, 16, 2, 148) == 240
+    assert ops.linrec_segment_tokens([5, 90], 16, 2, 148) == 64
+
+
 def test_the_switch_of_dependent_launches_takes_every_word_for_off(tmp_path):
     """``PHOTON_PDL``: unset, empty and 1 leave the launches on, everything else turns them off."""
     import os

@@ -22,16 +22,24 @@ def _step(lens, slots=None):
                        error_flag=torch.zeros(4, dtype=torch.int32, device=DEV), host_state_slots=slots)
 
 
-@pytest.mark.parametrize("mixer,portion,others", [("delta", 520, 9), ("delta", 77, 40), ("delta", 2048, 3)])
+@pytest.mark.parametrize("mixer,portion,others", [("delta", 520, 9), ("delta", 77, 40), ("delta", 2048, 3), ("gla", 520, 9),
+                                                  ("gla", 1093, 40), ("mlstm", 520, 9), ("mlstm", 1093, 40), ("mamba2", 600, 9), ("mamba2", 1093, 40),
+                                                  ("hgrn2", 800, 0), ("hgrn2", 800, 9)])
 def test_a_portion_beside_decoded_tokens(mixer, portion, others):
     """The step that continuous batching runs, at the sizes of a real layer and above the sizes from which long portions have kernels
     of their own, against 64 bits."""
     from perf import cases
+    from photon_infer_b200.kernels import ops
+    lens, mode = [portion] + [1] * others, {"gla": "decay_rows", "mlstm": "matrix_memory", "mamba2": "state_space", "hgrn2": "forget_write"}.get(mixer)
+    if mode:
+        assert ops.linrec_segments_supported(mode, 128, lens, 16) == (mixer != "hgrn2" or not others)
     case = dict(kind="mixer", mixer=mixer, width=2048, requests=1 + others, new=1, context=512, ragged=False, dtype="bf16", portion=portion)
     got = cases.run(cases.prepare(case, 3))
     want, limit = cases.exact(case, 3), cases.tolerance(case)
     for x, y in zip(got, want):
         assert _rel(x.reshape(y.shape), y) < limit["rel"]
+        if not others:
+            continue
         short = slice(portion, None) if x.dim() == 2 and x.shape[0] == portion + others else slice(1, None)
         assert _rel(x.reshape(y.shape)[short], y[short]) < limit["rel"]
 
@@ -64,13 +72,53 @@ def test_delta_rule_chooses_per_request(lens, monkeypatch):
         assert torch.equal(got[0][rows], want[0][rows]) and torch.equal(got[1][s], want[1][s]), (s, n)
 
 
-def test_recurrent_parts_choose_per_request():
-    """The rules: what a request is run by depends on its own tokens; the others of the step only say whether there is enough work."""
+@pytest.mark.parametrize("mode", ["state_space", "matrix_memory", "forget_write", "decay_rows"])
+@pytest.mark.parametrize("lens", [[300, 1, 1, 128, 1], [1, 64, 1, 0, 65], [1] * 33 + [128] + [1] * 33 + [200, 129], [128], [1, 2, 64], [127, 700]])
+def test_segments_of_a_request_do_not_depend_on_the_others(mode, lens):
+    """Outputs, state and divisors of every request have the bits that they have when it is alone, at any place of the step."""
     from photon_infer_b200.kernels import ops
-    assert ops.delta_chunked_from(128, 128, [256] + [1] * 31, 32) == ops.DELTA_CHUNKED_MIN_TOKENS
-    assert ops.delta_chunked_from(128, 128, [64] + [1] * 200, 32) == 0           # the decoded tokens are no work for the chunks
-    assert ops.delta_chunked_from(128, 128, [63] * 100, 32) == 0
-    assert ops.delta_chunked_from(129, 128, [4096], 32) == 0 and ops.delta_chunked_from(128, 257, [4096], 32) == 0
+    torch.manual_seed(len(lens))
+    H, N, dv, T, S = 4, 64, 40, sum(lens), len(lens)
+    memory, rows = mode == "matrix_memory", mode in ("forget_write", "decay_rows")
+    g = torch.randn(T, 2 * H, device=DEV)
+    x = [torch.randn(T, H * N, device=DEV), torch.rand(T, H * N, device=DEV), torch.randn(T, H * dv, device=DEV),
+         torch.rand(T, H * N, device=DEV).sqrt() if mode == "decay_rows" else None, None if rows else g[:, :H], g[:, H:] if memory else None]
+    p = [None if rows else torch.zeros(H, device=DEV), None if rows else torch.zeros(H, device=DEV), torch.ones(H, device=DEV) if mode == "state_space" else None]
+    start, cu = torch.rand(S, H * N * dv + (H * N + H if memory else 0), device=DEV), [sum(lens[:s]) for s in range(S + 1)]
+
+    def run(at, lens_, slots):
+        o, s = torch.full((at.stop - at.start, H * dv), 7.0, device=DEV), start.clone()
+        den = ops.linrec_segments(mode, *(None if t is None else t[at] for t in x), *p, 5.0 if memory else 0.0, 0.1,
+                                  i32([sum(lens_[:i]) for i in range(len(lens_) + 1)]), i32(slots), s, o, lens_, H, H, N, dv, None, segment=64)
+        return o, s, den
+    whole = run(slice(0, T), lens, list(range(S)))
+    for s, n in enumerate(lens):
+        at = slice(cu[s], cu[s + 1])
+        if n == 0:
+            assert torch.equal(whole[1][s], start[s])
+            continue
+        alone = run(at, [n], [s])
+        assert torch.equal(whole[0][at], alone[0]) and torch.equal(whole[1][s], alone[1][s]), (s, n)
+        assert not memory or torch.equal(whole[2][at], alone[2])
+
+
+def test_division_beside_a_norm_of_odd_parts(monkeypatch):
+    """The matrix memory's heads of 30 numbers, whose norm does not divide: segments against token by token."""
+    from photon_infer_b200.kernels import ops
+    from photon_infer_b200.parts.matrix_memory import MatrixMemoryMixer
+    torch.manual_seed(0)
+    H, dim, dv, lens = 16, 32, 30, [500, 1, 3]
+    mixer = MatrixMemoryMixer(256, H, dim, dv, 15.0, 1e-5)
+    mixer.load({s.name: (1.0 + 0.1 * torch.randn(s.concrete_shape(), device=DEV) if s.init == "norm" else 0.1 * torch.randn(s.concrete_shape(), device=DEV))
+                .bfloat16() for s in mixer.tensor_specs()})
+    h = torch.randn(sum(lens), 256, device=DEV).bfloat16()
+    outs = []
+    for least in (7000, 10 ** 9):
+        monkeypatch.setitem(ops.LINREC_SEGMENTS_FROM, "matrix_memory", least)
+        assert ops.linrec_segments_supported("matrix_memory", dim, lens, H) == (least == 7000)
+        state = torch.zeros(3, *mixer.state_spec().shape, device=DEV)
+        outs.append((mixer.forward(h, _step(lens), LayerCache(state=state)), state))
+    assert _rel(outs[0][0], outs[1][0]) < 2e-3 and _rel(outs[0][1], outs[1][1]) < 5e-6     # a bfloat16 product behind 32-bit sums
 
 
 def _rel(x, y):
