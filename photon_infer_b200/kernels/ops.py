@@ -1835,6 +1835,13 @@ def linrec_segments_supported(mode: str, dim: int, query_lens, heads: int) -> bo
     return sum(query_lens) * heads >= LINREC_SEGMENTS_FROM[mode]
 
 
+#: Where the other requests of a step fill the GPU, a portion is done beside them, and its cut would only add a pass: up to this many tokens
+#: for every round of their blocks.  us, not cut first, 32 heads, 63 decoded tokens (14 rounds), state space 256 tokens 242 and 279, 512 306 and
+#: 337, 640 364 and 374, 768 408 and 393; 31 decoded tokens, gated linear attention 256 tokens 206 and 228, 400 259 and 260, 512 321 and 300;
+#: 16 heads, 63 decoded tokens, matrix memory 400 tokens 206 and 176.
+LINREC_SEGMENTS_BESIDE = 45
+
+
 def linrec_segment_blocks(dim: int, vdim: int) -> int:
     """Blocks of one (segment, head)."""
     return int(load_module("linrec_segments").photon_linrec_segment_blocks(dim, vdim))
@@ -1844,12 +1851,13 @@ def linrec_segment_tokens(query_lens, heads: int, blocks: int, sms: int) -> int:
     """Tokens of a segment, a multiple of 16: the fewest with which the segments of the step's long requests (at least 128 tokens, or
     the longest) fit the GPU at once at two blocks a streaming multiprocessor (one block more would wait for a whole segment), but no fewer
     than 64 (every segment but the first costs a pass over its tokens without queries and a fold of its end state).  The others are
-    done within a segment's time and take no place.  The longest request's tokens where there are no more places than long requests."""
+    done within a segment's time and take no place.  The longest request's tokens where there are no more places than long requests, or where the
+    others take as long as it does."""
     longest = max(query_lens)
     longs = [n for n in query_lens if n >= LINREC_SEGMENTS_MIN_TOKENS] or [longest]
     places, total = max(1, 2 * sms // (heads * blocks)), sum(longs)
     whole = max(4, -(-longest // 16))
-    if places <= len(longs):
+    if places <= len(longs) or longest * 2 * sms <= LINREC_SEGMENTS_BESIDE * (len(query_lens) - len(longs)) * heads * blocks:
         return whole * 16
     # fewer sixteens than `low` cannot fit; `high` fits, since a request's last segment is less than one above its share
     low, high = max(4, -(-total // (16 * places))), max(4, min(whole, -(-total // (16 * (places - len(longs))))))
