@@ -62,3 +62,20 @@ def test_router_of_many_tokens(T, H, E, gate, scoring):
     assert torch.equal(counts.cpu().long(), torch.bincount(ids.flatten().long().cpu(), minlength=E))
     if gate:
         assert float((got[3].double().flatten() - torch.sigmoid(h.double() @ wsg[0].double())).abs().max()) < 2e-5
+
+
+@pytest.mark.parametrize("T,H,E,shift", [(2048, 2048, 16, 0.0), (1024, 4096, 16, 0.0), (8192, 512, 64, 0.0), (2048, 2048, 32, 0.5), (16384, 256, 8, 0.0)])
+def test_router_of_many_tokens_is_as_exact_as_that_of_few(T, H, E, shift):
+    """The same tokens in one step, whose logits the tensor cores form, and in steps too small for that: the error against 64 bits
+    (root mean square) is no larger.  All experts are chosen, so that every logit shows in a weight."""
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(T + E)
+    h, wr = (torch.randn(T, H, device=DEV) + shift).bfloat16(), (torch.randn(E, H, device=DEV) * H ** -0.5).bfloat16()
+    b = torch.randn(E, device=DEV) * 0.1
+    many = ops.moe_route(h, wr, b, E, "sigmoid")
+    few = [ops.moe_route(p, wr, b, E, "sigmoid") for p in h.split(T // 2)]
+    want = torch.sigmoid(h.double() @ wr.double().t() + b.double())
+    error = lambda ids, weights: float((weights.double() - want.gather(1, ids.long())).pow(2).mean().sqrt())
+    e = error(many[0], many[1]), error(torch.cat([f[0] for f in few]), torch.cat([f[1] for f in few]))
+    print("errors of many and of few:", e)
+    assert e[0] <= 1.02 * e[1], e
