@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) moe_route_kernel(const 
 // square; the kernel above in brackets): 2,048 x 2,048, 16 experts 2.60e-8 (2.75e-8), 1,024 x 4,096 2.82e-8 (2.93e-8), 8,192 x 512, 64
 // experts 2.40e-8 (2.52e-8), 16,384 x 256, 8 experts 2.30e-8 (2.43e-8).
 #define MOE_ROUTE_MANY 16
-#define MOE_MANY_FROM 4000000L
+#define MOE_MANY_FROM 2800000L
 template <int NT>
 __global__ void __launch_bounds__(256)
 moe_route_many_kernel(const bf16* __restrict__ h, long h_stride, const bf16* __restrict__ Wr, const void* __restrict__ bias, int bias_bf16,
@@ -368,8 +368,9 @@ PHOTON_API int photon_moe_route_ex(const void* h, long h_stride, int dtype, cons
   // 64 outputs are what a warp's registers hold; rows that its 16-byte loads cannot read, other types and logits that were formed
   // before go to the kernel above
   const int tiles = (E + (Wsg ? 1 : 0) + 7) / 8;
-  // .. and so do fewer numbers than MOE_MANY_FROM, whose few blocks of 16 tokens take as long as many (a routed feed-forward of 16 experts,
-  // us, that kernel first: 1,200 tokens x 2,048 217 and 226, 2,048 x 2,048 294 and 286, 1,200 x 4,096 600 and 588)
+  // .. and so do fewer numbers than MOE_MANY_FROM, whose few blocks of 16 tokens take as long as many.  A routed feed-forward of 16 experts,
+  // us, that kernel first: 1,000 tokens x 2,048 220 and 222, 1,200 218 and 219, 1,400 205 and 200, 1,600 215 and 197, 1,800 226 and 209, 2,048
+  // 253 and 243; 700 x 4,096 500 and 500, 900 543 and 539, 1,200 586 and 571
   if (!few && (long)T_ * H >= MOE_MANY_FROM && dtype == PHOTON_BF16 && logits == nullptr && tiles <= 8 && H % 32 == 0 && h_stride % 8 == 0 && ((uintptr_t)h & 15) == 0 &&
       ((uintptr_t)Wr & 15) == 0 && ((uintptr_t)Wsg & 15) == 0) {
     const int nt = tiles <= 2 ? 2 : tiles <= 3 ? 3 : tiles <= 4 ? 4 : 8;
