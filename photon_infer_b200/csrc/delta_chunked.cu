@@ -30,7 +30,8 @@
 // barrier a chunk.
 //
 // Measured, 2,048 tokens, 16 heads of 128 x 128: prep 52 us, walk 176 us, against 616 us for the token-by-token kernel, whose chain
-// from one token to the next is 300 ns; 64 tokens 10 + 8 us against 22 us and more for its walk.  The error against 64 bits is
+// from one token to the next is 300 ns (the look for outputs that are not finite came later: a mixer's step of these tokens 340 -> 355 us);
+// 64 tokens 10 + 8 us against 22 us and more for its walk.  The error against 64 bits is
 // 2.4e-7 (outputs) and 1.8e-7 (state) where the token-by-token kernel has 2.6e-7 and 2.1e-7.
 // What bounds the prep: its blocks' loads and stores (100 MB, 15 us of them) and the gaps between a block's steps; with the keys and queries
 // read 4 bytes at a time in turn, and the values only when the substitution asks for them, it took 103 us.  Three or four blocks an SM

@@ -34,7 +34,9 @@
 // warps at 16 heads of 128 x 128; the portion is cut into as many segments as give the GPU LS_BLOCKS_PER_SM blocks an SM.
 // Measured, heads of 128 x 128 (gates, both passes): state space, 16 heads, 2,048 tokens 379 -> 153 us; matrix memory, two requests of
 // 2,815 tokens 411 -> 234 us; forget and write 240 -> 155 us (777 tokens 94 -> 77 us); gated linear attention 416 us (chunks of
-// 32 tokens joined by a scan) -> 156 us and 37 us for its inputs.  Half of the time is the FP32 pipe; the rest is the barriers of a
+// 32 tokens joined by a scan) -> 156 us and 37 us for its inputs.  That was before decays near 1 were carried by what they lack to
+// 1, which takes 3 to 7 % of a mixer's step (2,048 tokens of 16 heads: gated linear attention 281 -> 300 us, state space 277 -> 284;
+// two requests of 2,815, matrix memory 365 -> 380; 777 tokens, forget and write 136 -> 143).  Half of the time is the FP32 pipe; the rest is the barriers of a
 // chunk, the folds and the blocks' start, which two or three blocks an SM hide equally (100 us either way for the second pass).
 #include "linrec.cuh"
 #include "portions.cuh"

@@ -1822,7 +1822,7 @@ LINREC_SEGMENT_MODES = {"state_space": 0, "matrix_memory": 1, "forget_write": 2,
 #: tokens, and the segments' additional launches and second pass cost more than they save.  B200, heads of 128 x 128, a mixer's
 #: step, us, without segments first: gated linear attention 300 tokens x 16 heads 139 and 148, 3 x 130 x 16 250 and 148; matrix
 #: memory 3 x 130 x 16 105 and 132, 500 x 16 161 and 131; state space 500 x 16 151 and 154, 300 x 32 168 and 157.
-#: Forget and write: 600 x 16 146 and 149, 850 x 16 165 and 145, 2,000 x 16 332 and 245; its one-pass kernel fills the GPU from 32 (request,
+#: Forget and write: 600 x 16 123 and 130, 640 x 16 127 and 130, 720 x 16 139 and 133, 800 x 16 153 and 144, 2,048 x 16 332 and 264; its one-pass kernel fills the GPU from 32 (request,
 #: head) pairs on: 2 x 700 x 16 187 and 197, 2,000 x 32 574 and 557, 2 x 1,400 x 32 722 and 755.
 LINREC_SEGMENTS_FROM = {"decay_rows": 6000, "matrix_memory": 7000, "state_space": 9000, "forget_write": 12000}
 
