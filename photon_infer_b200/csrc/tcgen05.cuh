@@ -7,6 +7,15 @@
 #define TC_WAIT_LIMIT (1u << 20)
 #endif
 
+// One lane of a warp that is here as a whole; the rest of the role's loop (waits too) is run by all lanes, and what one thread
+// issues stands in `if (elected)`.  Behind `lane == 0` instead the compiler cannot know that one thread is left and
+// serialises over the lanes that might be: a product then takes its thread 45 cycles instead of 9, a wait for a barrier that is ready
+// 206 instead of 72 (N = 16; measured with nothing else in the loop).
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t e;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void tc_mbar_init(uint64_t* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(bar)), "r"(count));

@@ -502,6 +502,14 @@ PHOTON_EXPORT int photon_attention_decode(const void* q, long q_stride, void* ou
 PHOTON_EXPORT int photon_sgemm_nt(const float* A, long lda, const float* W, long ldw, float* C, long ldc, int M, int N, int K,
                     cudaStream_t stream);
 
+/* ------------------------------------------------------------------ gemm_f32_tc.cu: 32-bit product as tensor-core products of
+ * bfloat16 parts.  W: 16-byte aligned, K % 4 == 0, ldw % 4 == 0; A, C: any row stride.  one_launch (M <= 16): one kernel and
+ * no scratch, for calls whose launches the host pays for; else scratch: 16-byte aligned, at least photon_sgemm_tc_scratch(M, N, K)
+ * bytes, written before it is read.  The same bits either way. */
+PHOTON_EXPORT long photon_sgemm_tc_scratch(int M, int N, int K);
+PHOTON_EXPORT int photon_sgemm_tc(const float* A, long lda, const float* W, long ldw, float* C, long ldc, int M, int N, int K,
+                    int one_launch, void* scratch, long scratch_bytes, int* err, cudaStream_t stream);
+
 /* ------------------------------------------------------------------ gemm_skinny.cu: bfloat16, M <= 64 (32 with SwiGLU) */
 /* epilogue 0: bfloat16 out; 1: float out; 2: SwiGLU (W = [gate rows; up rows], out [M, N / 2]).  K % 8 == 0,
  * 16-byte aligned rows.  scratch (float) and tickets (int, zero between launches) serve the split of K; launches

@@ -77,13 +77,13 @@ def _check(status: int, what: str) -> None:
 _sigs_done = set()
 
 
-def _fn(module: str, name: str, argtypes, defines=None):
+def _fn(module: str, name: str, argtypes, defines=None, restype=c_int):
     lib = load_module(module, defines)
     f = getattr(lib, name)
     key = (id(lib), name)
     if key not in _sigs_done:
         f.argtypes = argtypes
-        f.restype = c_int
+        f.restype = restype
         _sigs_done.add(key)
     return f
 
@@ -1048,9 +1048,47 @@ def gemm_tc_qkv(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, posit
              k_cache.shape[2], k_cache.shape[0] * k_cache.shape[2], _ptr(err), _stream()), "gemm_tc_qkv")
 
 
+SGEMM_TC_MIN = 1024         # rows and columns of a 32-bit weight, and
+SGEMM_TC_SIZE = 1 << 22     # numbers in it, from which its products run on the tensor cores
+
+
+def sgemm_tc_supported(weight: torch.Tensor) -> bool:
+    """Whether 32-bit products with this weight are sums of tensor-core products (``gemm_f32_tc.cu``).  The weight alone
+    decides, never the rows that meet it: one row has the bits that it has among many."""
+    N, K = weight.shape
+    return min(N, K) >= SGEMM_TC_MIN and N * K >= SGEMM_TC_SIZE and K % 4 == 0 and weight.data_ptr() % 16 == 0
+
+
+def sgemm_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, err: Optional[torch.Tensor] = None) -> None:
+    """``out = x @ weight^T`` in 32-bit accuracy, each number split into three bfloat16 parts whose products run on the
+    tcgen05 tensor cores.  float32 ``x [M, K]`` and ``out [M, N]`` with any row stride, ``weight`` contiguous with K a
+    multiple of 4 and a 16-byte aligned base."""
+    _cuda(x, weight, out, err)
+    M, K = x.shape
+    N = weight.shape[0]
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or out.dtype != torch.float32:
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, "sgemm_tc: float32 operands and output")
+    if weight.shape[1] != K or out.shape != (M, N) or x.stride(1) != 1 or out.stride(1) != 1 or not weight.is_contiguous():
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"sgemm_tc: x [M, {K}] against weight {tuple(weight.shape)}")
+    if err is None:
+        err = _error_word(x.device)
+    # few rows: one launch where the host would feel three, the faster three in a captured step and where the GPU takes longer
+    # than the host (one row against 128,256 x 2,048: 262 us in one launch); the same bits
+    one_launch = M <= 16 and N * K <= 1 << 25 and not torch.cuda.is_current_stream_capturing()
+    n, scratch = 0, None
+    if not one_launch:
+        n = _fn("gemm_f32_tc", "photon_sgemm_tc_scratch", [c_int, c_int, c_int], restype=c_long)(M, N, K)
+        scratch = torch.empty((n,), dtype=torch.uint8, device=x.device)
+    f = _fn("gemm_f32_tc", "photon_sgemm_tc",
+            [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p])
+    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, int(one_launch), _ptr(scratch), n,
+             _ptr(err), _stream()), "sgemm_tc")
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``x [M, K] @ weight[N, K]^T``.  float32: this package's FMA kernel (true 32-bit).
+    """``x [M, K] @ weight[N, K]^T``.  float32: this package's own kernels in 32-bit accuracy (weights of
+    1,024 x 1,024 and more as sums of tensor-core products, others as chains of multiply-adds).
     bfloat16: up to 8 rows the weight-streaming kernel; with enough 128 x 256 tiles to fill the
     GPU the tcgen05 kernel; in between the library product (cuBLAS through torch), where the
     reference's engine also calls the library (src/ops/kernels/cuda/matmul_dequant_cached.cu:193-207)."""
@@ -1078,6 +1116,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
             raise PhotonError(ErrorCode.INVALID_ARGUMENT, "linear: a float32 product gives float32")
         if out is None:
             out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+        if sgemm_tc_supported(weight):
+            sgemm_tc(x, weight, out)
+            return out
         f = _fn("gemm_f32", "photon_sgemm_nt",
                 [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int, c_void_p])
         _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, _stream()),

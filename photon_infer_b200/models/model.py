@@ -135,7 +135,7 @@ class CausalLM:
         """What this model launches in this dtype: module names and (name, definitions) pairs."""
         mods: List[object] = ["elementwise", "sampling"] + (["row_norms"] if self.spec.logit_softcap is not None else [])
         if self.dtype == torch.float32:
-            mods.append("gemm_f32")
+            mods += ["gemm_f32", "gemm_f32_tc"]
         for _, part in self._skeleton.named_parts():
             for m in part.required_kernels(self.dtype):
                 if m not in mods:
