@@ -12,8 +12,8 @@
 //
 // Keys and values come by TMA: one 2-D box per page part (16 keys x 64 features with pages of 16), 128-byte
 // swizzle, into a ring of stages, completion on an mbarrier.  Four producer warps (they give their registers
-// to the others with setmaxnreg) issue a page part each, because a TMA instruction costs its thread 150 to 200
-// cycles and a tile is eight or sixteen of them; one of them draws the items and hands them to the consumers
+// to the others with setmaxnreg) issue a page part each, because a tile is eight or sixteen such copies
+// (an elected lane of each warp issues); one of them draws the items and hands them to the consumers
 // through a small queue.  (The 2,048 cp.async instructions with their address arithmetic that a tile costs in
 // attention_flash.cu made that kernel issue-bound: 47 % of all issue slots at 18 % occupancy.)  The four
 // consumer warps take 16 keys of every tile each: scores and weighted sums as mma.m16n8k16 with fragments read
@@ -349,13 +349,14 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   const int nprod = parts < 4 ? parts : 4;                       // producer warps with work
   if (warp >= 4) {
     // ------------------------------------------------------------------ producers: Q rows and K/V tiles by TMA
-    // A TMA instruction costs its issuing thread some 150 to 200 cycles, and a tile of 64 keys in pages of 16 is
-    // 8 or 16 of them: one issuing thread would bound the block at 18 GB/s.  Four warps issue a page part each.
+    // Four warps issue a page part each of a tile's 8 or 16 copies (pages of 16); each warp waits as a whole and an elected lane
+    // issues (behind `lane == 0` a copy cost its thread 150 to 200 cycles; a layer's decode step of 56 requests 139 us, now 133).
     // They give most of their registers to the consumers.
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     const int pw = warp - 4;
     if (pw >= nprod) return;
     const bool leader = pw == 0;                                 // draws the items and brings Q
+    const bool elected = tc_elect();
     const int ppw = (parts + 3) / 4;                             // parts of this warp per tile: pw, pw + 4
     uint32_t n = 0;                                              // tiles issued so far: stage and parity follow
     uint32_t items = 0;
@@ -421,11 +422,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           if (page >= 0 && page < P.num_pages) rowc[pp] = (page * P.n_kv + it.g) * P.page_size + (key % P.page_size);
           else if (page != -2 && lane == 0) report_error(P.err, PHOTON_DEV_BAD_PAGE, it.tok0, key, page);
         }
-        if (lane == 0) {
-          AD_T(const long long t0 = clock64();)
-          ok = tc_wait(&empty_bar[s], ((n / AD_STAGES) & 1u) ^ 1u, &abort_flag) ? 1 : 0;
-          AD_T(t_wait += clock64() - t0;)
-          if (ok) {
+        AD_T(const long long t0 = clock64();)
+        ok = __all_sync(0xffffffffu, tc_wait(&empty_bar[s], ((n / AD_STAGES) & 1u) ^ 1u, &abort_flag));
+        AD_T(t_wait += clock64() - t0;)
+        if (!ok) break;
+        if (elected) {
             tc_mbar_expect_tx(&full_bar[s], (uint32_t)(ppw * P.box_rows * 128 * AD_DH * 2));
             for (int pp = 0; pp < ppw; ++pp) {
               unsigned char* kst = ring + (size_t)s * AD_STAGE_BYTES + (pw + 4 * pp) * P.box_rows * 128;
@@ -434,10 +435,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
               for (int h = 0; h < AD_DH; ++h) tc_tma_load(kst + AD_KV_BYTES + h * AD_HALF_BYTES, &map_v, h * 64, rowc[pp], &full_bar[s]);
             }
-          }
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
       }
       if (!ok) break;
     }

@@ -103,7 +103,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tc_mbar_init(q_full, 1);
     for (int s = 0; s < LT_KST; ++s) { tc_mbar_init(&k_full[s], 1); tc_mbar_init(&k_empty[s], 1); }
@@ -123,11 +123,12 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
   pdl_wait();                                       // queries, keys and values come from the kernels before
 
   if (warp == 8) {
-    // ---------------- producer
-    if (lane == 0) {
-      tc_mbar_expect_tx(q_full, 2 * LT_Q_BYTES);
+    // ---------------- producer: the warp waits, one of its lanes issues
+    const bool elected = tc_elect();
+    {
+      if (elected) tc_mbar_expect_tx(q_full, 2 * LT_Q_BYTES);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
+      for (int j = 0; j < 2 && elected; ++j) {
         unsigned char* qt = q_s + j * LT_Q_BYTES;
         const int t = q.tok0 + t0 + j * LT_ROWS;
 #pragma unroll
@@ -141,11 +142,13 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
         if (!tc_wait(&k_empty[s], ((kn / LT_KST) & 1) ^ 1, abort_flag)) return false;
         unsigned char* dst = k_s + s * LT_K_BYTES;
         const int row = row_lo + kn * LT_KT;
-        tc_mbar_expect_tx(&k_full[s], LT_K_BYTES);
+        if (elected) {
+          tc_mbar_expect_tx(&k_full[s], LT_K_BYTES);
 #pragma unroll
-        for (int c = 0; c < LT_NU; ++c) tc_tma_load3(dst + c * (LT_KT * 128), &map_ku, c * 64, head, row, &k_full[s]);
+          for (int c = 0; c < LT_NU; ++c) tc_tma_load3(dst + c * (LT_KT * 128), &map_ku, c * 64, head, row, &k_full[s]);
 #pragma unroll
-        for (int c = 0; c < LT_NR; ++c) tc_tma_load(dst + (LT_NU + c) * (LT_KT * 128), &map_kr, c * 64, row, &k_full[s]);
+          for (int c = 0; c < LT_NR; ++c) tc_tma_load(dst + (LT_NU + c) * (LT_KT * 128), &map_kr, c * 64, row, &k_full[s]);
+        }
         ++kn;
         return true;
       };
@@ -154,9 +157,11 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
         if (!tc_wait(&v_empty[s], ((vn / LT_VST) & 1) ^ 1, abort_flag)) return false;
         unsigned char* dst = v_s + s * LT_V_BYTES;
         const int row = row_lo + vn * LT_VH;
-        tc_mbar_expect_tx(&v_full[s], LT_V_BYTES);
+        if (elected) {
+          tc_mbar_expect_tx(&v_full[s], LT_V_BYTES);
 #pragma unroll
-        for (int c = 0; c < LT_NV; ++c) tc_tma_load3(dst + c * (LT_VH * 128), &map_v, c * 64, head, row, &v_full[s]);
+          for (int c = 0; c < LT_NV; ++c) tc_tma_load3(dst + c * (LT_VH * 128), &map_v, c * 64, head, row, &v_full[s]);
+        }
         ++vn;
         return true;
       };
@@ -167,7 +172,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
         ok = load_v() && load_v();
         if (ok && kn < ntiles) ok = load_k();
       }
-      if (*abort_flag) {
+      if (elected && *abort_flag) {
         // copies already issued still write into this block's shared memory: wait for them, bounded
         for (uint32_t w = 0; w < TC_WAIT_LIMIT && !tc_mbar_try(q_full, 0); ++w) {}
         for (int n = (kn > LT_KST ? kn - LT_KST : 0); n < kn; ++n)
@@ -177,8 +182,9 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
       }
     }
   } else if (warp == 9) {
-    // ---------------- MMA issuer
-    if (lane == 0) {
+    // ---------------- MMA issuer: the warp waits, one of its lanes issues
+    const bool elected = tc_elect();
+    {
       const uint32_t idesc_s = tc_idesc(LT_ROWS, LT_KT);
       const uint32_t idesc_o = tc_idesc(LT_ROWS, 64 * LT_NV) | TC_IDESC_B_MN;
       // the scores of key tile i for query tile j; the second query tile is the last to read the keys
@@ -186,6 +192,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
         const int s = i % LT_KST;
         if (!tc_wait(&k_full[s], (i / LT_KST) & 1, abort_flag)) return false;
         tc_fence_after();
+        if (!elected) return true;
         const uint32_t q_addr = tc_smem(q_s + j * LT_Q_BYTES), k_addr = tc_smem(k_s + s * LT_K_BYTES);
 #pragma unroll
         for (int kk = 0; kk < LT_NK * 4; ++kk)
@@ -205,6 +212,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
             const int n = 2 * i + half, s = n % LT_VST;
             if (!tc_wait(&v_full[s], (n / LT_VST) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
+            if (!elected) continue;
             const uint32_t v_addr = tc_smem(v_s + s * LT_V_BYTES);
 #pragma unroll
             for (int kk = 0; kk < LT_VH / 16; ++kk)  // P: 8 columns of packed pairs per 16 keys
@@ -213,7 +221,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __g
             if (j == 1) tc_commit(&v_empty[s]);
           }
           if (!ok) break;
-          tc_commit(&pv_done[j]);
+          if (elected) tc_commit(&pv_done[j]);
           // the next scores go where this tile's P was; the tensor core runs the products in the order of issue
           if (i + 1 < ntiles) ok = issue_scores(i + 1, j);
         }

@@ -172,7 +172,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tc_mbar_init(q_full, 1);
     for (int s = 0; s < AT_STAGES; ++s) { tc_mbar_init(&k_full[s], 1); tc_mbar_init(&v_full[s], 1); tc_mbar_init(&kv_empty[s], 1); }
@@ -191,7 +191,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (warp == 4) {
     // ---------------- producer
-    if (lane == 0) {
+    const bool elected = tc_elect();
+    if (elected) {
       tc_mbar_expect_tx(q_full, P.tile_rows * 128 * AT_DH);       // rows beyond tile_rows stay as they are: nobody uses them
 #pragma unroll
       for (int h = 0; h < AT_DH; ++h)
@@ -213,23 +214,22 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           else rowc = (page * P.n_kv + g) * P.page_size + slot;
         }
       }
-      int ok = 1;
-      if (lane == 0) ok = tc_wait(&kv_empty[s], ((i / AT_STAGES) & 1) ^ 1, abort_flag) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      if (lane == 0) { tc_mbar_expect_tx(&k_full[s], AT_K_BYTES); tc_mbar_expect_tx(&v_full[s], AT_V_BYTES); }
-      __syncwarp();
-      if (lane < boxes) {
-        unsigned char* kst = kv_s + s * AT_STAGE_BYTES + lane * P.box_rows * 128;
-        unsigned char* vst = kst + AT_K_BYTES;
+      if (!__all_sync(0xffffffffu, tc_wait(&kv_empty[s], ((i / AT_STAGES) & 1) ^ 1, abort_flag))) break;
+      if (elected) { tc_mbar_expect_tx(&k_full[s], AT_K_BYTES); tc_mbar_expect_tx(&v_full[s], AT_V_BYTES); }
+      // one thread issues all parts: the lanes that know their pages would be served one by one, and slower
+      unsigned char* kst = kv_s + s * AT_STAGE_BYTES;
+      for (int part = 0; part < boxes; ++part, kst += P.box_rows * 128) {
+        const int row = __shfl_sync(0xffffffffu, rowc, part);
+        if (elected) {
 #pragma unroll
-        for (int h = 0; h < AT_DH; ++h) tc_tma_load(kst + h * AT_HALF_BYTES, &map_k, h * 64, rowc, &k_full[s]);
+          for (int h = 0; h < AT_DH; ++h) tc_tma_load(kst + h * AT_HALF_BYTES, &map_k, h * 64, row, &k_full[s]);
 #pragma unroll
-        for (int h = 0; h < AT_VH; ++h) tc_tma_load(vst + h * AT_HALF_BYTES, &map_v, h * 64, rowc, &v_full[s]);
+          for (int h = 0; h < AT_VH; ++h) tc_tma_load(kst + AT_K_BYTES + h * AT_HALF_BYTES, &map_v, h * 64, row, &v_full[s]);
+        }
       }
       issued = i + 1;
     }
-    if (lane == 0 && *abort_flag) {
+    if (elected && *abort_flag) {
       // copies already issued still write into this block's shared memory: wait for them, bounded
       for (uint32_t w = 0; w < TC_WAIT_LIMIT && !tc_mbar_try(q_full, 0); ++w) {}
       for (int j = (issued > AT_STAGES ? issued - AT_STAGES : 0); j < issued; ++j) {
@@ -238,8 +238,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
   } else if (warp == 5) {
-    // ---------------- MMA issuer
-    if (lane == 0) {
+    // ---------------- MMA issuer: the warp waits, one of its lanes issues
+    const bool elected = tc_elect();
+    {
       const uint32_t idesc_s = tc_idesc(AT_ROWS, AT_KT);
       const uint32_t idesc_o = tc_idesc(AT_ROWS, 64 * AT_VH) | TC_IDESC_B_MN;
       const uint32_t q_addr = tc_smem(q_s);
@@ -247,12 +248,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int s = i % AT_STAGES;
         if (!tc_wait(&k_full[s], (i / AT_STAGES) & 1, abort_flag)) return false;
         tc_fence_after();
-        const uint32_t k_addr = tc_smem(kv_s + s * AT_STAGE_BYTES);
+        if (elected) {
+          const uint32_t k_addr = tc_smem(kv_s + s * AT_STAGE_BYTES);
 #pragma unroll
-        for (int kk = 0; kk < (HEAD_DIM + 15) / 16; ++kk)
-          tc_mma(tmem_base + (i % AT_NBUF) * AT_KT, tc_desc(q_addr + (kk >> 2) * (AT_ROWS * 128) + (kk & 3) * 32),
-                 tc_desc(k_addr + (kk >> 2) * AT_HALF_BYTES + (kk & 3) * 32), idesc_s, kk > 0 ? 1u : 0u);
-        tc_commit(&s_full[i % AT_NBUF]);
+          for (int kk = 0; kk < (HEAD_DIM + 15) / 16; ++kk)
+            tc_mma(tmem_base + (i % AT_NBUF) * AT_KT, tc_desc(q_addr + (kk >> 2) * (AT_ROWS * 128) + (kk & 3) * 32),
+                   tc_desc(k_addr + (kk >> 2) * AT_HALF_BYTES + (kk & 3) * 32), idesc_s, kk > 0 ? 1u : 0u);
+          tc_commit(&s_full[i % AT_NBUF]);
+        }
         return true;
       };
       bool ok = tc_wait(q_full, 0, abort_flag);
@@ -265,19 +268,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (!tc_wait(&p_full[i % AT_NBUF], (i / AT_NBUF) & 1, abort_flag)) { ok = false; break; }
         if (!tc_wait(&v_full[s], (i / AT_STAGES) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t p_addr = tc_smem(p_s + (i & 1) * AT_P_BYTES);
-        const uint32_t v_addr = tc_smem(kv_s + s * AT_STAGE_BYTES + AT_K_BYTES);
+        if (elected) {
+          const uint32_t p_addr = tc_smem(p_s + (i & 1) * AT_P_BYTES);
+          const uint32_t v_addr = tc_smem(kv_s + s * AT_STAGE_BYTES + AT_K_BYTES);
 #pragma unroll
-        for (int kk = 0; kk < AT_KT / 16; ++kk) {  // 16 keys: two groups of 8 rows of V
-          if (AT_P_TMEM)                           // P: 8 columns of packed pairs per 16 keys, where the tile's scores were
-            at_mma_ts(tmem_base + AT_O_COL, tmem_base + (i % AT_NBUF) * AT_KT + kk * 8, tc_desc_mn(v_addr + kk * 2048, AT_HALF_BYTES, 1024),
-                      idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
-          else                                     // P: 32 bytes along a row of the swizzled tile in shared memory
-            tc_mma(tmem_base + AT_O_COL, tc_desc(p_addr + kk * 32), tc_desc_mn(v_addr + kk * 2048, AT_HALF_BYTES, 1024),
-                   idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < AT_KT / 16; ++kk) {  // 16 keys: two groups of 8 rows of V
+            if (AT_P_TMEM)                         // P: 8 columns of packed pairs per 16 keys, where the tile's scores were
+              at_mma_ts(tmem_base + AT_O_COL, tmem_base + (i % AT_NBUF) * AT_KT + kk * 8, tc_desc_mn(v_addr + kk * 2048, AT_HALF_BYTES, 1024),
+                        idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+            else                                   // P: 32 bytes along a row of the swizzled tile in shared memory
+              tc_mma(tmem_base + AT_O_COL, tc_desc(p_addr + kk * 32), tc_desc_mn(v_addr + kk * 2048, AT_HALF_BYTES, 1024),
+                     idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+          }
+          tc_commit(&kv_empty[s]);
+          tc_commit(&pv_done[i % AT_NBUF]);
         }
-        tc_commit(&kv_empty[s]);
-        tc_commit(&pv_done[i % AT_NBUF]);
         if (AT_NBUF == 1 && i + 1 < ntiles) ok = issue_scores(i + 1);
       }
       pdl_launch_dependents();                      // all products of this block are issued

@@ -62,7 +62,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * TC_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_kb = (K + TC_BK - 1) / TC_BK;
   constexpr int TILE_COLS = (EPI == TC_EPI_SWIGLU) ? TC_BN / 2 : TC_BN;      // output columns of a tile
 
@@ -84,8 +84,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   pdl_wait();                                     // A is the output of the kernel before; the set-up above overlapped its tail
 
   if (warp == 0) {
-    // ---------------- producer: one lane issues the TMA loads, the ring runs on across tiles
-    if (lane == 0) {
+    // ---------------- producer: the warp waits, one lane issues the TMA loads; the ring runs on across tiles
+    const bool elected = tc_elect();
+    {
       int it = 0;                                   // k blocks issued so far
       bool ok = true;
 #ifdef TC_TEST_NO_LOADS
@@ -96,6 +97,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % TC_STAGES;
           if (!tc_wait(&empty[s], ((it / TC_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (!elected) continue;
           unsigned char* a_dst = tiles + s * TC_STAGE_BYTES;
           unsigned char* b_dst = a_dst + TC_A_BYTES;
           tc_mbar_expect_tx(&full[s], TC_STAGE_BYTES);
@@ -108,15 +110,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
-      if (*abort_flag) {
+      if (elected && *abort_flag) {
         // copies already issued still write into this block's shared memory: wait for them, bounded
         for (int j = (it > TC_STAGES ? it - TC_STAGES : 0); j < it; ++j)
           for (uint32_t i = 0; i < TC_WAIT_LIMIT && !tc_mbar_try(&full[j % TC_STAGES], (j / TC_STAGES) & 1); ++i) {}
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer: one lane
-    if (lane == 0) {
+    // ---------------- MMA issuer: the warp waits, one lane issues
+    const bool elected = tc_elect();
+    {
       const uint32_t idesc = tc_idesc(TC_BM, TC_BN);
       int it = 0, local = 0;
       bool ok = true;
@@ -130,6 +133,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const int s = it % TC_STAGES;
           if (!tc_wait(&full[s], (it / TC_STAGES) & 1, abort_flag)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (!elected) continue;
           const uint32_t a_addr = tc_smem(tiles + s * TC_STAGE_BYTES);
           const uint32_t b_addr = a_addr + TC_A_BYTES;
 #pragma unroll
@@ -139,7 +143,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
           tc_commit(&empty[s]);                     // the stage is free once these products have read it
         }
-        if (ok) tc_commit(&acc_ready[buf]);         // the accumulator is complete once all products are done
+        if (ok && elected) tc_commit(&acc_ready[buf]);         // the accumulator is complete once all products are done
       }
       pdl_launch_dependents();                      // all products of this block are issued
     }

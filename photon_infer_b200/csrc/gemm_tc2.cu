@@ -111,7 +111,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T2_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = t2_cta_rank();            // 0 or 1 inside the pair
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int num_kb = (K + T2_BK - 1) / T2_BK;
@@ -136,8 +136,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   pdl_wait();                                     // A is the output of the kernel before
 
   if (warp == 0) {
-    // ---------------- producer (one lane in each block): this block's rows of A and its half of the W tile
-    if (lane == 0) {
+    // ---------------- producer (one lane in each block; the warp waits): this block's rows of A and its half of the W tile
+    const bool elected = tc_elect();
+    {
       int it = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -145,6 +146,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % T2_STAGES;
           if (!t2_wait(&empty[s], ((it / T2_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (!elected) continue;
           unsigned char* a_dst = tiles + s * T2_STAGE_BYTES;
           unsigned char* b_dst = a_dst + T2_A_BYTES;
           if (rank == 0) tc_mbar_expect_tx(&full[s], 2 * T2_STAGE_BYTES);     // both blocks' bytes
@@ -156,7 +158,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer: one lane of block 0 issues for the pair
-    if (lane == 0 && rank == 0) {
+    const bool elected = tc_elect();
+    if (rank == 0) {
       const uint32_t idesc = tc_idesc(2 * T2_BM, T2_BN);
       int it = 0, local = 0;
       bool ok = true;
@@ -169,6 +172,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           const int s = it % T2_STAGES;
           if (!t2_wait(&full[s], (it / T2_STAGES) & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
+          if (!elected) continue;
           const uint32_t a_addr = tc_smem(tiles + s * T2_STAGE_BYTES);
           const uint32_t b_addr = a_addr + T2_A_BYTES;
 #pragma unroll
@@ -176,7 +180,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             t2_mma(d_tmem, tc_desc(a_addr + k * 32), tc_desc(b_addr + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
           t2_commit_both(&empty[s]);                // both blocks may refill the stage once these products have read it
         }
-        if (ok) t2_commit_both(&acc_ready[buf]);
+        if (ok && elected) t2_commit_both(&acc_ready[buf]);
       }
       pdl_launch_dependents();
     }
