@@ -132,10 +132,6 @@ PHOTON_API int photon_conv_state(const void* x, long x_stride, int x_dtype, int 
 #define LR_COLS 16
 #define LR_THREADS 128
 
-// Mode 2's inputs.
-__device__ __forceinline__ float lr_silu(float x) { return x / (1.0f + expf(-x)); }
-__device__ __forceinline__ float lr_write_gate(float z, float bias, float lower) { return (1.0f - lower) / (1.0f + expf(z + bias)); }
-
 // A thread owns four neighbouring channels of LR_GATE_TOK tokens (V 1: one channel).
 #define LR_GATE_TOK 4
 template <int V>

@@ -339,6 +339,17 @@ PHOTON_EXPORT int photon_linrec_segments(int mode, const float* q, long q_stride
                               float* out, long out_stride, float* den, float* scratch, int T, int S, int H, int qk_heads,
                               int N, int dv, int seg, int segs, int cuts, int cut_segs, int* err, cudaStream_t stream);
 
+/* ------------------------------------------------------------------ linrec_chunks.cu: the same on the tensor cores, in chunks of 128 tokens */
+/* As photon_linrec_segments; `chunks`: the sum over the requests of their tokens / 128, rounded up.  N, dv <= 128 and multiples of
+ * 4, rows and bases 16-byte aligned.  mode 2: p0, p1 [qk_heads * N] (raw q and gates k, as for photon_linrec) or null.  mode 1: den has room for (T + chunks) * H floats.  scratch: 16-byte aligned. */
+PHOTON_EXPORT long photon_linrec_chunks_scratch(int mode, int T, int chunks, int H, int N, int dv);
+PHOTON_EXPORT int photon_linrec_chunks(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
+                              long v_stride, const float* a, long a_stride, const float* ga, const float* gb, long g_stride,
+                              const float* p0, const float* p1, const float* p2, float cap, float q_scale,
+                              const int* cu_tokens, const int* state_slots, float* state, long state_stride, int num_slots,
+                              float* out, long out_stride, float* den, float* scratch, int T, int S, int H, int qk_heads,
+                              int N, int dv, int chunks, int* err, cudaStream_t stream);
+
 /* ------------------------------------------------------------------ attention_talk.cu: attention whose heads' scores are mixed */
 /* Bias (float, may be null) on q [T][H * d] and k [T][G * d] of in_dtype, rotation of the first rot_dims numbers of a head
  * (number j with j + rot_dims / 2, angle positions[t] * inv_freq[j]); q_out of out_dtype; the rotated key goes to k_cache, the

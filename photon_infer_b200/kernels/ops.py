@@ -1911,6 +1911,86 @@ def linrec_segment_tokens(query_lens, heads: int, blocks: int, sms: int) -> int:
     return low * 16
 
 
+def _check_linrec(what, mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, query_lens, heads, qk_heads, dim,
+                  vdim, err) -> None:
+    """What ``linrec_segments`` and ``linrec_chunks`` take."""
+    _cuda(q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, err)
+    if mode not in LINREC_SEGMENT_MODES:
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, f"{what}: unknown mode {mode!r}")
+    T, S = q.shape[0], len(query_lens)
+    for t, w, name in ((q, qk_heads * dim, "q"), (k, qk_heads * dim, "k"), (v, heads * vdim, "v"), (a, qk_heads * dim, "a"),
+                       (gate_a, heads, "gate_a"), (gate_b, heads, "gate_b"), (out, heads * vdim, "out")):
+        if t is not None and (t.dtype != torch.float32 or t.shape != (T, w) or t.stride(1) != 1):
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"{what}: {name} must be a float32 [T, {w}] view")
+    if gate_b is not None and (gate_a is None or gate_b.stride(0) != gate_a.stride(0)):
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"{what}: both gates must have one row stride")
+    if (mode == "matrix_memory") != (gate_b is not None) or (mode in ("state_space", "matrix_memory")) != (gate_a is not None) \
+            or (mode == "decay_rows") != (a is not None):
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, f"{what}: the matrix memory has two gates per head, the state-space layer one, "
+                          "the others none beside their rows' gates or decays")
+    for t, name in ((p0, "p0"), (p1, "p1"), (p2, "p2")):
+        if t is not None and (t.dtype != torch.float32 or t.numel() != heads or not t.is_contiguous()):
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"{what}: {name} must be float32 [{heads}]")
+    if mode in ("state_space", "matrix_memory") and (p0 is None or p1 is None or (p2 is None and mode == "state_space")):
+        raise PhotonError(ErrorCode.INVALID_ARGUMENT, f"{what}: the gates' parameters are missing")
+    need = heads * dim * vdim + (heads * dim + heads if mode == "matrix_memory" else 0)
+    if state.dtype != torch.float32 or state.dim() != 2 or not state.is_contiguous() or state.shape[1] < need:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"{what}: state must be contiguous float32 [slots, row]")
+    _int32(cu_tokens, "cu_tokens")
+    _int32(state_slots, "state_slots")
+    if cu_tokens.numel() < S + 1 or state_slots.numel() < S or sum(query_lens) > T:
+        raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"{what}: cu_tokens and state_slots must cover every request")
+
+
+LINREC_CHUNK = 128
+LINREC_CHUNKS_MIN_TOKENS = 64
+#: Tokens x heads of a step from which the chunks are the faster way (below, a step waits for the host, and they are one launch more than the
+#: segments).  B200, heads of 128 x 128, a mixer's step, us, as before first: gated linear attention 640 tokens x 16 heads 160 and 149, 2,048 x
+#: 16 302 and 225, 256 x 32 155 and 153, 400 x 32 208 and 166; matrix memory 640 x 16 154 and 131, 400 x 16 136 and 132, 2,048 x 16 296 and 199;
+#: state space 640 x 16 160 and 149, 256 x 32 147 and 150, 2,048 x 16 294 and 221; forget and write 1,000 x 16 177 and 146, 640 x 32 213 and 220.
+LINREC_CHUNKS_FROM = {"decay_rows": 10000, "matrix_memory": 10000, "state_space": 10000, "forget_write": 12000}
+
+
+def linrec_chunks_supported(mode: str, dim: int, vdim: int, query_lens, heads: int, *rows: Optional[torch.Tensor]) -> bool:
+    """Whether a bfloat16 step of long portions runs its recurrences in chunks of 128 tokens on the tensor cores (``linrec_chunks.cu``):
+    states of up to 128 x 128, no request that would leave a chunk mostly empty, enough work, and ``rows`` (the inputs, the state)
+    that start on 16 bytes."""
+    return (dim <= LINREC_CHUNK and vdim <= LINREC_CHUNK and dim % 4 == 0 and vdim % 4 == 0 and min(query_lens) >= LINREC_CHUNKS_MIN_TOKENS
+            and sum(query_lens) * heads >= LINREC_CHUNKS_FROM[mode]
+            and all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0) for t in rows))
+
+
+def linrec_chunks(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: Optional[torch.Tensor], gate_a: Optional[torch.Tensor],
+                  gate_b: Optional[torch.Tensor], p0: Optional[torch.Tensor], p1: Optional[torch.Tensor], p2: Optional[torch.Tensor],
+                  cap: float, q_scale: float, cu_tokens: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor, out: torch.Tensor,
+                  query_lens, heads: int, qk_heads: int, dim: int, vdim: int, err: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """``linrec_segments`` on the tensor cores, in 32-bit accuracy: the chunks' sums of k v^T side by side, a pass from chunk to chunk, and
+    the outputs of all chunks side by side.  ``forget_write``: ``q`` and ``k`` as ``linrec_gates`` leaves them or, with ``p0, p1
+    [qk_heads * dim]``, raw as for ``linrec``."""
+    gates = mode == "forget_write" and p0 is not None
+    _check_linrec("linrec_chunks", mode, q, k, v, a, gate_a, gate_b, None if gates else p0, None if gates else p1, p2, cu_tokens, state_slots,
+                  state, out, query_lens, heads, qk_heads, dim, vdim, err)
+    for t in (p0, p1) if gates else ():
+        if t is None or t.dtype != torch.float32 or t.numel() != qk_heads * dim or not t.is_contiguous():
+            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"linrec_chunks: p0 and p1 must be float32 [{qk_heads * dim}]")
+    T, S, code = q.shape[0], len(query_lens), LINREC_SEGMENT_MODES[mode]
+    chunks = sum(-(-n // LINREC_CHUNK) for n in query_lens)
+    n = _fn("linrec_chunks", "photon_linrec_chunks_scratch", [c_int] * 6, restype=c_long)(code, T, chunks, heads, dim, vdim)
+    scratch = torch.empty(n, dtype=torch.float32, device=q.device)
+    den = torch.empty((T + chunks, heads), dtype=torch.float32, device=q.device) if mode == "matrix_memory" else None
+    f = _fn("linrec_chunks", "photon_linrec_chunks",
+            [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_long, c_void_p, c_void_p,
+             c_void_p, c_float, c_float, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(code, _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(a), a.stride(0) if a is not None else 0,
+             _ptr(gate_a), _ptr(gate_b), gate_a.stride(0) if gate_a is not None else 0, _ptr(p0), _ptr(p1), _ptr(p2), float(cap),
+             float(q_scale), _ptr(cu_tokens), _ptr(state_slots), _ptr(state), state.stride(0), state.shape[0], _ptr(out), out.stride(0),
+             _ptr(den), _ptr(scratch), T, S, heads, qk_heads, dim, vdim, chunks, _ptr(err), _stream()), "linrec_chunks")
+    global _launch_count
+    _launch_count += 2 + (mode in ("state_space", "matrix_memory"))
+    return den[:T] if den is not None else None
+
+
 def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: Optional[torch.Tensor], gate_a: Optional[torch.Tensor],
                     gate_b: Optional[torch.Tensor], p0: Optional[torch.Tensor], p1: Optional[torch.Tensor], p2: Optional[torch.Tensor],
                     cap: float, q_scale: float, cu_tokens: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor, out: torch.Tensor,
@@ -1923,32 +2003,12 @@ def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     ``q`` and ``k`` as ``linrec_gates`` leaves them.  ``decay_rows``: ``S <- diag(a) S + k v^T``, ``a [T, qk_heads * dim]``.
     ``matrix_memory``: ``out`` is not divided; returns ``[T, heads]``, what it is to be divided by.  ``query_lens``: the requests'
     tokens in the step (host)."""
-    _cuda(q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, err)
-    if mode not in LINREC_SEGMENT_MODES:
-        raise PhotonError(ErrorCode.INVALID_ARGUMENT, f"linrec_segments: unknown mode {mode!r}")
+    if segment is None and linrec_chunks_supported(mode, dim, vdim, query_lens, heads, state, q, k, v, a):
+        return linrec_chunks(mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cap, q_scale, cu_tokens, state_slots, state, out, query_lens,
+                             heads, qk_heads, dim, vdim, err)
+    _check_linrec("linrec_segments", mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, query_lens, heads,
+                  qk_heads, dim, vdim, err)
     T, S = q.shape[0], len(query_lens)
-    for t, w, what in ((q, qk_heads * dim, "q"), (k, qk_heads * dim, "k"), (v, heads * vdim, "v"), (a, qk_heads * dim, "a"),
-                       (gate_a, heads, "gate_a"), (gate_b, heads, "gate_b"), (out, heads * vdim, "out")):
-        if t is not None and (t.dtype != torch.float32 or t.shape != (T, w) or t.stride(1) != 1):
-            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"linrec_segments: {what} must be a float32 [T, {w}] view")
-    if gate_b is not None and (gate_a is None or gate_b.stride(0) != gate_a.stride(0)):
-        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: both gates must have one row stride")
-    if (mode == "matrix_memory") != (gate_b is not None) or (mode in ("state_space", "matrix_memory")) != (gate_a is not None) \
-            or (mode == "decay_rows") != (a is not None):
-        raise PhotonError(ErrorCode.INVALID_ARGUMENT, "linrec_segments: the matrix memory has two gates per head, the state-space layer one, "
-                          "the others none beside their rows' gates or decays")
-    for t, what in ((p0, "p0"), (p1, "p1"), (p2, "p2")):
-        if t is not None and (t.dtype != torch.float32 or t.numel() != heads or not t.is_contiguous()):
-            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"linrec_segments: {what} must be float32 [{heads}]")
-    if mode in ("state_space", "matrix_memory") and (p0 is None or p1 is None or (p2 is None and mode == "state_space")):
-        raise PhotonError(ErrorCode.INVALID_ARGUMENT, "linrec_segments: the gates' parameters are missing")
-    need = heads * dim * vdim + (heads * dim + heads if mode == "matrix_memory" else 0)
-    if state.dtype != torch.float32 or state.dim() != 2 or not state.is_contiguous() or state.shape[1] < need:
-        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: state must be contiguous float32 [slots, row]")
-    _int32(cu_tokens, "cu_tokens")
-    _int32(state_slots, "state_slots")
-    if cu_tokens.numel() < S + 1 or state_slots.numel() < S or sum(query_lens) > T:
-        raise PhotonError(ErrorCode.SHAPE_MISMATCH, "linrec_segments: cu_tokens and state_slots must cover every request")
     seg = int(segment) if segment else linrec_segment_tokens(query_lens, heads, linrec_segment_blocks(dim, vdim), sm_count(q.device))
     pieces = [-(-n // seg) for n in query_lens]
     cut = [n for n in pieces if n > 1]

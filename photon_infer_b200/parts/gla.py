@@ -27,7 +27,7 @@ from .registry import register_mixer
 
 
 class GatedLinearAttention(Mixer):
-    kernel_modules = ("gla", "linrec_segments", "delta")
+    kernel_modules = ("gla", "linrec_segments", "linrec_chunks", "delta")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, tau: float, eps: float,

@@ -32,7 +32,7 @@ DEFAULT_NAMES = {"q": "q", "k": "k", "v": "v", "g": "g", "o": "o", "norm": "norm
 
 
 class MatrixMemoryMixer(Mixer):
-    kernel_modules = ("linrec", "linrec_segments", "row_norms")
+    kernel_modules = ("linrec", "linrec_segments", "linrec_chunks", "row_norms")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, gate_cap: float, eps: float,

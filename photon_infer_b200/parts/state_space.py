@@ -32,7 +32,7 @@ DEFAULT_NAMES = {"in": "in", "conv": "conv", "conv_bias": "conv.b", "dt_bias": "
 
 
 class StateSpaceMixer(Mixer):
-    kernel_modules = ("linrec", "linrec_segments", "row_norms")
+    kernel_modules = ("linrec", "linrec_segments", "linrec_chunks", "row_norms")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, vdim: int, state: int, taps: int, eps: float, groups: int = 1,

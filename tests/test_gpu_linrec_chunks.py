@@ -1,0 +1,126 @@
+"""The recurrences in chunks of 128 tokens on the tensor cores (linrec_chunks.cu) against the same recurrence token by token in 64
+bits: chunks that are not full, states that are not zero, reused and negative slots, small states, decays of nearly nothing, and
+values that are not finite; and over 2,048 tokens an error that is not larger than the walk's."""
+import pytest
+import torch
+
+import test_gpu_linrec_segments as segments
+from test_gpu_linrec_segments import _rel, _walk, i32
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+MODES = ["state_space", "matrix_memory", "forget_write", "decay_rows"]
+
+
+@pytest.fixture(autouse=True)
+def any_size(monkeypatch):
+    """Chunks for steps of any size."""
+    from photon_infer_b200.kernels import ops
+    monkeypatch.setattr(ops, "LINREC_CHUNKS_FROM", dict.fromkeys(ops.LINREC_CHUNKS_FROM, 0))
+
+
+def _case(mode, H, G, N, dv, lens, slots, strong, seed, poison=None):
+    from photon_infer_b200.kernels import ops
+    gen = torch.Generator().manual_seed(seed)
+    T = sum(lens)
+    rows = torch.randn(T, 3 * G * N + H * dv + 2 * H + 4 - 2 * H % 4, generator=gen)
+    a0 = 3 * G * N
+    b0 = a0 + H * dv
+    rows[:, 2 * G * N:a0] = torch.sigmoid(rows[:, 2 * G * N:a0] + 2.0) ** (40 if strong else 1)
+    if mode == "forget_write":
+        rows[:, G * N:2 * G * N] = torch.sigmoid(rows[:, G * N:2 * G * N] * (4.0 if strong else 1.0) + (4.0 if strong else -2.0))
+    if strong and mode == "decay_rows":
+        rows[7, 2 * G * N] = 0.0
+    p0, p1, p2 = (0.5 * torch.randn(H, generator=gen) for _ in range(3))
+    p1 = p1 + ((-3.0 if strong else 3.0) if mode == "matrix_memory" else -1.0)
+    p0 = p0 + (2.0 if strong and mode == "state_space" else 0.0)
+    memory, per_head = mode == "matrix_memory", mode in ("matrix_memory", "state_space")
+    width = H * N * dv + (H * N + H if memory else 0)
+    width += 4 + -width % 4
+    state = torch.randn(7, width, generator=gen)
+    if poison is not None:
+        rows[poison[0], a0 + poison[1]] = poison[2]
+    st, r = state.to(DEV), rows.to(DEV)
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    out, err = torch.full((T, H * dv), float("nan"), device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+    cap, scale = (6.0 if memory else 0.0), N ** -0.5
+    args = (r[:, :G * N], r[:, G * N:2 * G * N], r[:, a0:b0], r[:, 2 * G * N:a0] if mode == "decay_rows" else None)
+    assert ops.linrec_chunks_supported(mode, N, dv, lens, H, st, *args)
+    den = ops.linrec_segments(mode, *args, r[:, b0:b0 + H] if per_head else None, r[:, b0 + H:b0 + 2 * H] if memory else None,
+                              p0.to(DEV) if per_head else None, p1.to(DEV) if per_head else None, p2.to(DEV) if mode == "state_space" else None,
+                              cap, scale, i32(cu), i32(slots), st, out, lens, H, G, N, dv, err)
+    if memory:
+        out = (out.view(T, H, dv) / den.unsqueeze(-1)).view(T, H * dv)
+    assert err.cpu().tolist()[0] == 0
+    wants = []
+    for i, L in enumerate(lens):
+        x = rows[cu[i]:cu[i + 1]].double()
+        heads = lambda z: z.reshape(L, G, N).repeat_interleave(H // G, dim=1)
+        s0 = state[slots[i]].double() if slots[i] >= 0 else torch.zeros(width, dtype=torch.float64)
+        S, n = s0[:H * N * dv].view(H, N, dv), s0[H * N * dv:H * N * dv + H * N].view(H, N) if memory else None
+        m = s0[H * N * (dv + 1):H * N * (dv + 1) + H] if memory else None
+        wants.append(_walk(mode, heads(x[:, :G * N]), heads(x[:, G * N:2 * G * N]), x[:, a0:b0].reshape(L, H, dv), heads(x[:, 2 * G * N:a0]),
+                           x[:, b0:b0 + H], x[:, b0 + H:b0 + 2 * H], p0.double(), p1.double(), p2.double(), cap, scale, S, n, m))
+    return out.cpu(), st.cpu(), state, wants, cu
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("H,G,N,dv", [(2, 2, 128, 128), (4, 2, 128, 40), (3, 3, 64, 12), (2, 1, 8, 128), (1, 1, 100, 4)])
+@pytest.mark.parametrize("strong", [False, True])
+def test_chunks_match_the_walk(mode, H, G, N, dv, strong):
+    """The tolerances of the segments' test; ``strong``: blocks of 32 tokens whose decays multiply to less than 2^-40."""
+    G = H if mode == "matrix_memory" else G
+    lens, slots = [130, 64, 255, 128, 300, 97], [3, 0, 6, -1, 1, 5]
+    got, after, state, wants, cu = _case(mode, H, G, N, dv, lens, slots, strong, N + dv)
+    memory = mode == "matrix_memory"
+    for i, (want, S, n, m) in enumerate(wants):
+        assert _rel(got[cu[i]:cu[i + 1]], want) < (5e-5 if memory else 2e-5), i
+        if slots[i] >= 0:
+            row = after[slots[i]]
+            assert _rel(row[:H * N * dv], S.flatten()) < 2e-5
+            if memory:
+                assert _rel(row[H * N * dv:H * N * (dv + 1)], n.flatten()) < 2e-5
+                assert float((row[H * N * (dv + 1):H * N * (dv + 1) + H].double() - m).abs().max()) < 1e-5
+            assert torch.equal(row[-4:], state[slots[i], -4:])
+    for slot in {2, 4}:
+        assert torch.equal(after[slot], state[slot])
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(mode, value):
+    H, N, dv, lens, t, col = 2, 32, 16, [200, 130], 150, 3
+    got, after, _, wants, cu = _case(mode, H, H, N, dv, lens, [0, 1], False, 9, poison=(t, col, value))
+    clean, clean_after, _, _, _ = _case(mode, H, H, N, dv, lens, [0, 1], False, 9)
+    other = [c for c in range(H * dv) if c != col]
+    assert torch.equal(got[:, other], clean[:, other]) and torch.equal(got[:t, col], clean[:t, col]) and torch.equal(got[200:], clean[200:])
+    assert not bool(torch.isfinite(got[t:200, col]).any())
+    S = after[0, :H * N * dv].view(H, N, dv)
+    assert not bool(torch.isfinite(S[0, :, col]).any()) and torch.equal(after[1], clean_after[1])
+    assert torch.equal(S[:, :, 4:], clean_after[0, :H * N * dv].view(H, N, dv)[:, :, 4:])
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("gates", ["constant", "nearly constant", "ordinary"])
+def test_slow_decays_keep_their_bits(mode, gates):
+    segments.test_slow_decays_keep_their_bits(mode, gates)
+
+
+@pytest.mark.parametrize("C", [128, 40])
+def test_raw_gates_are_those_of_the_gates_kernel(C):
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(3)
+    H, dv, lens = 2, 64, [200, 70]
+    T = sum(lens)
+    q, z, v = torch.randn(T, H * C, device=DEV), 3 * torch.randn(T, H * C, device=DEV), torch.randn(T, H * dv, device=DEV)
+    bias, lower = torch.randn(H * C, device=DEV), 0.5 * torch.rand(H * C, device=DEV)
+    results = []
+    for raw in (True, False):
+        st, out, qk = torch.ones(2, H * C * dv, device=DEV), torch.empty(T, H * dv, device=DEV), (q, z)
+        if not raw:
+            qk = torch.empty(T, H * C, device=DEV), torch.empty(T, H * C, device=DEV)
+            ops.linrec_gates(q, z, bias, lower, *qk)
+        ops.linrec_chunks("forget_write", *qk, v, None, None, None, bias if raw else None, lower if raw else None, None, 0.0, 1.0, i32([0, 200, 270]),
+                          i32([0, 1]), st, out, lens, H, H, C, dv, None)
+        results.append((out, st))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
