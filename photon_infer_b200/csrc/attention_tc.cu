@@ -17,7 +17,7 @@
 //     tensor memory (the second product takes its A operand from there), and rescale O in tensor memory only when
 //     a row's maximum has grown by more than 2^8 since the last rescale (the sum and O stay
 //     relative to the maximum in use, so the result is the same up to rounding).
-// The scores of tile i + 1 are computed while the softmax of tile i runs.
+// The scores of tile i + 1 are computed while the softmax of tile i runs.  (attention_tc_pairs_kernel below: two such tiles a block.)
 //
 // Formula: include/photon/ops/kernels/mha_kernel.hpp:188-229 (scores (q.k)/sqrt(d) for the
 // keys up to the token's own position, softmax, weighted sum of values; head h uses
@@ -97,6 +97,78 @@ struct AttnTcParams {
   const bf16* gate; long gate_stride;              // may be null: [T, n_q * dv]; every output is multiplied by sigmoid(gate)
 };
 
+// The grid has a block per `per` tiles of the requests that have tiles here (few rows: the split-key kernel takes the
+// request), one request behind the other: every warp walks the requests, 32 at a time, to the one that holds the block's
+// tiles.  A grid of (requests x tiles of the longest) was 8,528 blocks where 208 had work, a portion of 1,093
+// tokens beside 40 decoded ones (24/8 heads of 128): 105 us, against 70 us without the empty blocks, each of which took
+// the shared memory of a full one.
+__device__ __forceinline__ bool at_find(const AttnTcParams& P, int per, int index, int& seq, int& before) {
+  seq = 0; before = 0;                             // `before`: blocks of the requests in front of `seq`
+  if (P.num_seqs <= 1) return true;
+  const int lane = threadIdx.x & 31;
+  int total = 0;
+  for (int s0 = 0; s0 < P.num_seqs; s0 += 32) {
+    const int s = s0 + lane;
+    int n = 0;
+    if (s < P.num_seqs) {
+      const int r = (P.cu_tokens[s + 1] - P.cu_tokens[s]) * P.group;
+      if (r > 16) n = (min((r + P.tile_rows - 1) / P.tile_rows, P.tiles_per_seq) + per - 1) / per;
+    }
+    int upto = n;                                  // inclusive sum over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, total + upto > index);
+    if (hit != 0) {
+      const int l = __ffs(hit) - 1;
+      seq = s0 + l;
+      before = total + __shfl_sync(0xffffffffu, upto - n, l);
+      return true;
+    }
+    total += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+
+// The output of a row: its O divided by its sum, times the gate; columns of tensor memory from `o_addr` on.
+__device__ __forceinline__ void at_write(const AttnTcParams& P, uint32_t o_addr, bool valid, int tok, int head, float m_used, float l) {
+  // the sink's weight, relative to the maximum in use
+  if (P.sinks && valid) l += exp2f(fmaf(P.sinks[head], 1.4426950408889634f, -m_used));
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  bf16* dst = P.out + (size_t)tok * P.out_stride + (size_t)head * VALUE_DIM;
+  const bf16* gt = P.gate ? P.gate + (size_t)tok * P.gate_stride + (size_t)head * VALUE_DIM : nullptr;
+#pragma unroll 1
+  for (int cc = 0; cc < VALUE_DIM; cc += 32) {
+    uint32_t ov[32];
+    tc_ld32(o_addr + cc, ov);
+    if (valid) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+        if (VALUE_DIM % 32 != 0 && cc + j >= VALUE_DIM) continue;
+        if (gt) {
+          // eight gates of this row (16 bytes): the output times sigmoid(gate), folded into the numbers before `inv`
+          const uint4 gz = *reinterpret_cast<const uint4*>(gt + cc + j);
+          const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gz);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float2 z = __bfloat1622float2(gp[u]);
+            ov[j + 2 * u] = __float_as_uint(__fdividef(__uint_as_float(ov[j + 2 * u]), 1.0f + __expf(-z.x)));
+            ov[j + 2 * u + 1] = __float_as_uint(__fdividef(__uint_as_float(ov[j + 2 * u + 1]), 1.0f + __expf(-z.y)));
+          }
+        }
+        uint4 v4;
+        v4.x = at_pack(__uint_as_float(ov[j]) * inv, __uint_as_float(ov[j + 1]) * inv);
+        v4.y = at_pack(__uint_as_float(ov[j + 2]) * inv, __uint_as_float(ov[j + 3]) * inv);
+        v4.z = at_pack(__uint_as_float(ov[j + 4]) * inv, __uint_as_float(ov[j + 5]) * inv);
+        v4.w = at_pack(__uint_as_float(ov[j + 6]) * inv, __uint_as_float(ov[j + 7]) * inv);
+        *reinterpret_cast<uint4*>(dst + cc + j) = v4;
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(AT_THREADS, AT_BLOCKS_PER_SM)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const AttnTcParams P) {
@@ -104,41 +176,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int g = blockIdx.x;
   const int G = P.group;
   pdl_wait();                                      // q, the cache and the step's tables come from kernels before
-  // The grid has a block per tile of the requests that have tiles here (few rows: the split-key kernel takes the
-  // request), one request behind the other: every warp walks the requests, 32 at a time, to the one that holds tile
-  // blockIdx.y.  A grid of (requests x tiles of the longest) was 8,528 blocks where 208 had work, a portion of 1,093
-  // tokens beside 40 decoded ones (24/8 heads of 128): 105 us, against 70 us without the empty blocks, each of which took
-  // the shared memory of a full one.
-  int seq = 0, before = 0;                         // `before`: tiles of the requests in front of `seq`
-  if (P.num_seqs > 1) {
-    const int lane = threadIdx.x & 31;
-    int total = 0;
-    bool found = false;
-    for (int s0 = 0; s0 < P.num_seqs && !found; s0 += 32) {
-      const int s = s0 + lane;
-      int n = 0;
-      if (s < P.num_seqs) {
-        const int r = (P.cu_tokens[s + 1] - P.cu_tokens[s]) * G;
-        if (r > 16) n = min((r + P.tile_rows - 1) / P.tile_rows, P.tiles_per_seq);
-      }
-      int upto = n;                                // inclusive sum over the lanes
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += v;
-      }
-      const unsigned hit = __ballot_sync(0xffffffffu, total + upto > (int)blockIdx.y);
-      if (hit != 0) {
-        const int l = __ffs(hit) - 1;
-        found = true;
-        seq = s0 + l;
-        before = total + __shfl_sync(0xffffffffu, upto - n, l);
-      } else {
-        total += __shfl_sync(0xffffffffu, upto, 31);
-      }
-    }
-    if (!found) return;
-  }
+  int seq, before;
+  if (!at_find(P, 1, (int)blockIdx.y, seq, before)) return;
   const int tok0 = P.cu_tokens[seq], ntok = P.cu_tokens[seq + 1] - tok0;
   const int rows = ntok * G;
   const int seq_tiles = min((rows + P.tile_rows - 1) / P.tile_rows, P.tiles_per_seq);
@@ -292,8 +331,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int r = threadIdx.x;                      // 0..127
     const int row = row0 + r;
     const bool valid = r < P.tile_rows && row < rows;
-    const int pos = valid ? P.positions[tok0 + row / G] : -1;
-    const int lo = (P.window > 0 && pos - P.window + 1 > 0) ? pos - P.window + 1 : 0;
+    // rows that nobody reads see every key: masking them would keep their warp busy at every tile (groups of 3: 2 rows of 128)
+    const int pos = valid ? P.positions[tok0 + row / G] : 0x7fffffff;
+    const int lo = (valid && P.window > 0 && pos - P.window + 1 > 0) ? pos - P.window + 1 : 0;
     const int kept = P.keep_first;
     const float cap = P.softcap, cap_in = P.cap_in * 2.8853900817779268f;     // tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1)
     const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
@@ -418,39 +458,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (ok && ntiles > 0 && wait_all(&pv_done[(ntiles - 1) % AT_NBUF], ((ntiles - 1) / AT_NBUF) & 1)) {
       tc_fence_after();
       const int tk = valid ? row / G : 0, h = valid ? row - tk * G : 0;
-      // the sink's weight, relative to the maximum in use
-      if (P.sinks && valid) l += exp2f(fmaf(P.sinks[g * G + h], 1.4426950408889634f, -m_used));
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      bf16* dst = P.out + (size_t)(tok0 + tk) * P.out_stride + (size_t)(g * G + h) * VALUE_DIM;
-      const bf16* gt = P.gate ? P.gate + (size_t)(tok0 + tk) * P.gate_stride + (size_t)(g * G + h) * VALUE_DIM : nullptr;
-#pragma unroll 1
-      for (int cc = 0; cc < VALUE_DIM; cc += 32) {
-        uint32_t ov[32];
-        tc_ld32(lane_addr + AT_O_COL + cc, ov);
-        if (valid) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            if (VALUE_DIM % 32 != 0 && cc + j >= VALUE_DIM) continue;
-            if (gt) {
-              // eight gates of this row (16 bytes): the output times sigmoid(gate), folded into the numbers before `inv`
-              const uint4 gz = *reinterpret_cast<const uint4*>(gt + cc + j);
-              const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&gz);
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const float2 z = __bfloat1622float2(gp[u]);
-                ov[j + 2 * u] = __float_as_uint(__fdividef(__uint_as_float(ov[j + 2 * u]), 1.0f + __expf(-z.x)));
-                ov[j + 2 * u + 1] = __float_as_uint(__fdividef(__uint_as_float(ov[j + 2 * u + 1]), 1.0f + __expf(-z.y)));
-              }
-            }
-            uint4 v4;
-            v4.x = at_pack(__uint_as_float(ov[j]) * inv, __uint_as_float(ov[j + 1]) * inv);
-            v4.y = at_pack(__uint_as_float(ov[j + 2]) * inv, __uint_as_float(ov[j + 3]) * inv);
-            v4.z = at_pack(__uint_as_float(ov[j + 4]) * inv, __uint_as_float(ov[j + 5]) * inv);
-            v4.w = at_pack(__uint_as_float(ov[j + 6]) * inv, __uint_as_float(ov[j + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + cc + j) = v4;
-          }
-        }
-      }
+      at_write(P, lane_addr + AT_O_COL, valid, tok0 + tk, g * G + h, m_used, l);
     }
   }
   // ---------------- teardown
@@ -462,6 +470,316 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
   if (threadIdx.x == 0 && *abort_flag) report_error(P.err, PHOTON_DEV_WAIT_TIMEOUT, blockIdx.x, blockIdx.y, 0);
 }
+
+// ---------------------------------------------------------------- two query tiles a block
+// Heads of more than 64 numbers and long contexts: a block of 384 threads owns an SM and two tiles of 128 rows of one request and
+// walks the keys that either sees in tiles of 128.  Scores have 128 columns a query tile (a product with N 64 reads 6 KB of
+// shared memory in 48 cycles where 32 would do; N 128 takes 64 either way), and while one tile's softmax runs, the tensor cores
+// work for the other:
+//   * warp 8 brings key and value tiles into rings of their own;
+//   * one thread of warp 9 issues, for the two query tiles in turn, O += P V in halves of 64 keys, each as soon as its P lies in
+//     tensor memory, and the next S = Q K^T, which takes the place of that P (the tensor cores run products in the order of issue,
+//     so scores that are there also say that the O before is);
+//   * warps 0-3 and 4-7: the rows of a query tile each.  They have 232 registers (the launch gives 168, the other four warps
+//     keep 40: 128 x 40 + 256 x 232 = 64,512 = 384 x 168), so that a row's 128 scores stay in registers.
+// Bound by the softmax warps (4,500 cycles for a pair of tiles of 128 keys, of which the exponentials take 2,048 at 16 a cycle and SM and the
+// products as many).  2,048 tokens behind 14,336, 32/8 heads of 128: 657 us with a tile a block, 482 so (1,070 TFLOP/s);
+// 2,048 from the start 59 and 51.  Heads of 64 gain nothing at any length (2,048 tokens 43 and 46 us; with columns of its own for P 42 and 48).
+#if HEAD_DIM > 64
+#define AP_KT 128
+#define AP_THREADS 384
+#define AP_K_BYTES (AP_KT * 128 * AT_DH)
+#define AP_V_BYTES (AP_KT * 128 * AT_VH)
+#define AP_HALF (AP_KT * 128)                      // one 64-wide half of a K or V tile
+#define AP_STAGES (AT_DH + AT_VH == 2 ? 3 : 2)
+#define AP_SMEM_BYTES (2 * AT_Q_BYTES + AP_STAGES * (AP_K_BYTES + AP_V_BYTES) + 1024 + 256)
+static_assert(AP_SMEM_BYTES <= 227 * 1024, "shared memory of a block");
+#define AP_O_COL 256                               // scores: 2 x 128 columns; O: 2 x 128
+
+__global__ void __launch_bounds__(AP_THREADS, 1)
+attention_tc_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                          const __grid_constant__ CUtensorMap map_v, const AttnTcParams P) {
+  const int g = blockIdx.x;
+  const int G = P.group;
+  pdl_wait();                                      // q, the cache and the step's tables come from kernels before
+  int seq, before;
+  if (!at_find(P, 2, (int)blockIdx.y, seq, before)) return;
+  const int tok0 = P.cu_tokens[seq], ntok = P.cu_tokens[seq + 1] - tok0;
+  const int rows = ntok * G;
+  const int seq_tiles = min((rows + P.tile_rows - 1) / P.tile_rows, P.tiles_per_seq);
+  const int pair = (seq_tiles + 1) / 2 - 1 - ((int)blockIdx.y - before);           // most keys first
+  if (rows <= 16 || pair < 0) return;
+  const int row0 = pair * 2 * P.tile_rows;
+  const int nq = 2 * pair + 1 < seq_tiles ? 2 : 1;
+  const int tile_tokens = P.tile_rows / G;
+  const int t_first = row0 / G, t_last = (min(row0 + nq * P.tile_rows, rows) - 1) / G;
+  const int pos_first = P.positions[tok0 + t_first], pos_last = P.positions[tok0 + t_last];
+  const int key_lo = (P.window > 0 && pos_first - P.window + 1 > 0) ? pos_first - P.window + 1 : 0;
+  const int tile_begin = key_lo / AP_KT;
+  const int kept_tiles = (P.keep_first > 0 && key_lo > 0) ? min((P.keep_first + AP_KT - 1) / AP_KT, tile_begin) : 0;
+  const int ntiles = kept_tiles + pos_last / AP_KT + 1 - tile_begin;
+  auto tile_of = [&](int i) { return i < kept_tiles ? i : tile_begin + i - kept_tiles; };
+
+  extern __shared__ unsigned char at_dyn[];
+  unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)at_dyn + 1023) & ~(uintptr_t)1023);
+  unsigned char* q_s = base;
+  unsigned char* k_s = q_s + 2 * AT_Q_BYTES;
+  unsigned char* v_s = k_s + AP_STAGES * AP_K_BYTES;
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(v_s + AP_STAGES * AP_V_BYTES);
+  uint64_t* k_full = q_full + 1;                    // [AP_STAGES] TMA -> MMA
+  uint64_t* k_empty = k_full + AP_STAGES;           // [AP_STAGES] MMA -> TMA
+  uint64_t* v_full = k_empty + AP_STAGES;
+  uint64_t* v_empty = v_full + AP_STAGES;
+  uint64_t* s_full = v_empty + AP_STAGES;           // [query tile] MMA -> softmax: the scores, and the O before
+  uint64_t* p_full = s_full + 2;                    // [query tile][half] softmax -> MMA (one arrival per warp)
+  uint64_t* o_full = p_full + 4;                    // [query tile] MMA -> softmax: all of O
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    tc_mbar_init(q_full, 1);
+    for (int s = 0; s < AP_STAGES; ++s) {
+      tc_mbar_init(&k_full[s], 1); tc_mbar_init(&k_empty[s], 1); tc_mbar_init(&v_full[s], 1); tc_mbar_init(&v_empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) { tc_mbar_init(&s_full[b], 1); tc_mbar_init(&o_full[b], 1); }
+    for (int b = 0; b < 4; ++b) tc_mbar_init(&p_full[b], 4);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_slot)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 8) {
+      // ---------------- producer
+      const bool elected = tc_elect();
+      if (elected) {
+        tc_mbar_expect_tx(q_full, nq * P.tile_rows * 128 * AT_DH);     // rows beyond tile_rows stay as they are: nobody uses them
+        for (int j = 0; j < nq; ++j)
+#pragma unroll
+          for (int h = 0; h < AT_DH; ++h)
+            tc_tma_load3(q_s + j * AT_Q_BYTES + h * (AT_ROWS * 128), &map_q, h * 64, g * G, tok0 + t_first + j * tile_tokens, q_full);
+      }
+      const int* table = P.block_table + (size_t)seq * P.max_pages;
+      const int boxes = AP_KT / P.box_rows;         // parts of a tile that may lie in different pages
+      // the row of this lane's part of a tile; outside the map: the part is filled with zeros
+      auto row_of = [&](int i) {
+        int rowc = P.total_rows;
+        if (lane < boxes) {
+          const int key = tile_of(i) * AP_KT + lane * P.box_rows;
+          if (key <= pos_last && (key + P.box_rows - 1 >= key_lo || key < P.keep_first)) {
+            const int pidx = key / P.page_size, slot = key - pidx * P.page_size;
+            const int page = table[pidx];
+            if (page < 0 || page >= P.num_pages) report_error(P.err, PHOTON_DEV_BAD_PAGE, tok0, key, page);
+            else rowc = (page * P.n_kv + g) * P.page_size + slot;
+          }
+        }
+        return rowc;
+      };
+      int kn = 0, vn = 0;                           // key and value tiles asked for so far
+      auto load = [&](int n, unsigned char* ring, int bytes, int halves, const CUtensorMap* map, uint64_t* full, uint64_t* empty) -> bool {
+        const int s = n % AP_STAGES, rowc = row_of(n);
+        if (!__all_sync(0xffffffffu, tc_wait(&empty[s], ((n / AP_STAGES) & 1) ^ 1, abort_flag))) return false;
+        if (elected) tc_mbar_expect_tx(&full[s], bytes);
+        unsigned char* dst = ring + s * bytes;
+        for (int part = 0; part < boxes; ++part, dst += P.box_rows * 128) {
+          const int row = __shfl_sync(0xffffffffu, rowc, part);
+          if (elected)
+            for (int h = 0; h < halves; ++h) tc_tma_load(dst + h * AP_HALF, map, h * 64, row, &full[s]);
+        }
+        return true;
+      };
+      auto load_k = [&]() { const bool ok = load(kn, k_s, AP_K_BYTES, AT_DH, &map_k, k_full, k_empty); kn += ok; return ok; };
+      auto load_v = [&]() { const bool ok = load(vn, v_s, AP_V_BYTES, AT_VH, &map_v, v_full, v_empty); vn += ok; return ok; };
+      // in the order in which room appears: the scores of tile i free a key tile before the products of tile i free values
+      bool ok = true;
+      for (int n = 0; n < AP_STAGES && n < ntiles && ok; ++n) ok = load_k();
+      for (int i = 0; i < ntiles && ok; ++i) {
+        ok = load_v();
+        if (ok && kn < ntiles) ok = load_k();
+      }
+      if (elected && *abort_flag) {
+        // copies already issued still write into this block's shared memory: wait for them, bounded
+        for (uint32_t w = 0; w < TC_WAIT_LIMIT && !tc_mbar_try(q_full, 0); ++w) {}
+        for (int n = (kn > AP_STAGES ? kn - AP_STAGES : 0); n < kn; ++n)
+          for (uint32_t w = 0; w < TC_WAIT_LIMIT && !tc_mbar_try(&k_full[n % AP_STAGES], (n / AP_STAGES) & 1); ++w) {}
+        for (int n = (vn > AP_STAGES ? vn - AP_STAGES : 0); n < vn; ++n)
+          for (uint32_t w = 0; w < TC_WAIT_LIMIT && !tc_mbar_try(&v_full[n % AP_STAGES], (n / AP_STAGES) & 1); ++w) {}
+      }
+    } else if (warp == 9) {
+      // ---------------- MMA issuer: the warp waits, one of its lanes issues
+      const bool elected = tc_elect();
+      const uint32_t idesc_s = tc_idesc(AT_ROWS, AP_KT);
+      const uint32_t idesc_o = tc_idesc(AT_ROWS, 64 * AT_VH) | TC_IDESC_B_MN;
+      auto issue_scores = [&](int i, int j) -> bool {
+        const int s = i % AP_STAGES;
+        if (!tc_wait(&k_full[s], (i / AP_STAGES) & 1, abort_flag)) return false;
+        tc_fence_after();
+        if (elected) {
+          const uint32_t q_addr = tc_smem(q_s + j * AT_Q_BYTES), k_addr = tc_smem(k_s + s * AP_K_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < (HEAD_DIM + 15) / 16; ++kk)
+            tc_mma(tmem + j * 128, tc_desc(q_addr + (kk >> 2) * (AT_ROWS * 128) + (kk & 3) * 32),
+                   tc_desc(k_addr + (kk >> 2) * AP_HALF + (kk & 3) * 32), idesc_s, kk > 0 ? 1u : 0u);
+          tc_commit(&s_full[j]);
+          if (j == nq - 1) tc_commit(&k_empty[s]);
+        }
+        return true;
+      };
+      bool ok = tc_wait(q_full, 0, abort_flag);
+      for (int j = 0; j < nq && ok; ++j) ok = issue_scores(0, j);
+      for (int i = 0; i < ntiles && ok; ++i) {
+        const int s = i % AP_STAGES;
+        for (int j = 0; j < nq && ok; ++j) {
+          if (!tc_wait(&v_full[s], (i / AP_STAGES) & 1, abort_flag)) { ok = false; break; }
+#pragma unroll
+          for (int half = 0; half < 2 && ok; ++half) {
+            if (!tc_wait(&p_full[2 * j + half], i & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            if (elected) {
+              const uint32_t v_addr = tc_smem(v_s + s * AP_V_BYTES) + half * 4 * 2048;
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)        // 16 keys: P's 8 columns of packed pairs, two groups of 8 rows of V
+                at_mma_ts(tmem + AP_O_COL + j * 128, tmem + j * 128 + half * 32 + kk * 8, tc_desc_mn(v_addr + kk * 2048, AP_HALF, 1024),
+                          idesc_o, (i > 0 || half > 0 || kk > 0) ? 1u : 0u);
+            }
+          }
+          if (!ok) break;
+          if (elected) {
+            if (j == nq - 1) tc_commit(&v_empty[s]);
+            if (i + 1 == ntiles) tc_commit(&o_full[j]);
+          }
+          if (i + 1 < ntiles) ok = issue_scores(i + 1, j);
+        }
+      }
+      pdl_launch_dependents();                      // all products of this block are issued
+    }
+  } else {
+    // ---------------- softmax: thread = row of query tile j
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    const int j = warp >> 2;
+    const int r = threadIdx.x & 127;
+    const int row = row0 + j * P.tile_rows + r;
+    const bool valid = j < nq && r < P.tile_rows && row < rows;
+    // rows that nobody reads see every key: masking them would keep their warp busy at every tile (groups of 3: 2 rows of 128)
+    const int pos = valid ? P.positions[tok0 + row / G] : 0x7fffffff;
+    const int lo = (valid && P.window > 0 && pos - P.window + 1 > 0) ? pos - P.window + 1 : 0;
+    const int kept = P.keep_first;
+    const float cap = P.softcap, cap_in = P.cap_in * 2.8853900817779268f;     // tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1)
+    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t s_addr = lane_addr + j * 128, o_addr = lane_addr + AP_O_COL + j * 128;
+    const float c = P.scale_log2;
+    float m_used = -INFINITY, l = 0.f;
+    bool ok = true;
+    // the warp goes on or gives up together: tcgen05.ld/st need all of its lanes
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, tc_wait(bar, parity, abort_flag) ? 1 : 0) != 0;
+    };
+    for (int i = 0; i < ntiles && j < nq; ++i) {
+      if (!wait_all(&s_full[j], i & 1)) { ok = false; break; }
+      tc_fence_after();
+      const int key_base = tile_of(i) * AP_KT;
+      uint32_t sv[AP_KT];
+#pragma unroll
+      for (int u = 0; u < AP_KT; u += 32) tc_ld32_issue(s_addr + u, sv + u);
+      tc_ld_wait();
+      if (cap > 0.f) {
+#pragma unroll
+        for (int u = 0; u < AP_KT; ++u) {
+          const float e = at_exp2(__uint_as_float(sv[u]) * cap_in);
+          sv[u] = __float_as_uint(cap - __fdividef(2.0f * cap, e + 1.0f));
+        }
+      }
+      if (!(key_base + AP_KT - 1 <= pos && key_base >= lo)) {
+        // keys this row does not see: those before offset a (but for the kept ones, before k) or behind offset b of the tile
+        const int a = lo - key_base, b = pos - key_base, k = kept - key_base;
+#pragma unroll
+        for (int u = 0; u < AP_KT; ++u) sv[u] = ((u >= a || u < k) && u <= b) ? sv[u] : 0xff800000u;       // -inf
+      }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int u = 0; u < AP_KT; u += 8) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mx4[w] = at_max3(mx4[w], __uint_as_float(sv[u + 2 * w]), __uint_as_float(sv[u + 2 * w + 1]));
+      }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      // the maximum in use lags behind the true one by at most AT_RESCALE_STEP
+      const float cand = fmaxf(m_used, mx * c);
+      float factor = 1.f;
+      const bool grow = cand > m_used + AT_RESCALE_STEP;          // also the first finite maximum
+      if (grow) { factor = at_exp2(m_used - cand); m_used = cand; l *= factor; }
+      const float nsub = (m_used == -INFINITY) ? 0.f : -m_used;
+      // rescale O: the products of the tile before have landed, because they were issued before these scores
+      if (i > 0 && __any_sync(0xffffffffu, grow)) {
+#pragma unroll 1
+        for (int cc = 0; cc < VALUE_DIM; cc += 32) {
+          uint32_t ov[32];
+          tc_ld32(o_addr + cc, ov);
+#pragma unroll
+          for (int u = 0; u < 32; ++u) ov[u] = __float_as_uint(__uint_as_float(ov[u]) * factor);
+          tc_st32(o_addr + cc, ov);
+        }
+        tc_st_wait();
+      }
+      if (j == 0 && i == ntiles - 1 && pos_last - key_base + 1 < AP_KT) {
+        // value rows beyond the request's last key: zeros instead of whatever the page holds.  The first tile's warps write them
+        // before their P is ready, and the second tile's products are issued after the first's.
+        const int nvalid = pos_last - key_base + 1, nzero = AP_KT - nvalid;
+        const int s = i % AP_STAGES;
+        if (!wait_all(&v_full[s], (i / AP_STAGES) & 1)) { ok = false; break; }
+        unsigned char* vst = v_s + s * AP_V_BYTES;
+        for (int e = r; e < nzero * 8 * AT_VH; e += AT_ROWS) {
+          const int half = e / (nzero * 8), rem = e - half * (nzero * 8);
+          *reinterpret_cast<uint4*>(vst + half * AP_HALF + (nvalid + (rem >> 3)) * 128 + ((rem & 7) << 4)) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> the tensor core's reads
+      }
+      // P = exp2(score * c - max in use), packed pairs over the scores they came from (32 columns per 64 keys)
+      float sum8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t pk[32];
+#pragma unroll
+        for (int u = 0; u < 64; u += 2) {
+          float x0, x1;
+          at_fma2(x0, x1, __uint_as_float(sv[half * 64 + u]), __uint_as_float(sv[half * 64 + u + 1]), c, nsub);
+          const float p0 = at_exp2(x0), p1 = at_exp2(x1);
+          at_add2(sum8[u & 6], sum8[(u & 6) + 1], p0, p1);
+          pk[u >> 1] = at_pack(p0, p1);
+        }
+        tc_st32(s_addr + half * 32, pk);
+        tc_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(&p_full[2 * j + half]);
+      }
+      l += ((sum8[0] + sum8[1]) + (sum8[2] + sum8[3])) + ((sum8[4] + sum8[5]) + (sum8[6] + sum8[7]));
+    }
+    if (ok && j < nq && ntiles > 0 && wait_all(&o_full[j], 0)) {
+      tc_fence_after();
+      const int tk = valid ? row / G : 0, h = valid ? row - tk * G : 0;
+      at_write(P, o_addr, valid, tok0 + tk, g * G + h, m_used, l);
+    }
+  }
+  // ---------------- teardown
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
+  }
+  if (threadIdx.x == 0 && *abort_flag) report_error(P.err, PHOTON_DEV_WAIT_TIMEOUT, blockIdx.x, blockIdx.y, 0);
+}
+
+#endif
 
 PHOTON_API int photon_attention_tc_head_dim() { return HEAD_DIM; }
 
@@ -543,5 +861,20 @@ PHOTON_API int photon_attention_tc_ex(const void* q, long q_stride, void* out, l
   dim3 grid(n_kv, (unsigned)(most < (long)S * P.tiles_per_seq ? most : (long)S * P.tiles_per_seq));
   if (S == 1) grid.y = P.tiles_per_seq;
   if (grid.y == 0) return 0;                        // no request of the step has more than 16 rows
+#if HEAD_DIM > 64
+  // Two tiles a block from 2,048 keys on, 4,096 beside other requests (the block table's width is the longest request's, which may not be
+  // the portion).  us, one and two tiles a block, 24/8 heads: 1,093 tokens from the start 30 and 33, 2,048 51 and 48, 512 behind
+  // 2,048 52 and 53, 1,024 behind 2,048 66 and 62, 512 behind 8,192 151 and 144; three requests of 300 to 600 tokens 22 and 25.
+#ifndef AT_PAIRS_KEYS
+#define AT_PAIRS_KEYS 2048
+#endif
+  if ((long)max_pages * page_size >= (S == 1 ? 1L : 2L) * AT_PAIRS_KEYS) {
+    cudaError_t e = cudaFuncSetAttribute(attention_tc_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    // a request's last tile may be alone in its block
+    const unsigned y = (unsigned)(S == 1 ? (grid.y + 1) / 2 : (grid.y + (part < (long)grid.y ? part : (long)grid.y) + 1) / 2);
+    return launch_pdl(attention_tc_pairs_kernel, dim3(n_kv, y), dim3(AP_THREADS), (size_t)AP_SMEM_BYTES, stream, map_q, map_k, map_v, P);
+  }
+#endif
   return launch_pdl(attention_tc_kernel, grid, dim3(AT_THREADS), (size_t)AT_SMEM_BYTES, stream, map_q, map_k, map_v, P);
 }
