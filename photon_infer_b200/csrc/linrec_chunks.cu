@@ -132,6 +132,11 @@ lc_gates_kernel(const float* __restrict__ ga, const float* __restrict__ gb, long
   if (h >= A.H || place.seq < 0) return;
   const int b0 = A.cu_tokens[place.seq] + ((int)blockIdx.x - place.before) * LC_T, b1 = min(A.cu_tokens[place.seq + 1], b0 + LC_T);
   const size_t TH = (size_t)A.T * A.H;
+  if (MODE == 1 && lane == 0 && (int)blockIdx.x == place.before) {                  // the maximum before the step: one block of the scan overwrites
+    const int slot = A.state_slots[place.seq];                                      // the slot while others may not have started
+    A.den[TH + (size_t)blockIdx.x * A.H + h] =
+        slot >= 0 && slot < A.num_slots ? A.state[(size_t)slot * A.state_stride + (size_t)A.H * A.N * (A.dv + 1) + h] : 0.f;
+  }
   const double a_h = MODE == 0 ? (double)expf(p0[h]) : 0.0;
   double sum = 0.0, last = -INFINITY;                 // the sum before these 32; mode 1: the largest i - sum so far
   for (int t = b0; t < b1; t += 32) {
@@ -433,7 +438,7 @@ lc_scan_kernel(const LcArgs A) {
   const int i = vec ? threadIdx.x * 4 : (blockIdx.x * 256 + threadIdx.x) * 4, end = vec ? A.N : size;
   float* slot_at = row0 ? row0 + (vec ? (size_t)A.H * size + (size_t)h * A.N : (size_t)h * size) + i : nullptr;
   float* slot_m = row0 ? row0 + (size_t)A.H * size + (size_t)A.H * A.N + h : nullptr;
-  float m = MODE == 1 && row0 ? *slot_m : 0.f;
+  float m = MODE == 1 ? A.den[(size_t)A.T * A.H + (size_t)before * A.H + h] : 0.f;  // from lc_gates_kernel
   float4 S = i < end && row0 ? *reinterpret_cast<const float4*>(slot_at) : make_float4(0.f, 0.f, 0.f, 0.f);
   const size_t step = vec ? (size_t)A.H * A.N : (size_t)A.H * size;
   float* at = (vec ? A.vecs + ((size_t)before * A.H + h) * A.N : A.ends + ((size_t)before * A.H + h) * size) + i;
@@ -468,7 +473,7 @@ lc_scan_kernel(const LcArgs A) {
       S.z = MODE == 1 ? fmaf(c2, U.z, lc_apply(code, S.z)) : lc_apply(code, S.z) + U.z;
       S.w = MODE == 1 ? fmaf(c2, U.w, lc_apply(code, S.w)) : lc_apply(code, S.w) + U.w;
     }
-    if (vec && threadIdx.x == 0) A.den[(size_t)A.T * A.H + ((size_t)(before + c)) * A.H + h] = m_start;
+    if (vec && threadIdx.x == 0 && c > 0) A.den[(size_t)A.T * A.H + ((size_t)(before + c)) * A.H + h] = m_start;
   }
   pdl_launch_dependents();
   if (i < end && slot_at) *reinterpret_cast<float4*>(slot_at) = S;
