@@ -196,7 +196,7 @@ linrec_kernel(const float* __restrict__ q, long q_stride, const float* __restric
               long g_stride, const float* __restrict__ p0, const float* __restrict__ p1, const float* __restrict__ p2,
               float cap, float q_scale, const int* __restrict__ cu_tokens, const int* __restrict__ state_slots,
               float* __restrict__ state, long state_stride, int num_slots, float* __restrict__ out, long out_stride,
-              int H, int qk_heads, int N, int dv, int vec, int* err) {
+              int H, int qk_heads, int N, int dv, int vec, float* __restrict__ fresh, int* err) {
   constexpr int NPS = 8 * (RPL + 4);                   // a staged row: 8 lanes' rows, each lane's share 16 bytes further on
   constexpr int REAL = MODE == 1 ? LR_COLS - 1 : LR_COLS;   // columns of S per block
   extern __shared__ __align__(16) float lr_smem[];
@@ -347,12 +347,28 @@ linrec_kernel(const float* __restrict__ q, long q_stride, const float* __restric
 #pragma unroll
       for (int i = 0; i < RPL; ++i) { const int r = sub * RPL + i; if (r < N) S_h[(size_t)r * dv + c] = S[i]; }
     } else if (blockIdx.x == 0) {
+      // every block of this (request, head) starts from the slot's n and m, and one that starts late must still find the old
+      // ones: the new ones wait in `fresh` for linrec_store_kernel
 #pragma unroll
-      for (int i = 0; i < RPL; ++i) { const int r = sub * RPL + i; if (r < N) n_h[r] = S[i]; }
+      for (int i = 0; i < RPL; ++i) { const int r = sub * RPL + i; if (r < N) fresh[((size_t)s * H + h) * (N + 1) + r] = S[i]; }
     }
   }
   __syncthreads();
-  if (MODE == 1 && m_h && tid == 0 && blockIdx.x == 0) *m_h = m_run;
+  if (MODE == 1 && m_h && tid == 0 && blockIdx.x == 0) fresh[((size_t)s * H + h) * (N + 1) + N] = m_run;
+}
+
+// Mode 1: the new n and m [S][H][N + 1] go to the requests' slots once no block reads the old ones any more.  Bound by its launch.
+__global__ void __launch_bounds__(128)
+linrec_store_kernel(const float* __restrict__ fresh, const int* __restrict__ state_slots, float* __restrict__ state, long state_stride,
+                    int num_slots, int H, int N, int dv) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int h = blockIdx.x, s = blockIdx.y, slot = state_slots[s];
+  if (slot < 0 || slot >= num_slots) return;
+  float* n0 = state + (size_t)slot * state_stride + (size_t)H * N * dv;
+  const float* from = fresh + ((size_t)s * H + h) * (N + 1);
+  for (int r = threadIdx.x; r < N; r += 128) n0[(size_t)h * N + r] = from[r];
+  if (threadIdx.x == 0) n0[(size_t)H * N + h] = from[N];
 }
 
 template <int MODE, int RPL>
@@ -360,15 +376,18 @@ static int linrec_go(dim3 grid, cudaStream_t stream, const float* q, long q_stri
                      long v_stride, const float* ga, const float* gb, long g_stride, const float* p0, const float* p1,
                      const float* p2, float cap, float q_scale, const int* cu_tokens, const int* state_slots, float* state,
                      long state_stride, int num_slots, float* out, long out_stride, int H, int qk_heads, int N, int dv, int vec,
-                     int* err) {
+                     float* fresh, int* err) {
   const size_t smem = ((size_t)4 * LR_CHUNK * 8 * (RPL + 4) + 2 * LR_CHUNK * LR_COLS + 4 * LR_CHUNK) * sizeof(float);
   if (smem > 36 * 1024) {                              // with the 9 KB of static arrays this passes the default limit
     cudaError_t e = cudaFuncSetAttribute(linrec_kernel<MODE, RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
   linrec_kernel<MODE, RPL><<<grid, LR_THREADS, smem, stream>>>(q, q_stride, k, k_stride, v, v_stride, ga, gb, g_stride, p0, p1, p2, cap,
-      q_scale, cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, vec, err);
-  return launch_status();
+      q_scale, cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, vec, fresh, err);
+  const int st = launch_status();
+  if (MODE != 1 || st != 0) return st;
+  return launch_pdl(linrec_store_kernel, dim3(H, grid.z), dim3(128), 0, stream, (const float*)fresh, state_slots, state, state_stride, num_slots, H,
+                    N, dv);
 }
 
 template <int MODE>
@@ -376,11 +395,11 @@ static int linrec_launch(int rpl, dim3 grid, cudaStream_t stream, const float* q
                          const float* v, long v_stride, const float* ga, const float* gb, long g_stride, const float* p0,
                          const float* p1, const float* p2, float cap, float q_scale, const int* cu_tokens,
                          const int* state_slots, float* state, long state_stride, int num_slots, float* out, long out_stride,
-                         int H, int qk_heads, int N, int dv, int* err) {
+                         int H, int qk_heads, int N, int dv, float* fresh, int* err) {
   // 16-byte copies of keys and queries when every row piece is aligned
   const int vec = (N % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)k & 15) == 0) ? 1 : 0;
 #define LR_GO(R) return linrec_go<MODE, R>(grid, stream, q, q_stride, k, k_stride, v, v_stride, ga, gb, g_stride, p0, p1, p2, cap, q_scale, \
-      cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, vec, err)
+      cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, vec, fresh, err)
   if (rpl <= 4) LR_GO(4);
   if (rpl <= 8) LR_GO(8);
   if (rpl <= 12) LR_GO(12);
@@ -639,16 +658,16 @@ static int linrec_rows_go(cudaStream_t stream, const float* q, long q_stride, co
 // [H] (mode 0: A_log, dt_bias, D; mode 1: the input gate's bias, the forget gate's bias, unused).  cap: the gates' bound
 // (mode 1).  Mode 2: k holds the raw gates z, p0 and p1 float [qk_heads * N] their biases and lower bounds; p0 null: q and k
 // hold silu(q) and the write gates already (photon_linrec_gates); ga, gb are not read.  q_scale multiplies the queries.  out float [T][H * dv] (row stride out_stride).  Head h reads query/key head
-// h / (H / qk_heads).  state: float [num_slots][state_stride], see the top of the file.
+// h / (H / qk_heads).  state: float [num_slots][state_stride], see the top of the file.  fresh (mode 1): scratch, float [S][H][N + 1].
 PHOTON_API int photon_linrec(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
                              long v_stride, const float* ga, const float* gb, long g_stride, const float* p0, const float* p1,
                              const float* p2, float cap, float q_scale, const int* cu_tokens, const int* state_slots,
                              float* state, long state_stride, int num_slots, float* out, long out_stride, int S, int H,
-                             int qk_heads, int N, int dv, int* err, cudaStream_t stream) {
+                             int qk_heads, int N, int dv, float* fresh, int* err, cudaStream_t stream) {
   if (S <= 0) return 0;
   if (mode < 0 || mode > 2 || (mode == 2 && (p0 == nullptr) != (p1 == nullptr))) return PHOTON_ERR_ARGUMENT;
   if (H <= 0 || qk_heads <= 0 || H % qk_heads || N <= 0 || dv <= 0) return PHOTON_ERR_ARGUMENT;
-  if (mode == 1 && !(cap > 0.f)) return PHOTON_ERR_ARGUMENT;
+  if (mode == 1 && (!(cap > 0.f) || fresh == nullptr)) return PHOTON_ERR_ARGUMENT;
   if (N > 512 || H > 65535 || S > 65535) return PHOTON_ERR_UNSUPPORTED;
   if (mode == 2) {
 #define LR_ROWS(L, R) return linrec_rows_go<L, R>(stream, q, q_stride, k, k_stride, v, v_stride, p0, p1, q_scale, cu_tokens, state_slots, \
@@ -664,7 +683,7 @@ PHOTON_API int photon_linrec(int mode, const float* q, long q_stride, const floa
   dim3 grid((dv + real - 1) / real, H, S);
   if (mode == 0)
     return linrec_launch<0>(rpl, grid, stream, q, q_stride, k, k_stride, v, v_stride, ga, gb, g_stride, p0, p1, p2, cap, q_scale,
-                            cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, err);
+                            cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, nullptr, err);
   return linrec_launch<1>(rpl, grid, stream, q, q_stride, k, k_stride, v, v_stride, ga, gb, g_stride, p0, p1, p2, cap, q_scale,
-                          cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, err);
+                          cu_tokens, state_slots, state, state_stride, num_slots, out, out_stride, H, qk_heads, N, dv, fresh, err);
 }

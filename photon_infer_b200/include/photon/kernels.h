@@ -315,12 +315,12 @@ PHOTON_EXPORT int photon_conv_state(const void* x, long x_stride, int x_dtype, i
  * dt_bias, D).  mode 1: a matrix memory with capped log gates and a running maximum (ga, gb the raw input and forget
  * gates, p0, p1 their biases; out = o / (max(|n . q|, exp(-m)) + 1e-6); n [H][N] and m [H] follow S in the state row).
  * mode 2: a gate per row, S_t = S_(t-1) + k (v^T - S_(t-1)), k = (1 - p1) / (1 + exp(z + p0)) with the raw gates z in k and p0,
- * p1 [qk_heads * N], queries silu(q); p0 null: q and k come from photon_linrec_gates. */
+ * p1 [qk_heads * N], queries silu(q); p0 null: q and k come from photon_linrec_gates.  fresh (mode 1): scratch [S][H][N + 1]. */
 PHOTON_EXPORT int photon_linrec(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
                      long v_stride, const float* ga, const float* gb, long g_stride, const float* p0, const float* p1,
                      const float* p2, float cap, float q_scale, const int* cu_tokens, const int* state_slots, float* state,
                      long state_stride, int num_slots, float* out, long out_stride, int S, int H, int qk_heads, int N, int dv,
-                     int* err, cudaStream_t stream);
+                     float* fresh, int* err, cudaStream_t stream);
 /* Mode 2's inputs of a long portion: q_out = silu(q), k_out = (1 - lower) / (1 + exp(z + bias)); q, z float [T][C] views. */
 PHOTON_EXPORT int photon_linrec_gates(const float* q, long q_stride, const float* z, long z_stride, const float* bias,
                            const float* lower, float* q_out, float* k_out, long out_stride, int T, int C, cudaStream_t stream);

@@ -1846,11 +1846,12 @@ def linrec(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate_a:
     f = _fn("linrec", "photon_linrec",
             [c_int, c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_void_p,
              c_float, c_float, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_long, c_int, c_int, c_int, c_int, c_int,
-             c_void_p, c_void_p])
+             c_void_p, c_void_p, c_void_p])
+    fresh = torch.empty((num_seqs * heads * (dim + 1),), dtype=torch.float32, device=q.device) if mode == "matrix_memory" else None
     _check(f(LINREC_MODES[mode], _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(gate_a), _ptr(gate_b),
              gate_a.stride(0) if gate_a is not None else 0, _ptr(p0), _ptr(p1), _ptr(p2), float(cap), float(q_scale), _ptr(cu_tokens), _ptr(state_slots),
              _ptr(state), state.stride(0), state.shape[0], _ptr(out), out.stride(0), int(num_seqs), heads, qk_heads, dim, vdim,
-             _ptr(err), _stream()), "linrec")
+             _ptr(fresh), _ptr(err), _stream()), "linrec")
 
 
 #: A bfloat16 step in which some request brings at least this many tokens cuts its recurrences into segments: two of 64 tokens are the
