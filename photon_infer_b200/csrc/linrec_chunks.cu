@@ -121,8 +121,9 @@ __device__ __forceinline__ void lc_product(uint32_t d, uint32_t a, uint32_t b, i
 // ---------------------------------------------------------------- 1: gates
 // With F the sum of the logarithms of the decays since the chunk's start, mode 0 needs exp(F_t - F_s) dt_s.  Mode 1 needs exp(F_t - F_s +
 // i_s - m_t) with the running maximum m_t = F_t + max(m before the chunk, M_t), M_t the largest i_s - F_s so far: exp((i_s - F_s) -
-// max(m, M_t)), from which F_t has gone.  What is subtracted is kept as two floats of a 64-bit sum.
-// Planes: mode 0 F (high, low), dt; mode 1 i - F (high, low), M (high, low), F.  A warp per (chunk, head), 32 tokens at a time.
+// max(m, M_t)), from which F_t has gone.  What is subtracted is kept as two floats of a 64-bit sum; so is F_t, because m_t itself is
+// the outputs' floor exp(-m_t) and F_t and M_t, hundreds each, cancel there.
+// Planes: mode 0 F (high, low), dt; mode 1 i - F (high, low), M (high, low), F (high, low).  A warp per (chunk, head), 32 tokens at a time.
 template <int MODE>
 __global__ void __launch_bounds__(128)
 lc_gates_kernel(const float* __restrict__ ga, const float* __restrict__ gb, long g_stride, const float* __restrict__ p0,
@@ -179,7 +180,9 @@ lc_gates_kernel(const float* __restrict__ ga, const float* __restrict__ gb, long
         A.gates[2 * TH + at] = take;
       } else {
         const float mh = (float)most;
-        A.gates[2 * TH + at] = mh; A.gates[3 * TH + at] = (float)(most - (double)mh); A.gates[4 * TH + at] = (float)F;
+        const float fh = (float)F;
+        A.gates[2 * TH + at] = mh; A.gates[3 * TH + at] = (float)(most - (double)mh);
+        A.gates[4 * TH + at] = fh; A.gates[5 * TH + at] = (float)(F - (double)fh);
       }
     }
     sum = __shfl_sync(0xffffffffu, F, 31);
@@ -198,7 +201,7 @@ struct LcShared {
   uint64_t bar;
   uint32_t tmem;
   int abort;
-  float hi[LC_T], lo[LC_T], take[LC_T];               // modes 0, 1: a token's F or i - F, and dt
+  float hi[LC_T], lo[LC_T], take[LC_T];               // modes 0, 1: a token's F or i - F, and dt or exp(-m_t)
   float m[LC_T], ml[LC_T];                            // mode 1: max(m before the chunk, M)
   float by[LC_T];                                     // modes 0, 1: the weight of S_0 in a token's output
   float group[8][LC_T], lacks[8][LC_T];               // modes 2, 3: the decay through 16 tokens and what it lacks to 1
@@ -527,7 +530,8 @@ lc_out_kernel(const LcArgs A) {
         const bool before = m0 > mh;                  // NaN: the token's own
         sh.m[tid] = before ? m0 : mh;
         sh.ml[tid] = before ? 0.f : ml;
-        sh.take[tid] = in ? A.gates[4 * TH + at] : 0.f;     // F
+        // high parts first: their sum is rounded relative to itself, however large they are
+        sh.take[tid] = in ? expf(-((A.gates[4 * TH + at] + sh.m[tid]) + (A.gates[5 * TH + at] + sh.ml[tid]))) : 0.f;
         sh.by[tid] = expf((m0 - sh.m[tid]) - sh.ml[tid]);
       }
     }
@@ -709,7 +713,7 @@ lc_out_kernel(const LcArgs A) {
     if (tid < p.cnt) {
       const float nq = ((sh.den[0][tid] + sh.den[1][tid]) + (sh.den[2][tid] + sh.den[3][tid])) +
                        sh.by[tid] * sh.qn[tid];
-      A.den[(size_t)(p.t0 + tid) * A.H + p.h] = fmaxf(fabsf(nq * A.q_scale), expf(-(sh.take[tid] + sh.m[tid]))) + 1e-6f;
+      A.den[(size_t)(p.t0 + tid) * A.H + p.h] = fmaxf(fabsf(nq * A.q_scale), sh.take[tid]) + 1e-6f;
     }
   }
   uint32_t in[32];
@@ -746,7 +750,7 @@ lc_out_kernel(const LcArgs A) {
 // ---------------------------------------------------------------- host side
 static void lc_parts(int mode, int T, int chunks, int H, int N, int dv, long (&part)[4]) {
   auto four = [](long n) { return (n + 3) & ~3L; };
-  part[0] = four(mode == 0 ? 3L * T * H : mode == 1 ? 5L * T * H : 0);
+  part[0] = four(mode == 0 ? 3L * T * H : mode == 1 ? 6L * T * H : 0);
   part[1] = four((long)chunks * H * N * dv);
   part[2] = four((long)chunks * H * N);
   part[3] = four((long)chunks * H * 4);

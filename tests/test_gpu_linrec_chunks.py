@@ -106,6 +106,36 @@ def test_slow_decays_keep_their_bits(mode, gates):
     segments.test_slow_decays_keep_their_bits(mode, gates)
 
 
+@pytest.mark.parametrize("forget", [2.0, -3.0, -15.0])
+def test_floors_of_the_matrix_memory_keep_their_bits(forget):
+    """Small queries, so that an output is divided by exp(-m_t), and forget gates whose logarithms since the chunk's start add up to
+    1,900: m_t stays as small as the input gates.  The outputs are no further from 64 bits than the walk's, or within four roundings
+    (the gates, the exponential, the division, the sum)."""
+    from photon_infer_b200.kernels import ops
+    gen = torch.Generator().manual_seed(11)
+    H, N, dv, T = 2, 64, 32, 300
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)
+    q, k, v = 1e-4 * rand(T, H * N), rand(T, H * N), rand(T, H * dv)
+    gates = torch.cat([-3.0 + rand(T, H), forget + rand(T, H)], dim=1)
+    zero, scale, width = torch.zeros(H, device=DEV), N ** -0.5, H * N * dv + H * N + 4
+    outs = []
+    for chunks in (True, False):
+        st, out = torch.zeros(1, width, device=DEV), torch.empty(T, H * dv, device=DEV)
+        args = (gates[:, :H], gates[:, H:], zero, zero, None, 15.0, scale, i32([0, T]), i32([0]), st, out)
+        if chunks:
+            den = ops.linrec_chunks("matrix_memory", q, k, v, None, *args, [T], H, H, N, dv, None)
+            out = (out.view(T, H, dv) / den.unsqueeze(-1)).view(T, H * dv)
+        else:
+            ops.linrec("matrix_memory", q, k, v, *args, 1, H, H, N, dv, None)
+        outs.append(out)
+    heads, d = (lambda x: x.double().view(T, H, -1)), (lambda x: x.double())
+    none = lambda *shape: torch.zeros(*shape, dtype=torch.float64, device=DEV)
+    want, _, _, _ = _walk("matrix_memory", heads(q), heads(k), heads(v), None, d(gates[:, :H]), d(gates[:, H:]), d(zero), d(zero), None, 15.0, scale,
+                          none(H, N, dv), none(H, N), none(H))
+    errors = [_rel(o, want) for o in outs]
+    assert errors[0] <= max(1.1 * errors[1], 2.0 ** -22), errors
+
+
 @pytest.mark.parametrize("C", [128, 40])
 def test_raw_gates_are_those_of_the_gates_kernel(C):
     from photon_infer_b200.kernels import ops
