@@ -49,10 +49,6 @@ __device__ __forceinline__ void ft_st8(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-__device__ __forceinline__ void ft_ld8(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
-}
 // Two neighbours of K as packed parts.
 __device__ __forceinline__ void ft_split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = at_pack(x, y);
@@ -363,7 +359,7 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       for (int q = 0; q < HC; q += STEP) {
         uint32_t v[STEP];
 #pragma unroll
-        for (int i = 0; i < STEP; i += 8) ft_ld8(tmem + buf * Shape::d_cols + lanes + col0 + q + i, v + i);
+        for (int i = 0; i < STEP; i += 8) tc_ld8_issue(tmem + buf * Shape::d_cols + lanes + col0 + q + i, v + i);
         tc_ld_wait();
         if (q + STEP >= HC) {
           tc_fence_before();

@@ -103,6 +103,11 @@ __device__ __forceinline__ void lc_put4(unsigned char* plane, int row, int col, 
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(d + i * LC_PART) = p[i];
 }
 // D = A B over 128 of K.  An operand is K-major (a row for every M or N) or MN-major (a row for every K).
+// The tensor cores truncate what they add to an accumulator, so each 32 of K have one of their own, 128 columns apart: two large
+// products each instead of eight in a row, and the four are added up in registers, rounded (lc_sum32).  Error of the outputs against 64
+// bits, 777 tokens of 128 x 128, one accumulator, four, and the segments: row decays near 1 2.5e-7, 1.5e-7, 2.3e-7, ordinary ones 2.0e-7, 1.5e-7,
+// 1.4e-7 (their state 8.1e-8, 8.4e-8, 1.2e-7); state space 9.6e-8, 6.8e-8, 4.4e-7.  It takes 1.5 % of a mixer's step (2,048 tokens, row decays, 221 ->
+// 225 us).  What the operands' products lost to rounding, carried in the third parts, gave 1 to 3 % of the error for 1 to 5 % of the step: not kept.
 template <bool A_MN, bool B_MN>
 __device__ __forceinline__ void lc_product(uint32_t d, uint32_t a, uint32_t b, int n) {
   const uint32_t idesc = tc_idesc(128, n) | (A_MN ? 1u << 15 : 0u) | (B_MN ? TC_IDESC_B_MN : 0u);
@@ -113,7 +118,25 @@ __device__ __forceinline__ void lc_product(uint32_t d, uint32_t a, uint32_t b, i
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const uint32_t kmajor = ((k >> 2) * LC_HALF + (k & 3) * 32) >> 4, mnmajor = k * 2048 >> 4;
-      tc_mma(d, aj + (A_MN ? mnmajor : kmajor), bj + (B_MN ? mnmajor : kmajor), idesc, (j > 0 || k > 0) ? 1u : 0u);
+      tc_mma(d + (k >> 1) * 128, aj + (A_MN ? mnmajor : kmajor), bj + (B_MN ? mnmajor : kmajor), idesc, (j > 0 || (k & 1)) ? 1u : 0u);
+    }
+  }
+}
+// 32 columns of a lane, the four accumulators added up; eight columns at a time, for the registers' sake.
+__device__ __forceinline__ void lc_sum32(uint32_t taddr, float* sum) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 8) {
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      uint32_t u[16];
+      tc_ld8_issue(taddr + i * 128 + c, u);
+      tc_ld8_issue(taddr + i * 128 + 128 + c, u + 8);
+      tc_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float pair = __uint_as_float(u[j]) + __uint_as_float(u[j + 8]);
+        sum[c + j] = i == 0 ? pair : sum[c + j] + pair;
+      }
     }
   }
 }
@@ -244,7 +267,7 @@ __device__ __forceinline__ void lc_put_value(unsigned char* plane, LcShared& sh,
   lc_put4(plane, t, col, v);
 }
 
-__device__ __forceinline__ void lc_set_up(LcShared& sh, int cols) {
+__device__ __forceinline__ void lc_set_up(LcShared& sh) {
   if (threadIdx.x == 0) {
     tc_mbar_init(&sh.bar, 1);
     sh.abort = 0;
@@ -254,21 +277,19 @@ __device__ __forceinline__ void lc_set_up(LcShared& sh, int cols) {
   if (threadIdx.x < 4) sh.direct[threadIdx.x] = 0;
   if (threadIdx.x == 0) sh.blocks = 1;
   if ((threadIdx.x >> 5) == 1) {
-    if (cols == 128) asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(tc_smem(&sh.tmem)) : "memory");
-    else asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc_smem(&sh.tmem)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc_smem(&sh.tmem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
 }
-__device__ __forceinline__ void lc_tear_down(LcShared& sh, int cols, int* err) {
+__device__ __forceinline__ void lc_tear_down(LcShared& sh, int* err) {
   tc_fence_before();
   __syncthreads();
   if ((threadIdx.x >> 5) == 1) {
     tc_fence_after();
-    if (cols == 128) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(sh.tmem) : "memory");
-    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(sh.tmem) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(sh.tmem) : "memory");
   }
   if (threadIdx.x == 0 && sh.abort) report_error(err, PHOTON_DEV_WAIT_TIMEOUT, blockIdx.x, blockIdx.y, 0);
 }
@@ -321,7 +342,7 @@ lc_ends_kernel(const LcArgs A) {
   pdl_wait();
   if (!lc_place(A, p)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  lc_set_up(sh, 128);
+  lc_set_up(sh);
   const float* v0 = A.v + (size_t)p.t0 * A.v_stride + (size_t)p.h * A.dv;
   if (MODE < 2) {
     const float* k0 = A.k + (size_t)p.t0 * A.k_stride + (size_t)p.hq * A.N;
@@ -405,17 +426,17 @@ lc_ends_kernel(const LcArgs A) {
   pdl_launch_dependents();
   {
     const int col = (warp & 3) * 32 + lane, n0 = (warp >> 2) * 32;
-    uint32_t u[32];
-    tc_ld32(sh.tmem + ((uint32_t)((warp & 3) * 32) << 16) + n0, u);
+    float u[32];
+    lc_sum32(sh.tmem + ((uint32_t)((warp & 3) * 32) << 16) + n0, u);
     if (col < A.dv) {
       float* dst = A.ends + p.at * A.N * A.dv + (size_t)n0 * A.dv + col;
       const bool bad = sh.bad[col] < LC_T;
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        if (n0 + j < A.N) dst[(size_t)j * A.dv] = bad ? NAN : __uint_as_float(u[j]);
+        if (n0 + j < A.N) dst[(size_t)j * A.dv] = bad ? NAN : u[j];
     }
   }
-  lc_tear_down(sh, 128, A.err);
+  lc_tear_down(sh, A.err);
 }
 
 // ---------------------------------------------------------------- 3: from chunk to chunk
@@ -495,11 +516,11 @@ lc_out_kernel(const LcArgs A) {
   pdl_wait();
   if (!lc_place(A, p)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  lc_set_up(sh, 512);
+  lc_set_up(sh);
   uint32_t parity = 0;
   const uint32_t x = tc_smem(X), y = tc_smem(Y);
-  const uint32_t tp = sh.tmem, t_in = sh.tmem + 128, t_self = sh.tmem + 256;     // P^T, O^T from S_0, O^T from the chunk itself
-  const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+  const uint32_t acc = sh.tmem;                       // in turn P^T, O^T from S_0, O^T from the chunk itself: each takes all columns
+  const uint32_t mine = acc + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 32;
   const float* q0 = A.q + (size_t)p.t0 * A.q_stride + (size_t)p.hq * A.N;
   const float* v0 = A.v + (size_t)p.t0 * A.v_stride + (size_t)p.h * A.dv;
   const float* S0 = A.ends + p.at * A.N * A.dv;
@@ -553,7 +574,7 @@ lc_out_kernel(const LcArgs A) {
         if (lane == 0) sh.qn[t] = d;
       }
     }
-    lc_run(sh, [&]() { lc_product<false, false>(tp, y, x, 128); });                // P^T [s][t]
+    lc_run(sh, [&]() { lc_product<false, false>(acc, y, x, 128); });               // P^T [s][t]
     fetch_state();
     lc_done(sh, parity);
   } else {
@@ -637,7 +658,7 @@ lc_out_kernel(const LcArgs A) {
           lc_put2(Y, tg * 16 + i, n, direct ? 0.f : key[i].x / bx, direct ? 0.f : key[i].y / by);
         }
       }
-      lc_run(sh, [&]() { lc_product<false, false>(tp + t0, y, x + t0 * 128, span * 16); });      // P^T [s][t0 ..]
+      lc_run(sh, [&]() { lc_product<false, false>(acc + t0, y, x + t0 * 128, span * 16); });     // P^T [s][t0 ..]
       lc_done(sh, parity);
     }
     if (blocks > 1) put_queries(through(0, tg));                      // as S_0 sees them
@@ -673,19 +694,18 @@ lc_out_kernel(const LcArgs A) {
   }
   if (MODE >= 2) fetch_state();                       // no earlier: the keys' registers
   put_state();
-  lc_run(sh, [&]() { lc_product<true, false>(t_in, y, x, 128); });                 // O^T [dv][t]: rows of S_0 are K
   float pw[32];                                       // P^T of token s (this lane's row), 32 tokens t
   const int s = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
+  lc_sum32(mine, pw);
+  lc_run(sh, [&]() { lc_product<true, false>(acc, y, x, 128); });                  // O^T [dv][t]: rows of S_0 are K
   {
-    uint32_t u[32];
-    tc_ld32(tp + lanes + c0, u);
     const float fs_hi = MODE < 2 ? sh.hi[s] : 0.f, fs_lo = MODE < 2 ? sh.lo[s] : 0.f, take = MODE < 2 ? sh.take[s] : 0.f;
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
       const int t = c0 + j;
       float w = 0.f;
       if (s <= t && t < p.cnt) {
-        w = __uint_as_float(u[j]);
+        w = pw[j];
         if (MODE < 2) {
           w *= MODE == 0 ? expf((sh.hi[t] - fs_hi) + (sh.lo[t] - fs_lo)) * take : expf((fs_hi - sh.m[t]) + (fs_lo - sh.ml[t]));
         }
@@ -705,7 +725,9 @@ lc_out_kernel(const LcArgs A) {
   for (int i = 0; i < 8; ++i) lc_put_value(Y, sh, warp + i * 16, lane * 4, ahead[i]);
 #pragma unroll
   for (int j = 0; j < 32; j += 4) lc_put4(X, s, c0 + j, make_float4(pw[j], pw[j + 1], pw[j + 2], pw[j + 3]));
-  lc_run(sh, [&]() { lc_product<true, true>(t_self, y, x, 128); });                // O^T [dv][t]: tokens s are K of both
+  float in[32];
+  lc_sum32(mine, in);
+  lc_run(sh, [&]() { lc_product<true, true>(acc, y, x, 128); });                   // O^T [dv][t]: tokens s are K of both
   if (MODE == 1) {
     lr_meet<16, 32>(pw, lane);                        // lane l: the sum over the warp's 32 tokens s for token c0 + l
     sh.den[warp & 3][c0 + lane] = pw[0];
@@ -716,13 +738,11 @@ lc_out_kernel(const LcArgs A) {
       A.den[(size_t)(p.t0 + tid) * A.H + p.h] = fmaxf(fabsf(nq * A.q_scale), sh.take[tid]) + 1e-6f;
     }
   }
-  uint32_t in[32];
-  tc_ld32(t_in + lanes + c0, in);
   lc_done(sh, parity);
   pdl_launch_dependents();
   {
-    uint32_t u[32];
-    tc_ld32(t_self + lanes + c0, u);
+    float u[32];
+    lc_sum32(mine, u);
     const int col = (warp & 3) * 32 + lane;
     if (col < A.dv) {
       const float skip = MODE == 0 ? A.d_skip[p.h] : 0.f;
@@ -732,8 +752,7 @@ lc_out_kernel(const LcArgs A) {
       float o[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float a = __uint_as_float(in[j]), b = __uint_as_float(u[j]);
-        o[j] = (MODE < 2 ? fmaf(sh.by[c0 + j], a, b) : a + b) * A.q_scale;
+        o[j] = (MODE < 2 ? fmaf(sh.by[c0 + j], in[j], u[j]) : in[j] + u[j]) * A.q_scale;
         if (MODE == 0) o[j] = fmaf(skip, j < last ? vv[(size_t)j * A.v_stride] : 0.f, o[j]);
       }
       if (bad < LC_T) {
@@ -744,7 +763,7 @@ lc_out_kernel(const LcArgs A) {
       for (int j = 0; j < 32; ++j) if (j < last) dst[(size_t)j * A.out_stride] = o[j];
     }
   }
-  lc_tear_down(sh, 512, A.err);
+  lc_tear_down(sh, A.err);
 }
 
 // ---------------------------------------------------------------- host side

@@ -1,10 +1,9 @@
 """The recurrences in chunks of 128 tokens on the tensor cores (linrec_chunks.cu) against the same recurrence token by token in 64
 bits: chunks that are not full, states that are not zero, reused and negative slots, small states, decays of nearly nothing, and
-values that are not finite; and over 2,048 tokens an error that is not larger than the walk's."""
+values that are not finite; and an error against 64 bits that is not larger than the segments'."""
 import pytest
 import torch
 
-import test_gpu_linrec_segments as segments
 from test_gpu_linrec_segments import _rel, _walk, i32
 
 pytestmark = pytest.mark.gpu
@@ -100,10 +99,41 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(mode, value):
     assert torch.equal(S[:, :, 4:], clean_after[0, :H * N * dv].view(H, N, dv)[:, :, 4:])
 
 
-@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("mode", ["state_space", "matrix_memory", "decay_rows"])
 @pytest.mark.parametrize("gates", ["constant", "nearly constant", "ordinary"])
-def test_slow_decays_keep_their_bits(mode, gates):
-    segments.test_slow_decays_keep_their_bits(mode, gates)
+@pytest.mark.parametrize("H,N,dv,T", [(2, 64, 32, 2048), (4, 128, 128, 777)])
+def test_errors_are_not_larger_than_the_segments(mode, gates, H, N, dv, T):
+    """Against 64 bits, decays of nearly 1 and ordinary ones, on the same inputs; a tenth for two orders of the same roundings."""
+    from photon_infer_b200.kernels import ops
+    gen = torch.Generator().manual_seed(len(mode) + len(gates))
+    vary = {"constant": 0.0, "nearly constant": 0.01, "ordinary": 1.0}[gates]
+    slow, memory = gates != "ordinary", mode == "matrix_memory"
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(DEV)
+    full = lambda x: torch.full((H,), x, device=DEV)
+    q, k, v = rand(T, H * N), rand(T, H * N), rand(T, H * dv)
+    a = ga = gb = p0 = p1 = p2 = None
+    if mode == "decay_rows":
+        per_row = torch.rand(H * N, generator=gen).to(DEV)
+        a = torch.exp(torch.nn.functional.logsigmoid((4 + 3 * per_row if slow else per_row) + vary * rand(T, H * N)) / 16)
+    elif mode == "state_space":
+        ga, p0, p1, p2 = -4 + vary * rand(T, H), full(-3.0 if slow else 0.0), full(0.1), full(1.0)
+    else:
+        both = torch.cat([0.3 * rand(T, H), (6.0 if slow else 2.0) + vary * rand(T, H)], dim=1)
+        ga, gb, p0, p1 = both[:, :H], both[:, H:], full(0.0), full(0.0)
+    cap, scale, size = (15.0 if memory else 0.0), N ** -0.5, H * N * dv + (H * N + H if memory else 0)
+    results = []
+    for way in (ops.linrec_chunks, ops.linrec_segments):
+        st, out = torch.zeros(1, size + -size % 4, device=DEV), torch.empty(T, H * dv, device=DEV)
+        length = {} if way is ops.linrec_chunks else {"segment": ops.linrec_segment_tokens([T], H, ops.linrec_segment_blocks(N, dv), ops.sm_count(st.device))}
+        den = way(mode, q, k, v, a, ga, gb, p0, p1, p2, cap, scale, i32([0, T]), i32([0]), st, out, [T], H, H, N, dv, None, **length)
+        results.append(((out.view(T, H, dv) / den.unsqueeze(-1)).view(T, H * dv) if memory else out, st))
+    d = lambda x: None if x is None else x.double()
+    heads = lambda x: None if x is None else x.double().view(T, H, -1)
+    zero = lambda *shape: torch.zeros(*shape, dtype=torch.float64, device=DEV)
+    want, S, n, m = _walk(mode, heads(q), heads(k), heads(v), heads(a), d(ga), d(gb), d(p0), d(p1), d(p2), cap, scale, zero(H, N, dv), zero(H, N), zero(H))
+    errors = [(_rel(out, want), _rel(st[0, :H * N * dv], S.flatten())) for out, st in results]
+    print("chunks and segments (outputs, state):", errors)
+    assert errors[0][0] <= 1.1 * errors[1][0] and errors[0][1] <= 1.1 * errors[1][1], errors
 
 
 @pytest.mark.parametrize("forget", [2.0, -3.0, -15.0])
