@@ -2,8 +2,10 @@
 // accuracy.
 //
 //   S_t = keep_t S_(t-1) + take_t k_t v_t^T        modes 0 (state space) and 1 (matrix memory): one number per head and token
-//   S_t = S_(t-1) + k_t (v_t^T - S_(t-1))           mode 2 (forget and write): a number per row
 //   S_t = diag(a_t) S_(t-1) + k_t v_t^T             mode 3 (gated linear attention): a number per row
+//
+// Mode 2 (forget and write) stays with the segments: the error of its outputs against 64 bits was 1.2e-7 to 1.3e-7 here and 0.9e-7 to 1.0e-7 there
+// (ordinary gates), and write gates near 1 took the blocks below one by one (512 tokens of 16 heads, 374 us against 68).
 //
 // With w(t, s) the decay from token s to token t (times what s takes) and w(t) that from the chunk's start S_0,
 //   o_t = w(t) q_t^T S_0 + sum over s <= t of w(t, s) (q_t . k_s) v_s        S_128 = w(128) S_0 + sum over s of w(128, s) k_s v_s^T
@@ -17,7 +19,7 @@
 // swizzled halves; whether a product reads them along the rows or across is a bit of its descriptors, so nothing is transposed.  Of
 // the nine products of parts the six largest are formed, the small ones first.
 //
-// Modes 2 and 3: w(t, s) differs from row to row of the state, so it has to be in the operands: q_t b_t and k_s / b_s with b the
+// Mode 3: w(t, s) differs from row to row of the state, so it has to be in the operands: q_t b_t and k_s / b_s with b the
 // product of the decays since a reference, the chunk's start while no row's decays multiply to less than LC_SMALL there.  Else
 // blocks of 64 or 32 tokens take their own starts: for the queries of block j, keys of the blocks before it are multiplied by decays
 // up to the start of j (at most 1), those of j itself divided by theirs; and the weights of a block of 32 that is still out of range
@@ -29,7 +31,7 @@
 // longer.  Rows by bulk copies instead of loads into registers, and calls instead of inlined splits, changed nothing.
 // Measured, heads of 128 x 128, the recurrence alone, us, segments first: gated linear attention, 2,048 tokens of 16 heads 176 and 102
 // (26 for the sums, 14 from chunk to chunk, 62 for the outputs); matrix memory, two requests of 2,815 251 and 131; state space, 2,048 161
-// and 93; forget and write, 777 91 (with its gates) and 60.
+// and 93.
 //
 // A value that is not finite would reach earlier tokens of its chunk through products with weights of 0: it is left out of
 // the products, and its column is NaN from its token on.
@@ -46,11 +48,10 @@
 
 struct LcArgs {
   const float* q; long q_stride;                     // [T][qk_heads * N]
-  const float* k; long k_stride;                     // [T][qk_heads * N]: keys; mode 2: write gates
+  const float* k; long k_stride;                     // [T][qk_heads * N]
   const float* v; long v_stride;                     // [T][H * dv]
   const float* a; long a_stride;                     // mode 3: [T][qk_heads * N] decays
   const float* d_skip;                               // mode 0: [H]
-  const float* bias; const float* lower;             // mode 2: [qk_heads * N], or null: q and k as photon_linrec_gates leaves them
   float q_scale;
   const int* cu_tokens;
   const int* state_slots;
@@ -59,7 +60,7 @@ struct LcArgs {
   float* den;                                        // mode 1: [T][H], what the outputs are to be divided by
   float* gates;                                      // planes [T][H], see lc_gates_kernel
   float* ends;                                       // [chunks][H][N * dv]: U, then S_0
-  float* vecs;                                       // [chunks][H][N]: mode 1 the sum of keys, then n at the start; modes 2, 3 the rows' decay (lc_code)
+  float* vecs;                                       // [chunks][H][N]: mode 1 the sum of keys, then n at the start; mode 3 the rows' decay (lc_code)
   float* scale;                                      // [chunks][H][4]: the chunk's F (high, low); mode 1 also F + M
   int T, S, H, qk_heads, N, dv, chunks;
   int* err;
@@ -227,10 +228,10 @@ struct LcShared {
   float hi[LC_T], lo[LC_T], take[LC_T];               // modes 0, 1: a token's F or i - F, and dt or exp(-m_t)
   float m[LC_T], ml[LC_T];                            // mode 1: max(m before the chunk, M)
   float by[LC_T];                                     // modes 0, 1: the weight of S_0 in a token's output
-  float group[8][LC_T], lacks[8][LC_T];               // modes 2, 3: the decay through 16 tokens and what it lacks to 1
+  float group[8][LC_T], lacks[8][LC_T];               // mode 3: the decay through 16 tokens and what it lacks to 1
   int bad[LC_T];                                      // the first token whose value in this column is not finite
   float qn[LC_T], den[4][LC_T];                       // mode 1
-  int blocks;                                         // modes 2, 3: blocks with references of their own
+  int blocks;                                         // mode 3: blocks with references of their own
   int direct[4];                                      // those of 32 whose weights are formed one by one,
   float self[4][32][33];                              // and those: [block][s][t]
 };
@@ -311,23 +312,12 @@ __device__ __forceinline__ void lc_done(LcShared& sh, uint32_t& parity) {
   tc_fence_after();
 }
 
-// Modes 2 and 3, two rows of a token: the keys (mode 2: the write gates), and the decays as they lie in memory (mode 3); then the decays and what they lack to 1.
-// Tokens behind the chunk and rows behind the state keep everything.
-template <int MODE>
-__device__ __forceinline__ void lc_row_gate(const LcArgs& A, const LcPlace& p, int t, int n, float2& key, float2& raw) {
-  key = make_float2(0.f, 0.f); raw = make_float2(1.f, 1.f);
+// Mode 3, two rows of a token: the keys, and the decays.  Tokens behind the chunk and rows behind the state keep everything.
+__device__ __forceinline__ void lc_row_gate(const LcArgs& A, const LcPlace& p, int t, int n, float2& key, float2& decay) {
+  key = make_float2(0.f, 0.f); decay = make_float2(1.f, 1.f);
   if (t >= p.cnt || n >= A.N) return;
   key = *reinterpret_cast<const float2*>(A.k + (size_t)(p.t0 + t) * A.k_stride + (size_t)p.hq * A.N + n);
-  if (MODE == 2 && A.lower != nullptr) {
-    const float2 b = *reinterpret_cast<const float2*>(A.bias + p.hq * A.N + n), l = *reinterpret_cast<const float2*>(A.lower + p.hq * A.N + n);
-    key = make_float2(lr_write_gate(key.x, b.x, l.x), lr_write_gate(key.y, b.y, l.y));
-  }
-  if (MODE == 3) raw = *reinterpret_cast<const float2*>(A.a + (size_t)(p.t0 + t) * A.a_stride + (size_t)p.hq * A.N + n);
-}
-template <int MODE>
-__device__ __forceinline__ void lc_row_decay(float2 key, float2 raw, float2& decay, float2& gone) {
-  if (MODE == 3) { decay = raw; gone = make_float2(1.0f - raw.x, 1.0f - raw.y); }
-  else { gone = key; decay = make_float2(1.0f - key.x, 1.0f - key.y); }
+  decay = *reinterpret_cast<const float2*>(A.a + (size_t)(p.t0 + t) * A.a_stride + (size_t)p.hq * A.N + n);
 }
 
 // ---------------------------------------------------------------- 2: the chunks' sums
@@ -373,15 +363,14 @@ lc_ends_kernel(const LcArgs A) {
     float2 key[16], e[16];
     float2 b = make_float2(1.f, 1.f), B = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) lc_row_gate<MODE>(A, p, tg * 16 + i, n, key[i], e[i]);
+    for (int i = 0; i < 16; ++i) lc_row_gate(A, p, tg * 16 + i, n, key[i], e[i]);
     // the decay behind each token to the end of the 16, from the last on
 #pragma unroll
     for (int i = 15; i >= 0; --i) {
-      float2 decay, gone;
-      lc_row_decay<MODE>(key[i], e[i], decay, gone);
+      const float2 decay = e[i];
       e[i] = b;
-      lc_decay(decay.x * b.x, gone.x, b.x, B.x);
-      lc_decay(decay.y * b.y, gone.y, b.y, B.y);
+      lc_decay(decay.x * b.x, 1.0f - decay.x, b.x, B.x);
+      lc_decay(decay.y * b.y, 1.0f - decay.y, b.y, B.y);
     }
     *reinterpret_cast<float2*>(&sh.group[tg][n]) = b;
     *reinterpret_cast<float2*>(&sh.lacks[tg][n]) = B;
@@ -466,7 +455,7 @@ lc_scan_kernel(const LcArgs A) {
   float4 S = i < end && row0 ? *reinterpret_cast<const float4*>(slot_at) : make_float4(0.f, 0.f, 0.f, 0.f);
   const size_t step = vec ? (size_t)A.H * A.N : (size_t)A.H * size;
   float* at = (vec ? A.vecs + ((size_t)before * A.H + h) * A.N : A.ends + ((size_t)before * A.H + h) * size) + i;
-  const float* rows = A.vecs + ((size_t)before * A.H + h) * A.N + (i < size ? i / A.dv : 0);     // modes 2, 3: the row's decay
+  const float* rows = A.vecs + ((size_t)before * A.H + h) * A.N + (i < size ? i / A.dv : 0);     // mode 3: the row's decay
   float* sc = A.scale + ((size_t)before * A.H + h) * 4;
   float4 next = make_float4(0.f, 0.f, 0.f, 0.f), after = next;
   if (i < end) { next = *reinterpret_cast<const float4*>(at); if (nc > 1) after = *reinterpret_cast<const float4*>(at + step); }
@@ -583,13 +572,11 @@ lc_out_kernel(const LcArgs A) {
     float2 key[16], bq[16];                           // bq: first the decays as they lie in memory, then from the start of the sixteen on
     float2 b = make_float2(1.f, 1.f), B = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) lc_row_gate<MODE>(A, p, tg * 16 + i, n, key[i], bq[i]);
+    for (int i = 0; i < 16; ++i) lc_row_gate(A, p, tg * 16 + i, n, key[i], bq[i]);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      float2 decay, gone;
-      lc_row_decay<MODE>(key[i], bq[i], decay, gone);
-      lc_decay(decay.x * b.x, gone.x, b.x, B.x);
-      lc_decay(decay.y * b.y, gone.y, b.y, B.y);
+      lc_decay(bq[i].x * b.x, 1.0f - bq[i].x, b.x, B.x);
+      lc_decay(bq[i].y * b.y, 1.0f - bq[i].y, b.y, B.y);
       bq[i] = b;
     }
     *reinterpret_cast<float2*>(&sh.group[tg][n]) = b;
@@ -621,7 +608,6 @@ lc_out_kernel(const LcArgs A) {
         for (int i = 0; i < 8; ++i) {
           const int t = tg * 16 + g + i;
           q[i] = t < p.cnt && n < A.N ? *reinterpret_cast<const float2*>(q0 + (size_t)t * A.q_stride + n) : make_float2(0.f, 0.f);
-          if (MODE == 2 && A.lower != nullptr) q[i] = make_float2(lr_silu(q[i].x), lr_silu(q[i].y));
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) lc_put2(X, tg * 16 + g + i, n, q[i].x * (bq[g + i].x * f.x), q[i].y * (bq[g + i].y * f.y));
@@ -638,16 +624,14 @@ lc_out_kernel(const LcArgs A) {
         float2 d = make_float2(1.f, 1.f), l = make_float2(0.f, 0.f);               // behind a token to the end of its sixteen
 #pragma unroll
         for (int i0 = 12; i0 >= 0; i0 -= 4) {         // the decays once more, a few at a time: registers that spill go to L2 here
-          float2 raw[4], again;
+          float2 decay[4], again;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) lc_row_gate<MODE>(A, p, tg * 16 + i0 + i, n, again, raw[i]);
+          for (int i = 0; i < 4; ++i) lc_row_gate(A, p, tg * 16 + i0 + i, n, again, decay[i]);
 #pragma unroll
           for (int i = 3; i >= 0; --i) {
-            float2 decay, gone;
             lc_put2(Y, tg * 16 + i0 + i, n, key[i0 + i].x * (d.x * f.x), key[i0 + i].y * (d.y * f.y));
-            lc_row_decay<MODE>(key[i0 + i], raw[i], decay, gone);
-            lc_decay(decay.x * d.x, gone.x, d.x, l.x);
-            lc_decay(decay.y * d.y, gone.y, d.y, l.y);
+            lc_decay(decay[i].x * d.x, 1.0f - decay[i].x, d.x, l.x);
+            lc_decay(decay[i].y * d.y, 1.0f - decay[i].y, d.y, l.y);
           }
         }
       } else if (blk == j) {
@@ -668,22 +652,16 @@ lc_out_kernel(const LcArgs A) {
       if (blocks < 4 || !sh.direct[j]) continue;
       const int s = j * 32 + (tid >> 4), n8 = (tid & 15) * 8, last = min(p.cnt, j * 32 + 32);
       const size_t kb = (size_t)p.hq * A.N;
-      auto key_at = [&](int t, int u) {
-        const float k = A.k[(size_t)(p.t0 + t) * A.k_stride + kb + n8 + u];
-        return MODE == 2 && A.lower != nullptr ? lr_write_gate(k, A.bias[kb + n8 + u], A.lower[kb + n8 + u]) : k;
-      };
       float d[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) d[u] = s < last && n8 + u < A.N ? key_at(s, u) : 0.f;
+      for (int u = 0; u < 8; ++u) d[u] = s < last && n8 + u < A.N ? A.k[(size_t)(p.t0 + s) * A.k_stride + kb + n8 + u] : 0.f;
       for (int t = j * 32; t < last; ++t) {           // all lanes, for the sums' sake; before s nothing
         float o = 0.f;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           if (n8 + u < A.N) {
-            float q = q0[(size_t)t * A.q_stride + n8 + u];
-            if (MODE == 2 && A.lower != nullptr) q = lr_silu(q);
-            if (t > s) d[u] *= MODE == 3 ? A.a[(size_t)(p.t0 + t) * A.a_stride + kb + n8 + u] : 1.0f - key_at(t, u);
-            o = fmaf(d[u], q, o);
+            if (t > s) d[u] *= A.a[(size_t)(p.t0 + t) * A.a_stride + kb + n8 + u];
+            o = fmaf(d[u], q0[(size_t)t * A.q_stride + n8 + u], o);
           }
         }
 #pragma unroll
@@ -692,7 +670,7 @@ lc_out_kernel(const LcArgs A) {
       }
     }
   }
-  if (MODE >= 2) fetch_state();                       // no earlier: the keys' registers
+  if (MODE == 3) fetch_state();                       // no earlier: the keys' registers
   put_state();
   float pw[32];                                       // P^T of token s (this lane's row), 32 tokens t
   const int s = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
@@ -713,7 +691,7 @@ lc_out_kernel(const LcArgs A) {
       pw[j] = w;
     }
   }
-  if (MODE >= 2 && sh.blocks == 4 && sh.direct[warp >> 2] && (warp & 3) == (warp >> 2)) {
+  if (MODE == 3 && sh.blocks == 4 && sh.direct[warp >> 2] && (warp & 3) == (warp >> 2)) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) if (c0 + j >= s && c0 + j < p.cnt) pw[j] = sh.self[warp >> 2][lane][j];
   }
@@ -803,8 +781,8 @@ static int lc_go(const LcArgs& A, const float* ga, const float* gb, long g_strid
 }
 
 // As photon_linrec_segments, in chunks of 128 tokens on the tensor cores: `chunks` of them, the sum over the requests of their tokens / 128,
-// rounded up.  Mode 2: p0 and p1 float [qk_heads * N] (bias and lower bound: q and k raw) or null (q and k from photon_linrec_gates).  N and dv up to 128, multiples of 4; rows and bases 16-byte aligned.  Mode 1: den has T * H floats for the caller and chunks * H
-// behind them.  scratch: photon_linrec_chunks_scratch floats, 16-byte aligned.
+// rounded up.  Modes 0, 1 and 3.  N and dv up to 128, multiples of 4; rows and bases 16-byte aligned.  Mode 1: den has T * H floats for the
+// caller and chunks * H behind them.  scratch: photon_linrec_chunks_scratch floats, 16-byte aligned.
 PHOTON_API int photon_linrec_chunks(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
                                     long v_stride, const float* a, long a_stride, const float* ga, const float* gb, long g_stride,
                                     const float* p0, const float* p1, const float* p2, float cap, float q_scale,
@@ -812,17 +790,16 @@ PHOTON_API int photon_linrec_chunks(int mode, const float* q, long q_stride, con
                                     float* out, long out_stride, float* den, float* scratch, int T, int S, int H, int qk_heads,
                                     int N, int dv, int chunks, int* err, cudaStream_t stream) {
   if (S <= 0 || T <= 0) return 0;
-  if (mode < 0 || mode > 3 || H <= 0 || qk_heads <= 0 || H % qk_heads || N <= 0 || dv <= 0 || chunks <= 0) return PHOTON_ERR_ARGUMENT;
+  if (mode < 0 || mode > 3 || mode == 2 || H <= 0 || qk_heads <= 0 || H % qk_heads || N <= 0 || dv <= 0 || chunks <= 0) return PHOTON_ERR_ARGUMENT;
   if (scratch == nullptr || ((uintptr_t)scratch & 15) || (mode == 1 && (!(cap > 0.f) || den == nullptr)) || (mode == 3) != (a != nullptr))
     return PHOTON_ERR_ARGUMENT;
   if (N > LC_T || dv > LC_T || (N & 3) || (dv & 3) || H > 65535 || S > 65535 || (q_stride & 3) || (k_stride & 3) || (v_stride & 3) ||
       (a_stride & 3) || (state_stride & 3) || ((uintptr_t)q & 15) || ((uintptr_t)k & 15) || ((uintptr_t)v & 15) || ((uintptr_t)a & 15) ||
-      ((uintptr_t)state & 15) || (mode == 2 && (((uintptr_t)p0 & 7) || ((uintptr_t)p1 & 7))))
+      ((uintptr_t)state & 15))
     return PHOTON_ERR_UNSUPPORTED;
-  if (mode == 2 && (p0 == nullptr) != (p1 == nullptr)) return PHOTON_ERR_ARGUMENT;
   LcArgs A;
   A.q = q; A.q_stride = q_stride; A.k = k; A.k_stride = k_stride; A.v = v; A.v_stride = v_stride; A.a = a; A.a_stride = a_stride;
-  A.d_skip = p2; A.bias = mode == 2 ? p0 : nullptr; A.lower = mode == 2 ? p1 : nullptr; A.q_scale = q_scale; A.cu_tokens = cu_tokens; A.state_slots = state_slots; A.state = state; A.state_stride = state_stride;
+  A.d_skip = p2; A.q_scale = q_scale; A.cu_tokens = cu_tokens; A.state_slots = state_slots; A.state = state; A.state_stride = state_stride;
   A.num_slots = num_slots; A.out = out; A.out_stride = out_stride; A.den = den;
   A.T = T; A.S = S; A.H = H; A.qk_heads = qk_heads; A.N = N; A.dv = dv; A.chunks = chunks; A.err = err;
   long part[4];
@@ -833,6 +810,5 @@ PHOTON_API int photon_linrec_chunks(int mode, const float* q, long q_stride, con
   A.scale = A.vecs + part[2];
   if (mode == 0) return lc_go<0>(A, ga, gb, g_stride, p0, p1, cap, stream);
   if (mode == 1) return lc_go<1>(A, ga, gb, g_stride, p0, p1, cap, stream);
-  if (mode == 2) return lc_go<2>(A, ga, gb, g_stride, p0, p1, cap, stream);
   return lc_go<3>(A, ga, gb, g_stride, p0, p1, cap, stream);
 }

@@ -340,8 +340,8 @@ PHOTON_EXPORT int photon_linrec_segments(int mode, const float* q, long q_stride
                               int N, int dv, int seg, int segs, int cuts, int cut_segs, int* err, cudaStream_t stream);
 
 /* ------------------------------------------------------------------ linrec_chunks.cu: the same on the tensor cores, in chunks of 128 tokens */
-/* As photon_linrec_segments; `chunks`: the sum over the requests of their tokens / 128, rounded up.  N, dv <= 128 and multiples of
- * 4, rows and bases 16-byte aligned.  mode 2: p0, p1 [qk_heads * N] (raw q and gates k, as for photon_linrec) or null.  mode 1: den has room for (T + chunks) * H floats.  scratch: 16-byte aligned. */
+/* As photon_linrec_segments, without mode 2; `chunks`: the sum over the requests of their tokens / 128, rounded up.  N, dv <= 128 and
+ * multiples of 4, rows and bases 16-byte aligned.  mode 1: den has room for (T + chunks) * H floats.  scratch: 16-byte aligned. */
 PHOTON_EXPORT long photon_linrec_chunks_scratch(int mode, int T, int chunks, int H, int N, int dv);
 PHOTON_EXPORT int photon_linrec_chunks(int mode, const float* q, long q_stride, const float* k, long k_stride, const float* v,
                               long v_stride, const float* a, long a_stride, const float* ga, const float* gb, long g_stride,

@@ -1948,15 +1948,15 @@ LINREC_CHUNKS_MIN_TOKENS = 64
 #: Tokens x heads of a step from which the chunks are the faster way (below, a step waits for the host, and they are one launch more than the
 #: segments).  B200, heads of 128 x 128, a mixer's step, us, as before first: gated linear attention 640 tokens x 16 heads 160 and 149, 2,048 x
 #: 16 302 and 225, 256 x 32 155 and 153, 400 x 32 208 and 166; matrix memory 640 x 16 154 and 131, 400 x 16 136 and 132, 2,048 x 16 296 and 199;
-#: state space 640 x 16 160 and 149, 256 x 32 147 and 150, 2,048 x 16 294 and 221; forget and write 1,000 x 16 177 and 146, 640 x 32 213 and 220.
-LINREC_CHUNKS_FROM = {"decay_rows": 10000, "matrix_memory": 10000, "state_space": 10000, "forget_write": 12000}
+#: state space 640 x 16 160 and 149, 256 x 32 147 and 150, 2,048 x 16 294 and 221.  Forget and write stays with the segments (linrec_chunks.cu).
+LINREC_CHUNKS_FROM = {"decay_rows": 10000, "matrix_memory": 10000, "state_space": 10000}
 
 
 def linrec_chunks_supported(mode: str, dim: int, vdim: int, query_lens, heads: int, *rows: Optional[torch.Tensor]) -> bool:
     """Whether a bfloat16 step of long portions runs its recurrences in chunks of 128 tokens on the tensor cores (``linrec_chunks.cu``):
     states of up to 128 x 128, no request that would leave a chunk mostly empty, enough work, and ``rows`` (the inputs, the state)
     that start on 16 bytes."""
-    return (dim <= LINREC_CHUNK and vdim <= LINREC_CHUNK and dim % 4 == 0 and vdim % 4 == 0 and min(query_lens) >= LINREC_CHUNKS_MIN_TOKENS
+    return (mode in LINREC_CHUNKS_FROM and dim <= LINREC_CHUNK and vdim <= LINREC_CHUNK and dim % 4 == 0 and vdim % 4 == 0 and min(query_lens) >= LINREC_CHUNKS_MIN_TOKENS
             and sum(query_lens) * heads >= LINREC_CHUNKS_FROM[mode]
             and all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0) for t in rows))
 
@@ -1966,14 +1966,9 @@ def linrec_chunks(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
                   cap: float, q_scale: float, cu_tokens: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor, out: torch.Tensor,
                   query_lens, heads: int, qk_heads: int, dim: int, vdim: int, err: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """``linrec_segments`` on the tensor cores, in 32-bit accuracy: the chunks' sums of k v^T side by side, a pass from chunk to chunk, and
-    the outputs of all chunks side by side.  ``forget_write``: ``q`` and ``k`` as ``linrec_gates`` leaves them or, with ``p0, p1
-    [qk_heads * dim]``, raw as for ``linrec``."""
-    gates = mode == "forget_write" and p0 is not None
-    _check_linrec("linrec_chunks", mode, q, k, v, a, gate_a, gate_b, None if gates else p0, None if gates else p1, p2, cu_tokens, state_slots,
-                  state, out, query_lens, heads, qk_heads, dim, vdim, err)
-    for t in (p0, p1) if gates else ():
-        if t is None or t.dtype != torch.float32 or t.numel() != qk_heads * dim or not t.is_contiguous():
-            raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"linrec_chunks: p0 and p1 must be float32 [{qk_heads * dim}]")
+    the outputs of all chunks side by side.  Not ``forget_write``."""
+    _check_linrec("linrec_chunks", mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, query_lens, heads, qk_heads,
+                  dim, vdim, err)
     T, S, code = q.shape[0], len(query_lens), LINREC_SEGMENT_MODES[mode]
     chunks = sum(-(-n // LINREC_CHUNK) for n in query_lens)
     n = _fn("linrec_chunks", "photon_linrec_chunks_scratch", [c_int] * 6, restype=c_long)(code, T, chunks, heads, dim, vdim)

@@ -29,7 +29,7 @@ DEFAULT_NAMES = {"q": "q", "f": "f", "f_bias": "f.b", "lower": "lower", "v": "v"
 
 
 class Hgrn2Mixer(Mixer):
-    kernel_modules = ("linrec", "linrec_segments", "linrec_chunks", "row_norms")
+    kernel_modules = ("linrec", "linrec_segments", "row_norms")
     state_skips_negative_slots = True
 
     def __init__(self, hidden_size: int, heads: int, dim: int, vdim: int, eps: float, names: Optional[Dict[str, str]] = None):
@@ -68,17 +68,12 @@ class Hgrn2Mixer(Mixer):
         rows = project(h, self.w_in, out_dtype=torch.float32)       # [q | f | v]
         q, k, v = rows[:, :nd], rows[:, nd:2 * nd], rows[:, 2 * nd:]
         bias, lower = self.f_bias, self.lower
-        lens = list(ctx.host_query_lens)
-        o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
-        if h.dtype == torch.bfloat16 and lens and ops.linrec_chunks_supported("forget_write", self.dim, self.vdim, lens, H, cache.state, q, k, v):
-            # long portions alone: chunks of tokens on the tensor cores, which form the gates themselves
-            ops.linrec_chunks("forget_write", q, k, v, None, None, None, bias, lower, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots,
-                              cache.state, o, lens, H, H, self.dim, self.vdim, ctx.error_flag)
-            return self._finish(o, h)
         if max(list(ctx.host_query_lens) or [T]) >= GATES_MIN_TOKENS:
             y = torch.empty((T, 2 * nd), dtype=torch.float32, device=h.device)
             ops.linrec_gates(q, k, bias, lower, y[:, :nd], y[:, nd:])
             q, k, bias, lower = y[:, :nd], y[:, nd:], None, None
+        o = torch.empty((T, nv), dtype=torch.float32, device=h.device)
+        lens = list(ctx.host_query_lens)
         if h.dtype == torch.bfloat16 and lens and bias is None and ops.linrec_segments_supported("forget_write", self.dim, lens, H):
             # long portions: segments of tokens side by side
             ops.linrec_segments("forget_write", q, k, v, None, None, None, None, None, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots,
@@ -86,11 +81,8 @@ class Hgrn2Mixer(Mixer):
         else:
             ops.linrec("forget_write", q, k, v, None, None, bias, lower, None, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o,
                        ctx.num_seqs, H, H, self.dim, self.vdim, ctx.error_flag)
-        return self._finish(o, h)
-
-    def _finish(self, o: torch.Tensor, h: torch.Tensor) -> torch.Tensor:
-        out = torch.empty(o.shape, dtype=h.dtype, device=h.device)
-        ops.group_rmsnorm(o, self.norm, self.eps, self.heads, out=out)
+        out = torch.empty((T, nv), dtype=h.dtype, device=h.device)
+        ops.group_rmsnorm(o, self.norm, self.eps, H, out=out)
         return project(out, self.w_o)
 
 

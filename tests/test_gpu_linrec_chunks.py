@@ -8,7 +8,7 @@ from test_gpu_linrec_segments import _rel, _walk, i32
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-MODES = ["state_space", "matrix_memory", "forget_write", "decay_rows"]
+MODES = ["state_space", "matrix_memory", "decay_rows"]
 
 
 @pytest.fixture(autouse=True)
@@ -26,8 +26,6 @@ def _case(mode, H, G, N, dv, lens, slots, strong, seed, poison=None):
     a0 = 3 * G * N
     b0 = a0 + H * dv
     rows[:, 2 * G * N:a0] = torch.sigmoid(rows[:, 2 * G * N:a0] + 2.0) ** (40 if strong else 1)
-    if mode == "forget_write":
-        rows[:, G * N:2 * G * N] = torch.sigmoid(rows[:, G * N:2 * G * N] * (4.0 if strong else 1.0) + (4.0 if strong else -2.0))
     if strong and mode == "decay_rows":
         rows[7, 2 * G * N] = 0.0
     p0, p1, p2 = (0.5 * torch.randn(H, generator=gen) for _ in range(3))
@@ -99,7 +97,7 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(mode, value):
     assert torch.equal(S[:, :, 4:], clean_after[0, :H * N * dv].view(H, N, dv)[:, :, 4:])
 
 
-@pytest.mark.parametrize("mode", ["state_space", "matrix_memory", "decay_rows"])
+@pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("gates", ["constant", "nearly constant", "ordinary"])
 @pytest.mark.parametrize("H,N,dv,T", [(2, 64, 32, 2048), (4, 128, 128, 777)])
 def test_errors_are_not_larger_than_the_segments(mode, gates, H, N, dv, T):
@@ -164,23 +162,3 @@ def test_floors_of_the_matrix_memory_keep_their_bits(forget):
                           none(H, N, dv), none(H, N), none(H))
     errors = [_rel(o, want) for o in outs]
     assert errors[0] <= max(1.1 * errors[1], 2.0 ** -22), errors
-
-
-@pytest.mark.parametrize("C", [128, 40])
-def test_raw_gates_are_those_of_the_gates_kernel(C):
-    from photon_infer_b200.kernels import ops
-    torch.manual_seed(3)
-    H, dv, lens = 2, 64, [200, 70]
-    T = sum(lens)
-    q, z, v = torch.randn(T, H * C, device=DEV), 3 * torch.randn(T, H * C, device=DEV), torch.randn(T, H * dv, device=DEV)
-    bias, lower = torch.randn(H * C, device=DEV), 0.5 * torch.rand(H * C, device=DEV)
-    results = []
-    for raw in (True, False):
-        st, out, qk = torch.ones(2, H * C * dv, device=DEV), torch.empty(T, H * dv, device=DEV), (q, z)
-        if not raw:
-            qk = torch.empty(T, H * C, device=DEV), torch.empty(T, H * C, device=DEV)
-            ops.linrec_gates(q, z, bias, lower, *qk)
-        ops.linrec_chunks("forget_write", *qk, v, None, None, None, bias if raw else None, lower if raw else None, None, 0.0, 1.0, i32([0, 200, 270]),
-                          i32([0, 1]), st, out, lens, H, H, C, dv, None)
-        results.append((out, st))
-    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
