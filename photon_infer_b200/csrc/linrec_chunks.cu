@@ -646,28 +646,41 @@ lc_out_kernel(const LcArgs A) {
       lc_done(sh, parity);
     }
     if (blocks > 1) put_queries(through(0, tg));                      // as S_0 sees them
-    // Blocks whose decays are too small for a common reference: thread (token s, 8 rows) multiplies the decays up from s on and meets the
-    // queries on the way; the 16 threads of a token share a half warp.
+    // Blocks whose decays are too small for a common reference: 16 threads share a token s, eight rows each; they multiply the decays up
+    // from s on and meet the queries on the way.  Keys, decays and queries of the 32 tokens lie in shared memory, where the keys' parts
+    // were.  Read from memory by every token that comes before, as they were, such blocks made 2,048 tokens of 16 heads (the recurrence, one row in
+    // 128 with decays of 0.1) take 280 us; 164 so, 177 in segments, 102 where no block is like that.
     for (int j = 0; j < 4; ++j) {
       if (blocks < 4 || !sh.direct[j]) continue;
-      const int s = j * 32 + (tid >> 4), n8 = (tid & 15) * 8, last = min(p.cnt, j * 32 + 32);
-      const size_t kb = (size_t)p.hq * A.N;
-      float d[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) d[u] = s < last && n8 + u < A.N ? A.k[(size_t)(p.t0 + s) * A.k_stride + kb + n8 + u] : 0.f;
-      for (int t = j * 32; t < last; ++t) {           // all lanes, for the sums' sake; before s nothing
-        float o = 0.f;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          if (n8 + u < A.N) {
-            if (t > s) d[u] *= A.a[(size_t)(p.t0 + t) * A.a_stride + kb + n8 + u];
-            o = fmaf(d[u], q0[(size_t)t * A.q_stride + n8 + u], o);
-          }
-        }
-#pragma unroll
-        for (int w = 8; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
-        if ((tid & 15) == 0) sh.self[j][tid >> 4][t - j * 32] = o;
+      float *ks = reinterpret_cast<float*>(Y), *as = ks + 32 * LC_T, *qs = as + 32 * LC_T;
+      const float* k0 = A.k + (size_t)p.t0 * A.k_stride + (size_t)p.hq * A.N;
+      const float* a0 = A.a + (size_t)p.t0 * A.a_stride + (size_t)p.hq * A.N;
+      for (int i = warp; i < 32; i += 16) {
+        *reinterpret_cast<float4*>(ks + i * LC_T + lane * 4) = lc_piece(k0, A.k_stride, j * 32 + i, p.cnt, lane * 4, A.N);
+        *reinterpret_cast<float4*>(as + i * LC_T + lane * 4) = lc_piece(a0, A.a_stride, j * 32 + i, p.cnt, lane * 4, A.N);
+        *reinterpret_cast<float4*>(qs + i * LC_T + lane * 4) = lc_piece(q0, A.q_stride, j * 32 + i, p.cnt, lane * 4, A.N);
       }
+      __syncthreads();
+      const int s = tid >> 4, l = tid & 15;
+      float4 d1 = *reinterpret_cast<const float4*>(ks + s * LC_T + l * 4), d2 = *reinterpret_cast<const float4*>(ks + s * LC_T + 64 + l * 4);
+#pragma unroll 1
+      for (int t0 = (warp * 2) & ~7; t0 < 32; t0 += 8) {                             // from the warp's first token on
+        float o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float *at = as + (t0 + i) * LC_T + l * 4, *qt = qs + (t0 + i) * LC_T + l * 4;
+          const float4 a1 = *reinterpret_cast<const float4*>(at), a2 = *reinterpret_cast<const float4*>(at + 64);
+          const float4 q1 = *reinterpret_cast<const float4*>(qt), q2 = *reinterpret_cast<const float4*>(qt + 64);
+          if (t0 + i > s) {
+            d1.x *= a1.x; d1.y *= a1.y; d1.z *= a1.z; d1.w *= a1.w;
+            d2.x *= a2.x; d2.y *= a2.y; d2.z *= a2.z; d2.w *= a2.w;
+          }
+          o[i] = fmaf(d1.x, q1.x, fmaf(d1.y, q1.y, fmaf(d1.z, q1.z, d1.w * q1.w))) + fmaf(d2.x, q2.x, fmaf(d2.y, q2.y, fmaf(d2.z, q2.z, d2.w * q2.w)));
+        }
+        lr_meet<8, 8>(o, lane);                       // lanes 2 i and 2 i + 1 of the sixteen: the sum for token t0 + i
+        if (!(l & 1)) sh.self[j][s][t0 + (l >> 1)] = o[0];
+      }
+      __syncthreads();                                // the plane takes the next block's, or the state
     }
   }
   if (MODE == 3) fetch_state();                       // no earlier: the keys' registers
