@@ -8,6 +8,7 @@ correctly refuses it (``UNSUPPORTED_SIZE``) instead of giving a wrong result.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_long, c_void_p
 from typing import Optional
@@ -1945,17 +1946,39 @@ def _check_linrec(what, mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens,
 
 LINREC_CHUNK = 128
 LINREC_CHUNKS_MIN_TOKENS = 64
-#: Tokens x heads of a step from which the chunks are the faster way (below, a step waits for the host, and they are one launch more than the
-#: segments).  B200, heads of 128 x 128, a mixer's step, us, as before first: gated linear attention 640 tokens x 16 heads 160 and 149, 2,048 x
-#: 16 302 and 225, 256 x 32 155 and 153, 400 x 32 208 and 166; matrix memory 640 x 16 154 and 131, 400 x 16 136 and 132, 2,048 x 16 296 and 199;
-#: state space 640 x 16 160 and 149, 256 x 32 147 and 150, 2,048 x 16 294 and 221.  Forget and write stays with the segments (linrec_chunks.cu).
+#: Tokens x heads of a step from which chunks are looked at: below, a step waits for the host, and they are one launch more than the segments.
+#: Forget and write stays with the segments (linrec_chunks.cu).
 LINREC_CHUNKS_FROM = {"decay_rows": 10000, "matrix_memory": 10000, "state_space": 10000}
+#: What a round of chunks (a block an SM, whatever its chunk holds) is worth in tokens that the segments' blocks walk on an SM.  A round takes 38 (state
+#: space), 39 (matrix memory), 48 us (row decays) with heads of 128 x 128 and 29 to 38 with small ones, a token 0.15 to 0.19 us, half of that
+#: for less than 64 rows, where the chunks gain nothing.
+LINREC_CHUNK_ROUND = {"state_space": 225, "matrix_memory": 200, "decay_rows": 260}
+LINREC_CHUNK_START = 75         # what a pass of the segments costs beside its tokens (a launch, the folds), in the same tokens
+
+
+@functools.lru_cache(maxsize=1024)
+def linrec_chunks_faster(mode: str, dim: int, query_lens: tuple, heads: int, blocks: int, sms: int) -> bool:
+    """Whether the chunks' rounds take less than the segments' passes, two where a request is cut and one where the step's requests fill the
+    GPU as they are.  B200, the recurrence alone, us, segments and chunks: row decays of 128 x 128, 16 heads 1,152 tokens 112 and 44, 1,200 115
+    and 78, 5 x 130 (10 chunks that hold 65 tokens each) 60 and 76; 32 heads 640 118 and 74, 3 x 130 61 and 76, 4 x 700 291 and 279; 64 heads of
+    64 x 64, 4 x 700 282 and 460, 2,048 327 and 311; state space of 128 x 128, 32 heads 3 x 130 45 and 62.  Over 1,062 steps (19 shapes of
+    heads, 22 of requests) the way that this takes is 0.5 % slower than the better one in the mean, 9 % at worst where it is the chunks."""
+    if dim <= 32:
+        return False
+    seg = linrec_segment_tokens(query_lens, heads, blocks, sms)
+    cut = max(query_lens) > seg
+    walked = sum(query_lens) * heads * blocks / sms
+    if not cut:                                         # as many blocks of the longest request as an SM gets
+        longs = sum(n >= LINREC_SEGMENTS_MIN_TOKENS for n in query_lens)
+        walked = max(walked, max(query_lens) * -(-longs * heads * blocks // sms))
+    rounds = -(-sum(-(-n // LINREC_CHUNK) for n in query_lens) * heads // sms)
+    return rounds * LINREC_CHUNK_ROUND[mode] <= (2 if cut else 1) * (walked + LINREC_CHUNK_START)
 
 
 def linrec_chunks_supported(mode: str, dim: int, vdim: int, query_lens, heads: int, *rows: Optional[torch.Tensor]) -> bool:
-    """Whether a bfloat16 step of long portions runs its recurrences in chunks of 128 tokens on the tensor cores (``linrec_chunks.cu``):
-    states of up to 128 x 128, no request that would leave a chunk mostly empty, enough work, and ``rows`` (the inputs, the state)
-    that start on 16 bytes."""
+    """Whether a bfloat16 step of long portions may run its recurrences in chunks of 128 tokens on the tensor cores (``linrec_chunks.cu``):
+    states of up to 128 x 128, no request of fewer than 64 tokens, enough work, and ``rows`` (the inputs, the state) that start on 16
+    bytes.  ``linrec_chunks_faster`` says whether it should."""
     return (mode in LINREC_CHUNKS_FROM and dim <= LINREC_CHUNK and vdim <= LINREC_CHUNK and dim % 4 == 0 and vdim % 4 == 0 and min(query_lens) >= LINREC_CHUNKS_MIN_TOKENS
             and sum(query_lens) * heads >= LINREC_CHUNKS_FROM[mode]
             and all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0) for t in rows))
@@ -1998,8 +2021,9 @@ def linrec_segments(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     reached.  ``forget_write``:
     ``q`` and ``k`` as ``linrec_gates`` leaves them.  ``decay_rows``: ``S <- diag(a) S + k v^T``, ``a [T, qk_heads * dim]``.
     ``matrix_memory``: ``out`` is not divided; returns ``[T, heads]``, what it is to be divided by.  ``query_lens``: the requests'
-    tokens in the step (host)."""
-    if segment is None and linrec_chunks_supported(mode, dim, vdim, query_lens, heads, state, q, k, v, a):
+    tokens in the step (host).  Without ``segment``, a step for which they are the faster way goes to ``linrec_chunks``."""
+    if segment is None and linrec_chunks_supported(mode, dim, vdim, query_lens, heads, state, q, k, v, a) \
+            and linrec_chunks_faster(mode, dim, tuple(query_lens), heads, linrec_segment_blocks(dim, vdim), sm_count(q.device)):
         return linrec_chunks(mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cap, q_scale, cu_tokens, state_slots, state, out, query_lens,
                              heads, qk_heads, dim, vdim, err)
     _check_linrec("linrec_segments", mode, q, k, v, a, gate_a, gate_b, p0, p1, p2, cu_tokens, state_slots, state, out, query_lens, heads,

@@ -13,9 +13,10 @@ MODES = ["state_space", "matrix_memory", "decay_rows"]
 
 @pytest.fixture(autouse=True)
 def any_size(monkeypatch):
-    """Chunks for steps of any size."""
+    """Chunks for steps of any size and shape."""
     from photon_infer_b200.kernels import ops
     monkeypatch.setattr(ops, "LINREC_CHUNKS_FROM", dict.fromkeys(ops.LINREC_CHUNKS_FROM, 0))
+    monkeypatch.setattr(ops, "linrec_chunks_faster", lambda *args: True)
 
 
 def _case(mode, H, G, N, dv, lens, slots, strong, seed, poison=None):
