@@ -797,6 +797,32 @@ PHOTON_API int photon_attention_tc(const void* q, long q_stride, void* out, long
                                 nullptr, 0, stream);
 }
 
+// Whether blocks own two query tiles (attention_tc_pairs_kernel).  `keys`: of the longest request that runs here; `tiles`, `pairs`: blocks of
+// one and of two tiles.  The pairs' keys cost less and their set-up more: us, one and two tiles a block, without a window
+//   keys 4,096 and more: 64 tokens behind 4,096 73 and 71, 2,048 behind 14,336 675 and 512 (32/8 heads of 128), 512 behind 8,192 147 and 140 (24/8);
+//   one tile a request, so that no block waits for two: 128 behind 1,536 33 and 29, 128 behind 512 16 and 15, 17 behind 512 15 and 16 (16/16);
+//   more tiles than SMs: 1,024 behind 1,536 50 and 49, 1,024 behind 512 33 and 34 (32/8), 2,048 from the start 40 and 42 (16/16);
+//   more than two an SM: 2,048 from the start 55 and 48 (32/8), 47 and 44 (24/8), 67 and 69 (40/2: 342 pairs, a third round);
+//   fewer: 512 behind 2,048 48 and 49, 1,093 beside 40 decoded tokens 27 and 30 (24/8), 200 beside requests of 14,000 keys 12 and 17.
+// Under a window both ends of a row's keys are masked: 2,048 tokens, windows of 128, 512 and 1,024 22 and 30, 34 and 41, 46 and 48; of
+// 4,096 behind 8,192 160 and 153, 512 tokens there 74 and 76 (24/8: 76 and 79).  It counts for half of its keys, but with one tile a
+// request (17 tokens under windows of 1,024 and 2,048: 23 and 23, 39 and 36).
+#ifndef AT_PAIRS_KEYS
+#define AT_PAIRS_KEYS 4096
+#endif
+static bool at_two_tiles(long keys, int window, int tiles_per_seq, long tiles, long pairs, int sms) {
+  const bool cut = window > 0 && window < keys;
+  const long seen = cut ? window / 2 : keys, full = AT_PAIRS_KEYS;
+  if (seen >= full) return true;
+  if (tiles_per_seq == 1) return (cut ? window : keys) >= full * 3 / 8;
+  if (tiles <= sms) return false;
+  return seen >= full * 5 / 8 || (seen >= full / 2 && tiles > 2 * sms && pairs <= 2 * sms);
+}
+// The rule alone, for a device of `sms` multiprocessors (heads of 64 and less always have one tile).
+PHOTON_API int photon_attention_tc_two_tiles(long keys, int window, int tiles_per_seq, long tiles, long pairs, int sms) {
+  return HEAD_DIM > 64 && at_two_tiles(keys, window, tiles_per_seq, tiles, pairs, sms);
+}
+
 // The same with kept first keys, sinks and bounded scores (see AttnTcParams), and an optional gate: bfloat16
 // [T, n_q * dv] with row stride gate_stride (16-byte aligned rows); every output is multiplied by sigmoid(gate).
 PHOTON_API int photon_attention_tc_ex(const void* q, long q_stride, void* out, long out_stride, const void* k_cache,
@@ -804,6 +830,19 @@ PHOTON_API int photon_attention_tc_ex(const void* q, long q_stride, void* out, l
                                       const int* positions, int S, int max_tokens_per_seq, int T, int n_q, int n_kv, int d,
                                       int page_size, int num_pages, int window, float scale, int* err, int keep_first,
                                       const float* sinks, float softcap, const void* gate, long gate_stride, cudaStream_t stream) {
+  return photon_attention_tc_keys(q, q_stride, out, out_stride, k_cache, v_cache, block_table, max_pages, cu_tokens, positions, S,
+                                  max_tokens_per_seq, T, n_q, n_kv, d, page_size, num_pages, window, scale, err, keep_first, sinks,
+                                  softcap, gate, gate_stride, 0, stream);
+}
+
+// The same, told how many keys the longest request that runs here has, which decides between kernels; 0: not known (the block table's width
+// where the step is one request, else few).
+PHOTON_API int photon_attention_tc_keys(const void* q, long q_stride, void* out, long out_stride, const void* k_cache,
+                                        const void* v_cache, const int* block_table, int max_pages, const int* cu_tokens,
+                                        const int* positions, int S, int max_tokens_per_seq, int T, int n_q, int n_kv, int d,
+                                        int page_size, int num_pages, int window, float scale, int* err, int keep_first,
+                                        const float* sinks, float softcap, const void* gate, long gate_stride, int keys,
+                                        cudaStream_t stream) {
   if (S <= 0 || T <= 0) return 0;
   if (keep_first < 0 || softcap < 0.f) return PHOTON_ERR_ARGUMENT;
   if (d != HEAD_DIM || n_kv <= 0 || n_q % n_kv || !(scale > 0.f)) return PHOTON_ERR_UNSUPPORTED;
@@ -862,17 +901,12 @@ PHOTON_API int photon_attention_tc_ex(const void* q, long q_stride, void* out, l
   if (S == 1) grid.y = P.tiles_per_seq;
   if (grid.y == 0) return 0;                        // no request of the step has more than 16 rows
 #if HEAD_DIM > 64
-  // Two tiles a block from 2,048 keys on, 4,096 beside other requests (the block table's width is the longest request's, which may not be
-  // the portion).  us, one and two tiles a block, 24/8 heads: 1,093 tokens from the start 30 and 33, 2,048 51 and 48, 512 behind
-  // 2,048 52 and 53, 1,024 behind 2,048 66 and 62, 512 behind 8,192 151 and 144; three requests of 300 to 600 tokens 22 and 25.
-#ifndef AT_PAIRS_KEYS
-#define AT_PAIRS_KEYS 2048
-#endif
-  if ((long)max_pages * page_size >= (S == 1 ? 1L : 2L) * AT_PAIRS_KEYS) {
+  // a request's last tile may be alone in its block
+  const unsigned y = (unsigned)(S == 1 ? (grid.y + 1) / 2 : (grid.y + (part < (long)grid.y ? part : (long)grid.y) + 1) / 2);
+  const long longest = keys > 0 ? keys : S == 1 ? (long)max_pages * page_size : 0;
+  if (at_two_tiles(longest, window, P.tiles_per_seq, (long)grid.y * n_kv, (long)y * n_kv, photon_sm_count())) {
     cudaError_t e = cudaFuncSetAttribute(attention_tc_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
-    // a request's last tile may be alone in its block
-    const unsigned y = (unsigned)(S == 1 ? (grid.y + 1) / 2 : (grid.y + (part < (long)grid.y ? part : (long)grid.y) + 1) / 2);
     return launch_pdl(attention_tc_pairs_kernel, dim3(n_kv, y), dim3(AP_THREADS), (size_t)AP_SMEM_BYTES, stream, map_q, map_k, map_v, P);
   }
 #endif

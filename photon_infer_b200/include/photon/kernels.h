@@ -493,6 +493,13 @@ PHOTON_EXPORT int photon_attention_tc_ex(const void* q, long q_stride, void* out
                            const int* positions, int S, int max_tokens_per_seq, int T, int n_q, int n_kv, int d,
                            int page_size, int num_pages, int window, float scale, int* err, int keep_first, const float* sinks,
                            float softcap, const void* gate, long gate_stride, cudaStream_t stream);
+/* The same with the keys of the longest of those requests (0: not known), which decide between kernels; and that rule alone. */
+PHOTON_EXPORT int photon_attention_tc_keys(const void* q, long q_stride, void* out, long out_stride, const void* k_cache,
+                             const void* v_cache, const int* block_table, int max_pages, const int* cu_tokens,
+                             const int* positions, int S, int max_tokens_per_seq, int T, int n_q, int n_kv, int d,
+                             int page_size, int num_pages, int window, float scale, int* err, int keep_first, const float* sinks,
+                             float softcap, const void* gate, long gate_stride, int keys, cudaStream_t stream);
+PHOTON_EXPORT int photon_attention_tc_two_tiles(long keys, int window, int tiles_per_seq, long tiles, long pairs, int sms);
 
 /* ------------------------------------------------------------------ attention_decode.cu (-DHEAD_DIM=64|128; bfloat16; TMA) */
 PHOTON_EXPORT int photon_attention_decode_head_dim(void);

@@ -750,11 +750,12 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
                  num_seqs: int, max_tokens_per_seq: int, n_q: int, n_kv: int, head_dim: int,
                  window: Optional[int], scale: float, err: Optional[torch.Tensor], keep_first: int = 0,
                  sink: Optional[torch.Tensor] = None, softcap: Optional[float] = None, gate: Optional[torch.Tensor] = None,
-                 value_dim: Optional[int] = None) -> None:
+                 value_dim: Optional[int] = None, keys: Optional[int] = None) -> None:
     """Paged causal attention of the requests that bring more than 16 rows (tokens x heads per
     group) in this step, on the tcgen05 tensor cores; the rows of the other requests are left
     untouched (``flash_attention`` with ``keys_mode`` takes them).  ``keep_first``, ``sink``, ``softcap``, ``gate``,
-    ``value_dim``: as in ``paged_attention`` (the gate's rows must start on 16-byte boundaries: ``gate_fusable``)."""
+    ``value_dim``: as in ``paged_attention`` (the gate's rows must start on 16-byte boundaries: ``gate_fusable``).
+    ``keys``: of the longest of those requests, where the caller knows it; it decides whether blocks own two query tiles."""
     _check_gate(gate, q, out)
     _check_sink(sink, n_q)
     dv = value_dim or head_dim
@@ -774,16 +775,16 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
         _int32(t, name)
     if cu_tokens.numel() < num_seqs + 1 or block_table.shape[0] < num_seqs:
         raise PhotonError(ErrorCode.SHAPE_MISMATCH, "attention_tc: cu_tokens and block_table must cover every request")
-    f = _fn("attention_tc", "photon_attention_tc_ex",
+    f = _fn("attention_tc", "photon_attention_tc_keys",
             [c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_float,
-             c_void_p, c_long, c_void_p],
+             c_void_p, c_long, c_int, c_void_p],
             defines=value_defines(head_dim, value_dim))
     _check(f(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_cache), _ptr(v_cache), _ptr(block_table),
              block_table.shape[1], _ptr(cu_tokens), _ptr(positions), int(num_seqs), int(max_tokens_per_seq), T,
              n_q, n_kv, head_dim, k_cache.shape[2], k_cache.shape[0], int(window) if window else 0, float(scale),
              _ptr(err), int(keep_first or 0), _ptr(sink), float(softcap or 0.0), _ptr(gate),
-             gate.stride(0) if gate is not None else 0, _stream()), "attention_tc")
+             gate.stride(0) if gate is not None else 0, int(keys or 0), _stream()), "attention_tc")
 
 
 # ----------------------------------------------------------------------------- matrix products

@@ -214,9 +214,10 @@ def attend_tensor_cores(mixer, q: torch.Tensor, out: torch.Tensor, ctx: StepCont
     if rows_mode and ops.USE_ATTENTION_TC and \
             ops.attention_tc_supported(q.dtype, self.head_dim, gsize, cache.k.shape[2], value_dim):
         # prompt portions: tensor memory and TMA; the split-key kernel keeps the decoded tokens
+        held = [n for n, f in zip(ctx.host_context_lens, few) if not f]
         ops.attention_tc(q, out, cache.k, cache.v, group.block_table, ctx.cu_tokens, ctx.positions,
                          ctx.num_seqs, ctx.max_query_len, self.n_q, self.n_kv, self.head_dim, self.window,
-                         self.scale, ctx.error_flag, **extras)
+                         self.scale, ctx.error_flag, keys=max(held, default=None), **extras)
         rows_mode = False
     if decode_tma:
         chunk, chunks, items = plan
