@@ -36,6 +36,7 @@
 //
 // Compiled per model with -DHEAD_DIM=<d> and, where a value has another width than a key, -DVALUE_DIM=<dv>.
 #include "attention_tc.cuh"
+#include <type_traits>
 #include <math.h>
 
 #ifndef HEAD_DIM
@@ -482,17 +483,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 //     so scores that are there also say that the O before is);
 //   * warps 0-3 and 4-7: the rows of a query tile each.  They have 232 registers (the launch gives 168, the other four warps
 //     keep 40: 128 x 40 + 256 x 232 = 64,512 = 384 x 168), so that a row's 128 scores stay in registers.
+// The first tile's products end with its own last key: a value that is not finite, of a token that only the second tile sees, meets
+// weights of 0 there, and 0 times it would be NaN.  The 16 keys among which it ends come with zeros behind it from a place of their own
+// (0.9 us a block: 2,048 tokens from the start 48.3 and 50.1).
 // Bound by the softmax warps (4,500 cycles for a pair of tiles of 128 keys, of which the exponentials take 2,048 at 16 a cycle and SM and the
 // products as many).  2,048 tokens behind 14,336, 32/8 heads of 128: 657 us with a tile a block, 482 so (1,070 TFLOP/s);
-// 2,048 from the start 59 and 51.  Heads of 64 gain nothing at any length (2,048 tokens 43 and 46 us; with columns of its own for P 42 and 48).
+// 2,048 from the start 54 and 50.  Heads of 64 gain nothing at any length (2,048 tokens 43 and 46 us; with columns of its own for P 42 and 48).
 #if HEAD_DIM > 64
 #define AP_KT 128
 #define AP_THREADS 384
 #define AP_K_BYTES (AP_KT * 128 * AT_DH)
 #define AP_V_BYTES (AP_KT * 128 * AT_VH)
 #define AP_HALF (AP_KT * 128)                      // one 64-wide half of a K or V tile
-#define AP_STAGES (AT_DH + AT_VH == 2 ? 3 : 2)
-#define AP_SMEM_BYTES (2 * AT_Q_BYTES + AP_STAGES * (AP_K_BYTES + AP_V_BYTES) + 1024 + 256)
+#define AP_STAGES 2
+#define AP_EDGE_BYTES (AT_VH * 2048)                // 16 value rows
+#define AP_SMEM_BYTES (2 * AT_Q_BYTES + AP_STAGES * (AP_K_BYTES + AP_V_BYTES) + AP_EDGE_BYTES + 1024 + 256)
 static_assert(AP_SMEM_BYTES <= 227 * 1024, "shared memory of a block");
 #define AP_O_COL 256                               // scores: 2 x 128 columns; O: 2 x 128
 
@@ -519,13 +524,17 @@ attention_tc_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   const int kept_tiles = (P.keep_first > 0 && key_lo > 0) ? min((P.keep_first + AP_KT - 1) / AP_KT, tile_begin) : 0;
   const int ntiles = kept_tiles + pos_last / AP_KT + 1 - tile_begin;
   auto tile_of = [&](int i) { return i < kept_tiles ? i : tile_begin + i - kept_tiles; };
+  // the tile of keys behind the last one that the first query tile sees, and that tile's keys before
+  const int mid = nq == 2 ? P.positions[tok0 + t_first + tile_tokens - 1] + 1 : 0;
+  const int mid_tile = nq == 2 ? kept_tiles + mid / AP_KT - tile_begin : ntiles, mid_keys = mid & (AP_KT - 1);
 
   extern __shared__ unsigned char at_dyn[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)at_dyn + 1023) & ~(uintptr_t)1023);
   unsigned char* q_s = base;
   unsigned char* k_s = q_s + 2 * AT_Q_BYTES;
   unsigned char* v_s = k_s + AP_STAGES * AP_K_BYTES;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(v_s + AP_STAGES * AP_V_BYTES);
+  unsigned char* edge_s = v_s + AP_STAGES * AP_V_BYTES;
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(edge_s + AP_EDGE_BYTES);
   uint64_t* k_full = q_full + 1;                    // [AP_STAGES] TMA -> MMA
   uint64_t* k_empty = k_full + AP_STAGES;           // [AP_STAGES] MMA -> TMA
   uint64_t* v_full = k_empty + AP_STAGES;
@@ -636,30 +645,62 @@ attention_tc_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       };
       bool ok = tc_wait(q_full, 0, abort_flag);
       for (int j = 0; j < nq && ok; ++j) ok = issue_scores(0, j);
-      for (int i = 0; i < ntiles && ok; ++i) {
+      // EDGE: the tiles of keys in which the first query tile ends, and behind.  In one loop with the others, whose products it kept from
+      // issuing one behind the other, this took 15 % (2,048 tokens behind 14,336, 24/8 heads: 467 -> 540 us); it is rolled up because straight
+      // code that a block meets once costs more to fetch than to run.
+      auto products = [&](int i, auto edge) -> bool {
+        constexpr bool EDGE = decltype(edge)::value;
         const int s = i % AP_STAGES;
-        for (int j = 0; j < nq && ok; ++j) {
-          if (!tc_wait(&v_full[s], (i / AP_STAGES) & 1, abort_flag)) { ok = false; break; }
+        for (int j = 0; j < nq; ++j) {
+          if (!tc_wait(&v_full[s], (i / AP_STAGES) & 1, abort_flag)) return false;
+          const uint32_t o = tmem + AP_O_COL + j * 128, p = tmem + j * 128;          // P: 8 columns of packed pairs for 16 keys, halves 32 apart
+          const uint32_t v_addr = tc_smem(v_s + s * AP_V_BYTES);                     // 16 keys: two groups of 8 rows of V
+          if (EDGE) {
+            const int sees = j > 0 ? AP_KT : i == mid_tile ? mid_keys : 0;
+            if (j == 0 && i == mid_tile && (mid_keys & 15)) {
+              // the 16 values among which it ends
+              const unsigned char* from = v_s + s * AP_V_BYTES + (mid_keys >> 4) * 2048;
+#pragma unroll 1
+              for (int e = lane; e < 128; e += 32)
 #pragma unroll
-          for (int half = 0; half < 2 && ok; ++half) {
-            if (!tc_wait(&p_full[2 * j + half], i & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            if (elected) {
-              const uint32_t v_addr = tc_smem(v_s + s * AP_V_BYTES) + half * 4 * 2048;
+                for (int h = 0; h < AT_VH; ++h)
+                  *reinterpret_cast<uint4*>(edge_s + h * 2048 + e * 16) =
+                      (e >> 3) < (mid_keys & 15) ? *reinterpret_cast<const uint4*>(from + h * AP_HALF + e * 16) : make_uint4(0, 0, 0, 0);
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic writes -> the tensor core's reads
+              __syncwarp();
+            }
+#pragma unroll 1
+            for (int kk = 0; kk < 8; ++kk) {
+              if ((kk & 3) == 0) {
+                if (!tc_wait(&p_full[2 * j + (kk >> 2)], i & 1, abort_flag)) return false;
+                tc_fence_after();
+              }
+              if (elected && kk * 16 < sees)
+                at_mma_ts(o, p + kk * 8, kk * 16 + 16 <= sees ? tc_desc_mn(v_addr + kk * 2048, AP_HALF, 1024) : tc_desc_mn(tc_smem(edge_s), 2048, 1024),
+                          idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
+            }
+          } else {
 #pragma unroll
-              for (int kk = 0; kk < 4; ++kk)        // 16 keys: P's 8 columns of packed pairs, two groups of 8 rows of V
-                at_mma_ts(tmem + AP_O_COL + j * 128, tmem + j * 128 + half * 32 + kk * 8, tc_desc_mn(v_addr + kk * 2048, AP_HALF, 1024),
-                          idesc_o, (i > 0 || half > 0 || kk > 0) ? 1u : 0u);
+            for (int half = 0; half < 2; ++half) {
+              if (!tc_wait(&p_full[2 * j + half], i & 1, abort_flag)) return false;
+              tc_fence_after();
+              if (elected)
+#pragma unroll
+                for (int kk = half * 4; kk < half * 4 + 4; ++kk)
+                  at_mma_ts(o, p + kk * 8, tc_desc_mn(v_addr + kk * 2048, AP_HALF, 1024), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
             }
           }
-          if (!ok) break;
           if (elected) {
             if (j == nq - 1) tc_commit(&v_empty[s]);
             if (i + 1 == ntiles) tc_commit(&o_full[j]);
           }
-          if (i + 1 < ntiles) ok = issue_scores(i + 1, j);
+          if (i + 1 < ntiles && !issue_scores(i + 1, j)) return false;
         }
-      }
+        return true;
+      };
+      int i = 0;
+      for (; i < min(mid_tile, ntiles) && ok; ++i) ok = products(i, std::false_type());
+      for (; i < ntiles && ok; ++i) ok = products(i, std::true_type());
       pdl_launch_dependents();                      // all products of this block are issued
     }
   } else {
@@ -802,7 +843,7 @@ PHOTON_API int photon_attention_tc(const void* q, long q_stride, void* out, long
 //   keys 4,096 and more: 64 tokens behind 4,096 73 and 71, 2,048 behind 14,336 675 and 512 (32/8 heads of 128), 512 behind 8,192 147 and 140 (24/8);
 //   one tile a request, so that no block waits for two: 128 behind 1,536 33 and 29, 128 behind 512 16 and 15, 17 behind 512 15 and 16 (16/16);
 //   more tiles than SMs: 1,024 behind 1,536 50 and 49, 1,024 behind 512 33 and 34 (32/8), 2,048 from the start 40 and 42 (16/16);
-//   more than two an SM: 2,048 from the start 55 and 48 (32/8), 47 and 44 (24/8), 67 and 69 (40/2: 342 pairs, a third round);
+//   more than two an SM: 2,048 from the start 54 and 50 (32/8), 47 and 46 (24/8), 67 and 69 (40/2: 342 pairs, a third round);
 //   fewer: 512 behind 2,048 48 and 49, 1,093 beside 40 decoded tokens 27 and 30 (24/8), 200 beside requests of 14,000 keys 12 and 17.
 // Under a window both ends of a row's keys are masked: 2,048 tokens, windows of 128, 512 and 1,024 22 and 30, 34 and 41, 46 and 48; of
 // 4,096 behind 8,192 160 and 153, 512 tokens there 74 and 76 (24/8: 76 and 79).  It counts for half of its keys, but with one tile a

@@ -13,7 +13,7 @@ from photon_infer_b200.csrc.build import load_module
     (2112, 0, 2, 16, 8, False), (2560, 0, 13, 104, 56, False),
     # one tile a request
     (1664, 0, 1, 16, 16, True), (640, 0, 1, 16, 16, False), (14353, 2048, 1, 8, 8, True), (14353, 1024, 1, 8, 8, False),
-    # more tiles than multiprocessors (50 and 49, 33 and 34, 40 and 42), than two on each (55 and 48, 67 and 69)
+    # more tiles than multiprocessors (50 and 49, 33 and 34, 40 and 42), than two on each (54 and 50, 67 and 69)
     (2560, 0, 32, 256, 128, True), (1536, 0, 32, 256, 128, False), (2048, 0, 16, 256, 128, False), (2048, 0, 64, 512, 256, True),
     (2048, 0, 342, 684, 342, False),
     # short portions beside requests with long tables (12 and 17, 27 and 30)

@@ -69,3 +69,35 @@ def test_options_match_the_kernel_of_one_tile(d, dv, window, keep, sink, cap, ga
     assert not torch.isnan(outs[0]).any()
     assert float((outs[0] - outs[1]).abs().max()) <= 2.0 ** -7 * float(outs[1].abs().max())
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) <= 4e-3
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,dv", [(8, 2, 128, 128), (6, 2, 128, 64), (5, 1, 96, 96), (2, 2, 112, 112)])
+@pytest.mark.parametrize("held,value", [(0, float("nan")), (37, float("inf")), (128, float("nan"))])
+def test_values_that_are_not_finite_stay_out_of_earlier_query_tiles(n_q, n_kv, d, dv, held, value, monkeypatch):
+    """A token's values reach the tokens before it no further than with one query tile a block: not the tile before, which ends
+    between or at multiples of 16 keys, in the block's last tile of keys or in one before it."""
+    from photon_infer_b200.kernels import ops
+    _force(monkeypatch, 0)
+    gen = torch.Generator().manual_seed(8)
+    rnd = lambda *s: torch.randn(s, generator=gen).to(torch.bfloat16).to(DEV)
+    group, ps, T = n_q // n_kv, 16, 330
+    tile = 128 // group                                  # tokens of a query tile
+    pages = -(-(held + T) // ps)
+    q, kc, vc = rnd(T, n_q * d), rnd(pages, n_kv, ps, d), rnd(pages, n_kv, ps, dv)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+
+    def run(values):
+        out, err = torch.empty(T, n_q * dv, dtype=torch.bfloat16, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+        ops.attention_tc(q, out, kc, values, i32([list(range(pages))]), i32([0, T]), i32(list(range(held, held + T))), 1, T, n_q, n_kv, d, None,
+                         1.0 / math.sqrt(d), err, value_dim=dv)
+        assert err.cpu().tolist()[0] == 0
+        return out
+
+    clean = run(vc)
+    for first in range(tile, T, 2 * tile):               # the first token that only the second tile of a block sees, and one more
+        for token in {first, min(first + 5, T - 1)}:
+            bad = vc.clone()
+            bad[(held + token) // ps, :, (held + token) % ps] = value
+            out = run(bad)
+            assert torch.equal(out[:first], clean[:first]), token
+            assert not bool(torch.isfinite(out[token:]).any())
