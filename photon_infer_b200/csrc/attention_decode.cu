@@ -51,6 +51,7 @@ static_assert(HEAD_DIM == 64 || HEAD_DIM == 128, "head size of the TMA decode at
 #define AD_KD (HEAD_DIM / 16)
 #define AD_ND (HEAD_DIM / 8)
 #define AD_SORTED 128                               // requests up to which the items are ordered by length
+#define AD_SORT_TILES 8                             // key tiles of the longest from which they are
 #define AD_MAX_SEQS 512
 #ifndef AD_ADAPTIVE
 #define AD_ADAPTIVE 1                              // 0: the host's chunk size is used as it is (for comparisons)
@@ -207,7 +208,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   __shared__ uint64_t full_bar[AD_STAGES], empty_bar[AD_STAGES], q_full, q_empty, item_full[AD_QUEUE], item_empty[AD_QUEUE];
   __shared__ Item item_s[AD_QUEUE];
   __shared__ int chunk_prefix[AD_MAX_SEQS + 1];
-  __shared__ int order[AD_SORTED], tiles_s[AD_SORTED];
+  __shared__ int order[AD_SORTED];
+  __shared__ __align__(16) int length[AD_SORTED];                // of a request: its key tiles, and which comes first among equals
   __shared__ int s_flag;
   __shared__ int abort_flag;
 
@@ -227,7 +229,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   pdl_wait();
 
   // ---- chunks of every request, and their prefix sum
-  const bool sorted = P.S <= AD_SORTED && P.S * P.n_kv > (int)gridDim.x;
+  bool sorted = P.S <= AD_SORTED && P.S * P.n_kv > (int)gridDim.x;
   auto key_range = [&](int seq, int& tok0, int& ntok, int& ctx, int& tile_begin, int& tile_end) -> bool {
     tok0 = P.cu_tokens[seq];
     ntok = P.cu_tokens[seq + 1] - tok0;
@@ -268,8 +270,10 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       // least 0.8 of the longest).  Requests of mixed lengths fill one another's gaps, and the host's cut was measured
       // as good or better there (56 requests of 128 to 2,300 keys: 70 us with chunks of 22 tiles, 71 us whole).
       // Thread t tries p = fewest chunks + t chunks per request; the cheapest wins, the longer chunk on a tie.
+      const bool alike = (long)sum * 5 >= (long)tiles * few * 4;
+      sorted = sorted && !alike && tiles >= AD_SORT_TILES;
       int key = 0x7fffffff;
-      if (tiles > 0 && few > 0 && (long)sum * 5 >= (long)tiles * few * 4) {
+      if (tiles > 0 && few > 0 && alike) {
         const long cap = P.scratch_chunks / few;                       // chunks a request may have
         const int p_hi = (int)min((long)min(AD_MAX_CHUNKS, tiles), cap);
         const int p = (tiles + 63) / 64 + (int)threadIdx.x;
@@ -291,10 +295,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (key != 0x7fffffff) CH = 64 - (key & 127);
       __syncthreads();                                           // scan is used again below
     }
-    // Longest requests first: items are drawn in this order, so what is left at the end is short.  A layer of 56 requests of 128
-    // to 2,304 keys took 135 us in the order of the step, 130.7 us sorted; 96 requests of up to 3,000 keys 233 and 229 us, 64 of up to
-    // 8,000 253.5 and 252 us.  Not where every request and key/value head has a block to begin with (one round of items:
-    // 24 requests 105.1 us, sorted 106.0 us), and not above AD_SORTED requests: a block ranks them itself, S comparisons a thread.
+    // Longest requests first: items are drawn in this order, so what is left at the end is short.  A layer of 56 requests of 222 to
+    // 2,246 keys (24/8 heads of 128) took 135.0 us in the order of the step, 130.6 us sorted; 96 with every eighth of 2,304 keys, the others of
+    // 200, 131 and 121; 128 of 128 to 1,484 158 and 161 (heads of 64: 110 and 106).  Ranking takes 1 to 2 us.  Not where every request and
+    // key/value head has a block to begin with (one round of items: 24 requests 105.1 us, sorted 106.0), not for requests of nearly one length
+    // (38 of 2,304 148 and 150) or of a few tiles (128 of up to 200 keys 108 and 110), and not above AD_SORTED requests: a block ranks them itself.
     auto chunks_of = [&](int seq, int& tiles) -> int {
       int tok0, ntok, ctx, tb, te;
       tiles = key_range(seq, tok0, ntok, ctx, tb, te) ? te - tb : 0;
@@ -309,12 +314,17 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     int mine = 0;
     if (sorted) {                                                // one request a thread (span is 1)
       const int seq = threadIdx.x;
-      int tiles = 0, n = 0;
-      if (seq < P.S) { n = chunks_of(seq, tiles); tiles_s[seq] = tiles; }
+      int tiles = 0, n = 0, mine_at = -1;
+      if (seq < P.S) { n = chunks_of(seq, tiles); mine_at = tiles * AD_SORTED + AD_SORTED - 1 - seq; }
+      if (seq < AD_SORTED) length[seq] = mine_at;
       __syncthreads();
       if (seq < P.S) {
         int rank = 0;
-        for (int s = 0; s < P.S; ++s) rank += tiles_s[s] > tiles || (tiles_s[s] == tiles && s < seq);
+#pragma unroll 8
+        for (int s = 0; s < P.S; s += 4) {
+          const int4 l = *reinterpret_cast<const int4*>(length + s);
+          rank += (l.x > mine_at) + (l.y > mine_at) + (l.z > mine_at) + (l.w > mine_at);
+        }
         order[rank] = seq;
         chunk_prefix[rank + 1] = n;                              // counts first, sums below
       }
