@@ -181,6 +181,9 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   const int chunk0 = group0 * p.group_chunks, chunk1 = min(p.chunks, group1 * p.group_chunks);
 
   auto load_w = [&](int c, int stage) {
+#ifdef FT_TEST_NO_LOADS
+    return;
+#endif
     unsigned char* dst = w_ring + stage * FT_W_BYTES;
     tc_mbar_expect_tx(&w_full[stage], FT_W_BYTES);
     tc_tma_load(dst, &map_w, c * FT_BK, n0, &w_full[stage]);
@@ -292,7 +295,7 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     const uint32_t a0 = tmem_a + ((uint32_t)((warp & 3) * 32) << 16) + unit0 * 8;
     FtPlace at, two;
     for (int c = chunk0; c < chunk1; ++c, at.step(p.w_stages), two.step(2)) {
-      if (!tc_wait(&w_full[at.s], at.turn, abort_flag)) break;
+      if (!tc_wait_warp(&w_full[at.s], at.turn, abort_flag)) break;
       const unsigned char* row = w_ring + at.s * FT_W_BYTES + (unit0 >> 1) * (FT_W_BYTES / 2) + r * 128;
       uint32_t hi[UNITS][8], mid[UNITS][8], lo[UNITS][8];
 #pragma unroll
@@ -304,7 +307,7 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
           ft_cut2(v.z, v.w, hi[u][2 * j + 1], mid[u][2 * j + 1], lo[u][2 * j + 1]);
         }
       // all but the stores lies before the wait for the products that read this place
-      if (!tc_wait(&done[two.s], two.turn ^ 1, abort_flag)) break;
+      if (!tc_wait_warp(&done[two.s], two.turn ^ 1, abort_flag)) break;
       tc_fence_after();
 #pragma unroll
       for (int u = 0; u < UNITS; ++u) {
@@ -352,7 +355,7 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     };
     auto promote = [&](int it) {
       const int buf = it & 1;
-      if (!tc_wait(&done[buf], (it >> 1) & 1, abort_flag)) { ok = false; return; }
+      if (!tc_wait_warp(&done[buf], (it >> 1) & 1, abort_flag)) { ok = false; return; }
       tc_fence_after();
       constexpr int STEP = HC < 32 ? HC : HC == 32 ? 32 : 24;
 #pragma unroll
@@ -398,7 +401,7 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
       for (int i = 0; i < 4; ++i) { next[i][0] = fetch(chunk0 + i, row); next[i][1] = fetch(chunk0 + i, row + 8); }
       FtPlace at;
       auto put = [&](int c, float4* slot) {
-        if (!tc_wait(&b_empty[at.s], at.turn ^ 1, abort_flag)) { ok = false; return; }
+        if (!tc_wait_warp(&b_empty[at.s], at.turn ^ 1, abort_flag)) { ok = false; return; }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float4 v = slot[h];

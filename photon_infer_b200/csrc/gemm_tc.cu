@@ -154,7 +154,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     int local = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
       const int buf = local & 1;
-      if (!tc_wait(&acc_ready[buf], (local >> 1) & 1, abort_flag)) break;
+      if (!tc_wait_warp(&acc_ready[buf], (local >> 1) & 1, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int m0 = (tile / tiles_n) * TC_BM, n0 = (tile % tiles_n) * TILE_COLS;
       const int row = m0 + quad * 32 + lane;

@@ -191,7 +191,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     int local = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local) {
       const int buf = local & 1;
-      if (!t2_wait(&acc_ready[buf], (local >> 1) & 1, abort_flag)) break;
+      if (!__all_sync(0xffffffffu, t2_wait(&acc_ready[buf], (local >> 1) & 1, abort_flag))) break;      // tcgen05.ld needs all lanes
       tc_fence_after();
       const int m0 = (tile / tiles_n) * (2 * T2_BM) + (int)rank * T2_BM, n0 = (tile % tiles_n) * TILE_COLS;
       const int row = m0 + quad * 32 + lane;

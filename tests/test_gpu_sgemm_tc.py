@@ -83,3 +83,27 @@ def test_magnitudes_far_from_one(scale):
     torch.manual_seed(24)
     x, w = torch.randn(20, 2048, device=DEV), torch.randn(2048, 2048, device=DEV)
     assert torch.equal(ops.linear(x * scale, w / scale), ops.linear(x, w))
+
+
+@pytest.mark.parametrize("rows,one_launch", [(7, 1), (7, 0), (150, 0)])
+def test_a_wait_that_runs_out_is_reported(rows, one_launch):
+    """A build whose weights never come and whose waits give up after a few thousand polls: every warp gives up as a whole, the kernel
+    reports PHOTON_DEV_WAIT_TIMEOUT and returns; the stock build runs right afterwards."""
+    from ctypes import c_int, c_long, c_void_p
+    from photon_infer_b200.csrc.build import load_module
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(26)
+    N, K = 2048, 2048
+    x, w, out = torch.randn(rows, K, device=DEV), torch.randn(N, K, device=DEV), torch.zeros(rows, N, device=DEV)
+    err, scratch = torch.zeros(4, dtype=torch.int32, device=DEV), torch.empty(64 << 20, dtype=torch.uint8, device=DEV)
+    f = load_module("gemm_f32_tc", {"FT_TEST_NO_LOADS": 1, "TC_WAIT_LIMIT": 4096}).photon_sgemm_tc
+    f.argtypes = [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p]
+    f.restype = c_int
+    assert f(x.data_ptr(), K, w.data_ptr(), K, out.data_ptr(), N, rows, N, K, one_launch, scratch.data_ptr(), scratch.numel(), err.data_ptr(),
+             torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert err.cpu().tolist()[0] == 4
+    err.zero_()
+    ops.sgemm_tc(x, w, out, err)
+    assert err.cpu().tolist()[0] == 0
+    assert float((out.double() - x.double() @ w.double().t()).norm() / out.double().norm()) < 1e-6
