@@ -1052,6 +1052,7 @@ def gemm_tc_qkv(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, posit
 
 SGEMM_TC_MIN = 1024         # rows and columns of a 32-bit weight, and
 SGEMM_TC_SIZE = 1 << 22     # numbers in it, from which its products run on the tensor cores
+SGEMM_ONE_LAUNCH_SIZE = 1 << 24     # numbers in it, from which a product of few rows is three launches
 
 
 def sgemm_tc_supported(weight: torch.Tensor) -> bool:
@@ -1074,9 +1075,10 @@ def sgemm_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, err: Opti
         raise PhotonError(ErrorCode.SHAPE_MISMATCH, f"sgemm_tc: x [M, {K}] against weight {tuple(weight.shape)}")
     if err is None:
         err = _error_word(x.device)
-    # few rows: one launch where the host would feel three, the faster three in a captured step and where the GPU takes longer
-    # than the host (one row against 128,256 x 2,048: 262 us in one launch); the same bits
-    one_launch = M <= 16 and N * K <= 1 << 25 and not torch.cuda.is_current_stream_capturing()
+    # few rows: one launch where the host would feel three (some 22 us), the faster three in a captured step and where the GPU takes
+    # longer than the host (one row, us, one launch and three: 3,072 x 2,048 13 and 22, 1,024 x 8,192 20 and 22, 2,048 x 8,192 28 and 22,
+    # 16,384 x 2,048 38 and 31); the same bits
+    one_launch = M <= 16 and N * K < SGEMM_ONE_LAUNCH_SIZE and not torch.cuda.is_current_stream_capturing()
     n, scratch = 0, None
     if not one_launch:
         n = _fn("gemm_f32_tc", "photon_sgemm_tc_scratch", [c_int, c_int, c_int], restype=c_long)(M, N, K)

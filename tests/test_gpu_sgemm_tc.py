@@ -107,3 +107,15 @@ def test_a_wait_that_runs_out_is_reported(rows, one_launch):
     ops.sgemm_tc(x, w, out, err)
     assert err.cpu().tolist()[0] == 0
     assert float((out.double() - x.double() @ w.double().t()).norm() / out.double().norm()) < 1e-6
+
+
+@pytest.mark.parametrize("N,K", [(4095, 4096), (4096, 4096)])
+def test_both_sides_of_the_line_between_one_launch_and_three(N, K):
+    """The rows of a product of many: below 2^24 numbers one launch forms few rows, from there on three do."""
+    from photon_infer_b200.kernels import ops
+    torch.manual_seed(27)
+    assert ops.SGEMM_ONE_LAUNCH_SIZE == 4096 * 4096
+    x, w = torch.randn(40, K, device=DEV), torch.randn(N, K, device=DEV)
+    out = ops.linear(x, w)
+    for rows in (1, 3, 16):
+        assert torch.equal(ops.linear(x[:rows], w), out[:rows]), rows
