@@ -537,6 +537,15 @@ PHOTON_API long photon_sgemm_tc_scratch(int M, int N, int K) {
   return ft_parts_bytes(M, K) + (b.splits > 1 ? (long)b.groups * M * N * 4 : 0);
 }
 
+// Kernels that photon_sgemm_tc launches.
+PHOTON_API int photon_sgemm_tc_launches(int M, int N, int K, int one_launch) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (one_launch) return 1;
+  int n = 0;
+  for (; M > 0; M -= FT_SLAB) n += ft_plan(M < FT_SLAB ? M : FT_SLAB, N, K, false).splits > 1 ? 3 : 2;
+  return n;
+}
+
 template <int HC, bool FEW>
 static int ft_go(const CUtensorMap& mw, const CUtensorMap& mb, const FtArgs& a, int blocks, size_t smem, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(ft_kernel<HC, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -525,6 +525,7 @@ PHOTON_EXPORT int photon_sgemm_nt(const float* A, long lda, const float* W, long
  * no scratch, for calls whose launches the host pays for; else scratch: 16-byte aligned, at least photon_sgemm_tc_scratch(M, N, K)
  * bytes, written before it is read.  The same bits either way. */
 PHOTON_EXPORT long photon_sgemm_tc_scratch(int M, int N, int K);
+PHOTON_EXPORT int photon_sgemm_tc_launches(int M, int N, int K, int one_launch);      /* kernels that a call launches */
 PHOTON_EXPORT int photon_sgemm_tc(const float* A, long lda, const float* W, long ldw, float* C, long ldc, int M, int N, int K,
                     int one_launch, void* scratch, long scratch_bytes, int* err, cudaStream_t stream);
 

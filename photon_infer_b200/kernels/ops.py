@@ -1062,6 +1062,11 @@ def sgemm_tc_supported(weight: torch.Tensor) -> bool:
     return min(N, K) >= SGEMM_TC_MIN and N * K >= SGEMM_TC_SIZE and K % 4 == 0 and weight.data_ptr() % 16 == 0
 
 
+@functools.lru_cache(maxsize=4096)
+def _sgemm_tc_launches(M: int, N: int, K: int, one_launch: bool) -> int:
+    return _fn("gemm_f32_tc", "photon_sgemm_tc_launches", [c_int] * 4)(M, N, K, int(one_launch))
+
+
 def sgemm_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, err: Optional[torch.Tensor] = None) -> None:
     """``out = x @ weight^T`` in 32-bit accuracy, each number split into three bfloat16 parts whose products run on the
     tcgen05 tensor cores.  float32 ``x [M, K]`` and ``out [M, N]`` with any row stride, ``weight`` contiguous with K a
@@ -1087,6 +1092,8 @@ def sgemm_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, err: Opti
             [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int, c_int, c_void_p, c_long, c_void_p, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, int(one_launch), _ptr(scratch), n,
              _ptr(err), _stream()), "sgemm_tc")
+    global _launch_count
+    _launch_count += _sgemm_tc_launches(M, N, K, one_launch) - 1
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
@@ -1856,6 +1863,8 @@ def linrec(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate_a:
              gate_a.stride(0) if gate_a is not None else 0, _ptr(p0), _ptr(p1), _ptr(p2), float(cap), float(q_scale), _ptr(cu_tokens), _ptr(state_slots),
              _ptr(state), state.stride(0), state.shape[0], _ptr(out), out.stride(0), int(num_seqs), heads, qk_heads, dim, vdim,
              _ptr(fresh), _ptr(err), _stream()), "linrec")
+    global _launch_count
+    _launch_count += mode == "matrix_memory"              # the new n and m are stored by a launch of their own
 
 
 #: A bfloat16 step in which some request brings at least this many tokens cuts its recurrences into segments: two of 64 tokens are the
