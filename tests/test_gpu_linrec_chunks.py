@@ -19,7 +19,7 @@ def any_size(monkeypatch):
     monkeypatch.setattr(ops, "linrec_chunks_faster", lambda *args: True)
 
 
-def _case(mode, H, G, N, dv, lens, slots, strong, seed, poison=None):
+def _case(mode, H, G, N, dv, lens, slots, strong, seed, poison=None, what="v"):
     from photon_infer_b200.kernels import ops
     gen = torch.Generator().manual_seed(seed)
     T = sum(lens)
@@ -37,7 +37,8 @@ def _case(mode, H, G, N, dv, lens, slots, strong, seed, poison=None):
     width += 4 + -width % 4
     state = torch.randn(7, width, generator=gen)
     if poison is not None:
-        rows[poison[0], a0 + poison[1]] = poison[2]
+        first = {"q": 0, "k": G * N, "a": 2 * G * N, "v": a0, "gate_a": b0, "gate_b": b0 + H}[what]
+        rows[poison[0], first + poison[1]] = poison[2]
     st, r = state.to(DEV), rows.to(DEV)
     cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
     out, err = torch.full((T, H * dv), float("nan"), device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
@@ -96,6 +97,28 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(mode, value):
     S = after[0, :H * N * dv].view(H, N, dv)
     assert not bool(torch.isfinite(S[0, :, col]).any()) and torch.equal(after[1], clean_after[1])
     assert torch.equal(S[:, :, 4:], clean_after[0, :H * N * dv].view(H, N, dv)[:, :, 4:])
+
+
+@pytest.mark.parametrize("mode,what", [(m, w) for m in MODES for w in ("q", "k", "gate_a", "gate_b", "a")
+                                        if (w != "gate_a" or m != "decay_rows") and (w != "gate_b" or m == "matrix_memory") and (w != "a" or m == "decay_rows")])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("strong", [False, True])
+def test_inputs_that_are_not_finite_reach_no_earlier_token(mode, what, value, strong):
+    """Queries, keys, gates and decays: other heads, the other request and earlier tokens keep their bits (blocks of row decays may take
+    another form for the decay: their roundings), and what is not finite in the recurrence token by token is not finite here."""
+    H, N, dv, lens, t = 2, 32, 16, [200, 130], 75
+    got, after, _, wants, cu = _case(mode, H, H, N, dv, lens, [0, 1], strong, 9, poison=(t, 0, value), what=what)
+    clean, clean_after, _, _, _ = _case(mode, H, H, N, dv, lens, [0, 1], strong, 9)
+    assert torch.equal(got[:, dv:], clean[:, dv:]) and torch.equal(got[200:], clean[200:]) and torch.equal(after[1], clean_after[1])
+    if what == "a":
+        assert _rel(got[:t, :dv], clean[:t, :dv].double()) < 2e-6
+    else:
+        assert torch.equal(got[:t, :dv], clean[:t, :dv])
+    want = wants[0][0][:, :dv]
+    there = torch.isfinite(want)
+    assert not bool((torch.isfinite(got[:200, :dv]) & ~there).any())
+    if bool(there[t:].any()):                            # a query: its own token alone; a gate or a decay that only closes
+        assert _rel(torch.where(there, got[:200, :dv], 0.0), torch.where(there, want, 0.0)) < 5e-5
 
 
 @pytest.mark.parametrize("mode", MODES)
