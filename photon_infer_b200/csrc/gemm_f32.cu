@@ -7,7 +7,7 @@
 // row's result does not depend on M, on the kernel or tile it fell into or on the other rows:
 // the float32 path gives identical bits for every way of cutting a request into steps.  So K is never
 // split, and the kernels below differ only in how they bring the operands to the multiply-adds.
-// Weights of 2^22 numbers and more, 1,024 or more either way, do not come here but to gemm_f32_tc.cu (ops.sgemm_tc_supported).
+// Weights of 2^22 numbers, 1,024 rows and 2,048 columns and more do not come here but to gemm_f32_tc.cu (ops.sgemm_tc_supported).
 #include "common.cuh"
 
 __device__ __forceinline__ void sg_cp16(float* dst, const float* src, bool in) {      // nothing is read where `in` does not

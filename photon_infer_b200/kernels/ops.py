@@ -1050,8 +1050,10 @@ def gemm_tc_qkv(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, posit
              k_cache.shape[2], k_cache.shape[0] * k_cache.shape[2], _ptr(err), _stream()), "gemm_tc_qkv")
 
 
-SGEMM_TC_MIN = 1024         # rows and columns of a 32-bit weight, and
-SGEMM_TC_SIZE = 1 << 22     # numbers in it, from which its products run on the tensor cores
+# Rows and columns of a 32-bit weight, and numbers in it, from which its products run on the tensor cores.  One row, captured, weights from
+# memory, us, chain and tensor cores: 4,096 x 1,024 7 and 10, 8,192 x 1,024 9 and 14 (eight rows 20 and 15, 513 125 and 42: few columns are a
+# short chain), 2,048 x 2,048 10 and 10, 3,072 x 2,048 12 and 13, 16,384 x 2,048 31 and 30, 1,024 x 4,096 18 and 12, 2,048 x 8,192 34 and 19.
+SGEMM_TC_MIN_ROWS, SGEMM_TC_MIN_COLUMNS, SGEMM_TC_SIZE = 1024, 2048, 1 << 22
 SGEMM_ONE_LAUNCH_SIZE = 1 << 24     # numbers in it, from which a product of few rows is three launches
 
 
@@ -1059,7 +1061,8 @@ def sgemm_tc_supported(weight: torch.Tensor) -> bool:
     """Whether 32-bit products with this weight are sums of tensor-core products (``gemm_f32_tc.cu``).  The weight alone
     decides, never the rows that meet it: one row has the bits that it has among many."""
     N, K = weight.shape
-    return min(N, K) >= SGEMM_TC_MIN and N * K >= SGEMM_TC_SIZE and K % 4 == 0 and weight.data_ptr() % 16 == 0
+    return (N >= SGEMM_TC_MIN_ROWS and K >= SGEMM_TC_MIN_COLUMNS and N * K >= SGEMM_TC_SIZE and K % 4 == 0
+            and weight.data_ptr() % 16 == 0)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -1099,7 +1102,7 @@ def sgemm_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, err: Opti
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``x [M, K] @ weight[N, K]^T``.  float32: this package's own kernels in 32-bit accuracy (weights of
-    1,024 x 1,024 and more as sums of tensor-core products, others as chains of multiply-adds).
+    2^22 numbers, 1,024 rows and 2,048 columns and more as sums of tensor-core products, others as chains of multiply-adds).
     bfloat16: up to 8 rows the weight-streaming kernel; with enough 128 x 256 tiles to fill the
     GPU the tcgen05 kernel; in between the library product (cuBLAS through torch), where the
     reference's engine also calls the library (src/ops/kernels/cuda/matmul_dequant_cached.cu:193-207)."""

@@ -12,6 +12,14 @@ DEV = "cuda:0"
 SIZES = [(2048, 2048), (2050, 2052), (1030, 4100), (4160, 1020 + 8), (1024, 8192)]
 
 
+def _product(x, w):
+    """On the tensor cores, also weights of few columns, which ``linear`` leaves to the chain."""
+    from photon_infer_b200.kernels import ops
+    out = torch.empty(x.shape[0], w.shape[0], device=DEV)
+    ops.sgemm_tc(x, w, out)
+    return out
+
+
 def _chain(x, w):
     """The product as gemm_f32.cu forms it: a chain of multiply-adds."""
     from photon_infer_b200.kernels import ops
@@ -26,16 +34,16 @@ def test_accuracy_and_the_same_bits_for_every_row_count(N, K):
     from photon_infer_b200.kernels import ops
     torch.manual_seed(21)
     x, w = torch.randn(513, K, device=DEV), torch.randn(N, K, device=DEV)
-    assert ops.sgemm_tc_supported(w)
-    out = ops.linear(x, w)
+    out = _product(x, w)
+    assert not ops.sgemm_tc_supported(w) or torch.equal(out, ops.linear(x, w))
     want = x.double() @ w.double().t()
     error = (out.double() - want).abs()
     assert bool((error <= 20 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all())
     # no further from 64 bits than the chain of multiply-adds
     assert float(error.pow(2).mean()) <= float((_chain(x, w).double() - want).pow(2).mean())
     for rows in (1, 2, 15, 16, 17, 33, 64, 65, 96, 97, 200):
-        assert torch.equal(ops.linear(x[:rows], w), out[:rows]), rows
-    assert torch.equal(ops.linear(x[500:], w), out[500:])
+        assert torch.equal(_product(x[:rows], w), out[:rows]), rows
+    assert torch.equal(_product(x[500:], w), out[500:])
 
 
 @pytest.mark.parametrize("rows", [1, 16, 40])
@@ -57,11 +65,17 @@ def test_strided_rows_and_captured_launches(rows):
 
 
 def test_more_rows_than_one_round_takes():
-    from photon_infer_b200.kernels import ops
     torch.manual_seed(25)
     x, w = torch.randn(4096 + 33, 1024, device=DEV), torch.randn(4096, 1024, device=DEV)
-    out = ops.linear(x, w)
-    assert torch.equal(out[4090:], ops.linear(x[4090:], w)) and torch.equal(out[:40], ops.linear(x[:40], w))
+    out = _product(x, w)
+    assert torch.equal(out[4090:], _product(x[4090:], w)) and torch.equal(out[:40], _product(x[:40], w))
+
+
+@pytest.mark.parametrize("N,K,tensor", [(1024, 4096, True), (2048, 2048, True), (1023, 8192, False), (1024, 4092, False), (4096, 1024, False),
+                                        (8192, 2044, False)])
+def test_which_weights(N, K, tensor):
+    from photon_infer_b200.kernels import ops
+    assert ops.sgemm_tc_supported(torch.empty(N, K, device=DEV)) == tensor
 
 
 @pytest.mark.parametrize("rows", [9, 70])
