@@ -2,10 +2,11 @@
 //
 // A 32-bit number is the sum of three bfloat16 numbers, each what the ones before left (W's by cutting bits off, 8 + 8 + 8, the
 // tokens' by rounding; exact down to 2^-110, where the third one's last bits leave bfloat16's range).  Of the nine products of such
-// parts the six largest are formed; the three that are left out are below 2^-24 of the term, of either sign.  Six bfloat16
+// parts the six largest are formed.  Of a term w a with w and a in [1, 2), w's second and third parts are below 2^-7 and 2^-15, the tokens'
+// 2^-8 and 2^-17 at most: the three products left out are below 2^-23 + 2^-24 + 2^-32 of it (2^-22.4), of either sign.  Six bfloat16
 // products a term are still six times what the FP32 pipe does (1.6 PFLOP/s / 6 against 31 to 46 TFLOP/s of gemm_f32.cu's
 // tiles).  Measured, 513 rows, against those: 3072 x 2048 46 us (190), 2048 x 2048 42 (141), 16384 x 2048 212 (870), 2048 x 8192
-// 135 (545); one row 19, 15, 39 and 27 (16, 14, 37 and 39).  Error against 64 bits (rms, K = 2048): 1.1e-7, the chain's 8.1e-7.
+// 135 (545); one row, captured, weights from memory, 13, 10, 30 and 19 (12, 10, 31 and 34).  Error against 64 bits (rms, K = 2048): 1.1e-7, the chain's 8.1e-7.
 // What bounds it: at 513 rows the products (1.1 PFLOP/s of bfloat16 with ragged tiles and a last round), with 69 KB a chunk
 // and SM from L2 close behind; up to 64 rows W's bytes.
 //

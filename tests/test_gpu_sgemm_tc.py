@@ -29,8 +29,9 @@ def _chain(x, w):
 @pytest.mark.parametrize("N,K", SIZES)
 def test_accuracy_and_the_same_bits_for_every_row_count(N, K):
     """Error: in a chunk of 64 the four additions of the large products are truncated, at most two units of 2^-23 each with the
-    alignment inside the instruction; up to 16 chunks a group and 8 groups are rounded (2^-24 each); the small products and the
-    terms left out add less than one: 8 + 8 + 4 = 20 units of 2^-23 of the sum of magnitudes."""
+    alignment inside the instruction, 8 units; up to 15 sums of chunks in a group and 7 of groups are rounded (half a unit each), 11;
+    the products left out are below 1.51 units of their terms, and the truncations of the small products, twenty of two units of 2^-7 of
+    the sum, below 0.32: 21 units of 2^-23 of the sum of magnitudes."""
     from photon_infer_b200.kernels import ops
     torch.manual_seed(21)
     x, w = torch.randn(513, K, device=DEV), torch.randn(N, K, device=DEV)
@@ -38,7 +39,7 @@ def test_accuracy_and_the_same_bits_for_every_row_count(N, K):
     assert not ops.sgemm_tc_supported(w) or torch.equal(out, ops.linear(x, w))
     want = x.double() @ w.double().t()
     error = (out.double() - want).abs()
-    assert bool((error <= 20 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all())
+    assert bool((error <= 21 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all())
     # no further from 64 bits than the chain of multiply-adds
     assert float(error.pow(2).mean()) <= float((_chain(x, w).double() - want).pow(2).mean())
     for rows in (1, 2, 15, 16, 17, 33, 64, 65, 96, 97, 200):
