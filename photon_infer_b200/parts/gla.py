@@ -11,7 +11,8 @@ slot between steps; decays, their logarithms and the recurrence itself are 32-bi
 
 One fused product gives ``[q | k | v | g | W_a1 h]``.  For few tokens one kernel forms the decay logits from the low-rank part,
 runs the recurrence over the tokens of a step and applies the norm and the gate in its epilogue; a step with a long portion
-forms the decays of all tokens first, runs the recurrence in segments side by side (``linrec_segments.cu``), and then norm and gate.  Portions in
+forms the decays of all tokens first, runs the recurrence in segments side by side (``linrec_segments.cu``) or in chunks on the tensor
+cores (``linrec_chunks.cu``), and then norm and gate.  Portions in
 between run chunks of 32 tokens from zero states side by side, joined by a scan.
 """
 from __future__ import annotations
@@ -77,7 +78,7 @@ class GatedLinearAttention(Mixer):
         v, g = fused[:, 2 * nd:2 * nd + nv], fused[:, 2 * nd + nv:2 * nd + 2 * nv]
         low = fused[:, 2 * nd + 2 * nv:]
         out = torch.empty((T, nv), dtype=h.dtype, device=h.device)
-        # a step with a long bfloat16 portion runs in segments of tokens side by side; everything else (and the float32 run, whose
+        # a step with a long bfloat16 portion runs in segments or chunks of tokens side by side; everything else (and the float32 run, whose
         # sums depend on nothing but the token's place in its request) goes token by token
         lens = list(ctx.host_query_lens)
         if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("decay_rows", self.dim, lens, self.heads) \

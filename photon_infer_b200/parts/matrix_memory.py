@@ -13,7 +13,7 @@ Each head's ``o`` is divided by its root mean square; the heads are concatenated
 the request's state slot between steps; everything after the input product is 32-bit.
 
 Kernels of a step: ONE product ``[q | k | v | g | i | f]`` with 32-bit rows; the recurrence over the tokens of the step
-(``linrec.cu``; the vector ``n`` rides along as one more column of ``S``); norm and gate in one pass (``row_norms.cu``);
+(``linrec.cu``; the vector ``n`` rides along as one more column of ``S``; long portions ``linrec_segments.cu`` or ``linrec_chunks.cu``); norm and gate in one pass (``row_norms.cu``);
 the output product.
 """
 from __future__ import annotations
@@ -76,7 +76,7 @@ class MatrixMemoryMixer(Mixer):
         g0 = 2 * nd + nv
         lens = list(ctx.host_query_lens)
         if h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("matrix_memory", self.dim, lens, H):
-            # long portions: segments of tokens side by side; the division rides in the norm
+            # long portions: segments or chunks of tokens side by side; the division rides in the norm
             den = ops.linrec_segments("matrix_memory", rows[:, :nd], rows[:, nd:2 * nd], rows[:, 2 * nd:g0], None, rows[:, g0 + nv:g0 + nv + H],
                                       rows[:, g0 + nv + H:], self.i_bias, self.f_bias, None, self.gate_cap, self.dim ** -0.5, ctx.cu_tokens,
                                       ctx.state_slots, cache.state, o, lens, H, H, self.dim, self.vdim, ctx.error_flag)

@@ -91,7 +91,7 @@ class StateSpaceMixer(Mixer):
         lens = list(ctx.host_query_lens)
         long = h.dtype == torch.bfloat16 and lens and ops.linrec_segments_supported("state_space", self.state, lens, self.heads)
         if long:
-            # long portions: segments of tokens side by side
+            # long portions: segments or chunks of tokens side by side
             ops.linrec_segments("state_space", y[:, inner + GN:], y[:, inner:inner + GN], y[:, :inner], None, rows[:, inner + C:], None,
                                 self.a_log, self.dt_bias, self.d_skip, 0.0, 1.0, ctx.cu_tokens, ctx.state_slots, cache.state, o, lens,
                                 self.heads, self.groups, self.state, self.vdim, ctx.error_flag)
