@@ -486,8 +486,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 // The first tile's products end with its own last key: a value that is not finite, of a token that only the second tile sees, meets
 // weights of 0 there, and 0 times it would be NaN.  The 16 keys among which it ends come with zeros behind it from a place of their own
 // (0.9 us a block: 2,048 tokens from the start 48.3 and 50.1).
-// Bound by the softmax warps (4,500 cycles for a pair of tiles of 128 keys, of which the exponentials take 2,048 at 16 a cycle and SM and the
-// products as many).  2,048 tokens behind 14,336, 32/8 heads of 128: 657 us with a tile a block, 482 so (1,070 TFLOP/s);
+// Bound by the softmax warps (3,700 cycles for a pair of tiles of 128 keys, of which the exponentials take 2,048 at 16 a cycle and SM and the
+// products as many: both units are active for 55 % of the time).  2,048 tokens behind 14,336, 32/8 heads of 128: 657 us with a tile a block, 482 so (1,070 TFLOP/s);
 // 2,048 from the start 54 and 50.  Heads of 64 gain nothing at any length (2,048 tokens 43 and 46 us; with columns of its own for P 42 and 48).
 #if HEAD_DIM > 64
 #define AP_KT 128

@@ -33,3 +33,11 @@ __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
+// Two 32-bit numbers as three packed bfloat16 parts, each the rounding of what the ones before left.
+__device__ __forceinline__ void at_split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = at_pack(x, y);
+  x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xffff0000u);          // exact
+  mid = at_pack(x, y);
+  x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xffff0000u);
+  lo = at_pack(x, y);
+}

@@ -37,8 +37,8 @@
 #define FT_GROUPS 8
 #define FT_FEW 16                     // tokens up to which one launch does all
 #define FT_A_COLS 96                  // tensor memory columns of a chunk's parts of W
-// Warps of a block: four that issue, those that split W (with eight a chunk of many tokens took 1,400 cycles, waits in a row and
-// half-rate bit operations), those that add the chunks up.  Up to FT_FEW tokens half as many, so that two blocks fit an SM.
+// Warps of a block: four that issue, those that split W (eight were slower with many tokens: waits in a row and half-rate bit
+// operations), those that add the chunks up.  Up to FT_FEW tokens half as many, so that two blocks fit an SM.
 template <bool FEW> struct FtShape {
   static constexpr int splitters = FEW ? 8 : 16, adders = FEW ? 4 : 8, threads = (4 + splitters + adders) * 32;
   static constexpr int d_cols = FEW ? 32 : 96, tmem_cols = FEW ? 256 : 512;     // of an accumulator; of all (a power of two)
@@ -50,16 +50,7 @@ __device__ __forceinline__ void ft_st8(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-// Two neighbours of K as packed parts.
-__device__ __forceinline__ void ft_split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = at_pack(x, y);
-  x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xffff0000u);          // exact
-  mid = at_pack(x, y);
-  x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xffff0000u);
-  lo = at_pack(x, y);
-}
-
-// The same by cutting bits off: 8 + 8 + 8 bits, all of them.
+// at_split2 by cutting bits off: 8 + 8 + 8 bits, all of them.
 __device__ __forceinline__ void ft_cut2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
   x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u); y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
@@ -105,8 +96,8 @@ ft_split_kernel(const float* __restrict__ A, long lda, int M, int K, int Kp, bf1
       if (k + 3 < K) v.w = src[3];
     }
     uint2 p[3];
-    ft_split2(v.x, v.y, p[0].x, p[1].x, p[2].x);
-    ft_split2(v.z, v.w, p[0].y, p[1].y, p[2].y);
+    at_split2(v.x, v.y, p[0].x, p[1].x, p[2].x);
+    at_split2(v.z, v.w, p[0].y, p[1].y, p[2].y);
 #pragma unroll
     for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(parts + j * plane + (size_t)m * Kp + k) = p[j];
   }
@@ -408,8 +399,8 @@ ft_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
           const float4 v = slot[h];
           slot[h] = fetch(c + 4, row + 8 * h);
           uint2 q[3];
-          ft_split2(v.x, v.y, q[0].x, q[1].x, q[2].x);
-          ft_split2(v.z, v.w, q[0].y, q[1].y, q[2].y);
+          at_split2(v.x, v.y, q[0].x, q[1].x, q[2].x);
+          at_split2(v.z, v.w, q[0].y, q[1].y, q[2].y);
           // as TMA would lay them: 128 bytes a row, 16-byte pieces swizzled by the row
           unsigned char* dst = b_ring + at.s * b_bytes + (row + 8 * h) * 128 + (((quad4 >> 1) ^ (row & 7)) << 4) + (quad4 & 1) * 8;
 #pragma unroll

@@ -9,6 +9,18 @@ __device__ __forceinline__ float lr_logsigmoid(float x) { return fminf(x, 0.f) -
 // Inputs of mode 2 (forget and write).
 __device__ __forceinline__ float lr_silu(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float lr_write_gate(float z, float bias, float lower) { return (1.0f - lower) / (1.0f + expf(z + bias)); }
+// The product b of decays and what it lacks to 1, B = 1 - b, brought forward by a decay that lacks `gone` to 1 (`scaled` is that
+// decay times b).  Near 1 a product rounds to 2^-25 of itself at every token, always alike where the decays hardly change, which over
+// hundreds of tokens is far more than the state's own roundings; B keeps all its bits there.  Below 1/2 the product is the exact one.
+__device__ __forceinline__ void lr_decay(float scaled, float gone, float& b, float& B) {
+  B = fmaf(gone, b, B);
+  b = B < 0.5f ? 1.0f - B : scaled;
+}
+// A decay as one number: -B (minus zero for a decay of 1) where B lies between 0 and 1/2, else b (also behind a decay that the
+// rounding of a running maximum has put above 1).  x decays to fma(code, x, x or 0): the sign says which.
+__device__ __forceinline__ float lr_code(float b, float B) { return B >= 0.f && B < 0.5f ? -fabsf(B) : b; }
+__device__ __forceinline__ uint32_t lr_mask(float code) { return (uint32_t)(__float_as_int(code) >> 31); }
+__device__ __forceinline__ float lr_apply(float code, float x) { return fmaf(code, x, __uint_as_float(__float_as_uint(x) & lr_mask(code))); }
 __device__ __forceinline__ void lr_cp4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
 }

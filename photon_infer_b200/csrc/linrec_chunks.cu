@@ -23,15 +23,14 @@
 // product of the decays since a reference, the chunk's start while no row's decays multiply to less than LC_SMALL there.  Else
 // blocks of 64 or 32 tokens take their own starts: for the queries of block j, keys of the blocks before it are multiplied by decays
 // up to the start of j (at most 1), those of j itself divided by theirs; and the weights of a block of 32 that is still out of range
-// are formed one by one in 32 bits.  Products of decays near 1 are carried by what they lack to 1 (lc_decay), as in linrec_segments.cu.
+// are formed one by one in 32 bits.  Products of decays near 1 are carried by what they lack to 1 (lr_decay), as in linrec_segments.cu.
 //
-// What bounds it: none of the tensor cores (a chunk's 150 to 200 products take 5 us of the 22 to 40 that a block of lc_out_kernel takes),
-// memory (384 KB a block) or issue slots (38 % used) alone, but one block an SM whose phases (rows in, parts, products, weights, rows
+// What bounds it: none of the tensor cores (active for 12 to 15 % of lc_ends_kernel's and lc_out_kernel's time), memory (384 KB a block, 15 to 20 %
+// of the DRAM rate) or issue slots (32 to 40 % used) alone, but one block an SM whose phases (rows in, parts, products, weights, rows
 // out) follow one another.  Straight-line code is fetched once a block: with the products' loop unrolled the same block took 10 to 15 %
 // longer.  Rows by bulk copies instead of loads into registers, and calls instead of inlined splits, changed nothing.
-// Measured, heads of 128 x 128, the recurrence alone, us, segments first: gated linear attention, 2,048 tokens of 16 heads 176 and 102
-// (26 for the sums, 14 from chunk to chunk, 62 for the outputs); matrix memory, two requests of 2,815 251 and 131; state space, 2,048 161
-// and 93.
+// Measured, 2,048 tokens of 16 heads of 128 x 128, the recurrence alone, us, segments first: gated linear attention 176 and 102, matrix memory 183
+// and 96, state space 155 and 84.
 //
 // A value that is not finite would reach earlier tokens of its chunk through products with weights of 0: it is left out of
 // the products, and its column is NaN from its token on.
@@ -60,45 +59,27 @@ struct LcArgs {
   float* den;                                        // mode 1: [T][H], what the outputs are to be divided by
   float* gates;                                      // planes [T][H], see lc_gates_kernel
   float* ends;                                       // [chunks][H][N * dv]: U, then S_0
-  float* vecs;                                       // [chunks][H][N]: mode 1 the sum of keys, then n at the start; mode 3 the rows' decay (lc_code)
+  float* vecs;                                       // [chunks][H][N]: mode 1 the sum of keys, then n at the start; mode 3 the rows' decay (lr_code)
   float* scale;                                      // [chunks][H][4]: the chunk's F (high, low); mode 1 also F + M
   int T, S, H, qk_heads, N, dv, chunks;
   int* err;
 };
 
-// ---------------------------------------------------------------- decays (see linrec_segments.cu)
-__device__ __forceinline__ void lc_decay(float scaled, float gone, float& b, float& B) {
-  B = fmaf(gone, b, B);
-  b = B < 0.5f ? 1.0f - B : scaled;
-}
-__device__ __forceinline__ float lc_code(float b, float B) { return B >= 0.f && B < 0.5f ? -fabsf(B) : b; }
-__device__ __forceinline__ float lc_apply(float code, float x) {
-  return fmaf(code, x, __uint_as_float(__float_as_uint(x) & (uint32_t)(__float_as_int(code) >> 31)));
-}
-
 // ---------------------------------------------------------------- operands in shared memory
-// Two neighbours as packed parts, each the rounding of what the ones before left.
-__device__ __forceinline__ void lc_split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = at_pack(x, y);
-  x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xffff0000u);          // exact
-  mid = at_pack(x, y);
-  x -= __uint_as_float(mid << 16); y -= __uint_as_float(mid & 0xffff0000u);
-  lo = at_pack(x, y);
-}
 __device__ __forceinline__ unsigned char* lc_at(unsigned char* plane, int row, int col) {      // col even
   return plane + (col >> 6) * LC_HALF + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4) + (col & 7) * 2;
 }
 __device__ __forceinline__ void lc_put2(unsigned char* plane, int row, int col, float x, float y) {
   uint32_t p[3];
-  lc_split2(x, y, p[0], p[1], p[2]);
+  at_split2(x, y, p[0], p[1], p[2]);
   unsigned char* d = lc_at(plane, row, col);
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(d + i * LC_PART) = p[i];
 }
 __device__ __forceinline__ void lc_put4(unsigned char* plane, int row, int col, const float4& v) {
   uint2 p[3];
-  lc_split2(v.x, v.y, p[0].x, p[1].x, p[2].x);
-  lc_split2(v.z, v.w, p[0].y, p[1].y, p[2].y);
+  at_split2(v.x, v.y, p[0].x, p[1].x, p[2].x);
+  at_split2(v.z, v.w, p[0].y, p[1].y, p[2].y);
   unsigned char* d = lc_at(plane, row, col);
 #pragma unroll
   for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(d + i * LC_PART) = p[i];
@@ -369,8 +350,8 @@ lc_ends_kernel(const LcArgs A) {
     for (int i = 15; i >= 0; --i) {
       const float2 decay = e[i];
       e[i] = b;
-      lc_decay(decay.x * b.x, 1.0f - decay.x, b.x, B.x);
-      lc_decay(decay.y * b.y, 1.0f - decay.y, b.y, B.y);
+      lr_decay(decay.x * b.x, 1.0f - decay.x, b.x, B.x);
+      lr_decay(decay.y * b.y, 1.0f - decay.y, b.y, B.y);
     }
     *reinterpret_cast<float2*>(&sh.group[tg][n]) = b;
     *reinterpret_cast<float2*>(&sh.lacks[tg][n]) = B;
@@ -378,17 +359,17 @@ lc_ends_kernel(const LcArgs A) {
     b = make_float2(1.f, 1.f); B = make_float2(0.f, 0.f);
     for (int g = 7; g > tg; --g) {
       const float2 d = *reinterpret_cast<const float2*>(&sh.group[g][n]), l = *reinterpret_cast<const float2*>(&sh.lacks[g][n]);
-      lc_decay(d.x * b.x, l.x, b.x, B.x);
-      lc_decay(d.y * b.y, l.y, b.y, B.y);
+      lr_decay(d.x * b.x, l.x, b.x, B.x);
+      lr_decay(d.y * b.y, l.y, b.y, B.y);
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i) lc_put2(X, tg * 16 + i, n, key[i].x * (e[i].x * b.x), key[i].y * (e[i].y * b.y));
     if (tg == 0) {
       const float2 d = *reinterpret_cast<const float2*>(&sh.group[0][n]), l = *reinterpret_cast<const float2*>(&sh.lacks[0][n]);
-      lc_decay(d.x * b.x, l.x, b.x, B.x);
-      lc_decay(d.y * b.y, l.y, b.y, B.y);
+      lr_decay(d.x * b.x, l.x, b.x, B.x);
+      lr_decay(d.y * b.y, l.y, b.y, B.y);
       float* vec = A.vecs + p.at * A.N;
-      if (n < A.N) { vec[n] = lc_code(b.x, B.x); vec[n + 1] = lc_code(b.y, B.y); }
+      if (n < A.N) { vec[n] = lr_code(b.x, B.x); vec[n + 1] = lr_code(b.y, B.y); }
     }
     float4 vv[8];
 #pragma unroll
@@ -481,10 +462,10 @@ lc_scan_kernel(const LcArgs A) {
     }
     if (i < end) {
       *reinterpret_cast<float4*>(at) = S;
-      S.x = MODE == 1 ? fmaf(c2, U.x, lc_apply(code, S.x)) : lc_apply(code, S.x) + U.x;
-      S.y = MODE == 1 ? fmaf(c2, U.y, lc_apply(code, S.y)) : lc_apply(code, S.y) + U.y;
-      S.z = MODE == 1 ? fmaf(c2, U.z, lc_apply(code, S.z)) : lc_apply(code, S.z) + U.z;
-      S.w = MODE == 1 ? fmaf(c2, U.w, lc_apply(code, S.w)) : lc_apply(code, S.w) + U.w;
+      S.x = MODE == 1 ? fmaf(c2, U.x, lr_apply(code, S.x)) : lr_apply(code, S.x) + U.x;
+      S.y = MODE == 1 ? fmaf(c2, U.y, lr_apply(code, S.y)) : lr_apply(code, S.y) + U.y;
+      S.z = MODE == 1 ? fmaf(c2, U.z, lr_apply(code, S.z)) : lr_apply(code, S.z) + U.z;
+      S.w = MODE == 1 ? fmaf(c2, U.w, lr_apply(code, S.w)) : lr_apply(code, S.w) + U.w;
     }
     if (vec && threadIdx.x == 0 && c > 0) A.den[(size_t)A.T * A.H + ((size_t)(before + c)) * A.H + h] = m_start;
   }
@@ -575,8 +556,8 @@ lc_out_kernel(const LcArgs A) {
     for (int i = 0; i < 16; ++i) lc_row_gate(A, p, tg * 16 + i, n, key[i], bq[i]);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      lc_decay(bq[i].x * b.x, 1.0f - bq[i].x, b.x, B.x);
-      lc_decay(bq[i].y * b.y, 1.0f - bq[i].y, b.y, B.y);
+      lr_decay(bq[i].x * b.x, 1.0f - bq[i].x, b.x, B.x);
+      lr_decay(bq[i].y * b.y, 1.0f - bq[i].y, b.y, B.y);
       bq[i] = b;
     }
     *reinterpret_cast<float2*>(&sh.group[tg][n]) = b;
@@ -586,8 +567,8 @@ lc_out_kernel(const LcArgs A) {
       float2 d = make_float2(1.f, 1.f), l = make_float2(0.f, 0.f);
       for (int g = g0; g < g1; ++g) {
         const float2 dg = *reinterpret_cast<const float2*>(&sh.group[g][n]), lg = *reinterpret_cast<const float2*>(&sh.lacks[g][n]);
-        lc_decay(dg.x * d.x, lg.x, d.x, l.x);
-        lc_decay(dg.y * d.y, lg.y, d.y, l.y);
+        lr_decay(dg.x * d.x, lg.x, d.x, l.x);
+        lr_decay(dg.y * d.y, lg.y, d.y, l.y);
       }
       return d;
     };
@@ -630,8 +611,8 @@ lc_out_kernel(const LcArgs A) {
 #pragma unroll
           for (int i = 3; i >= 0; --i) {
             lc_put2(Y, tg * 16 + i0 + i, n, key[i0 + i].x * (d.x * f.x), key[i0 + i].y * (d.y * f.y));
-            lc_decay(decay[i].x * d.x, 1.0f - decay[i].x, d.x, l.x);
-            lc_decay(decay[i].y * d.y, 1.0f - decay[i].y, d.y, l.y);
+            lr_decay(decay[i].x * d.x, 1.0f - decay[i].x, d.x, l.x);
+            lr_decay(decay[i].y * d.y, 1.0f - decay[i].y, d.y, l.y);
           }
         }
       } else if (blk == j) {

@@ -19,7 +19,7 @@
 //
 // Everything is 32-bit as in the token-by-token kernels; what differs is the scale in which a chunk's state is held (below) and
 // the fold (one multiply-add per segment and state element, two where the decay is one number per row).  Decays near 1 are
-// carried by what they lack to 1 (ls_decay).  Error of the state against 64 bits, 2,048 tokens, token by token in brackets:
+// carried by what they lack to 1 (lr_decay).  Error of the state against 64 bits, 2,048 tokens, token by token in brackets:
 // write gates of 1e-5 to 1e-2 that hardly change 2.3e-7 (3.3e-7), of 0.01 to 0.5 6.2e-8 (5.2e-8); row decays of 0.999 to
 // 0.9999 2.9e-7 (1.0e-6), of 0.96 1.2e-7 (1.4e-7).  With products of rounded decays the first was 5.8e-6, the third 2.7e-6.
 //
@@ -49,19 +49,7 @@
 
 struct alignas(16) LsCols { float x[LS_C]; };        // the lane's columns of one row
 
-// The product b of decays and what it lacks to 1, B = 1 - b, brought forward by a decay that lacks `gone` to 1 (`scaled` is that
-// decay times b).  Near 1 a product rounds to 2^-25 of itself at every token, always alike where the decays hardly change, which over
-// hundreds of tokens is far more than the state's own roundings; B keeps all its bits there.  Below 1/2 the product is the exact one.
-__device__ __forceinline__ void ls_decay(float scaled, float gone, float& b, float& B) {
-  B = fmaf(gone, b, B);
-  b = B < 0.5f ? 1.0f - B : scaled;
-}
-// A decay as one number: -B (minus zero for a decay of 1) where B lies between 0 and 1/2, else b (also behind a decay that the
-// rounding of a running maximum has put above 1).  x decays to fma(code, x, x or 0): the sign says which.
-__device__ __forceinline__ float ls_code(float b, float B) { return B >= 0.f && B < 0.5f ? -fabsf(B) : b; }
-__device__ __forceinline__ uint32_t ls_mask(float code) { return (uint32_t)(__float_as_int(code) >> 31); }
-__device__ __forceinline__ float ls_apply(float code, float x) { return fmaf(code, x, __uint_as_float(__float_as_uint(x) & ls_mask(code))); }
-__device__ __forceinline__ lr_pair ls_mask2(float c0, float c1) { return (lr_pair)ls_mask(c1) << 32 | ls_mask(c0); }
+__device__ __forceinline__ lr_pair ls_mask2(float c0, float c1) { return (lr_pair)lr_mask(c1) << 32 | lr_mask(c0); }
 
 struct LsArgs {
   const float* q; long q_stride;                     // [T][qk_heads * N]
@@ -77,7 +65,7 @@ struct LsArgs {
   float* out; long out_stride;                       // [T][H * dv]; mode 1: before the division
   float* den;                                        // mode 1: [T][H], what the outputs are to be divided by
   float* ends;                                       // [cut_segs][H][N * dv]: the requests of several segments
-  float* vecs;                                       // [cut_segs][H][N]: mode 1 n at the end; modes 2, 3 the rows' decay (ls_code)
+  float* vecs;                                       // [cut_segs][H][N]: mode 1 n at the end; modes 2, 3 the rows' decay (lr_code)
   float* scale;                                      // [segs][H][2]: mode 0 the decay; mode 1 F and L at the end
   float* first;                                      // [cuts][H][N * dv], then [cuts][H][N]: the state of those requests before the step
   float* first_m;                                    // [S][H]: mode 1, the running maximum before the step
@@ -173,7 +161,7 @@ ls_walk_kernel(const LsArgs A) {
   float* vs = as + (HAS_A ? 2 * LS_CHUNK * NP : 0);    // [2][CHUNK][BC]
   float* os = vs + 2 * LS_CHUNK * BC;                  // [CHUNK][BC], second pass
   __shared__ float keep_s[LS_CHUNK], take_s[LS_CHUNK], floor_s[LS_CHUNK], by_s[LS_CHUNK];
-  __shared__ __align__(16) float end_s[MODE < 2 ? 4 : NP];    // the decay through the chunk (ls_code), modes 2 and 3 per row
+  __shared__ __align__(16) float end_s[MODE < 2 ? 4 : NP];    // the decay through the chunk (lr_code), modes 2 and 3 per row
   __shared__ int plain_s;
   __shared__ float den_s[4][LS_CHUNK];
   const int N = A.N, dv = A.dv, H = A.H;
@@ -401,7 +389,7 @@ ls_walk_kernel(const LsArgs A) {
 #pragma unroll
       for (int o = 1; o < LS_CHUNK; o <<= 1) {
         float up = __shfl_up_sync(0xffffffffu, gb, o), upB = __shfl_up_sync(0xffffffffu, gB, o);
-        if (lane >= o) { ls_decay(gb * up, gB, up, upB); gb = up; gB = upB; }
+        if (lane >= o) { lr_decay(gb * up, gB, up, upB); gb = up; gB = upB; }
       }
       gplain = !(__shfl_sync(0xffffffffu, gb, LS_CHUNK - 1) >= LS_SMALL);
       if (!gplain) gt = gt / gb;
@@ -411,7 +399,7 @@ ls_walk_kernel(const LsArgs A) {
     if (SCALAR && tid < LS_CHUNK) {
       keep_s[tid] = gk; take_s[tid] = gt; floor_s[tid] = gfl; by_s[tid] = gplain ? 1.f : gb;
       if (tid == 0) plain_s = gplain;
-      if (tid == LS_CHUNK - 1) end_s[0] = ls_code(gb, gB);
+      if (tid == LS_CHUNK - 1) end_s[0] = lr_code(gb, gB);
     }
     __syncthreads();                                   // this chunk has landed for every thread
     float* kd = ks + (size_t)stage * LS_CHUNK * NP;
@@ -425,7 +413,7 @@ ls_walk_kernel(const LsArgs A) {
       // a thread per row: the row's decays multiplied up, then its keys and queries brought into the chunk's scale
       auto row_decay = [&](int at, float& b, float& B) {
         const float x = HAS_A ? ad[at] : kd[at];           // the decay, or what it lacks to 1
-        ls_decay(HAS_A ? x * b : fmaf(-x, b, b), HAS_A ? 1.0f - x : x, b, B);
+        lr_decay(HAS_A ? x * b : fmaf(-x, b, b), HAS_A ? 1.0f - x : x, b, B);
       };
       float b_end[RT];
       bool small = false;
@@ -434,9 +422,9 @@ ls_walk_kernel(const LsArgs A) {
         const int r = tid + i * LS_THREADS;
         float bt = 1.f, Bt = 0.f;
         if (r < N) for (int tt = 0; tt < cnt; ++tt) row_decay(tt * NP + r, bt, Bt);
-        b_end[i] = ls_code(bt, Bt);
+        b_end[i] = lr_code(bt, Bt);
         const float f = follow[i];
-        ls_decay(ls_apply(b_end[i], f), Bt, follow[i], lacks[i]);
+        lr_decay(lr_apply(b_end[i], f), Bt, follow[i], lacks[i]);
         small |= !(bt >= LS_SMALL);
       }
       plain = __syncthreads_or(small) != 0;
@@ -485,7 +473,7 @@ ls_walk_kernel(const LsArgs A) {
               if (HAS_Q) nq[tt] = fmaf(follow[i], qd[tt * NP + r], nq[tt]);
             }
           }
-          if (!plain) follow[i] = ls_apply(end_s[0], follow[i]);
+          if (!plain) follow[i] = lr_apply(end_s[0], follow[i]);
         }
       }
       if (HAS_Q) {
@@ -642,7 +630,7 @@ ls_walk_kernel(const LsArgs A) {
   }
   if (leads && vec != nullptr && (MODE == 1 || (PASS == 1 && !SCALAR))) {
 #pragma unroll
-    for (int i = 0; i < RT; ++i) if (tid + i * LS_THREADS < N) vec[tid + i * LS_THREADS] = MODE == 1 ? follow[i] : ls_code(follow[i], lacks[i]);
+    for (int i = 0; i < RT; ++i) if (tid + i * LS_THREADS < N) vec[tid + i * LS_THREADS] = MODE == 1 ? follow[i] : lr_code(follow[i], lacks[i]);
   }
 }
 
