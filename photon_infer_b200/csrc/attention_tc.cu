@@ -652,7 +652,8 @@ attention_tc_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         constexpr bool EDGE = decltype(edge)::value;
         const int s = i % AP_STAGES;
         for (int j = 0; j < nq; ++j) {
-          if (!tc_wait_warp(&v_full[s], (i / AP_STAGES) & 1, abort_flag)) return false;
+          // the copy below needs all lanes; the vote alone would take 4 % where the tensor cores wait for the issue
+          if (!(EDGE ? tc_wait_warp(&v_full[s], (i / AP_STAGES) & 1, abort_flag) : tc_wait(&v_full[s], (i / AP_STAGES) & 1, abort_flag))) return false;
           const uint32_t o = tmem + AP_O_COL + j * 128, p = tmem + j * 128;          // P: 8 columns of packed pairs for 16 keys, halves 32 apart
           const uint32_t v_addr = tc_smem(v_s + s * AP_V_BYTES);                     // 16 keys: two groups of 8 rows of V
           if (EDGE) {
